@@ -1,0 +1,942 @@
+// FP64 matrix products as exact sums of FP8 digit products (tcgen05), the bulk
+// arithmetic of the FP64 path and of the factorizations: GB300 runs FP64 FMAs
+// at about 1.2 TFLOP/s and kind::f8f6f4 MMAs at 4.5 PFLOP/s.
+//
+//   C = alpha * A * B^T + beta * C,  A: M rows, B: N rows, K elements a row.
+//
+// Digits.  Row r of an operand is scaled by a power of two, 2^ex, so that
+// |x| 2^-ex < 1/2, rounded to a multiple of 2^-60 and written in base 32 with
+// signed digits, x 2^-ex = sum_{s=1..12} d_s 32^-s, |d_s| <= 16: exact in E4M3.
+// The cut works on the bit pattern in integer instructions: the 60-bit fixed
+// point number plus sum_s 16 * 32^(12-s) has the digits d_s + 16 as its 5-bit
+// fields.
+//
+// Products.  A product of digits s and t has weight 32^-(s+t); level L is the
+// sum of all pairs with s + t = L.  Levels 2 .. 13 are kept (78 of the 144
+// pairs); what is dropped is below 2^-65 * 11 * 2^8 of the product of the row
+// scales per element, and of random sign, like the rounding of the digits:
+// less than the rounding of an FP64 accumulation.  Measured 2-norm errors over
+// 150 entries against exactly rounded sums, normal data, digits / FP64 kernel:
+// K = 128 5e-15 / 5e-14, K = 1000 3e-14 / 4e-13, K = 10000 1.2e-13 / 4.1e-12
+// (hard calls as one operand 1.8e-15).  A level's sum over K is an integer;
+// in units of the accumulator at most pairs * K * 2^8, so 65536 pairs x K of a
+// level are summed exactly in FP32 and then added to int32 sums.  At the end
+// the levels are combined in 128-bit integers and rounded once to FP64: no
+// FP64 instruction runs per element unless alpha or beta asks for one.
+// Operands with fewer digits (hard-call genotypes have one) have fewer pairs:
+// the digits in use per 256 rows are found while cutting.
+//
+// digit_gemm_kernel: persistent clusters of two CTAs, 256 x 256 tiles with
+// tcgen05.mma.cta_group::2 (M = 256, N = 256, K = 32), each CTA holding 128
+// rows of A and 128 of B.  Two levels run at once, L in TMEM columns 0-255 and
+// L + 1 in 256-511.  For a K-block the digits of B ascend, t = 1, 2, ..: the
+// A tile that level L + 1 needs at step t, digit L + 1 - t, is the one level L
+// used at step t - 1, so each 32 KB stage (one A tile, one B tile) feeds eight
+// MMAs and the previous stage's A tile is kept one step longer.  That is 28
+// bytes per clock and SM from L2, half of what one A and one B tile per four
+// MMAs would take.
+//   warp 0     TMA producer (each CTA its own 128 rows), six stages
+//   warp 1     MMA issue (pair leader), TMEM allocation
+//   warps 2-9  epilogue: q = 32 P_L + P_{L+1} as int32 into the CTA's own
+//              planes (L2-resident, 4 bytes per element and level pair); once a
+//              tile's last pass is stored its TMEM is released and the planes
+//              are combined while the next tile's MMAs run.
+// Every wait is bounded as in fgls_ozaki.cu.
+//
+// Bound by the FP8 pipe: 10000 x 4096 x 10000 takes 18.1 ms with both cuts (78
+// pairs: 3.5 PFLOP/s, 0.92 of twice the measured BF16 rate) and 4.5 ms with
+// hard calls (12 pairs), where the FP64 kernel takes 665 ms.
+#include <cuda.h>
+#include <cuda_fp8.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+
+#include "fgls_common.cuh"
+#include "fgls_digit_gemm.cuh"
+#include "fgls_kernels.cuh"
+#include "fgls_tc.cuh"
+
+namespace fgls {
+
+namespace {
+
+using namespace oz;
+
+constexpr int ND = DG_DIGITS;
+constexpr int ROW = 128;               // bytes (digits) of a K-step
+constexpr int TILE = 128 * ROW;        // 16 KB: 128 rows of one digit plane
+constexpr int STAGE = 2 * TILE;        // an A and a B tile
+constexpr int STAGES = 6;
+constexpr int SMEM = STAGES * STAGE + 1024 + 256;
+constexpr int NTHREADS = 320;
+constexpr int EPI_WARPS = 8;
+constexpr int MAXPASS = (ND + 1) / 2;  // level pairs
+constexpr int PLANE = 128 * 256;       // ints of one CTA's plane
+constexpr int BAD_ROW = 0x7fffffff;    // exponent of a row that holds a NaN or an infinity
+constexpr int PAIR_K = 512;            // K-steps x pairs one FP32 accumulator takes exactly (65536 elements)
+// int32 planes: 33 * 2^8 * pairs * K < 2^31 for 12 pairs
+constexpr int K_MAX_STEPS = 160;       // 20480 elements of K per launch
+// kind::f8f6f4: D=F32, A=B=E4M3, K-major, N=256, M=256 (the pair)
+constexpr uint32_t DG_IDESC = (1u << 4) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+
+__device__ __forceinline__ void tma_load_3d_cg2(void* dst, const CUtensorMap* tm, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
+      "%4}], [%5];" ::"r"(smem_u32(dst)),
+      "l"((uint64_t)tm), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
+
+struct DgArgs {
+  int M, N;
+  int kb0, nk;            // K-steps of this launch: [kb0, kb0 + nk)
+  int ksplit, kper;       // K split over units: split z takes steps [z*kper, ..) of the range
+  int tiles_m, tiles_n;   // 256 x 256 tiles
+  int lower_tiles;        // tiles are those with n_tile <= m_tile only, and only r >= c is written
+  int a_lower;            // row r of A is zero beyond column r
+  const int *exA, *exB, *ndA, *ndB;
+  double alpha, beta;
+  double* C;              // ksplit > 1: partial plane z at C + z * M * N
+  long long ldc;
+  int* planes;
+  int* err;
+  unsigned long long wait_ns;
+};
+
+// What the three roles need of a unit (an output tile and a range of K).
+struct Unit {
+  int mt, nt, z, kb, nk, da, db;
+};
+__device__ __forceinline__ int dg_units(const DgArgs& g) {
+  const int t = g.lower_tiles ? g.tiles_m * (g.tiles_m + 1) / 2 : g.tiles_m * g.tiles_n;
+  return t * g.ksplit;
+}
+// Unit u.  Lower-triangular A: row tiles with the most K first (the units are
+// dealt in order); else groups of eight row tiles, so that the tiles in flight
+// share operand tiles in L2.
+__device__ __forceinline__ Unit dg_unit(const DgArgs& g, int u) {
+  Unit U;
+  U.z = u % g.ksplit;
+  int t = u / g.ksplit;
+  if (g.lower_tiles) {
+    int m = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while (m * (m + 1) / 2 > t) m--;
+    while ((m + 1) * (m + 2) / 2 <= t) m++;
+    U.mt = m;
+    U.nt = t - m * (m + 1) / 2;
+  } else if (g.a_lower) {
+    U.mt = g.tiles_m - 1 - t / g.tiles_n;
+    U.nt = t % g.tiles_n;
+  } else {
+    const int per = 8 * g.tiles_n, grp = t / per;
+    const int gm = min(8, g.tiles_m - grp * 8);
+    const int in = t - grp * per;
+    U.mt = grp * 8 + in % gm;
+    U.nt = in / gm;
+  }
+  U.kb = g.kb0 + U.z * g.kper;
+  U.nk = min(g.kper, g.nk - U.z * g.kper);
+  if (g.a_lower) U.nk = min(U.nk, 2 * (U.mt + 1) - U.kb);  // 256 rows: 2 K-steps a row tile
+  U.da = max(1, g.ndA[U.mt]);
+  U.db = max(1, g.ndB[U.nt]);
+  return U;
+}
+
+// Level pair i of a unit: levels L and L + 1, the B digits t that take part.
+struct Pass {
+  int L, tlo, thi, has1, pro, chunk;  // pro: an A tile (digit L + 1 - tlo) precedes step tlo; chunk: K-steps a pass
+};
+__device__ __forceinline__ int dg_passes(const Unit& U) { return (min(ND + 1, U.da + U.db)) / 2; }
+__device__ __forceinline__ Pass dg_pass(const Unit& U, int i) {
+  Pass P;
+  const int lmax = min(ND + 1, U.da + U.db);
+  P.L = 2 + 2 * i;
+  P.has1 = P.L + 1 <= lmax;
+  P.tlo = max(1, P.L - U.da);
+  P.thi = P.has1 ? min(U.db, P.L) : min(U.db, P.L - 1);
+  P.pro = P.has1 && P.L + 1 - P.tlo <= U.da;
+  const int steps = max(1, U.nk), most = PAIR_K / (P.thi - P.tlo + 1);
+  const int n = (steps + most - 1) / most;
+  P.chunk = (steps + n - 1) / n;
+  return P;
+}
+
+// An integer |v| <= 2^24 held in a float, as an int without a conversion
+// instruction (those run at a quarter of the FP32 rate): the multiple of four
+// by the 1.5 * 2^25 addend, the rest by the 1.5 * 2^23 one.
+__device__ __forceinline__ int exact_f2i(float v) {
+  const float t = __fadd_rn(v, 50331648.0f);
+  const float r = __fsub_rn(v, __fsub_rn(t, 50331648.0f));
+  const float u = __fadd_rn(r, 12582912.0f);
+  return (int)(((uint32_t)__float_as_int(t) - 0x4C400000u) * 4u + ((uint32_t)__float_as_int(u) - 0x4B400000u));
+}
+
+// T * 2^e rounded to FP64 (to nearest even), in integer instructions.
+__device__ __forceinline__ double i128_to_double(__int128 T, int e) {
+  const bool neg = T < 0;
+  const unsigned __int128 U = neg ? (unsigned __int128)0 - (unsigned __int128)T : (unsigned __int128)T;
+  uint64_t hi = (uint64_t)(U >> 64), lo = (uint64_t)U;
+  int top;  // index of the highest set bit
+  if (hi) {
+    const int z = __clzll((long long)hi);
+    top = 127 - z;
+    if (z) {
+      hi = (hi << z) | (lo >> (64 - z));
+      lo <<= z;
+    }
+  } else {
+    if (!lo) return 0.0;
+    const int z = __clzll((long long)lo);
+    top = 63 - z;
+    hi = lo << z;
+    lo = 0;
+  }
+  uint64_t m = hi >> 11;
+  const uint32_t rest = (uint32_t)hi & 0x7ffu;
+  if (rest > 0x400u || (rest == 0x400u && (lo != 0 || (m & 1)))) m++;
+  const int ex = top + e;  // m in [2^52, 2^53]
+  if (ex < -1000 || ex > 1000) return ldexp(neg ? -(double)m : (double)m, ex - 52);
+  return __longlong_as_double((long long)((m + ((uint64_t)(ex + 1022) << 52)) | (neg ? 1ull << 63 : 0ull)));
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
+    digit_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                      const __grid_constant__ DgArgs g) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = (uint64_t*)(smem + STAGES * STAGE);  // [STAGES], used in the leader
+  uint64_t* empty = full + STAGES;                       // [STAGES]
+  uint64_t* tfull = empty + STAGES;
+  uint64_t* tempty = tfull + 1;  // used in the leader
+  uint64_t* drain = tempty + 1;
+  uint32_t* tbase_slot = (uint32_t*)(drain + 1);
+  volatile int* abort_flag = (volatile int*)(tbase_slot + 1);
+  static_assert((STAGES * 2 + 3) * 8 + 8 <= 256, "barriers fit the 256-byte tail");
+
+  const uint32_t rank = cluster_rank();
+  const bool lead = rank == 0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int units = dg_units(g);
+  const int cid = (int)(blockIdx.x >> 1), ncl = (int)(gridDim.x >> 1);
+  const uint16_t BOTH = 0x3;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; s++) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(tfull, 1);
+    mbar_init(tempty, 2 * EPI_WARPS);
+    mbar_init(drain, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {  // one warp of each CTA allocates the same columns in both
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tbase_slot)),
+                 "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  cluster_sync();  // both CTAs' barriers are initialised before either signals the other's
+  tc_fence_after();
+  const uint32_t tbase = *tbase_slot;
+  const uint32_t lead_full = cluster_addr(full, 0);
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      int issued[STAGES];
+      uint32_t issued_phase[STAGES];
+      for (int s = 0; s < STAGES; s++) issued[s] = 0;
+      bool ok = true;
+      // one stage: A digit sa (0: none) and B digit tb (0: none) of K-step kb
+      auto fill = [&](int kb, int ra, int sa, int rb, int tb) -> bool {
+        if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, g.err, 41, g.wait_ns)) return false;
+        issued[stage] = 0;
+        uint8_t* sb = smem + stage * STAGE;
+        const uint32_t fb = lead_full + 8u * (uint32_t)stage;
+        const int bytes = (sa > 0 ? TILE : 0) + (tb > 0 ? TILE : 0);
+        if (lead) mbar_expect_tx(&full[stage], 2 * bytes);  // both CTAs' copies
+        if (sa > 0) tma_load_3d_cg2(sb, &tmA, kb * ROW, ra, sa - 1, fb);
+        if (tb > 0) tma_load_3d_cg2(sb + TILE, &tmB, kb * ROW, rb, tb - 1, fb);
+        issued[stage] = 1;
+        issued_phase[stage] = phase;
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        return true;
+      };
+#pragma unroll 1
+      for (int u = cid; u < units && ok; u += ncl) {
+        const Unit U = dg_unit(g, u);
+        const int ra = U.mt * 256 + (int)rank * 128, rb = U.nt * 256 + (int)rank * 128;
+        const int np = dg_passes(U);
+#pragma unroll 1
+        for (int i = 0; i < np && ok; i++) {
+          const Pass P = dg_pass(U, i);
+#pragma unroll 1
+          for (int kb = 0; kb < U.nk && ok; kb++) {
+            if (P.pro) ok = fill(U.kb + kb, ra, P.L + 1 - P.tlo, rb, 0);
+#pragma unroll 1
+            for (int t = P.tlo; t <= P.thi && ok; t++) ok = fill(U.kb + kb, ra, P.L - t, rb, t);
+          }
+        }
+      }
+      if (ok) {
+        // every stage filled so far has been released by the leader's MMAs:
+        // no multicast commit is still on its way to this CTA
+#pragma unroll 1
+        for (int i = 0; i < STAGES; i++) {
+          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, g.err, 45, g.wait_ns)) break;
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
+      } else if (lead) {
+        const uint64_t deadline = globaltimer_ns() + WAIT_NS;
+        for (int s = 0; s < STAGES; s++)
+          if (issued[s]) mbar_drain_until(&full[s], issued_phase[s], deadline);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && lead) {
+      int stage = 0;
+      uint32_t phase = 0, q = 0;
+      bool ok = true, any = false;
+#pragma unroll 1
+      for (int u = cid; u < units && ok; u += ncl) {
+        const Unit U = dg_unit(g, u);
+        const int np = dg_passes(U);
+#pragma unroll 1
+        for (int i = 0; i < np && ok; i++) {
+          const Pass P = dg_pass(U, i);
+#pragma unroll 1
+          for (int k0 = 0; k0 < U.nk && ok; k0 += P.chunk, q++) {
+            {  // both CTAs' epilogues have drained the accumulators
+              const uint64_t t0 = globaltimer_ns();
+              uint32_t spin = 0;
+              while (!mbar_try_wait_cluster(tempty, (q & 1) ^ 1)) {
+                const bool every = (spin & 63) == 63, first = spin == 0;  // as in mbar_wait
+                spin++;
+                if ((every && (*abort_flag || *(volatile int*)g.err)) ||
+                    ((every || first) && globaltimer_ns() - t0 > g.wait_ns)) {
+                  *abort_flag = 1;
+                  atomicCAS(g.err, 0, 42);
+                  ok = false;
+                  break;
+                }
+              }
+              if (!ok) break;
+            }
+            tc_fence_after();
+            uint32_t use0 = 0, use1 = 0;
+            const int k1 = min(U.nk, k0 + P.chunk);
+#pragma unroll 1
+            for (int kb = k0; kb < k1 && ok; kb++) {
+              int prev = -1;  // the stage whose A tile level L + 1 uses next
+              if (P.pro) {
+                if (!mbar_wait(&full[stage], phase, abort_flag, g.err, 43, g.wait_ns)) { ok = false; break; }
+                prev = stage;
+                if (++stage == STAGES) { stage = 0; phase ^= 1; }
+              }
+#pragma unroll 1
+              for (int t = P.tlo; t <= P.thi; t++) {
+                if (!mbar_wait(&full[stage], phase, abort_flag, g.err, 43, g.wait_ns)) { ok = false; break; }
+                tc_fence_after();
+                uint8_t* sb = smem + stage * STAGE;
+                const uint64_t b = desc_sw128(sb + TILE);
+                if (P.L - t >= 1) {
+                  const uint64_t a = desc_sw128(sb);
+#pragma unroll
+                  for (int kk = 0; kk < ROW / 32; kk++) {
+                    mma_f8_cg2(tbase, a + 2 * kk, b + 2 * kk, DG_IDESC, use0);
+                    use0 = 1;
+                  }
+                }
+                if (prev >= 0) {
+                  const uint64_t a = desc_sw128(smem + prev * STAGE);
+#pragma unroll
+                  for (int kk = 0; kk < ROW / 32; kk++) {
+                    mma_f8_cg2(tbase + 256, a + 2 * kk, b + 2 * kk, DG_IDESC, use1);
+                    use1 = 1;
+                  }
+                  mma_commit_cg2(&empty[prev], BOTH);
+                }
+                any = true;
+                prev = P.has1 ? stage : -1;
+                if (!P.has1) mma_commit_cg2(&empty[stage], BOTH);
+                if (++stage == STAGES) { stage = 0; phase ^= 1; }
+              }
+              if (!ok) break;
+              if (prev >= 0) mma_commit_cg2(&empty[prev], BOTH);
+            }
+            if (!ok) break;
+            mma_commit_cg2(tfull, BOTH);
+          }
+        }
+      }
+      if (!ok && any) {
+        // all MMAs issued by this thread complete before TMEM is released
+        mma_commit_cg2(drain, 0x1);
+        mbar_drain(drain, 0);
+      }
+    }
+    __syncwarp();
+  } else {
+    const int lq = warp & 3;
+    const int cbeg = ((warp - 2) >> 2) * 128;
+    const int row = lq * 32 + lane;
+    const uint32_t ta = tbase + ((uint32_t)(lq * 32) << 16) + (uint32_t)cbeg;
+    const uint32_t lead_tempty = cluster_addr(tempty, 0);
+    int* plane0 = g.planes + (size_t)blockIdx.x * (MAXPASS * PLANE) + cbeg * 128 + row;
+    uint32_t q = 0;
+    bool ok = true;
+#pragma unroll 1
+    for (int u = cid; u < units && ok; u += ncl) {
+      const Unit U = dg_unit(g, u);
+      const int np = dg_passes(U);
+#pragma unroll 1
+      for (int i = 0; i < np && ok; i++) {
+        const Pass P = dg_pass(U, i);
+        int* pl = plane0 + i * PLANE;
+#pragma unroll 1
+        for (int k0 = 0; k0 < U.nk; k0 += P.chunk, q++) {
+          int okw = 1;
+          if (lane == 0) okw = mbar_wait(tfull, q & 1, abort_flag, g.err, 44, g.wait_ns) ? 1 : 0;
+          okw = __shfl_sync(0xffffffffu, okw, 0);
+          if (!okw) { ok = false; break; }
+          tc_fence_after();
+#pragma unroll 1
+          for (int c0 = 0; c0 < 128; c0 += 32) {
+            uint32_t v[32], w[32];
+            tmem_ld32(ta + c0, v);
+            if (P.has1) {
+              tmem_ld32(ta + 256 + c0, w);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 32; j++)
+                v[j] = (uint32_t)(exact_f2i(__uint_as_float(v[j])) * 32 + exact_f2i(__uint_as_float(w[j])));
+            } else {
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 32; j++) v[j] = (uint32_t)(exact_f2i(__uint_as_float(v[j])) * 32);
+            }
+            if (k0 > 0) {
+#pragma unroll
+              for (int j = 0; j < 32; j++) v[j] += (uint32_t)pl[(c0 + j) * 128];
+            }
+#pragma unroll
+            for (int j = 0; j < 32; j++) pl[(c0 + j) * 128] = (int)v[j];
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(lead_tempty);
+        }
+      }
+      if (!ok) break;
+      // combine the planes: T = sum_i q_i 2^(10 (np - 1 - i)), the element is
+      // T 2^(exA + exB - 5 (2 np + 1))
+      const int r = U.mt * 256 + (int)rank * 128 + row;
+      const int n0 = U.nt * 256 + cbeg;
+      const int ncols = min(128, g.N - n0);
+      if (r < g.M && ncols > 0) {
+        const int ea = g.exA[r];
+        const int h = min(np, 3);
+        double* crow = g.C + (g.ksplit > 1 ? (size_t)U.z * g.M * g.N : 0) + r + (long long)n0 * g.ldc;
+#pragma unroll 1
+        for (int c0 = 0; c0 < ncols; c0 += 4) {
+          int qv[4][MAXPASS];
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int i = 0; i < MAXPASS; i++) qv[j][i] = (i < np && U.nk > 0) ? plane0[i * PLANE + (c0 + j) * 128] : 0;
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const int c = c0 + j;
+            if (c >= ncols) break;
+            if (g.lower_tiles && r < n0 + c) continue;
+            long long W = 0, V = 0;
+#pragma unroll
+            for (int i = 0; i < MAXPASS; i++) {
+              if (i < h) W = W * 1024 + qv[j][i];
+              else if (i < np) V = V * 1024 + qv[j][i];
+            }
+            const __int128 T = ((__int128)W << (10 * (np - h))) + V;
+            const int eb = g.exB[n0 + c];
+            double v;
+            if (ea == BAD_ROW || eb == BAD_ROW) v = __longlong_as_double(0x7ff8000000000000ll);
+            else v = i128_to_double(T, ea + eb - 5 * (2 * np + 1));
+            double* cp = crow + (long long)c * g.ldc;
+            if (g.alpha != 1.0) v = g.alpha == -1.0 ? -v : v * g.alpha;
+            if (g.beta != 0.0) v = fma(g.beta, *cp, v);
+            *cp = v;
+          }
+        }
+      }
+      __syncwarp();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();  // the leader's MMAs into both CTAs' TMEM are complete
+  tc_fence_after();
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(512) : "memory");
+  // neither CTA exits while the other may still signal its barriers or copy
+  // into its shared memory (see gemm_pair in fgls_ozaki.cu)
+  cluster_sync();
+  if (*abort_flag) {
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 100000ull) {
+    }
+  }
+}
+
+// C = alpha * sum_z P_z + beta * C, z ascending (P_z: M x N, ld M)
+__global__ void __launch_bounds__(256) digit_split_sum_kernel(int M, int N, int splits, const double* __restrict__ P,
+                                                              double alpha, double beta, double* __restrict__ C,
+                                                              long long ldc) {
+  const long long total = (long long)M * N;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
+       e += (long long)gridDim.x * blockDim.x) {
+    double v = 0.0;
+    for (int z = 0; z < splits; z++) v += P[e + (long long)z * total];
+    double* c = C + e % M + (e / M) * ldc;
+    *c = beta != 0.0 ? fma(beta, *c, alpha * v) : alpha * v;
+  }
+}
+
+// ------------------------------------------------------------------- digits
+constexpr uint64_t DIGIT_BIAS = 16ull * (((1ull << 60) - 1) / 31);  // 16 in every 5-bit field
+
+// x 2^(60 - ex) rounded to an integer (|x| < 2^(ex-1)); exact zero stays zero.
+__device__ __forceinline__ long long to_fixed(double x, int ex) {
+  const long long b = __double_as_longlong(x);
+  int e = (int)((b >> 52) & 0x7ff);
+  unsigned long long m = (unsigned long long)b & 0xfffffffffffffull;
+  if (e) m |= 1ull << 52;
+  else e = 1;
+  const int sh = e - 1015 - ex;  // m 2^sh
+  unsigned long long f;
+  if (sh >= 0) f = m << min(sh, 11);
+  else if (sh > -55) f = (m + (1ull << (-sh - 1))) >> -sh;
+  else f = 0;
+  return b < 0 ? -(long long)f : (long long)f;
+}
+// the four digits of weight 32^-(s+1) of four biased numbers, as E4M3 bytes
+__device__ __forceinline__ uint32_t digit_word(const uint64_t (&u)[4], int s) {
+  float f[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const uint32_t d = s == 0 ? (uint32_t)(u[k] >> 55) : (uint32_t)(u[k] >> (55 - 5 * s)) & 31u;
+    f[k] = __fsub_rn(__uint_as_float(0x4B000000u | d), 8388624.0f);
+  }
+  const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(f[0], f[1]), __NV_SATFINITE, __NV_E4M3);
+  const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(f[2], f[3]), __NV_SATFINITE, __NV_E4M3);
+  return lo | (hi << 16);
+}
+// exponent of a row's scale from the largest biased exponent in it
+__device__ __forceinline__ int row_exponent(int top) { return top == 0x7ff ? BAD_ROW : top - 1021; }
+__device__ __forceinline__ int digits_used(unsigned long long bits) {  // of the OR of a row's fixed-point magnitudes
+  return bits ? ND - (__ffsll((long long)bits) - 1) / 5 : 0;
+}
+
+// One CTA of 256 threads (or one of eight warps, TPR = 32) per row whose
+// elements are contiguous in K.  The row is read twice, the second time mostly
+// from L2; bound by the writes (twelve bytes an element) and integer issue.
+// w > 0: row (i*w + c)*w + d is the product of columns i*w + c and i*w + d.
+template <int TPR>
+__global__ void __launch_bounds__(256) cut_contig_kernel(const double* __restrict__ X, long long ld, int rows, int K,
+                                                         int Kpad, int w, uint8_t* __restrict__ D,
+                                                         int* __restrict__ ex, int* __restrict__ nd) {
+  const int r = blockIdx.x * (256 / TPR) + (int)threadIdx.x / TPR;
+  const int l = threadIdx.x % TPR;
+  if (TPR == 32 && r >= rows) return;
+  const double *x = X + (long long)r * ld, *y = nullptr;
+  if (w > 0) {
+    x = X + (long long)(r / w) * ld;
+    y = X + (long long)(r / (w * w) * w + r % w) * ld;
+  }
+  auto value = [&](int k) -> double { return y ? x[k] * y[k] : x[k]; };
+  int top = 0;
+  for (int k = l; k < K; k += TPR)
+    top = max(top, (int)((__double_as_longlong(value(k)) >> 52) & 0x7ff));
+  __shared__ int stop[8];
+  __shared__ unsigned long long sbits[8];
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (TPR > 32) {
+    if ((threadIdx.x & 31) == 0) stop[threadIdx.x >> 5] = top;
+    __syncthreads();
+    for (int q = 0; q < 8; q++) top = max(top, stop[q]);
+  }
+  const int e = row_exponent(top);
+  if (l == 0) ex[r] = e;
+  const int es = e == BAD_ROW ? 1024 : e;  // finite digits in a bad row too
+  unsigned long long bits = 0;
+  for (int g = l; g < Kpad / 4; g += TPR) {
+    uint64_t u[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int k = 4 * g + j;
+      const long long f = k < K ? to_fixed(value(k), es) : 0;
+      bits |= (unsigned long long)(f < 0 ? -f : f);
+      u[j] = (uint64_t)f + DIGIT_BIAS;
+    }
+#pragma unroll
+    for (int s = 0; s < ND; s++) *(uint32_t*)(D + ((size_t)s * rows + r) * Kpad + 4 * g) = digit_word(u, s);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) bits |= __shfl_xor_sync(0xffffffffu, bits, o);
+  if (TPR > 32) {
+    if ((threadIdx.x & 31) == 0) sbits[threadIdx.x >> 5] = bits;
+    __syncthreads();
+    for (int q = 0; q < 8; q++) bits |= sbits[q];
+  }
+  if (l == 0) atomicMax(nd + (r >> 8), digits_used(bits));
+}
+
+// 32 rows per CTA, elements contiguous over the rows: digits of 32 x 64 tiles
+// turned in shared memory, so that both the loads (256 bytes a warp) and the
+// stores (64 bytes a row and plane) are coalesced.
+__global__ void __launch_bounds__(256) cut_strided_kernel(const double* __restrict__ X, long long ld, int rows, int K,
+                                                          int Kpad, uint8_t* __restrict__ D, int* __restrict__ ex,
+                                                          int* __restrict__ nd) {
+  __shared__ uint32_t t[ND][32][17];
+  __shared__ int stop[8][32];
+  __shared__ unsigned long long sbits[8];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int r0 = blockIdx.x * 32, r = r0 + lane;
+  const double* x = X + r;
+  int top = 0;
+  if (r < rows)
+    for (int k = wp; k < K; k += 8) top = max(top, (int)((__double_as_longlong(x[(long long)k * ld]) >> 52) & 0x7ff));
+  stop[wp][lane] = top;
+  __syncthreads();
+  for (int q = 0; q < 8; q++) top = max(top, stop[q][lane]);
+  const int e = row_exponent(top);
+  if (wp == 0 && r < rows) ex[r] = e;
+  const int es = e == BAD_ROW ? 1024 : e;
+  unsigned long long bits = 0;
+  for (int k0 = 0; k0 < Kpad; k0 += 64) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {  // two groups of four elements a thread
+      const int g = wp * 2 + h;
+      uint64_t u[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int k = k0 + 4 * g + j;
+        const long long f = (r < rows && k < K) ? to_fixed(x[(long long)k * ld], es) : 0;
+        bits |= (unsigned long long)(f < 0 ? -f : f);
+        u[j] = (uint64_t)f + DIGIT_BIAS;
+      }
+#pragma unroll
+      for (int s = 0; s < ND; s++) t[s][lane][g] = digit_word(u, s);
+    }
+    __syncthreads();
+    // 12 planes x 32 rows of 16 words: two rows a warp and step
+    for (int q = wp * 2 + (lane >> 4); q < ND * 32; q += 16) {
+      const int s = q >> 5, rr = q & 31;
+      if (r0 + rr < rows)
+        *(uint32_t*)(D + ((size_t)s * rows + r0 + rr) * Kpad + k0 + 4 * (lane & 15)) = t[s][rr][lane & 15];
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) bits |= __shfl_xor_sync(0xffffffffu, bits, o);
+  if (lane == 0) sbits[wp] = bits;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 0; q < 8; q++) bits |= sbits[q];
+    atomicMax(nd + (r0 >> 8), digits_used(bits));
+  }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encoder() {
+  static std::atomic<EncodeTiledFn> known{nullptr};
+  EncodeTiledFn fn = known.load(std::memory_order_acquire);
+  if (!fn) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      fn = (EncodeTiledFn)p;
+    known.store(fn, std::memory_order_release);
+  }
+  return fn;
+}
+
+// K-major rows of every digit plane, boxes of 128 digits x 128 rows; rows past
+// the matrix are filled with zeros, so no row padding is stored.
+cudaError_t digit_map(CUtensorMap* m, const DigitMat& d) {
+  EncodeTiledFn enc = encoder();
+  if (!enc) return cudaErrorNotSupported;
+  cuuint64_t dims[3] = {(cuuint64_t)d.Kpad, (cuuint64_t)d.rows, (cuuint64_t)ND};
+  cuuint64_t strides[2] = {(cuuint64_t)d.Kpad, (cuuint64_t)d.Kpad * (cuuint64_t)d.rows};
+  cuuint32_t box[3] = {ROW, 128, 1};
+  cuuint32_t es[3] = {1, 1, 1};
+  const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, d.d, dims, strides, box, es,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+// Clusters of two CTAs of the kernel that the current device holds at once,
+// queried once per device; 0 if none can launch.
+int dg_clusters() {
+  static std::atomic<int> known[64];  // clusters + 1; 0: not queried yet
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  const int v = known[dev].load(std::memory_order_relaxed);
+  if (v > 0) return v - 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2);
+  cfg.blockDim = dim3(NTHREADS);
+  cfg.dynamicSmemBytes = SMEM;
+  int n = 0;
+  if (cudaFuncSetAttribute(digit_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, (void*)digit_gemm_kernel, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    n = 0;
+  }
+  known[dev].store(n + 1, std::memory_order_relaxed);
+  return n;
+}
+
+}  // namespace
+
+struct DigitGemm {
+  int clusters = 0;
+  int* planes = nullptr;
+  int* err = nullptr;
+  double* part = nullptr;
+  size_t part_elems = 0;
+  void* op[2] = {nullptr, nullptr};
+  size_t op_bytes[2] = {0, 0};
+};
+
+size_t digit_mat_bytes(int rows, int K) {
+  const size_t Kpad = (size_t)(K + ROW - 1) / ROW * ROW;
+  return (size_t)ND * rows * Kpad + sizeof(int) * ((size_t)rows + (size_t)(rows + 255) / 256) + 512;
+}
+
+DigitMat digit_mat_at(void* mem, int rows, int K) {
+  DigitMat m;
+  m.rows = rows;
+  m.K = K;
+  m.Kpad = (K + ROW - 1) / ROW * ROW;
+  m.d = (uint8_t*)mem;
+  m.nd = (int*)(m.d + (((size_t)ND * rows * m.Kpad + 255) & ~(size_t)255));
+  m.ex = m.nd + (rows + 255) / 256;
+  return m;
+}
+
+namespace {
+cudaError_t cut(cudaStream_t s, const DigitMat& m, const double* X, long long ld, bool kcontig, int w) {
+  if (m.rows <= 0 || m.K <= 0) return cudaErrorInvalidValue;
+  FGLS_CUDA_TRY(cudaMemsetAsync(m.nd, 0, sizeof(int) * ((m.rows + 255) / 256), s));
+  if (!kcontig)
+    cut_strided_kernel<<<ceil_div(m.rows, 32), 256, 0, s>>>(X, ld, m.rows, m.K, m.Kpad, m.d, m.ex, m.nd);
+  else if (m.K <= 1024)
+    cut_contig_kernel<32><<<ceil_div(m.rows, 8), 256, 0, s>>>(X, ld, m.rows, m.K, m.Kpad, w, m.d, m.ex, m.nd);
+  else
+    cut_contig_kernel<256><<<m.rows, 256, 0, s>>>(X, ld, m.rows, m.K, m.Kpad, w, m.d, m.ex, m.nd);
+  note_launch();
+  return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t digit_cut(cudaStream_t s, const DigitMat& m, const double* X, long long ld, bool kcontig) {
+  return cut(s, m, X, ld, kcontig, 0);
+}
+
+cudaError_t digit_cut_products(cudaStream_t s, const DigitMat& m, const double* X, long long ld, int w) {
+  return cut(s, m, X, ld, true, w);
+}
+
+cudaError_t digit_gemm_create(DigitGemm** out) {
+  *out = nullptr;
+  const int n = dg_clusters();
+  if (n <= 0 || !encoder()) return cudaErrorNotSupported;
+  DigitGemm* g = new DigitGemm();
+  g->clusters = n;
+  cudaError_t r = cudaMalloc(&g->planes, sizeof(int) * (size_t)MAXPASS * PLANE * 2 * n);
+  if (r == cudaSuccess) r = cudaMalloc(&g->err, sizeof(int));
+  if (r == cudaSuccess) r = cudaMemset(g->err, 0, sizeof(int));
+  if (r == cudaSuccess) r = cudaDeviceSynchronize();  // the memset ran on the default stream
+  if (r != cudaSuccess) {
+    digit_gemm_destroy(g);
+    return r;
+  }
+  *out = g;
+  return cudaSuccess;
+}
+
+void digit_gemm_destroy(DigitGemm* g) {
+  if (!g) return;
+  void* ptrs[] = {g->planes, g->err, g->part, g->op[0], g->op[1]};
+  for (void* p : ptrs)
+    if (p) cudaFree(p);
+  delete g;
+}
+
+int* digit_gemm_error_word(DigitGemm* g) { return g->err; }
+
+cudaError_t digit_mul(DigitGemm* g, cudaStream_t s, const DigitMat& A, const DigitMat& B, double alpha, double beta,
+                      double* C, long long ldc, const DigitMulOpts& o) {
+  if (A.K != B.K) return cudaErrorInvalidValue;
+  CUtensorMap ma, mb;
+  FGLS_CUDA_TRY(digit_map(&ma, A));
+  FGLS_CUDA_TRY(digit_map(&mb, B));
+  DgArgs a;
+  a.M = A.rows;
+  a.N = B.rows;
+  a.tiles_m = ceil_div(A.rows, 256);
+  a.tiles_n = ceil_div(B.rows, 256);
+  a.lower_tiles = o.c_lower;
+  a.a_lower = o.a_lower;
+  a.exA = A.ex;
+  a.exB = B.ex;
+  a.ndA = A.nd;
+  a.ndB = B.nd;
+  a.alpha = alpha;
+  a.planes = g->planes;
+  a.err = g->err;
+  a.wait_ns = WAIT_NS;
+  const int tiles = o.c_lower ? a.tiles_m * (a.tiles_m + 1) / 2 : a.tiles_m * a.tiles_n;
+  const int nk_all = A.Kpad / ROW;
+  for (int kb = 0; kb < nk_all; kb += K_MAX_STEPS) {
+    a.kb0 = kb;
+    a.nk = std::min(K_MAX_STEPS, nk_all - kb);
+    a.beta = kb > 0 ? 1.0 : beta;
+    // few tiles: split K over the idle clusters, at least four K-steps each
+    int z = 1;
+    if (!o.a_lower && !o.c_lower && 2 * tiles <= g->clusters) z = std::min(g->clusters / tiles, a.nk / 4);
+    const size_t elems = (size_t)a.M * a.N;
+    if (z > 1 && g->part_elems < elems * z) {
+      if (g->part) cudaFree(g->part);
+      g->part = nullptr;
+      g->part_elems = 0;
+      if (cudaMalloc(&g->part, sizeof(double) * elems * z) == cudaSuccess) g->part_elems = elems * z;
+      else (void)cudaGetLastError();
+    }
+    if (z < 2 || g->part_elems < elems * z) z = 1;
+    a.kper = ceil_div(a.nk, z);
+    a.ksplit = ceil_div(a.nk, a.kper);
+    a.C = C;
+    a.ldc = ldc;
+    DgArgs b = a;
+    if (a.ksplit > 1) {
+      b.alpha = 1.0;
+      b.beta = 0.0;
+      b.C = g->part;
+      b.ldc = a.M;
+    }
+    const int cl = std::max(1, std::min(g->clusters, tiles * a.ksplit));
+    digit_gemm_kernel<<<2 * cl, NTHREADS, SMEM, s>>>(ma, mb, b);
+    note_launch();
+    if (a.ksplit > 1) {
+      digit_split_sum_kernel<<<(int)std::min<long long>((elems + 255) / 256, 152LL * 16), 256, 0, s>>>(
+          a.M, a.N, a.ksplit, g->part, a.alpha, a.beta, C, ldc);
+      note_launch();
+    }
+    FGLS_CUDA_TRY(cudaGetLastError());
+  }
+  return cudaSuccess;
+}
+
+// Estimates in microseconds, from measured products of 64 .. 10000 rows:
+//   FP64 kernel: 64 x 64 tiles, one wave of up to 152 takes 1.0 us per element
+//     of K (300 x 513 x 5000: 5.06 ms; 4096 x 4096 x 5000: 134.6 ms);
+//   digits: five launches (40 us), cutting at 6 ps an element, 0.16 us per
+//     element of K and wave of 76 tiles of 256 x 256, K split when there are
+//     fewer (300 x 513 x 5000: 0.31 ms; 4096 x 4096 x 5000: 4.2 ms).
+// They cross near K = 60 for one tile; 256 x 256 x 128 measures 0.16 ms both ways.
+bool digit_gemm_pays(long long M, long long N, long long K) {
+  const double t64 = (double)((M + 63) / 64) * (double)((N + 63) / 64);
+  const double t256 = (double)((M + 255) / 256) * (double)((N + 255) / 256);
+  const double fp64 = std::max(1.0, t64 / 152.0) * (double)K;
+  const double waves = t256 < 38.0 ? std::max(t256 / 76.0, 512.0 / (double)std::max(K, 512LL)) : std::ceil(t256 / 76.0);
+  const double digits = 40.0 + 6e-6 * (double)(M + N) * (double)K + 0.16 * (double)K * waves;
+  return K >= 64 && digits < fp64;
+}
+
+cudaError_t digit_dgemm(DigitGemm* g, cudaStream_t s, bool tA, bool tB, int M, int N, int K, double alpha,
+                        const double* A, long long lda, const double* B, long long ldb, double beta, double* C,
+                        long long ldc) {
+  if (g && digit_gemm_pays(M, N, K)) {
+    const size_t need[2] = {digit_mat_bytes(M, K), digit_mat_bytes(N, K)};
+    bool ok = true;
+    for (int q = 0; q < 2 && ok; q++) {
+      if (g->op_bytes[q] >= need[q]) continue;
+      if (g->op[q]) cudaFree(g->op[q]);
+      g->op[q] = nullptr;
+      g->op_bytes[q] = 0;
+      if (cudaMalloc(&g->op[q], need[q]) == cudaSuccess) {
+        g->op_bytes[q] = need[q];
+      } else {
+        (void)cudaGetLastError();
+        ok = false;
+      }
+    }
+    if (ok) {
+      const DigitMat a = digit_mat_at(g->op[0], M, K), b = digit_mat_at(g->op[1], N, K);
+      FGLS_CUDA_TRY(digit_cut(s, a, A, lda, tA));
+      FGLS_CUDA_TRY(digit_cut(s, b, B, ldb, !tB));
+      return digit_mul(g, s, a, b, alpha, beta, C, ldc);
+    }
+  }
+  return dgemm(s, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+}
+
+}  // namespace fgls
+
+// Diagnostic entry point (include/fgls_gb300.h).
+extern "C" int fglsgpu_selftest_dgemm(int transA, int transB, int M, int N, int K, double alpha, const double* A,
+                                      long long lda, const double* B, long long ldb, double beta, double* C,
+                                      long long ldc, int digits, double* ms) {
+  using namespace fgls;
+  if (M <= 0 || N <= 0 || K <= 0 || !A || !B || !C) return FGLSGPU_EINVAL;
+  if (lda < (transA ? K : M) || ldb < (transB ? N : K) || ldc < M) return FGLSGPU_EINVAL;
+  cudaStream_t s = nullptr;
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  DigitGemm* g = nullptr;
+  void* mem[2] = {nullptr, nullptr};
+  cudaError_t r = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  auto chk = [&](cudaError_t e) {
+    if (r == cudaSuccess) r = e;
+  };
+  for (auto& e : ev) chk(cudaEventCreate(&e));
+  if (digits) {
+    chk(digit_gemm_create(&g));
+    chk(cudaMalloc(&mem[0], digit_mat_bytes(M, K)));
+    chk(cudaMalloc(&mem[1], digit_mat_bytes(N, K)));
+  }
+  if (r == cudaSuccess) chk(cudaEventRecord(ev[0], s));
+  if (r == cudaSuccess && !digits)
+    chk(dgemm(s, transA != 0, transB != 0, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc));
+  if (r == cudaSuccess && digits) {
+    const DigitMat a = digit_mat_at(mem[0], M, K), b = digit_mat_at(mem[1], N, K);
+    chk(digit_cut(s, a, A, lda, transA != 0));
+    chk(digit_cut(s, b, B, ldb, transB == 0));
+    if (r == cudaSuccess) chk(digit_mul(g, s, a, b, alpha, beta, C, ldc));
+  }
+  if (r == cudaSuccess) chk(cudaEventRecord(ev[1], s));
+  if (s) chk(cudaStreamSynchronize(s));
+  int herr = 0;
+  float t = 0.f;
+  if (r == cudaSuccess && g) chk(cudaMemcpy(&herr, digit_gemm_error_word(g), sizeof(int), cudaMemcpyDeviceToHost));
+  if (r == cudaSuccess) chk(cudaEventElapsedTime(&t, ev[0], ev[1]));
+  if (ms) *ms = t;
+  for (void* p : mem)
+    if (p) cudaFree(p);
+  digit_gemm_destroy(g);
+  for (auto e : ev)
+    if (e) cudaEventDestroy(e);
+  if (s) cudaStreamDestroy(s);
+  if (r != cudaSuccess) return FGLSGPU_ECUDA;
+  return herr ? FGLSGPU_ETIMEOUT : FGLSGPU_OK;
+}

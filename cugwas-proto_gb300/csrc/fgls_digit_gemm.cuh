@@ -1,0 +1,57 @@
+// FP64 matrix products on the FP8 tensor cores (fgls_digit_gemm.cu): both
+// operands are cut into twelve signed base-32 digits per row (60 bits under a
+// power-of-two scale per row) and the digit products are summed exactly, so
+// the result carries at least the accuracy of an FP64 DGEMM.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace fgls {
+
+constexpr int DG_DIGITS = 12;
+
+// One operand as digits: `rows` rows (rows of op(A), columns of op(B)) of K
+// digits each, K innermost, rows of Kpad bytes, digit planes one after the
+// other; per row the exponent of its scale, per 256 rows the digits in use.
+struct DigitMat {
+  uint8_t* d = nullptr;
+  int* ex = nullptr;
+  int* nd = nullptr;
+  int rows = 0, K = 0, Kpad = 0;
+};
+size_t digit_mat_bytes(int rows, int K);
+// lays out a matrix of `rows` x K in `mem` (digit_mat_bytes, 256-byte aligned)
+DigitMat digit_mat_at(void* mem, int rows, int K);
+
+// Digits of a column-major FP64 matrix.  kcontig: row r's element k at
+// X[k + r*ld]; else at X[r + k*ld].  Rows holding a NaN or an infinity make every product with them NaN.
+cudaError_t digit_cut(cudaStream_t s, const DigitMat& m, const double* X, long long ld, bool kcontig);
+// rows r = (i*w + c)*w + d: the products of columns i*w + c and i*w + d of X
+cudaError_t digit_cut_products(cudaStream_t s, const DigitMat& m, const double* X, long long ld, int w);
+
+// Workspace of the digit GEMM for one stream at a time: partial sums of every
+// CTA, K-split partials, the operands of digit_dgemm, a wait error word.
+struct DigitGemm;
+cudaError_t digit_gemm_create(DigitGemm** out);  // cudaErrorNotSupported: no clusters of two
+void digit_gemm_destroy(DigitGemm* g);
+int* digit_gemm_error_word(DigitGemm* g);
+
+struct DigitMulOpts {
+  bool a_lower = false;    // row r of A is zero beyond column r
+  bool c_lower = false;    // square C: only r >= c is computed and written
+};
+// C (A.rows x B.rows, ld ldc) = alpha * A * B^T + beta * C; A.K == B.K.
+cudaError_t digit_mul(DigitGemm* g, cudaStream_t s, const DigitMat& A, const DigitMat& B, double alpha, double beta,
+                      double* C, long long ldc, const DigitMulOpts& o = DigitMulOpts());
+
+// As dgemm (fgls_common.cuh), through digits when the product is large enough
+// for that to pay and `g` is set, else the FP64 kernel.  Both operands' digits
+// live in g (grown on demand; without the memory for it the FP64 kernel runs).
+cudaError_t digit_dgemm(DigitGemm* g, cudaStream_t s, bool tA, bool tB, int M, int N, int K, double alpha,
+                        const double* A, long long lda, const double* B, long long ldb, double beta, double* C,
+                        long long ldc);
+// whether digit_dgemm takes the digits for this product
+bool digit_gemm_pays(long long M, long long N, long long K);
+
+}  // namespace fgls

@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "fgls_common.cuh"
+#include "fgls_digit_gemm.cuh"
 #include "fgls_kernels.cuh"
 #include "fgls_ozaki.cuh"
 
@@ -72,6 +73,15 @@ struct fglsgpu_engine {
   double *aGYLc = nullptr, *aGYLs = nullptr, *aGRc = nullptr, *aGRs = nullptr, *acontrib = nullptr, *ag = nullptr;
   double *agR = nullptr, *aacc = nullptr, *aU = nullptr, *aV2 = nullptr;
   bool adj_ready = false;
+  // FP64 products through digits (fgls_digit_gemm.cu): the resident operands,
+  // cut again only when they change, and the block's operand
+  DigitGemm* dg = nullptr;
+  bool dg_off = false;  // no CTA pairs or no memory for the digits: FP64 kernels throughout
+  DigitMat zdig, ayldig, ddig;  // eigen: Z^T, AYL^T, dinv^T rows
+  void *zmem = nullptr, *wmem = nullptr, *blkmem = nullptr;
+  size_t blk_bytes = 0;
+  bool z_cut = false, w_cut = false;
+  bool probing = false;  // the autotuner's FP64 block: no room for x_b SNPs
 };
 
 namespace {
@@ -111,18 +121,23 @@ cudaError_t dalloc(T** p, size_t count) {
 // follow the reference's error texts (src/fgls_chol.c:266-271, :309-314, :418-434).
 int check_status(fglsgpu_engine* e, const char* stage) {
   ENG_TRY(e, cudaMemcpyAsync(e->hst, e->dst, sizeof(DevStatus), cudaMemcpyDeviceToHost, e->comp), "status copy");
-  *e->hst_wait = 0;
+  e->hst_wait[0] = e->hst_wait[1] = 0;
   if (e->oz)
     ENG_TRY(e, cudaMemcpyAsync(e->hst_wait, ozaki_error_word(e->oz), sizeof(int), cudaMemcpyDeviceToHost, e->comp),
             "status copy");
+  if (e->dg)
+    ENG_TRY(e, cudaMemcpyAsync(e->hst_wait + 1, digit_gemm_error_word(e->dg), sizeof(int), cudaMemcpyDeviceToHost,
+                               e->comp),
+            "status copy");
   ENG_TRY(e, cudaStreamSynchronize(e->comp), stage);
   const DevStatus s = *e->hst;
-  const int wsite = *e->hst_wait;
+  const int wsite = e->hst_wait[0] ? e->hst_wait[0] : e->hst_wait[1];
   if (wsite) {
-    // the tcgen05 kernels of the split path gave up on a pipeline wait: their
-    // outputs since the last check are invalid; clear the word so that the
-    // next launches run normally
-    ENG_TRY(e, cudaMemsetAsync(ozaki_error_word(e->oz), 0, sizeof(int), e->comp), "status reset");
+    // the tcgen05 kernels gave up on a pipeline wait: their outputs since the
+    // last check are invalid; clear the words so that the next launches run
+    // normally
+    if (e->oz) ENG_TRY(e, cudaMemsetAsync(ozaki_error_word(e->oz), 0, sizeof(int), e->comp), "status reset");
+    if (e->dg) ENG_TRY(e, cudaMemsetAsync(digit_gemm_error_word(e->dg), 0, sizeof(int), e->comp), "status reset");
     ENG_TRY(e, cudaStreamSynchronize(e->comp), "status reset");
     return fail(e, FGLSGPU_ETIMEOUT, "device wait expired in %s (tensor-core kernel wait site %d)", stage, wsite);
   }
@@ -151,7 +166,7 @@ void free_all(fglsgpu_engine* e) {
                   e->dQ,   e->dGYL, e->dGR,  e->dB[0], e->dB[1], e->dV[0], e->dV[1], e->dU8, e->dst,
                   e->aWc, e->aAYLc, e->aAYLs, e->atopc, e->atops, e->areml, e->aGYLc, e->aGYLs, e->aGRc,
                   e->aGRs, e->acontrib, e->ag, e->agR, e->aacc, e->aU, e->aV2, e->dSE[0], e->dSE[1], e->dP[0],
-                  e->dP[1], e->dXw};
+                  e->dP[1], e->dXw, e->zmem, e->wmem, e->blkmem};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (e->hst) cudaFreeHost(e->hst);
@@ -162,6 +177,7 @@ void free_all(fglsgpu_engine* e) {
       cudaEventDestroy(ev.b);
     }
   if (e->oz) ozaki_destroy(e->oz);
+  digit_gemm_destroy(e->dg);
   for (int k = 0; k < 2; k++) {
     if (e->evH[k]) cudaEventDestroy(e->evH[k]);
     if (e->evC[k]) cudaEventDestroy(e->evC[k]);
@@ -226,6 +242,72 @@ long long geno_bytes_per_col(int fmt, int n) {
   return fmt == GENO_F64 ? 8LL * n : fmt == GENO_U8 ? (long long)n : (long long)(n + 3) / 4;
 }
 
+// Device memory of `bytes` at *p, kept in *have; false when there is none.
+bool grow(void** p, size_t* have, size_t bytes) {
+  if (*have >= bytes) return true;
+  if (*p) cudaFree(*p);
+  *p = nullptr;
+  *have = 0;
+  if (cudaMalloc(p, bytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    *p = nullptr;
+    return false;
+  }
+  *have = bytes;
+  return true;
+}
+
+void drop_digits(fglsgpu_engine* e) {
+  for (void** q : {&e->zmem, &e->wmem, &e->blkmem}) {
+    if (*q) cudaFree(*q);
+    *q = nullptr;
+  }
+  e->blk_bytes = 0;
+  e->z_cut = e->w_cut = false;
+}
+
+// Digits of the eigen variant's resident operands (Z once per problem, the
+// weighted null-model columns and the weights once per h, sigma) and room for
+// the digits of a block of x_b SNPs.  On return use = whether the block's
+// products run on them: the eigenvector product of `cols` columns is large
+// enough, and the device has the memory (twelve bytes an element).  A 4096-SNP
+// block of hard calls at n = 5000, t = 16 takes 2.0 ms on them and 179 ms on the
+// FP64 kernels, with the same error against exact arithmetic (1.4e-14).
+int eigen_digits(fglsgpu_engine* e, long long cols, bool* use) {
+  *use = false;
+  const fglsgpu_config& c = e->cfg;
+  const int n = c.n, nq = c.t * (1 + c.wXL);
+  if (e->dg_off || c.variant != FGLSGPU_VARIANT_EIGEN || !digit_gemm_pays(n, cols, n)) return FGLSGPU_OK;
+  const long long most = (e->probing ? cols : std::max<long long>(cols, (long long)c.x_b * c.wXR)) * c.wXR;
+  size_t none = 0;
+  bool ok = e->dg || digit_gemm_create(&e->dg) == cudaSuccess;
+  if (ok && !e->zmem) ok = grow(&e->zmem, &none, digit_mat_bytes(n, n));
+  none = 0;
+  const size_t wy = (digit_mat_bytes(nq, n) + 255) & ~(size_t)255;
+  if (ok && !e->wmem) ok = grow(&e->wmem, &none, wy + digit_mat_bytes(c.t, n));
+  if (ok) ok = grow(&e->blkmem, &e->blk_bytes, digit_mat_bytes((int)most, n));
+  if (!ok) {
+    (void)cudaGetLastError();
+    drop_digits(e);
+    e->dg_off = true;
+    return FGLSGPU_OK;
+  }
+  if (!e->z_cut) {
+    e->zdig = digit_mat_at(e->zmem, n, n);
+    ENG_TRY(e, digit_cut(e->comp, e->zdig, e->dZ, n, true), "digits of Z");
+    e->z_cut = true;
+  }
+  if (!e->w_cut) {
+    e->ayldig = digit_mat_at(e->wmem, nq, n);
+    e->ddig = digit_mat_at((char*)e->wmem + wy, c.t, n);
+    ENG_TRY(e, digit_cut(e->comp, e->ayldig, e->dAYL, n, true), "digits of the weighted columns");
+    ENG_TRY(e, digit_cut(e->comp, e->ddig, e->ddinv, n, true), "digits of the weights");
+    e->w_cut = true;
+  }
+  *use = true;
+  return FGLSGPU_OK;
+}
+
 // Compute one block already in device memory (n x x*wXR genotypes in format
 // `fmt` at dX) into dB/dV with the given trait strides, on e->comp.
 int compute_block(fglsgpu_engine* e, const void* dX, int fmt, int x, double* dB, double* dV, long long bstr,
@@ -277,18 +359,37 @@ int compute_block(fglsgpu_engine* e, const void* dX, int fmt, int x, double* dB,
     Prof pr(e, FGLSGPU_PROF_GRAM, s);
     ENG_TRY(e, gram_skinny(s, n, x, wXL, wXR, e->dWork, n, e->dWY, e->dGYL, e->dGR), "gram");
   } else {
-    {
-      Prof pr(e, FGLSGPU_PROF_FP64_GEMM, s);
-      ENG_TRY(e, dgemm(s, true, false, n, (int)cols, n, 1.0, e->dZ, n, dXin, n, 0.0, e->dWork, n), "Z^T XR");
-    }
-    Prof pr(e, FGLSGPU_PROF_GRAM, s);
-    ENG_TRY(e, dgemm(s, true, false, (int)cols, t * (1 + wXL), n, 1.0, e->dWork, n, e->dAYL, n, 0.0, e->dGYL,
-                     cols),
-            "gram YL");
+    bool digits = false;
+    const int rc = eigen_digits(e, cols, &digits);
+    if (rc) return rc;
     const long long qcols = cols * wXR;
-    ENG_TRY(e, quad_products(s, n, x, wXR, e->dWork, n, e->dQ, n), "quad");
-    ENG_TRY(e, dgemm(s, true, false, (int)qcols, t, n, 1.0, e->dQ, n, e->ddinv, n, 0.0, e->dGR, qcols),
-            "gram R");
+    if (digits) {
+      // hard-call columns have one digit: 12 of the 78 digit pairs
+      {
+        Prof pr(e, FGLSGPU_PROF_FP64_GEMM, s);
+        const DigitMat xd = digit_mat_at(e->blkmem, (int)cols, n);
+        ENG_TRY(e, digit_cut(s, xd, dXin, n, true), "digits of XR");
+        ENG_TRY(e, digit_mul(e->dg, s, e->zdig, xd, 1.0, 0.0, e->dWork, n), "Z^T XR");
+      }
+      Prof pr(e, FGLSGPU_PROF_GRAM, s);
+      const DigitMat rd = digit_mat_at(e->blkmem, (int)cols, n), qd = digit_mat_at(e->blkmem, (int)qcols, n);
+      ENG_TRY(e, digit_cut(s, rd, e->dWork, n, true), "digits of Z^T XR");
+      ENG_TRY(e, digit_mul(e->dg, s, rd, e->ayldig, 1.0, 0.0, e->dGYL, cols), "gram YL");
+      ENG_TRY(e, digit_cut_products(s, qd, e->dWork, n, wXR), "digits of the squares");
+      ENG_TRY(e, digit_mul(e->dg, s, qd, e->ddig, 1.0, 0.0, e->dGR, qcols), "gram R");
+    } else {
+      {
+        Prof pr(e, FGLSGPU_PROF_FP64_GEMM, s);
+        ENG_TRY(e, dgemm(s, true, false, n, (int)cols, n, 1.0, e->dZ, n, dXin, n, 0.0, e->dWork, n), "Z^T XR");
+      }
+      Prof pr(e, FGLSGPU_PROF_GRAM, s);
+      ENG_TRY(e, dgemm(s, true, false, (int)cols, t * (1 + wXL), n, 1.0, e->dWork, n, e->dAYL, n, 0.0, e->dGYL,
+                       cols),
+              "gram YL");
+      ENG_TRY(e, quad_products(s, n, x, wXR, e->dWork, n, e->dQ, n), "quad");
+      ENG_TRY(e, dgemm(s, true, false, (int)qcols, t, n, 1.0, e->dQ, n, e->ddinv, n, 0.0, e->dGR, qcols),
+              "gram R");
+    }
   }
   Prof pr(e, FGLSGPU_PROF_SOLVE, s);
   ENG_TRY(e, snp_solve(s, p, x, t, wXL, e->dtop, e->dGYL, 1, cols, e->dGR, cols * wXR, dB, bstr, dV, vstr, e->dst,
@@ -371,7 +472,9 @@ int tune_slices(fglsgpu_engine* e) {
     e->dQ = dQ;
   }
   c.precision = FGLSGPU_PREC_FP64;
+  e->probing = true;
   if (!rc) rc = compute_block(e, dX, GENO_F64, xp, dBr, dVr, (long long)xp * p, (long long)xp * p * p, 0);
+  e->probing = false;
   c.precision = FGLSGPU_PREC_SPLIT;
   e->dWork = keepW;
   e->dQ = keepQ;
@@ -431,6 +534,7 @@ int tune_slices(fglsgpu_engine* e) {
   }
   release();
   if (!rc) rc = check_status(e, "slice probe");
+  drop_digits(e);  // the FP64 probe's operands: the split path needs the memory itself
   if (rc) return rc;
   ENG_TRY(e, ozaki_set_run_slices(e->oz, s, chosen), "slice choice");
   ENG_TRY(e, cudaStreamSynchronize(s), "slice choice");
@@ -499,7 +603,7 @@ int fglsgpu_create(const fglsgpu_config* cfg, fglsgpu_engine** out) {
   chk(dalloc(&e->dtop, t * e->topw));
   chk(dalloc(&e->dst, 1));
   chk(cudaMallocHost((void**)&e->hst, sizeof(DevStatus)));
-  chk(cudaMallocHost((void**)&e->hst_wait, sizeof(int)));
+  chk(cudaMallocHost((void**)&e->hst_wait, 2 * sizeof(int)));
   for (int k = 0; k < 2; k++) {
     chk(dalloc(&e->dX[k], n * xb * wXR));
     chk(dalloc(&e->dB[k], (long long)nt * xb * p));
@@ -576,12 +680,17 @@ int fglsgpu_set_problem(fglsgpu_engine* e, const double* Phi, const double* XL, 
     if (qfail) return fail(e, FGLSGPU_ENOCONV, "dsyevr failed (info: 1): QL iteration did not converge");
     ENG_TRY(e, dgemm(s, true, false, c.n, c.wXL, c.n, 1.0, e->dZ, n, e->dXL, n, 0.0, e->dZtXL, n), "Z^T XL");
     ENG_TRY(e, dgemm(s, true, false, c.n, c.t, c.n, 1.0, e->dZ, n, e->dY, n, 0.0, e->dZtY, n), "Z^T Y");
+    e->z_cut = e->w_cut = false;
     ENG_TRY(e, eigen_traits(s, c.n, c.t, c.wXL, e->dW, e->dh, e->dsig, e->dZtXL, e->dZtY, e->ddinv, e->dAYL,
                             e->dtop, e->dst),
             "trait weights");
     rc = check_status(e, "eigen setup");
     if (rc) return rc;
-    if (split(e)) {
+    if (!split(e)) {
+      bool use;
+      rc = eigen_digits(e, (long long)c.x_b * c.wXR, &use);
+      if (rc) return rc;
+    } else {
       if (!e->oz) {
         ENG_TRY(e, ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, /*eigen=*/1), "split plan");
         ozaki_set_wait_limit(e->oz, e->wait_ns);
@@ -1060,6 +1169,7 @@ int fglsgpu_set_hsigma(fglsgpu_engine* e, const double* h, const double* sigma) 
   int rc = reset_status(e);
   if (rc) return rc;
   e->problem_set = false;
+  e->w_cut = false;
   ENG_TRY(e, eigen_traits(s, c.n, c.t, c.wXL, e->dW, e->dh, e->dsig, e->dZtXL, e->dZtY, e->ddinv, e->dAYL,
                           e->dtop, e->dst),
           "trait weights");

@@ -66,6 +66,7 @@
 #include "fgls_kernels.cuh"
 #include "fgls_ozaki.cuh"
 #include "fgls_selfgram.cuh"
+#include "fgls_tc.cuh"
 #include "fgls_batch.cuh"
 
 namespace fgls {
@@ -102,181 +103,6 @@ constexpr int GROUP_M = 8;
 // tcgen05.mma instruction descriptor, kind::f8f6f4: D=F32, A=B=E4M3
 // (format 0), both K-major, N=256, M=128.
 constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ uint64_t globaltimer_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-constexpr uint64_t WAIT_NS = 2000000000ull;  // default limit of one wait: 2 s
-
-// Bounded wait: false if the phase does not complete within `limit_ns` (the
-// kernel-wide error word `err` then records `site`), or if this CTA or any
-// other CTA of the launch (or an earlier launch since the host last cleared
-// `err`) already gave up.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                          int* err, int site, uint64_t limit_ns) {
-  const uint64_t t0 = globaltimer_ns();
-  for (uint32_t it = 0;; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
-    // the clock after the first miss (a short limit takes effect at once)
-    // and every 64; the error words, which cost a memory load, every 64
-    const bool every = (it & 63) == 63;
-    if (every && (*abort_flag || *(volatile int*)err)) {
-      *abort_flag = 1;
-      return false;
-    }
-    if ((every || it == 0) && globaltimer_ns() - t0 > limit_ns) {
-      *abort_flag = 1;
-      atomicCAS(err, 0, site);
-      return false;
-    }
-  }
-}
-
-// Drain wait of a CTA pair's leader on the abort path: one deadline for all
-// its stages (a stage may never complete when the peer gave up before its
-// copies; the leader's own copies land within microseconds).
-__device__ __forceinline__ void mbar_drain_until(uint64_t* bar, uint32_t parity, uint64_t deadline) {
-  while (!mbar_try_wait(bar, parity) && globaltimer_ns() < deadline) {
-  }
-}
-
-// Bounded drain wait used on the abort path only (always the default limit,
-// so that no copy or MMA of this CTA outlives its shared memory or TMEM).
-__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
-  const uint64_t t0 = globaltimer_ns();
-  while (!mbar_try_wait(bar, parity) && globaltimer_ns() - t0 < WAIT_NS) {
-  }
-}
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tm, int x, int y, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-          smem_u32(dst)),
-      "l"((uint64_t)tm), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// 2-SM (cluster of two CTAs) forms.  `bar` below is a shared::cluster
-// address, possibly of the peer CTA's barrier (mapa).
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {  // the same variable in CTA `rank`
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-  return r;
-}
-// every thread of both CTAs (a superset of __syncthreads)
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// a copy into this CTA's shared memory that completes on the barrier at
-// cluster address `bar` (the pair leader's)
-__device__ __forceinline__ void tma_load_2d_cg2(void* dst, const CUtensorMap* tm, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
-      "[%4];" ::"r"(smem_u32(dst)),
-      "l"((uint64_t)tm), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
-
-__device__ __forceinline__ uint64_t desc_sw128(const void* p) {
-  const uint32_t a = smem_u32(p);
-  uint64_t d = 0;
-  d |= (uint64_t)((a & 0x3FFFFu) >> 4);  // start address
-  d |= (uint64_t)1 << 16;                // leading byte offset (unused for SW128 K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;      // stride byte offset: 8 rows x 128 B
-  d |= (uint64_t)1 << 46;                // descriptor version (sm_100 family)
-  d |= (uint64_t)2 << 61;                // 128B swizzle
-  return d;
-}
-
-__device__ __forceinline__ void mma_f8(uint32_t dt, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(dt),
-      "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-      : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-// 2-SM MMA (issued by the pair leader; operands from both CTAs' shared
-// memory at the same offsets, accumulator in both CTAs' TMEM)
-__device__ __forceinline__ void mma_f8_cg2(uint32_t dt, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(dt),
-      "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-      : "memory");
-}
-// arrive on the barrier at `bar`'s offset in each CTA of `mask` once the
-// leader's 2-SM MMAs so far have completed
-__device__ __forceinline__ void mma_commit_cg2(uint64_t* bar, uint16_t mask) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-                   smem_u32(bar)),
-               "h"(mask)
-               : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 struct GemmArgs {
   int M;            // valid rows of A

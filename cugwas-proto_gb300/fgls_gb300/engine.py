@@ -44,6 +44,7 @@ EXPORTS = (
     "fglsgpu_batch_profile_read", "fglsgpu_run_block_device_packed", "fglsgpu_run_snps_compact",
     "fglsgpu_reml_fit", "fglsgpu_set_hsigma", "fglsgpu_set_wait_limit", "fglsgpu_run_snps_u8",
     "fglsgpu_run_snps_packed", "fglsgpu_split_params", "fglsgpu_quad_digits", "fglsgpu_batch_tile",
+    "fglsgpu_selftest_dgemm",
 )
 PROF_CLASSES = ("genotypes", "split_gemm", "selfgram", "solve", "fp64_gemm", "trsm", "gram", "spare")
 
@@ -104,6 +105,7 @@ def lib():
     L.fglsgpu_last_error.restype = C.c_char_p
     L.fglsgpu_version.restype = I
     L.fglsgpu_selftest_split_gemm.argtypes = [I, I, I, I, P, P, P]
+    L.fglsgpu_selftest_dgemm.argtypes = [I, I, I, I, I, C.c_double, P, LL, P, LL, C.c_double, P, LL, I, P]
     L.fglsgpu_set_precision.argtypes = [P, I]
     L.fglsgpu_profile.argtypes = [P, I]
     L.fglsgpu_profile_read.argtypes = [P, P, P]

@@ -297,6 +297,16 @@ int fglsgpu_version(void);
 int fglsgpu_selftest_split_gemm(int M, int K, int N, int slices, const double *A, const double *X,
                                 double *C);
 
+/* Diagnostic: C = alpha * op(A) * op(B) + beta * C in FP64 (column-major,
+ * device pointers; op(A) M x K, op(B) K x N, transA / transB != 0 transpose)
+ * through the engine's FP64 kernel (digits = 0) or through its exact sums of
+ * FP8 digit products (digits != 0), the two forms the FP64 path picks from by
+ * size.  `ms` (may be NULL) receives the device time.  Returns when C is
+ * written.  No counterpart in the reference (its GEMMs are BLAS calls). */
+int fglsgpu_selftest_dgemm(int transA, int transB, int M, int N, int K, double alpha, const double *A,
+                           long long lda, const double *B, long long ldb, double beta, double *C,
+                           long long ldc, int digits, double *ms);
+
 /* The same split-precision GEMM for callers that may not allocate device
  * memory (code running under a framework that owns the device through its
  * own memory pool, or that must keep the device's footprint fixed).  All
