@@ -864,30 +864,44 @@ bool digit_gemm_pays(long long M, long long N, long long K) {
   return K >= 64 && digits < fp64;
 }
 
+namespace {
+bool reserve(DigitGemm* g, int q, size_t bytes) {
+  if (g->op_bytes[q] >= bytes) return true;
+  if (g->op[q]) cudaFree(g->op[q]);
+  g->op[q] = nullptr;
+  g->op_bytes[q] = 0;
+  if (cudaMalloc(&g->op[q], bytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    g->op[q] = nullptr;
+    return false;
+  }
+  g->op_bytes[q] = bytes;
+  return true;
+}
+}  // namespace
+
+bool digit_gemm_reserve(DigitGemm* g, int rows, int K) {
+  const size_t b = digit_mat_bytes(rows, K);
+  return reserve(g, 0, b) && reserve(g, 1, b);
+}
+
+void digit_gemm_trim(DigitGemm* g) {
+  if (!g) return;
+  for (int q = 0; q < 2; q++) {
+    if (g->op[q]) cudaFree(g->op[q]);
+    g->op[q] = nullptr;
+    g->op_bytes[q] = 0;
+  }
+}
+
 cudaError_t digit_dgemm(DigitGemm* g, cudaStream_t s, bool tA, bool tB, int M, int N, int K, double alpha,
                         const double* A, long long lda, const double* B, long long ldb, double beta, double* C,
                         long long ldc) {
-  if (g && digit_gemm_pays(M, N, K)) {
-    const size_t need[2] = {digit_mat_bytes(M, K), digit_mat_bytes(N, K)};
-    bool ok = true;
-    for (int q = 0; q < 2 && ok; q++) {
-      if (g->op_bytes[q] >= need[q]) continue;
-      if (g->op[q]) cudaFree(g->op[q]);
-      g->op[q] = nullptr;
-      g->op_bytes[q] = 0;
-      if (cudaMalloc(&g->op[q], need[q]) == cudaSuccess) {
-        g->op_bytes[q] = need[q];
-      } else {
-        (void)cudaGetLastError();
-        ok = false;
-      }
-    }
-    if (ok) {
-      const DigitMat a = digit_mat_at(g->op[0], M, K), b = digit_mat_at(g->op[1], N, K);
-      FGLS_CUDA_TRY(digit_cut(s, a, A, lda, tA));
-      FGLS_CUDA_TRY(digit_cut(s, b, B, ldb, !tB));
-      return digit_mul(g, s, a, b, alpha, beta, C, ldc);
-    }
+  if (g && digit_gemm_pays(M, N, K) && reserve(g, 0, digit_mat_bytes(M, K)) && reserve(g, 1, digit_mat_bytes(N, K))) {
+    const DigitMat a = digit_mat_at(g->op[0], M, K), b = digit_mat_at(g->op[1], N, K);
+    FGLS_CUDA_TRY(digit_cut(s, a, A, lda, tA));
+    FGLS_CUDA_TRY(digit_cut(s, b, B, ldb, !tB));
+    return digit_mul(g, s, a, b, alpha, beta, C, ldc);
   }
   return dgemm(s, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
 }

@@ -51,6 +51,11 @@ cudaError_t digit_mul(DigitGemm* g, cudaStream_t s, const DigitMat& A, const Dig
 cudaError_t digit_dgemm(DigitGemm* g, cudaStream_t s, bool tA, bool tB, int M, int N, int K, double alpha,
                         const double* A, long long lda, const double* B, long long ldb, double beta, double* C,
                         long long ldc);
+// room for operands of up to `rows` x K each (so that digit_dgemm allocates
+// nothing); false when the device has not the memory.  digit_gemm_trim gives
+// the operands' room back.
+bool digit_gemm_reserve(DigitGemm* g, int rows, int K);
+void digit_gemm_trim(DigitGemm* g);
 // whether digit_dgemm takes the digits for this product
 bool digit_gemm_pays(long long M, long long N, long long K);
 

@@ -20,6 +20,7 @@
 #include <cstdlib>
 
 #include "fgls_common.cuh"
+#include "fgls_digit_gemm.cuh"
 #include "fgls_kernels.cuh"
 
 namespace fgls {
@@ -318,29 +319,65 @@ __global__ void build_y_kernel(int n, int b, int nb, const double* __restrict__ 
   }
 }
 
-// Compact-WY factor T (nb x nb upper, ld nb, nb <= 256) of
-// H_b ... H_{b+nb-1} = I - Y T Y^T from tau and G = Y^T Y (forward,
-// columnwise): T_ii = tau_i, T[0:i, i] = -tau_i T[0:i, 0:i] G[0:i, i].  One
-// CTA of 256 threads, column by column.
-__global__ void __launch_bounds__(256) larft_kernel(int nb, const double* __restrict__ tau, const double* G,
-                                                    double* T) {
-  __shared__ double g[256];
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) T[e] = 0.0;
-  __syncthreads();
-  for (int i = 0; i < nb; i++) {
-    const double ti = tau[i];
-    if (threadIdx.x < i) g[threadIdx.x] = G[threadIdx.x + (long long)i * nb];
-    __syncthreads();
-    if (threadIdx.x < i) {
-      const int r = threadIdx.x;
-      double acc = 0.0;
-      for (int q = 0; q < i; q++)  // all threads read column q together (coalesced); T upper: rows r <= q
-        if (q >= r) acc += T[r + (long long)q * nb] * g[q];
-      T[r + (long long)i * nb] = -ti * acc;
-    }
-    if (threadIdx.x == 0) T[i + (long long)i * nb] = ti;
-    __syncthreads();
+// Compact-WY factor T (nb x nb upper, ld nb) of H_b ... H_{b+nb-1} =
+// I - Y T Y^T from tau and G = Y^T Y (forward, columnwise):
+//   T_ii = tau_i, T[0:i, i] = -tau_i T[0:i, 0:i] G[0:i, i].
+// Column by column that is one CTA's serial chain through global memory (2.0
+// ms at nb = 256).  Instead 32 x 32 diagonal blocks, one warp each, then
+// merges of neighbours, [T1, -T1 G12 T2; 0, T2], 32 -> 64 -> .. with one
+// thread per element and 16 x 16 outputs per CTA: seven launches, 0.05 ms.
+constexpr int LB = 32;
+__global__ void __launch_bounds__(LB) larft_base_kernel(int nb, const double* __restrict__ tau,
+                                                        const double* __restrict__ G, double* __restrict__ T) {
+  __shared__ double g[LB][LB + 1], t[LB][LB + 1];  // [column][row]
+  const int o = blockIdx.x * LB, m = min(LB, nb - o), r = threadIdx.x;
+  for (int i = 0; i < m; i++) {
+    g[i][r] = r < i ? G[(o + r) + (long long)(o + i) * nb] : 0.0;
+    t[i][r] = 0.0;
   }
+  __syncwarp();
+  for (int i = 0; i < m; i++) {
+    const double ti = tau[o + i];
+    double acc = 0.0;
+    for (int q = r; q < i; q++) acc = fma(t[q][r], g[i][q], acc);
+    if (r < i) t[i][r] = -ti * acc;
+    if (r == i) t[i][r] = ti;
+    __syncwarp();
+  }
+  for (int i = 0; i < m; i++)
+    if (r < m) T[(o + r) + (long long)(o + i) * nb] = t[i][r];
+}
+// Merge of the blocks [o, o + w) and [o + w, o + w + w2), o = 2 w blockIdx.z:
+// first P = G12 T2, then T12 = -T1 P.
+template <bool FIRST>
+__global__ void __launch_bounds__(256) larft_merge_kernel(int nb, int w, const double* __restrict__ G,
+                                                          double* __restrict__ T, double* __restrict__ P) {
+  const int o = 2 * w * blockIdx.z, w2 = min(w, nb - o - w);
+  const int r = blockIdx.x * 16 + (threadIdx.x & 15), c = blockIdx.y * 16 + (threadIdx.x >> 4);
+  if (r >= w || c >= w2) return;
+  double* p = P + (long long)blockIdx.z * w * w;
+  double acc = 0.0;
+  if (FIRST) {
+    for (int q = 0; q <= c; q++)
+      acc = fma(G[(o + r) + (long long)(o + w + q) * nb], T[(o + w + q) + (long long)(o + w + c) * nb], acc);
+    p[r + c * w] = acc;
+  } else {
+    for (int q = r; q < w; q++) acc = fma(T[(o + r) + (long long)(o + q) * nb], p[q + c * w], acc);
+    T[(o + r) + (long long)(o + w + c) * nb] = -acc;
+  }
+}
+// T from G and tau; P: scratch of nb^2 / 2 elements
+cudaError_t larft(cudaStream_t s, int nb, const double* tau, const double* G, double* T, double* P, long long* nl) {
+  FGLS_CUDA_TRY(cudaMemsetAsync(T, 0, sizeof(double) * nb * nb, s));
+  larft_base_kernel<<<ceil_div(nb, LB), LB, 0, s>>>(nb, tau, G, T);
+  (*nl)++;
+  for (int w = LB; w < nb; w *= 2) {
+    const dim3 grid(ceil_div(w, 16), ceil_div(w, 16), ceil_div(nb - w, 2 * w));
+    larft_merge_kernel<true><<<grid, 256, 0, s>>>(nb, w, G, T, P);
+    larft_merge_kernel<false><<<grid, 256, 0, s>>>(nb, w, G, T, P);
+    *nl += 2;
+  }
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -353,7 +390,7 @@ size_t eig_workspace_bytes(int n) {
   return sizeof(double) * ((size_t)n * 8 + nt + nr + nt * nt * ST) + sizeof(int) * (size_t)n + 256;
 }
 
-cudaError_t dsyev_device(cudaStream_t s, int n, const double* Phi, long long ldp, double* A, double* Z,
+cudaError_t dsyev_device(cudaStream_t s, DigitGemm* dg, int n, const double* Phi, long long ldp, double* A, double* Z,
                          double* W, void* work, int* fail_out, long long* launches) {
   double* d = (double*)work;
   double* e = d + n;
@@ -374,6 +411,11 @@ cudaError_t dsyev_device(cudaStream_t s, int n, const double* Phi, long long ldp
   auto mark = [&](int i) {
     if (timing) cudaEventRecord(ev[i], s);
   };
+  // the products' digits: largest operands n x n; given back below
+  if (dg && !(digit_gemm_pays(n, n, 256) && digit_gemm_reserve(dg, n, n))) {
+    digit_gemm_trim(dg);
+    dg = nullptr;
+  }
   mark(0);
   // A := Phi (lower) symmetrized
   FGLS_CUDA_TRY(cudaMemcpy2DAsync(A, sizeof(double) * n, Phi, sizeof(double) * ldp, sizeof(double) * n, n,
@@ -412,7 +454,7 @@ cudaError_t dsyev_device(cudaStream_t s, int n, const double* Phi, long long ldp
   FGLS_CUDA_TRY(cudaMalloc(&dcw, std::max(dc_workspace_bytes(n), bt_bytes)));
   int* dfail = rank;  // n ints of scratch; first used as the failure flag
   FGLS_CUDA_TRY(cudaMemsetAsync(dfail, 0, sizeof(int), s));
-  cudaError_t rc = dc_tridiag_eig(s, n, d, e, W, Z, dcw, dfail, &nl);
+  cudaError_t rc = dc_tridiag_eig(s, dg, n, d, e, W, Z, dcw, dfail, &nl);
   mark(3);
   // 4. Z := H_0 H_1 ... H_{n-3} Z, blocks of NB reflectors from the last one
   //    in compact-WY form (I - Y T Y^T): three DGEMMs per block, 2 n^3 flops
@@ -430,21 +472,23 @@ cudaError_t dsyev_device(cudaStream_t s, int n, const double* Phi, long long ldp
       const int mr = n - b - 1;
       double* Zs = Z + (b + 1);  // rows b+1 .. n-1, all n columns (ld n)
       build_y_kernel<<<grid_for((long long)mr * nb), 256, 0, s>>>(n, b, nb, A, n, Yb);
-      // G = Y^T Y has only (nb/64)^2 output tiles: K split over the SMs, W2 as scratch
-      rc = dgemm_splitk(s, true, false, nb, nb, mr, 1.0, Yb, mr, Yb, mr, 0.0, G, nb, W2, (long long)NB * n);
-      if (rc == cudaSuccess) {
-        larft_kernel<<<1, 256, 0, s>>>(nb, tau + b, G, Tm);
-        rc = dgemm(s, true, false, nb, n, mr, 1.0, Yb, mr, Zs, n, 0.0, Wb, nb);
-      }
-      if (rc == cudaSuccess) rc = dgemm(s, false, false, nb, n, nb, 1.0, Tm, nb, Wb, nb, 0.0, W2, nb);
-      if (rc == cudaSuccess) rc = dgemm(s, false, false, mr, n, nb, -1.0, Yb, mr, W2, nb, 1.0, Zs, n);
-      nl += 2;
+      // G = Y^T Y has few output tiles: K split over the SMs either way (W2 as scratch)
+      if (dg && digit_gemm_pays(nb, nb, mr))
+        rc = digit_dgemm(dg, s, true, false, nb, nb, mr, 1.0, Yb, mr, Yb, mr, 0.0, G, nb);
+      else
+        rc = dgemm_splitk(s, true, false, nb, nb, mr, 1.0, Yb, mr, Yb, mr, 0.0, G, nb, W2, (long long)NB * n);
+      if (rc == cudaSuccess) rc = larft(s, nb, tau + b, G, Tm, W2, &nl);
+      if (rc == cudaSuccess) rc = digit_dgemm(dg, s, true, false, nb, n, mr, 1.0, Yb, mr, Zs, n, 0.0, Wb, nb);
+      if (rc == cudaSuccess) rc = digit_dgemm(dg, s, false, false, nb, n, nb, 1.0, Tm, nb, Wb, nb, 0.0, W2, nb);
+      if (rc == cudaSuccess) rc = digit_dgemm(dg, s, false, false, mr, n, nb, -1.0, Yb, mr, W2, nb, 1.0, Zs, n);
+      nl++;
     }
   }
   int hfail = 0;
   if (rc == cudaSuccess) rc = cudaMemcpyAsync(&hfail, dfail, sizeof(int), cudaMemcpyDeviceToHost, s);
   if (rc == cudaSuccess) rc = cudaStreamSynchronize(s);
   cudaFree(dcw);
+  digit_gemm_trim(dg);
   FGLS_CUDA_TRY(rc);
   *fail_out = hfail;
   mark(4);

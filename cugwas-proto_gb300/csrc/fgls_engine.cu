@@ -535,6 +535,7 @@ int tune_slices(fglsgpu_engine* e) {
   release();
   if (!rc) rc = check_status(e, "slice probe");
   drop_digits(e);  // the FP64 probe's operands: the split path needs the memory itself
+  digit_gemm_trim(e->dg);
   if (rc) return rc;
   ENG_TRY(e, ozaki_set_run_slices(e->oz, s, chosen), "slice choice");
   ENG_TRY(e, cudaStreamSynchronize(s), "slice choice");
@@ -675,11 +676,16 @@ int fglsgpu_set_problem(fglsgpu_engine* e, const double* Phi, const double* XL, 
   e->problem_set = false;
   if (c.variant == FGLSGPU_VARIANT_EIGEN) {
     int qfail = 0;
-    ENG_TRY(e, dsyev_device(s, c.n, e->dPhi, n, e->dL, e->dZ, e->dW, e->deigwork, &qfail, nullptr),
+    if (!e->dg && !e->dg_off && digit_gemm_create(&e->dg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      e->dg_off = true;
+    }
+    ENG_TRY(e, dsyev_device(s, e->dg, c.n, e->dPhi, n, e->dL, e->dZ, e->dW, e->deigwork, &qfail, nullptr),
             "eigendecomposition");
     if (qfail) return fail(e, FGLSGPU_ENOCONV, "dsyevr failed (info: 1): QL iteration did not converge");
-    ENG_TRY(e, dgemm(s, true, false, c.n, c.wXL, c.n, 1.0, e->dZ, n, e->dXL, n, 0.0, e->dZtXL, n), "Z^T XL");
-    ENG_TRY(e, dgemm(s, true, false, c.n, c.t, c.n, 1.0, e->dZ, n, e->dY, n, 0.0, e->dZtY, n), "Z^T Y");
+    ENG_TRY(e, digit_dgemm(e->dg, s, true, false, c.n, c.wXL, c.n, 1.0, e->dZ, n, e->dXL, n, 0.0, e->dZtXL, n),
+            "Z^T XL");
+    ENG_TRY(e, digit_dgemm(e->dg, s, true, false, c.n, c.t, c.n, 1.0, e->dZ, n, e->dY, n, 0.0, e->dZtY, n), "Z^T Y");
     e->z_cut = e->w_cut = false;
     ENG_TRY(e, eigen_traits(s, c.n, c.t, c.wXL, e->dW, e->dh, e->dsig, e->dZtXL, e->dZtY, e->ddinv, e->dAYL,
                             e->dtop, e->dst),
@@ -695,7 +701,7 @@ int fglsgpu_set_problem(fglsgpu_engine* e, const double* Phi, const double* XL, 
         ENG_TRY(e, ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, /*eigen=*/1), "split plan");
         ozaki_set_wait_limit(e->oz, e->wait_ns);
       }
-      ENG_TRY(e, ozaki_set_eigen(e->oz, s, e->dZ, e->dAYL, e->ddinv), "split operands");
+      ENG_TRY(e, ozaki_set_eigen(e->oz, s, e->dg, e->dZ, e->dAYL, e->ddinv), "split operands");
       ENG_TRY(e, cudaStreamSynchronize(s), "split operands");
       rc = tune_slices(e);
       if (rc) return rc;
@@ -951,7 +957,7 @@ int fglsgpu_set_precision(fglsgpu_engine* e, int precision) {
   if (precision == FGLSGPU_PREC_SPLIT && e->problem_set && c.variant == FGLSGPU_VARIANT_EIGEN) {
     if (!e->oz) ENG_TRY(e, ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, 1), "split plan");
     ozaki_set_wait_limit(e->oz, e->wait_ns);
-    ENG_TRY(e, ozaki_set_eigen(e->oz, e->comp, e->dZ, e->dAYL, e->ddinv), "split operands");
+    ENG_TRY(e, ozaki_set_eigen(e->oz, e->comp, e->dg, e->dZ, e->dAYL, e->ddinv), "split operands");
     ENG_TRY(e, cudaStreamSynchronize(e->comp), "split operands");
     const int rc = tune_slices(e);
     if (rc) return rc;
@@ -1178,7 +1184,7 @@ int fglsgpu_set_hsigma(fglsgpu_engine* e, const double* h, const double* sigma) 
   if (split(e)) {
     if (!e->oz) ENG_TRY(e, ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, 1), "split plan");
     ozaki_set_wait_limit(e->oz, e->wait_ns);
-    ENG_TRY(e, ozaki_set_eigen(e->oz, s, e->dZ, e->dAYL, e->ddinv), "split operands");
+    ENG_TRY(e, ozaki_set_eigen(e->oz, s, e->dg, e->dZ, e->dAYL, e->ddinv), "split operands");
     ENG_TRY(e, cudaStreamSynchronize(s), "split operands");
     rc = tune_slices(e);
     if (rc) return rc;

@@ -42,15 +42,17 @@ cudaError_t snp_solve(cudaStream_t s, int p, int x, int t, int wXL, const double
 
 // Eigendecomposition (fgls_eig.cu).  A and Z: n x n device scratch/outputs
 // (ld n); work: eig_workspace_bytes(n).  *fail_out = 1 if QL did not converge.
+// dg (may be null): its matrix products run as exact digit products.
+struct DigitGemm;
 size_t eig_workspace_bytes(int n);
-cudaError_t dsyev_device(cudaStream_t s, int n, const double* Phi, long long ldp, double* A, double* Z,
+cudaError_t dsyev_device(cudaStream_t s, DigitGemm* dg, int n, const double* Phi, long long ldp, double* A, double* Z,
                          double* W, void* work, int* fail_out, long long* launches);
 
 // Divide-and-conquer eigensolver of the tridiagonal (d, e) (fgls_dc.cu):
 // W ascending, V (n x n) eigenvectors; d, e are overwritten; fail_dev set
 // to 1 if a leaf iteration did not converge.
 size_t dc_workspace_bytes(int n);
-cudaError_t dc_tridiag_eig(cudaStream_t s, int n, double* d, double* e, double* W, double* V, void* work,
+cudaError_t dc_tridiag_eig(cudaStream_t s, DigitGemm* dg, int n, double* d, double* e, double* W, double* V, void* work,
                            int* fail_dev, long long* launches);
 
 // Batched cohorts: solves of all problems with p predictors listed in plist

@@ -63,6 +63,7 @@
 #include <vector>
 
 #include "fgls_common.cuh"
+#include "fgls_digit_gemm.cuh"
 #include "fgls_kernels.cuh"
 #include "fgls_ozaki.cuh"
 #include "fgls_selfgram.cuh"
@@ -2226,9 +2227,10 @@ cudaError_t selfgram(OzakiPlan* p, cudaStream_t s, int col0, int xq, int t, doub
 
 }  // namespace
 
-cudaError_t ozaki_set_eigen(OzakiPlan* p, cudaStream_t s, const double* Z, const double* AYL, const double* dinv) {
+cudaError_t ozaki_set_eigen(OzakiPlan* p, cudaStream_t s, DigitGemm* dg, const double* Z, const double* AYL,
+                            const double* dinv) {
   // U = Z * AYL (FP64, once per problem): x~^T y~_j = x^T U[:, j] etc.
-  FGLS_CUDA_TRY(dgemm(s, false, false, p->n, p->nU, p->n, 1.0, Z, p->n, AYL, p->n, 0.0, p->U, p->n));
+  FGLS_CUDA_TRY(digit_dgemm(dg, s, false, false, p->n, p->nU, p->n, 1.0, Z, p->n, AYL, p->n, 0.0, p->U, p->n));
   // rows of Z^T are the columns of Z (contiguous): ld n
   FGLS_CUDA_TRY(slice_operands(p, s, Z, p->n, p->n));
   split_pairs_kernel<<<p->t, 256, 0, s>>>(p->n, p->t, dinv, p->D, p->dmax);

@@ -17,7 +17,10 @@ struct OzakiPlan;
 cudaError_t ozaki_create(OzakiPlan** out, int n, int t, int wXL, int wXR, int x_b, int slices, int eigen);
 void ozaki_destroy(OzakiPlan* p);
 // eigen: Z (n x n), AYL (n x t(1+wXL)), dinv (n x t)
-cudaError_t ozaki_set_eigen(OzakiPlan* p, cudaStream_t s, const double* Z, const double* AYL, const double* dinv);
+// (dg, here and below: digit products for the FP64 operand setup; may be null)
+struct DigitGemm;
+cudaError_t ozaki_set_eigen(OzakiPlan* p, cudaStream_t s, DigitGemm* dg, const double* Z, const double* AYL,
+                            const double* dinv);
 // chol: L (n x n lower), WY = [y~ | XL~] (n x (1+wXL)) of the selected trait
 cudaError_t ozaki_set_chol(OzakiPlan* p, cudaStream_t s, const double* L, const double* WY);
 // A genotype block on the device in one of three formats (exactly one
