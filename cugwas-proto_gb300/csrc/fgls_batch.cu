@@ -45,6 +45,7 @@
 
 #include "fgls_batch.cuh"
 #include "fgls_common.cuh"
+#include "fgls_digit_gemm.cuh"
 #include "fgls_kernels.cuh"
 #include "fgls_ozaki.cuh"
 #include "fgls_selfgram.cuh"
@@ -422,8 +423,9 @@ int time_step(fglsgpu_batch* b, int x_b, double* rate) {
 // FP64-path beta on the probe block.  Scratch: L, Linv, LinvT (n x n), WY,
 // U (n x (1+wXL)), X64 / GYL / GR64 / Bp / Vp for the probe.
 struct Scratch {
-  double *L = nullptr, *Linv = nullptr, *LinvT = nullptr, *WY = nullptr, *U = nullptr;
-  double *X64 = nullptr, *GYL = nullptr, *GR64 = nullptr, *Vp = nullptr;
+  double *L = nullptr, *Linv = nullptr, *LinvT = nullptr, *WY = nullptr, *U = nullptr, *diag = nullptr;
+  DigitGemm* dg = nullptr;  // digit products of the FP64 setup; null: FP64 kernels
+  double *X64 = nullptr, *Xw = nullptr, *GYL = nullptr, *GR64 = nullptr, *Vp = nullptr;
   DevStatus* st = nullptr;
   cudaStream_t s = nullptr;
   cudaError_t alloc(int nmax, int wmax) {
@@ -431,9 +433,16 @@ struct Scratch {
     cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
     for (double** v : {&L, &Linv, &LinvT})
       if (e == cudaSuccess) e = dalloc(v, nn);
+    if (e == cudaSuccess) e = dalloc(&diag, 64 * 64);
+    if (e == cudaSuccess && (digit_gemm_create(&dg) != cudaSuccess || !digit_gemm_reserve(dg, nmax, nmax))) {
+      (void)cudaGetLastError();
+      digit_gemm_destroy(dg);
+      dg = nullptr;
+    }
     if (e == cudaSuccess) e = dalloc(&WY, (size_t)nmax * (1 + wmax));
     if (e == cudaSuccess) e = dalloc(&U, (size_t)nmax * (1 + wmax));
     if (e == cudaSuccess) e = dalloc(&X64, (size_t)nmax * PROBE);
+    if (e == cudaSuccess) e = dalloc(&Xw, (size_t)nmax * PROBE);
     if (e == cudaSuccess) e = dalloc(&GYL, (size_t)PROBE * (1 + wmax));
     if (e == cudaSuccess) e = dalloc(&GR64, (size_t)PROBE);
     if (e == cudaSuccess) e = dalloc(&Vp, (size_t)PROBE * FGLS_MAX_P * FGLS_MAX_P);
@@ -442,7 +451,8 @@ struct Scratch {
     return e;
   }
   void release() {
-    void* ptrs[] = {L, Linv, LinvT, WY, U, X64, GYL, GR64, Vp, st};
+    digit_gemm_destroy(dg);
+    void* ptrs[] = {L, Linv, LinvT, WY, U, diag, X64, Xw, GYL, GR64, Vp, st};
     for (void* v : ptrs)
       if (v) cudaFree(v);
     if (s) cudaStreamDestroy(s);
@@ -465,16 +475,23 @@ cudaError_t setup_problem(fglsgpu_batch* b, Scratch& w, const CohortInputs& ci, 
   const double h = in.h[q.j], sg = in.sigma[q.j];
   probe_genotypes_kernel<<<256, 256, 0, s>>>(q.c, n, PROBE, q.j == 0 ? b->co[q.c].probe : nullptr, w.X64);
   FGLS_CUDA_TRY(build_shifted(s, n, ci.Phi, n, h * sg, (1.0 - h) * sg, w.L, n));
-  FGLS_CUDA_TRY(dpotrf_lower(s, n, w.L, n, w.st));
-  FGLS_CUDA_TRY(cudaMemcpyAsync(w.WY, ci.Y + (size_t)q.j * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-  FGLS_CUDA_TRY(cudaMemcpyAsync(w.WY + n, ci.XL, sizeof(double) * n * wXL, cudaMemcpyDeviceToDevice, s));
-  FGLS_CUDA_TRY(dtrsm_llnn(s, n, 1 + wXL, w.L, n, w.WY, n));
+  FGLS_CUDA_TRY(dpotrf_lower(s, w.dg, n, w.L, n, w.diag, w.st));
+  FGLS_CUDA_TRY(lower_inverse(s, w.dg, n, w.L, n, w.Linv));
+  // [y | XL] whitened: a product with L^-1, or the solve for small cohorts
+  const bool product = w.dg && n >= 1024;
+  double* raw = product ? w.U : w.WY;
+  FGLS_CUDA_TRY(cudaMemcpyAsync(raw, ci.Y + (size_t)q.j * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+  FGLS_CUDA_TRY(cudaMemcpyAsync(raw + n, ci.XL, sizeof(double) * n * wXL, cudaMemcpyDeviceToDevice, s));
+  if (product)
+    FGLS_CUDA_TRY(digit_dgemm(w.dg, s, false, false, n, 1 + wXL, n, 1.0, w.Linv, n, w.U, n, 0.0, w.WY, n));
+  else
+    FGLS_CUDA_TRY(dtrsm_llnn(s, n, 1 + wXL, w.L, n, w.WY, n));
   FGLS_CUDA_TRY(null_model_chol(s, n, wXL, w.WY, q.top, w.st, 0));
-  FGLS_CUDA_TRY(split_chol_operand(s, n, wXL, w.L, w.WY, S_BUILT, q.Mpad, c.Kpad, q.A, q.scale_built, w.Linv, w.LinvT,
+  FGLS_CUDA_TRY(split_chol_operand(s, w.dg, n, wXL, w.Linv, w.WY, S_BUILT, q.Mpad, c.Kpad, q.A, q.scale_built, w.LinvT,
                                    w.U));
   // FP64 path on the probe block (the reference's chol per-block loop)
-  FGLS_CUDA_TRY(dtrsm_llnn(s, n, PROBE, w.L, n, w.X64, n));
-  FGLS_CUDA_TRY(gram_skinny(s, n, PROBE, wXL, 1, w.X64, n, w.WY, w.GYL, w.GR64));
+  FGLS_CUDA_TRY(digit_dgemm(w.dg, s, false, false, n, PROBE, n, 1.0, w.Linv, n, w.X64, n, 0.0, w.Xw, n));
+  FGLS_CUDA_TRY(gram_skinny(s, n, PROBE, wXL, 1, w.Xw, n, w.WY, w.GYL, w.GR64));
   FGLS_CUDA_TRY(snp_solve(s, p, PROBE, 1, wXL, q.top, w.GYL, 1, PROBE, w.GR64, PROBE, q.ref, 0, w.Vp, 0, w.st, 0));
   return cudaGetLastError();
 }
@@ -637,6 +654,15 @@ int fglsgpu_batch_create(const fglsgpu_cohort* cohorts, int count, const fglsgpu
           return bail(bfail(nullptr, hs.code == FGLSGPU_ENOTSPD ? FGLSGPU_ENOTSPD : hs.code,
                             "cohort %d: a trait's M or null model is not positive definite (info %d, item %lld)",
                             c, hs.info, hs.idx));
+        }
+        int gave_up = 0;
+        if (e == cudaSuccess && w[q].dg)
+          e = cudaMemcpy(&gave_up, digit_gemm_error_word(w[q].dg), sizeof(int), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess && gave_up) {
+          cudaEventDestroy(up);
+          release();
+          return bail(bfail(nullptr, FGLSGPU_ETIMEOUT, "device wait expired in the setup of cohort %d (site %d)", c,
+                            gave_up));
         }
       }
     }

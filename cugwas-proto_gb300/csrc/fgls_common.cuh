@@ -51,11 +51,14 @@ cudaError_t dgemm_lower(cudaStream_t s, bool transA, bool transB, int N, int K, 
                         double beta, double* C, long long ldc);
 
 // In-place lower Cholesky of the n x n matrix A (only the lower triangle is
-// read or written).  If `scale_alpha` is non-null the factored matrix is
-// alpha*A + beta*I (the reference's M = h*s*Phi + (1-h)*s*I), built from
-// Src's lower triangle into A first.  Returns cudaSuccess or a launch error;
-// a non-positive pivot is reported through `st` (info = 1-based column).
-cudaError_t dpotrf_lower(cudaStream_t s, int n, double* A, long long lda, DevStatus* st);
+// read; the strict upper triangle is scratch).  dg (may be null): the trailing
+// updates run as exact digit products (fgls_digit_gemm.cuh); dinv: scratch of
+// 64 x 64.  Returns cudaSuccess or a launch error; a non-positive pivot is
+// reported through `st` (info = 1-based column).
+struct DigitGemm;
+cudaError_t dpotrf_lower(cudaStream_t s, DigitGemm* dg, int n, double* A, long long lda, double* dinv, DevStatus* st);
+// Linv = L^-1 (n x n, ld n, zero above the diagonal) of the lower triangle of L.
+cudaError_t lower_inverse(cudaStream_t s, DigitGemm* dg, int n, const double* L, long long ldl, double* Linv);
 cudaError_t build_shifted(cudaStream_t s, int n, const double* Src, long long lds, double alpha,
                           double beta, double* A, long long lda);
 

@@ -10,6 +10,7 @@
 #include <algorithm>
 
 #include "fgls_common.cuh"
+#include "fgls_digit_gemm.cuh"
 #include "fgls_kernels.cuh"
 
 namespace fgls {
@@ -140,57 +141,177 @@ cudaError_t launch_dgemm(cudaStream_t s, bool tA, bool tB, int M, int N, int K, 
 // ---------------------------------------------------------------------------
 // Diagonal-block kernels (NB = 128).
 // ---------------------------------------------------------------------------
-constexpr int NB = 128;       // block size of potrf / trsm
+constexpr int NB = 128;       // block size of trsm
 constexpr int SCB = 64;       // RHS columns per CTA in the diagonal solve
 constexpr int DT = 256;       // threads of the diagonal kernels
+constexpr int PB = 64;        // diagonal block of potrf and of the inverse
+constexpr int PO = 512;       // outer panel of potrf, base block of the inverse
 
-// Factor the kb x kb diagonal block at A (lower, in place) in shared memory.
-__global__ void __launch_bounds__(DT) potf2_kernel(int kb, double* A, long long lda, int col0,
-                                                   DevStatus* st) {
-  extern __shared__ double sm[];
-  double* Ls = sm;  // [NB][NB+1], Ls[c * (NB+1) + r] = A(r, c)
-  const int ld = NB + 1;
-  for (int e = threadIdx.x; e < kb * kb; e += DT) {
-    int r = e % kb, c = e / kb;
-    Ls[c * ld + r] = (r >= c) ? A[r + (long long)c * lda] : 0.0;
-  }
-  __syncthreads();
-  __shared__ int bad;
-  if (threadIdx.x == 0) bad = 0;
+// Inverse of the kb x kb lower triangle in Ls ([c][r], rdiag[j] = 1 / L_jj) into
+// Xs ([c][r], zero above the diagonal): thread (c, g) holds column c's rows g,
+// g + 4, ..; all threads of the CTA call it.
+__device__ __forceinline__ void tri_inverse(int kb, const double (*Ls)[PB + 1], const double* rdiag,
+                                            double (*Xs)[PB + 1]) {
+  const int c = threadIdx.x & (PB - 1), g = threadIdx.x / PB;
+  for (int r = g; r < PB; r += DT / PB) Xs[c][r] = r == c ? 1.0 : 0.0;
   __syncthreads();
   for (int j = 0; j < kb; j++) {
-    double d = Ls[j * ld + j];
-    if (!(d > 0.0)) {
-      if (threadIdx.x == 0 && !bad) {
-        bad = 1;
-        set_status(st, FGLSGPU_ENOTSPD, col0 + j + 1, -1);
+    const double x = Xs[c][j] * rdiag[j];
+    __syncthreads();
+    if (g == (j & 3)) Xs[c][j] = x;
+    if (c <= j)
+      for (int r = j + 1 + ((g - (j + 1)) & 3); r < kb; r += 4) Xs[c][r] = fma(-Ls[j][r], x, Xs[c][r]);
+    __syncthreads();
+  }
+}
+
+// Factors the kb x kb diagonal block at A (lower, in place) and writes the
+// inverse of its factor to dinv (PB x PB, row c at dinv + c*PB, zero above the
+// diagonal and past kb).  One CTA, a serial chain of 2 kb steps: 64 columns
+// take 0.04 ms; the 128-column form was bound by one SM's FP64 rate.
+__global__ void __launch_bounds__(DT) potf2_inv_kernel(int kb, double* A, long long lda, int col0,
+                                                       double* __restrict__ dinv, DevStatus* st) {
+  extern __shared__ double sm[];
+  double(*Ls)[PB + 1] = (double(*)[PB + 1])sm;              // Ls[c][r] = A(r, c)
+  double(*Xs)[PB + 1] = (double(*)[PB + 1])(sm + PB * (PB + 1));
+  __shared__ double rdiag[PB];
+  for (int e = threadIdx.x; e < PB * PB; e += DT) {
+    const int r = e & (PB - 1), c = e / PB;
+    Ls[c][r] = (r >= c && r < kb) ? A[r + (long long)c * lda] : 0.0;
+  }
+  __syncthreads();
+  const int r = threadIdx.x & (PB - 1), g = threadIdx.x / PB;
+  bool bad = false;
+  for (int j = 0; j < kb; j++) {
+    const double d = Ls[j][j];
+    if (!(d > 0.0) && threadIdx.x == 0 && !bad) {
+      bad = true;
+      set_status(st, FGLSGPU_ENOTSPD, col0 + j + 1, -1);
+    }
+    const double piv = sqrt(d), ri = 1.0 / piv;
+    const double v = r > j ? Ls[j][r] * ri : r == j ? piv : 0.0;
+    __syncthreads();
+    if (g == 0 && r >= j) Ls[j][r] = v;
+    if (threadIdx.x == 0) rdiag[j] = ri;
+    __syncthreads();
+    // columns c > j of row r (the factor's column j in shared memory)
+    for (int c = j + 1 + ((g - (j + 1)) & 3); c <= r; c += DT / PB) Ls[c][r] = fma(-v, Ls[j][c], Ls[c][r]);
+    __syncthreads();
+  }
+  tri_inverse(kb, Ls, rdiag, Xs);
+  for (int e = threadIdx.x; e < PB * PB; e += DT) {
+    const int rr = e & (PB - 1), c = e / PB;
+    if (rr >= c && rr < kb) A[rr + (long long)c * lda] = Ls[c][rr];
+    // row c' = e / PB of dinv, element q = e % PB: Linv(c', q)
+    dinv[e] = (c < kb && rr <= c) ? Xs[rr][c] : 0.0;
+  }
+}
+
+// P (rows x kb) := P L^-T for the factored block, as a product with its
+// inverse: 32 rows a CTA.  FP64-issue-bound: rows * kb^2 / 2 FMAs over all SMs.
+__global__ void __launch_bounds__(256) panel_mul_kernel(int rows, int kb, double* __restrict__ P, long long lda,
+                                                        const double* __restrict__ dinv) {
+  __shared__ double Ps[PB][32], Di[PB][PB];  // Ps[q][r], Di[c][q]
+  const int r = threadIdx.x & 31, cg = threadIdx.x >> 5;
+  const int row = blockIdx.x * 32 + r;
+  for (int e = threadIdx.x; e < PB * PB; e += 256) Di[e / PB][e & (PB - 1)] = dinv[e];
+  for (int q = cg; q < PB; q += 8) Ps[q][r] = (row < rows && q < kb) ? P[row + (long long)q * lda] : 0.0;
+  __syncthreads();
+  double acc[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) acc[i] = 0.0;
+#pragma unroll
+  for (int qb = 0; qb < 8; qb++) {
+#pragma unroll
+    for (int q8 = 0; q8 < 8; q8++) {
+      const double p = Ps[qb * 8 + q8][r];
+#pragma unroll
+      for (int i = qb; i < 8; i++) acc[i] = fma(p, Di[cg + 8 * i][qb * 8 + q8], acc[i]);  // columns cg + 8 i
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+    if (row < rows && cg + 8 * i < kb) P[row + (long long)(cg + 8 * i) * lda] = acc[i];
+}
+
+// Inverses of the PB x PB diagonal blocks of L, one CTA each, into Linv.
+__global__ void __launch_bounds__(DT) tri_inv_kernel(int n, const double* __restrict__ L, long long ldl,
+                                                     double* __restrict__ Linv) {
+  extern __shared__ double sm[];
+  double(*Ls)[PB + 1] = (double(*)[PB + 1])sm;
+  double(*Xs)[PB + 1] = (double(*)[PB + 1])(sm + PB * (PB + 1));
+  __shared__ double rdiag[PB];
+  const int o = blockIdx.x * PB, kb = min(PB, n - o);
+  for (int e = threadIdx.x; e < PB * PB; e += DT) {
+    const int r = e & (PB - 1), c = e / PB;
+    Ls[c][r] = (r >= c && r < kb) ? L[(o + r) + (long long)(o + c) * ldl] : 0.0;
+  }
+  __syncthreads();
+  if (threadIdx.x < kb) rdiag[threadIdx.x] = 1.0 / Ls[threadIdx.x][threadIdx.x];
+  __syncthreads();
+  tri_inverse(kb, Ls, rdiag, Xs);
+  for (int e = threadIdx.x; e < PB * PB; e += DT) {
+    const int r = e & (PB - 1), c = e / PB;
+    if (r >= c && r < kb && c < kb) Linv[(o + r) + (long long)(o + c) * n] = Xs[c][r];
+  }
+}
+
+// Merge of neighbouring diagonal blocks [o, o + w) and [o + w, o + w + w2) of
+// the inverse, o = 2 w blockIdx.z: with L21 the block of L between them,
+//   FIRST:  T^T = A^-T L21^T   (into the zero block above the diagonal)
+//   second: X21 = -D^-1 T
+// 32 x 32 outputs a CTA; the zero halves of A^-1 and D^-1 are skipped.
+template <bool FIRST>
+__global__ void __launch_bounds__(256) tri_merge_kernel(int n, int w, const double* __restrict__ L, long long ldl,
+                                                        double* Linv) {
+  __shared__ double As[32][33], Bs[32][33];
+  const int o = 2 * w * blockIdx.z, w2 = min(w, n - o - w);
+  const int M = FIRST ? w : w2, N = FIRST ? w2 : w;
+  const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+  if (w2 <= 0 || i0 >= M || j0 >= N) return;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int kbeg = FIRST ? i0 : 0, kend = FIRST ? w : min(w2, i0 + 32);
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int k0 = kbeg; k0 < kend; k0 += 32) {
+    __syncthreads();
+    for (int q = ty; q < 32; q += 8) {
+      if (FIRST) {
+        // As[k][i] = A^-1(k, i): memory runs along k; Bs[k][j] = L21(j, k)
+        As[tx][q] = (k0 + tx < w && i0 + q < w) ? Linv[(o + k0 + tx) + (long long)(o + i0 + q) * n] : 0.0;
+        Bs[q][tx] = (j0 + tx < w2 && k0 + q < w) ? L[(o + w + j0 + tx) + (long long)(o + k0 + q) * ldl] : 0.0;
+      } else {
+        As[q][tx] = (i0 + tx < w2 && k0 + q < w2) ? Linv[(o + w + i0 + tx) + (long long)(o + w + k0 + q) * n] : 0.0;
+        Bs[q][tx] = (j0 + tx < w && k0 + q < w2) ? Linv[(o + j0 + tx) + (long long)(o + w + k0 + q) * n] : 0.0;
       }
     }
-    double piv = sqrt(d);
     __syncthreads();
-    // scale column j below the diagonal
-    for (int r = j + 1 + threadIdx.x; r < kb; r += DT) Ls[j * ld + r] /= piv;
-    __syncthreads();
-    if (threadIdx.x == 0) Ls[j * ld + j] = piv;
-    // rank-1 update of the trailing lower triangle
-    const int rem = kb - j - 1;
-    for (int e = threadIdx.x; e < rem * rem; e += DT) {
-      int r = j + 1 + e % rem, c = j + 1 + e / rem;
-      if (r >= c) Ls[c * ld + r] -= Ls[j * ld + r] * Ls[j * ld + c];
+#pragma unroll 8
+    for (int k = 0; k < 32; k++) {
+      const double a = As[k][tx];
+#pragma unroll
+      for (int u = 0; u < 4; u++) acc[u] = fma(a, Bs[k][ty * 4 + u], acc[u]);
     }
-    __syncthreads();
   }
-  for (int e = threadIdx.x; e < kb * kb; e += DT) {
-    int r = e % kb, c = e / kb;
-    if (r >= c) A[r + (long long)c * lda] = Ls[c * ld + r];
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    const int i = i0 + tx, j = j0 + ty * 4 + u;
+    if (i >= M || j >= N) continue;
+    if (FIRST) Linv[(o + i) + (long long)(o + w + j) * n] = acc[u];
+    else Linv[(o + w + i) + (long long)(o + j) * n] = -acc[u];
   }
+}
+
+// Zeros above the diagonal of every merged block, [o, o + w) x [o + w, ..).
+__global__ void __launch_bounds__(256) tri_clear_kernel(int n, int w, double* __restrict__ Linv) {
+  const int o = 2 * w * blockIdx.z, w2 = min(w, n - o - w);
+  for (int e = blockIdx.x * 256 + threadIdx.x; e < w * w2; e += gridDim.x * 256)
+    Linv[(o + e % w) + (long long)(o + w + e / w) * n] = 0.0;
 }
 
 // Forward substitution with the kb x kb lower block L on a set of right-hand
 // sides.  RHS element (i, c) lives at X[i*si + c*sc]; i < kb runs over the
 // block's rows, c < nrhs over the right-hand sides.  Used for
 //   TRSM:  X := L^-1 X        (si = 1, sc = ldx)
-//   POTRF: P := P L^-T        (rows of the panel are the RHS: si = lda, sc = 1)
 template <int SCB>
 __global__ void __launch_bounds__(DT) diag_solve_kernel(int kb, const double* L, long long ldl,
                                                         double* X, long long si, long long sc,
@@ -243,7 +364,7 @@ __global__ void __launch_bounds__(DT) diag_solve_kernel(int kb, const double* L,
   }
 }
 
-constexpr size_t POTF2_SMEM = sizeof(double) * NB * (NB + 1);
+constexpr size_t TRI_SMEM = sizeof(double) * 2 * PB * (PB + 1);  // a diagonal block and its inverse
 constexpr size_t DSOLVE_SMEM = sizeof(double) * (NB + SCB) * (NB + 1);
 constexpr int SCB_NARROW = 16;  // RHS per CTA when few right-hand sides (e.g. the 512-wide L^-1 panels)
 constexpr size_t DSOLVE_SMEM_NARROW = sizeof(double) * (NB + SCB_NARROW) * (NB + 1);
@@ -275,7 +396,8 @@ __global__ void build_shifted_kernel(int n, const double* __restrict__ S, long l
 bool g_attr_done = false;
 cudaError_t ensure_attrs() {
   if (g_attr_done) return cudaSuccess;
-  FGLS_CUDA_TRY(cudaFuncSetAttribute(potf2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)POTF2_SMEM));
+  FGLS_CUDA_TRY(cudaFuncSetAttribute(potf2_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRI_SMEM));
+  FGLS_CUDA_TRY(cudaFuncSetAttribute(tri_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRI_SMEM));
   FGLS_CUDA_TRY(cudaFuncSetAttribute(diag_solve_kernel<SCB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)DSOLVE_SMEM));
   FGLS_CUDA_TRY(cudaFuncSetAttribute(diag_solve_kernel<SCB_NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -344,26 +466,98 @@ cudaError_t build_shifted(cudaStream_t s, int n, const double* Src, long long ld
   return cudaGetLastError();
 }
 
-cudaError_t dpotrf_lower(cudaStream_t s, int n, double* A, long long lda, DevStatus* st) {
+// Blocked Cholesky: 64-column blocks (factor and its inverse in one CTA, the
+// panel below as a product with the inverse), updates within 512-column panels
+// after each block and of the whole trailing triangle after each panel, so that
+// the big update has K = 512.  With digits, n = 10000 takes ~30 ms against
+// 360 ms when every update ran on the FP64 kernel.
+cudaError_t dpotrf_lower(cudaStream_t s, DigitGemm* dg, int n, double* A, long long lda, double* dinv, DevStatus* st) {
   FGLS_CUDA_TRY(ensure_attrs());
-  for (int k = 0; k < n; k += NB) {
-    const int kb = std::min(NB, n - k);
-    double* Akk = A + k + (long long)k * lda;
-    potf2_kernel<<<1, DT, POTF2_SMEM, s>>>(kb, Akk, lda, k, st);
-    note_launch();
-    FGLS_CUDA_TRY(cudaGetLastError());
-    const int rest = n - k - kb;
-    if (rest > 0) {
+  for (int k0 = 0; k0 < n; k0 += PO) {
+    const int kw = std::min(PO, n - k0);
+    for (int k = k0; k < k0 + kw; k += PB) {
+      const int kb = std::min(PB, k0 + kw - k);
+      double* Akk = A + k + (long long)k * lda;
+      potf2_inv_kernel<<<1, DT, TRI_SMEM, s>>>(kb, Akk, lda, k, dinv, st);
+      note_launch();
+      const int rest = n - k - kb;
+      if (rest <= 0) break;
       double* P = A + (k + kb) + (long long)k * lda;  // rest x kb panel
-      // P := P L_kk^-T  (each panel row is a right-hand side)
-      launch_diag_solve(s, kb, Akk, lda, P, lda, 1, rest);
+      panel_mul_kernel<<<ceil_div(rest, 32), 256, 0, s>>>(rest, kb, P, lda, dinv);
       note_launch();
       FGLS_CUDA_TRY(cudaGetLastError());
-      double* T = A + (k + kb) + (long long)(k + kb) * lda;
-      FGLS_CUDA_TRY(dgemm_lower(s, false, true, rest, kb, -1.0, P, lda, P, lda, 1.0, T, lda));
+      const int in = k0 + kw - k - kb;  // columns of the panel still to factor
+      if (in > 0) {
+        double* T = A + (k + kb) + (long long)(k + kb) * lda;
+        DigitMat a;
+        if (dg && digit_gemm_pays(rest, in, kb)) a = digit_gemm_operand(dg, 0, rest, kb);
+        if (a.d) {
+          FGLS_CUDA_TRY(digit_cut(s, a, P, lda, false));
+          DigitMat b = a;  // the panel's first rows
+          b.rows = in;
+          FGLS_CUDA_TRY(digit_mul(dg, s, a, b, -1.0, 1.0, T, lda));
+        } else {
+          FGLS_CUDA_TRY(dgemm(s, false, true, rest, in, kb, -1.0, P, lda, P, lda, 1.0, T, lda));
+        }
+      }
+    }
+    const int rest = n - k0 - kw;
+    if (rest <= 0) break;
+    double* P = A + (k0 + kw) + (long long)k0 * lda;  // rest x kw
+    double* T = A + (k0 + kw) + (long long)(k0 + kw) * lda;
+    DigitMat a;
+    if (dg && digit_gemm_pays(rest, rest, kw)) a = digit_gemm_operand(dg, 0, rest, kw);
+    if (a.d) {
+      DigitMulOpts o;
+      o.c_lower = true;
+      FGLS_CUDA_TRY(digit_cut(s, a, P, lda, false));
+      FGLS_CUDA_TRY(digit_mul(dg, s, a, a, -1.0, 1.0, T, lda, o));
+    } else {
+      FGLS_CUDA_TRY(dgemm_lower(s, false, true, rest, kw, -1.0, P, lda, P, lda, 1.0, T, lda));
     }
   }
   return cudaSuccess;
+}
+
+namespace {
+// The block [off, off + size) of the inverse, its PO-blocks done: halves first,
+// then X21 = -D^-1 (L21 A^-1), with T^T = A^-T L21^T in the zero block above
+// the diagonal meanwhile.
+cudaError_t inverse_range(cudaStream_t s, DigitGemm* dg, int n, const double* L, long long ldl, double* Linv, int off,
+                          int size) {
+  if (size <= PO) return cudaSuccess;
+  int s1 = PO;
+  while (2 * s1 < size) s1 *= 2;
+  const int s2 = size - s1, o2 = off + s1;
+  FGLS_CUDA_TRY(inverse_range(s, dg, n, L, ldl, Linv, off, s1));
+  FGLS_CUDA_TRY(inverse_range(s, dg, n, L, ldl, Linv, o2, s2));
+  double* TT = Linv + off + (long long)o2 * n;
+  FGLS_CUDA_TRY(digit_dgemm(dg, s, true, true, s1, s2, s1, 1.0, Linv + off + (long long)off * n, n,
+                            L + o2 + (long long)off * ldl, ldl, 0.0, TT, n));
+  DigitMulOpts lower;
+  lower.a_lower = true;
+  FGLS_CUDA_TRY(digit_dgemm(dg, s, false, true, s2, s1, s2, -1.0, Linv + o2 + (long long)o2 * n, n, TT, n, 0.0,
+                            Linv + o2 + (long long)off * n, n, lower));
+  return cudaMemset2DAsync(TT, sizeof(double) * n, 0, sizeof(double) * s1, s2, s);
+}
+}  // namespace
+
+// 64 x 64 blocks by substitution, all at once; neighbours merged to 512 by one
+// launch a level; beyond that two products a merge, through digits.
+cudaError_t lower_inverse(cudaStream_t s, DigitGemm* dg, int n, const double* L, long long ldl, double* Linv) {
+  FGLS_CUDA_TRY(ensure_attrs());
+  FGLS_CUDA_TRY(cudaMemsetAsync(Linv, 0, sizeof(double) * (size_t)n * n, s));
+  tri_inv_kernel<<<ceil_div(n, PB), DT, TRI_SMEM, s>>>(n, L, ldl, Linv);
+  note_launch();
+  for (int w = PB; w < PO && w < n; w *= 2) {
+    const dim3 grid(w / 32, w / 32, ceil_div(n - w, 2 * w));
+    tri_merge_kernel<true><<<grid, 256, 0, s>>>(n, w, L, ldl, Linv);
+    tri_merge_kernel<false><<<grid, 256, 0, s>>>(n, w, L, ldl, Linv);
+    tri_clear_kernel<<<dim3(std::max(1, w * w / 2048), 1, grid.z), 256, 0, s>>>(n, w, Linv);
+    note_launch(3);
+  }
+  FGLS_CUDA_TRY(cudaGetLastError());
+  return inverse_range(s, dg, n, L, ldl, Linv, 0, n);
 }
 
 cudaError_t dtrsm_llnn(cudaStream_t s, int n, int nrhs, const double* L, long long ldl, double* X,

@@ -8,8 +8,8 @@
 // |x| 2^-ex < 1/2, rounded to a multiple of 2^-60 and written in base 32 with
 // signed digits, x 2^-ex = sum_{s=1..12} d_s 32^-s, |d_s| <= 16: exact in E4M3.
 // The cut works on the bit pattern in integer instructions: the 60-bit fixed
-// point number plus sum_s 16 * 32^(12-s) has the digits d_s + 16 as its 5-bit
-// fields.
+// point magnitude plus sum_s 16 * 32^(12-s) has the digits d_s + 16 as its
+// 5-bit fields.
 //
 // Products.  A product of digits s and t has weight 32^-(s+t); level L is the
 // sum of all pairs with s + t = L.  Levels 2 .. 13 are kept (78 of the 144
@@ -510,8 +510,9 @@ __global__ void __launch_bounds__(256) digit_split_sum_kernel(int M, int N, int 
 // ------------------------------------------------------------------- digits
 constexpr uint64_t DIGIT_BIAS = 16ull * (((1ull << 60) - 1) / 31);  // 16 in every 5-bit field
 
-// x 2^(60 - ex) rounded to an integer (|x| < 2^(ex-1)); exact zero stays zero.
-__device__ __forceinline__ long long to_fixed(double x, int ex) {
+
+// |x| 2^(60 - ex) rounded to an integer (|x| < 2^(ex-1)); sign: x's sign bit.
+__device__ __forceinline__ unsigned long long to_fixed(double x, int ex, uint32_t& sign) {
   const long long b = __double_as_longlong(x);
   int e = (int)((b >> 52) & 0x7ff);
   unsigned long long m = (unsigned long long)b & 0xfffffffffffffull;
@@ -522,15 +523,20 @@ __device__ __forceinline__ long long to_fixed(double x, int ex) {
   if (sh >= 0) f = m << min(sh, 11);
   else if (sh > -55) f = (m + (1ull << (-sh - 1))) >> -sh;
   else f = 0;
-  return b < 0 ? -(long long)f : (long long)f;
+  sign = (uint32_t)(b >> 32) & 0x80000000u;
+  return f;
 }
-// the four digits of weight 32^-(s+1) of four biased numbers, as E4M3 bytes
-__device__ __forceinline__ uint32_t digit_word(const uint64_t (&u)[4], int s) {
+// The four digits of weight 32^-(s+1) of four biased magnitudes, signs applied,
+// as E4M3 bytes.  Signs go on the digits because the digits of a magnitude lie
+// in [-16, 15], -1/2 on average: cut from signed numbers, the low digits would
+// share that mean whatever the signs, and the dropped digit pairs would add up
+// over K instead of averaging out.
+__device__ __forceinline__ uint32_t digit_word(const uint64_t (&u)[4], const uint32_t (&sg)[4], int s) {
   float f[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     const uint32_t d = s == 0 ? (uint32_t)(u[k] >> 55) : (uint32_t)(u[k] >> (55 - 5 * s)) & 31u;
-    f[k] = __fsub_rn(__uint_as_float(0x4B000000u | d), 8388624.0f);
+    f[k] = __uint_as_float(__float_as_uint(__fsub_rn(__uint_as_float(0x4B000000u | d), 8388624.0f)) ^ sg[k]);
   }
   const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(f[0], f[1]), __NV_SATFINITE, __NV_E4M3);
   const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(f[2], f[3]), __NV_SATFINITE, __NV_E4M3);
@@ -576,15 +582,16 @@ __global__ void __launch_bounds__(256) cut_contig_kernel(const double* __restric
   unsigned long long bits = 0;
   for (int g = l; g < Kpad / 4; g += TPR) {
     uint64_t u[4];
+    uint32_t sg[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       const int k = 4 * g + j;
-      const long long f = k < K ? to_fixed(value(k), es) : 0;
-      bits |= (unsigned long long)(f < 0 ? -f : f);
-      u[j] = (uint64_t)f + DIGIT_BIAS;
+      const unsigned long long f = to_fixed(k < K ? value(k) : 0.0, es, sg[j]);
+      bits |= f;
+      u[j] = f + DIGIT_BIAS;
     }
 #pragma unroll
-    for (int s = 0; s < ND; s++) *(uint32_t*)(D + ((size_t)s * rows + r) * Kpad + 4 * g) = digit_word(u, s);
+    for (int s = 0; s < ND; s++) *(uint32_t*)(D + ((size_t)s * rows + r) * Kpad + 4 * g) = digit_word(u, sg, s);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) bits |= __shfl_xor_sync(0xffffffffu, bits, o);
@@ -623,15 +630,16 @@ __global__ void __launch_bounds__(256) cut_strided_kernel(const double* __restri
     for (int h = 0; h < 2; h++) {  // two groups of four elements a thread
       const int g = wp * 2 + h;
       uint64_t u[4];
+      uint32_t sg[4];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int k = k0 + 4 * g + j;
-        const long long f = (r < rows && k < K) ? to_fixed(x[(long long)k * ld], es) : 0;
-        bits |= (unsigned long long)(f < 0 ? -f : f);
-        u[j] = (uint64_t)f + DIGIT_BIAS;
+        const unsigned long long f = to_fixed((r < rows && k < K) ? x[(long long)k * ld] : 0.0, es, sg[j]);
+        bits |= f;
+        u[j] = f + DIGIT_BIAS;
       }
 #pragma unroll
-      for (int s = 0; s < ND; s++) t[s][lane][g] = digit_word(u, s);
+      for (int s = 0; s < ND; s++) t[s][lane][g] = digit_word(u, sg, s);
     }
     __syncthreads();
     // 12 planes x 32 rows of 16 words: two rows a warp and step
@@ -675,7 +683,7 @@ cudaError_t digit_map(CUtensorMap* m, const DigitMat& d) {
   EncodeTiledFn enc = encoder();
   if (!enc) return cudaErrorNotSupported;
   cuuint64_t dims[3] = {(cuuint64_t)d.Kpad, (cuuint64_t)d.rows, (cuuint64_t)ND};
-  cuuint64_t strides[2] = {(cuuint64_t)d.Kpad, (cuuint64_t)d.Kpad * (cuuint64_t)d.rows};
+  cuuint64_t strides[2] = {(cuuint64_t)d.Kpad, (cuuint64_t)d.Kpad * (cuuint64_t)d.prow};
   cuuint32_t box[3] = {ROW, 128, 1};
   cuuint32_t es[3] = {1, 1, 1};
   const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, d.d, dims, strides, box, es,
@@ -725,7 +733,7 @@ size_t digit_mat_bytes(int rows, int K) {
 
 DigitMat digit_mat_at(void* mem, int rows, int K) {
   DigitMat m;
-  m.rows = rows;
+  m.rows = m.prow = rows;
   m.K = K;
   m.Kpad = (K + ROW - 1) / ROW * ROW;
   m.d = (uint8_t*)mem;
@@ -736,7 +744,7 @@ DigitMat digit_mat_at(void* mem, int rows, int K) {
 
 namespace {
 cudaError_t cut(cudaStream_t s, const DigitMat& m, const double* X, long long ld, bool kcontig, int w) {
-  if (m.rows <= 0 || m.K <= 0) return cudaErrorInvalidValue;
+  if (m.rows <= 0 || m.K <= 0 || m.prow != m.rows) return cudaErrorInvalidValue;
   FGLS_CUDA_TRY(cudaMemsetAsync(m.nd, 0, sizeof(int) * ((m.rows + 255) / 256), s));
   if (!kcontig)
     cut_strided_kernel<<<ceil_div(m.rows, 32), 256, 0, s>>>(X, ld, m.rows, m.K, m.Kpad, m.d, m.ex, m.nd);
@@ -880,6 +888,11 @@ bool reserve(DigitGemm* g, int q, size_t bytes) {
 }
 }  // namespace
 
+DigitMat digit_gemm_operand(DigitGemm* g, int q, int rows, int K) {
+  if (!reserve(g, q, digit_mat_bytes(rows, K))) return DigitMat();
+  return digit_mat_at(g->op[q], rows, K);
+}
+
 bool digit_gemm_reserve(DigitGemm* g, int rows, int K) {
   const size_t b = digit_mat_bytes(rows, K);
   return reserve(g, 0, b) && reserve(g, 1, b);
@@ -896,12 +909,12 @@ void digit_gemm_trim(DigitGemm* g) {
 
 cudaError_t digit_dgemm(DigitGemm* g, cudaStream_t s, bool tA, bool tB, int M, int N, int K, double alpha,
                         const double* A, long long lda, const double* B, long long ldb, double beta, double* C,
-                        long long ldc) {
+                        long long ldc, const DigitMulOpts& o) {
   if (g && digit_gemm_pays(M, N, K) && reserve(g, 0, digit_mat_bytes(M, K)) && reserve(g, 1, digit_mat_bytes(N, K))) {
     const DigitMat a = digit_mat_at(g->op[0], M, K), b = digit_mat_at(g->op[1], N, K);
     FGLS_CUDA_TRY(digit_cut(s, a, A, lda, tA));
     FGLS_CUDA_TRY(digit_cut(s, b, B, ldb, !tB));
-    return digit_mul(g, s, a, b, alpha, beta, C, ldc);
+    return digit_mul(g, s, a, b, alpha, beta, C, ldc, o);
   }
   return dgemm(s, tA, tB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
 }

@@ -19,6 +19,7 @@ struct DigitMat {
   int* ex = nullptr;
   int* nd = nullptr;
   int rows = 0, K = 0, Kpad = 0;
+  int prow = 0;  // rows between digit planes (rows, more in a view of the first rows)
 };
 size_t digit_mat_bytes(int rows, int K);
 // lays out a matrix of `rows` x K in `mem` (digit_mat_bytes, 256-byte aligned)
@@ -50,7 +51,10 @@ cudaError_t digit_mul(DigitGemm* g, cudaStream_t s, const DigitMat& A, const Dig
 // live in g (grown on demand; without the memory for it the FP64 kernel runs).
 cudaError_t digit_dgemm(DigitGemm* g, cudaStream_t s, bool tA, bool tB, int M, int N, int K, double alpha,
                         const double* A, long long lda, const double* B, long long ldb, double beta, double* C,
-                        long long ldc);
+                        long long ldc, const DigitMulOpts& o = DigitMulOpts());
+// scratch operands of g (0, 1) laid out for rows x K; d == nullptr when the
+// device has not the memory
+DigitMat digit_gemm_operand(DigitGemm* g, int q, int rows, int K);
 // room for operands of up to `rows` x K each (so that digit_dgemm allocates
 // nothing); false when the device has not the memory.  digit_gemm_trim gives
 // the operands' room back.

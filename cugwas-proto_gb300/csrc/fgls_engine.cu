@@ -78,6 +78,11 @@ struct fglsgpu_engine {
   DigitGemm* dg = nullptr;
   bool dg_off = false;  // no CTA pairs or no memory for the digits: FP64 kernels throughout
   DigitMat zdig, ayldig, ddig;  // eigen: Z^T, AYL^T, dinv^T rows
+  // chol: the selected trait's L^-1 (null: no memory for it, the blocks then
+  // run a blocked TRSM) and its rows' digits (valid when linv_cut), 64 x 64 scratch
+  double *dLinv = nullptr, *ddiag = nullptr;
+  DigitMat ldig;
+  bool linv_cut = false;
   void *zmem = nullptr, *wmem = nullptr, *blkmem = nullptr;
   size_t blk_bytes = 0;
   bool z_cut = false, w_cut = false;
@@ -85,6 +90,8 @@ struct fglsgpu_engine {
 };
 
 namespace {
+
+constexpr int TUNE_SNPS = 256;  // SNPs of the autotuner's probe block
 
 thread_local std::string tl_err;
 
@@ -166,7 +173,7 @@ void free_all(fglsgpu_engine* e) {
                   e->dQ,   e->dGYL, e->dGR,  e->dB[0], e->dB[1], e->dV[0], e->dV[1], e->dU8, e->dst,
                   e->aWc, e->aAYLc, e->aAYLs, e->atopc, e->atops, e->areml, e->aGYLc, e->aGYLs, e->aGRc,
                   e->aGRs, e->acontrib, e->ag, e->agR, e->aacc, e->aU, e->aV2, e->dSE[0], e->dSE[1], e->dP[0],
-                  e->dP[1], e->dXw, e->zmem, e->wmem, e->blkmem};
+                  e->dP[1], e->dXw, e->zmem, e->wmem, e->blkmem, e->dLinv, e->ddiag};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (e->hst) cudaFreeHost(e->hst);
@@ -214,11 +221,13 @@ struct Prof {
     ev = take(e, cls);
     cudaEventRecord(ev.a, s);
   }
-  ~Prof() {
+  void close() {
     if (!on) return;
+    on = false;
     cudaEventRecord(ev.b, s);
     e->pev_live.push_back(ev);
   }
+  ~Prof() { close(); }
 };
 
 // Stage hook of the split path: brackets each stage on the stream it runs on.
@@ -263,7 +272,42 @@ void drop_digits(fglsgpu_engine* e) {
     *q = nullptr;
   }
   e->blk_bytes = 0;
-  e->z_cut = e->w_cut = false;
+  e->z_cut = e->w_cut = e->linv_cut = false;
+}
+
+// The workspace of the digit products; null when the device cannot run them.
+DigitGemm* digit_work(fglsgpu_engine* e) {
+  if (!e->dg && !e->dg_off && digit_gemm_create(&e->dg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    e->dg_off = true;
+  }
+  return e->dg;
+}
+
+// Digits of the rows of L^-1 (once per select_trait) and room for the digits
+// of `cols` genotype columns; *use as in eigen_digits.
+int chol_digits(fglsgpu_engine* e, long long cols, bool* use) {
+  *use = false;
+  const fglsgpu_config& c = e->cfg;
+  const int n = c.n;
+  if (!e->dLinv || !digit_gemm_pays(n, cols, n) || !digit_work(e)) return FGLSGPU_OK;
+  const long long most = e->probing ? cols : std::max<long long>(cols, (long long)c.x_b * c.wXR);
+  size_t none = 0;
+  if (!((e->zmem || grow(&e->zmem, &none, digit_mat_bytes(n, n))) &&
+        grow(&e->blkmem, &e->blk_bytes, digit_mat_bytes((int)most, n)))) {
+    drop_digits(e);
+    e->dg_off = true;
+    digit_gemm_destroy(e->dg);
+    e->dg = nullptr;
+    return FGLSGPU_OK;
+  }
+  if (!e->linv_cut) {
+    e->ldig = digit_mat_at(e->zmem, n, n);
+    ENG_TRY(e, digit_cut(e->comp, e->ldig, e->dLinv, n, false), "digits of L^-1");
+    e->linv_cut = true;
+  }
+  *use = true;
+  return FGLSGPU_OK;
 }
 
 // Digits of the eigen variant's resident operands (Z once per problem, the
@@ -280,7 +324,7 @@ int eigen_digits(fglsgpu_engine* e, long long cols, bool* use) {
   if (e->dg_off || c.variant != FGLSGPU_VARIANT_EIGEN || !digit_gemm_pays(n, cols, n)) return FGLSGPU_OK;
   const long long most = (e->probing ? cols : std::max<long long>(cols, (long long)c.x_b * c.wXR)) * c.wXR;
   size_t none = 0;
-  bool ok = e->dg || digit_gemm_create(&e->dg) == cudaSuccess;
+  bool ok = digit_work(e) != nullptr;
   if (ok && !e->zmem) ok = grow(&e->zmem, &none, digit_mat_bytes(n, n));
   none = 0;
   const size_t wy = (digit_mat_bytes(nq, n) + 255) & ~(size_t)255;
@@ -350,12 +394,28 @@ int compute_block(fglsgpu_engine* e, const void* dX, int fmt, int x, double* dB,
     dXin = e->dXw;
   }
   if (c.variant == FGLSGPU_VARIANT_CHOL) {
-    {
-      Prof pr(e, FGLSGPU_PROF_TRSM, s);
+    bool digits = false;
+    const int rc = chol_digits(e, cols, &digits);
+    if (rc) return rc;
+    Prof pt(e, FGLSGPU_PROF_TRSM, s);
+    if (digits) {
+      // x~ = L^-1 x with the explicit inverse: 10000 x 4096 real dosages take
+      // 9 ms (hard calls 2) where the blocked TRSM takes 361, with the same
+      // error against exact arithmetic
+      const DigitMat xd = digit_mat_at(e->blkmem, (int)cols, n);
+      DigitMulOpts lower;
+      lower.a_lower = true;
+      ENG_TRY(e, digit_cut(s, xd, dXin, n, true), "digits of XR");
+      ENG_TRY(e, digit_mul(e->dg, s, e->ldig, xd, 1.0, 0.0, e->dWork, n, lower), "L^-1 XR");
+    } else if (e->dLinv && !e->dg_off) {
+      // small blocks: one product instead of a chain of 128-column solves
+      ENG_TRY(e, dgemm(s, false, false, n, (int)cols, n, 1.0, e->dLinv, n, dXin, n, 0.0, e->dWork, n), "L^-1 XR");
+    } else {
       ENG_TRY(e, cudaMemcpyAsync(e->dWork, dXin, sizeof(double) * n * cols, cudaMemcpyDeviceToDevice, s),
               "block copy");
       ENG_TRY(e, dtrsm_llnn(s, n, (int)cols, e->dL, n, e->dWork, n), "TRSM");
     }
+    pt.close();
     Prof pr(e, FGLSGPU_PROF_GRAM, s);
     ENG_TRY(e, gram_skinny(s, n, x, wXL, wXR, e->dWork, n, e->dWY, e->dGYL, e->dGR), "gram");
   } else {
@@ -430,7 +490,7 @@ __global__ void probe_genotypes_kernel(int n, int x, double* __restrict__ out) {
 // chosen the same way from 8..11.  Called after every build of the split
 // operands (they depend on the trait's weights or factor).
 constexpr double TUNE_TOL = 1e-10;
-constexpr int TUNE_SNPS = 256, TUNE_MIN_SLICES = 6, TUNE_MIN_QDIGITS = 8;
+constexpr int TUNE_MIN_SLICES = 6, TUNE_MIN_QDIGITS = 8;
 
 int tune_slices(fglsgpu_engine* e) {
   fglsgpu_config& c = e->cfg;
@@ -616,6 +676,7 @@ int fglsgpu_create(const fglsgpu_config* cfg, fglsgpu_engine** out) {
     chk(dalloc(&e->dL, n * n));
     chk(dalloc(&e->dWY, n * (1 + wXL)));
     chk(dalloc(&e->dWork, n * xb * wXR));
+    chk(dalloc(&e->ddiag, 64 * 64));
   } else {
     chk(dalloc(&e->dL, n * n));  // eigensolver scratch
     chk(dalloc(&e->dZ, n * n));
@@ -676,11 +737,7 @@ int fglsgpu_set_problem(fglsgpu_engine* e, const double* Phi, const double* XL, 
   e->problem_set = false;
   if (c.variant == FGLSGPU_VARIANT_EIGEN) {
     int qfail = 0;
-    if (!e->dg && !e->dg_off && digit_gemm_create(&e->dg) != cudaSuccess) {
-      (void)cudaGetLastError();
-      e->dg_off = true;
-    }
-    ENG_TRY(e, dsyev_device(s, e->dg, c.n, e->dPhi, n, e->dL, e->dZ, e->dW, e->deigwork, &qfail, nullptr),
+    ENG_TRY(e, dsyev_device(s, digit_work(e), c.n, e->dPhi, n, e->dL, e->dZ, e->dW, e->deigwork, &qfail, nullptr),
             "eigendecomposition");
     if (qfail) return fail(e, FGLSGPU_ENOCONV, "dsyevr failed (info: 1): QL iteration did not converge");
     ENG_TRY(e, digit_dgemm(e->dg, s, true, false, c.n, c.wXL, c.n, 1.0, e->dZ, n, e->dXL, n, 0.0, e->dZtXL, n),
@@ -726,21 +783,45 @@ int fglsgpu_select_trait(fglsgpu_engine* e, int j) {
   const double alpha = e->hh[j] * e->hs[j];          // src/fgls_chol.c:253
   const double beta = (1.0 - e->hh[j]) * e->hs[j];   // src/fgls_chol.c:254
   ENG_TRY(e, build_shifted(s, c.n, e->dPhi, n, alpha, beta, e->dL, n), "build M");
-  ENG_TRY(e, dpotrf_lower(s, c.n, e->dL, n, e->dst), "potrf");
+  DigitGemm* dg = digit_work(e);
+  ENG_TRY(e, dpotrf_lower(s, dg, c.n, e->dL, n, e->ddiag, e->dst), "potrf");
   rc = check_status(e, "potrf(M)");
   if (rc) return rc;
   ENG_TRY(e, cudaMemcpyAsync(e->dWY, e->dY + (long long)j * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, s),
           "copy y");
   ENG_TRY(e, cudaMemcpyAsync(e->dWY + n, e->dXL, sizeof(double) * n * c.wXL, cudaMemcpyDeviceToDevice, s),
           "copy XL");
-  ENG_TRY(e, dtrsm_llnn(s, c.n, 1 + c.wXL, e->dL, n, e->dWY, n), "whiten y, XL");
+  // L^-1: the split path's operand, and what the FP64 path multiplies by
+  // (n^2 doubles: without the memory the FP64 path solves with L instead)
+  if (!e->dLinv && dalloc(&e->dLinv, (size_t)n * n) != cudaSuccess) {
+    (void)cudaGetLastError();
+    e->dLinv = nullptr;
+    if (split(e)) return fail(e, FGLSGPU_ENOMEM, "no memory for the inverse of the factor");
+  }
+  e->linv_cut = false;
+  if (e->dLinv) ENG_TRY(e, lower_inverse(s, dg, c.n, e->dL, n, e->dLinv), "inverse of the factor");
+  bool digits = false;
+  rc = chol_digits(e, split(e) ? std::min((long long)TUNE_SNPS, (long long)c.x_b) : (long long)c.x_b * c.wXR, &digits);
+  if (rc) return rc;
+  if (digits && c.n >= 1024) {
+    // whitening as a product: four columns cost one tile column, the solve a
+    // chain of 128-column steps (24 ms at n = 10000)
+    DigitMat w = digit_gemm_operand(e->dg, 0, 1 + c.wXL, c.n);
+    if (!w.d) return fail(e, FGLSGPU_ENOMEM, "no memory for the whitening");
+    DigitMulOpts lower;
+    lower.a_lower = true;
+    ENG_TRY(e, digit_cut(s, w, e->dWY, n, true), "whiten y, XL");
+    ENG_TRY(e, digit_mul(e->dg, s, e->ldig, w, 1.0, 0.0, e->dWY, n, lower), "whiten y, XL");
+  } else {
+    ENG_TRY(e, dtrsm_llnn(s, c.n, 1 + c.wXL, e->dL, n, e->dWY, n), "whiten y, XL");
+  }
   ENG_TRY(e, null_model_chol(s, c.n, c.wXL, e->dWY, e->dtop, e->dst, 0), "null model");
   rc = check_status(e, "null model");
   if (rc) return rc;
   if (split(e)) {
     if (!e->oz) ENG_TRY(e, ozaki_create(&e->oz, c.n, 1, c.wXL, c.wXR, c.x_b, c.slices, /*eigen=*/0), "split plan");
     ozaki_set_wait_limit(e->oz, e->wait_ns);
-    ENG_TRY(e, ozaki_set_chol(e->oz, s, e->dL, e->dWY), "split operands");
+    ENG_TRY(e, ozaki_set_chol(e->oz, s, e->dg, e->dLinv, e->dWY), "split operands");
     ENG_TRY(e, cudaStreamSynchronize(s), "split operands");
     e->trait_sel = j;
     rc = tune_slices(e);

@@ -1827,13 +1827,6 @@ __global__ void __launch_bounds__(256) genotypes_packed_f8_kernel(int K, const u
   }
 }
 
-__global__ void eye_kernel(int n, double* A) {
-  const long long total = (long long)n * n;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x)
-    A[e] = (e % n == e / n) ? 1.0 : 0.0;
-}
-
 // B = A^T for n x n column-major, 32 x 32 tiles through shared memory
 __global__ void transpose_kernel(int n, const double* __restrict__ A, double* __restrict__ B) {
   __shared__ double tile[32][33];
@@ -1991,7 +1984,6 @@ struct OzakiPlan {
   CUtensorMap mapAd, mapDd;
   CUtensorMap mapDd56;  // trait digits in 56-row boxes (2-SM quadratic Gram, one-digit slot pairs)
   QuadPasses qp;
-  double* Linv = nullptr;       // chol: n x n, L^-1
   double* LinvT = nullptr;      // chol: n x n, (L^-1)^T (rows of L^-1 contiguous)
   float2* sqsum = nullptr;      // chol: Mpad/32 x Ncap sums of R^2 over 32-row groups (ld Ncap)
   int* err = nullptr;
@@ -2057,7 +2049,6 @@ cudaError_t ozaki_create(OzakiPlan** out, int n, int t, int wXL, int wXR, int x_
     chk(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev));
   }
   chk(cudaMalloc(&p->err, 3 * sizeof(int)));  // [wait error word, GEMM tile counter, finished CTAs]
-  if (!eigen) chk(cudaMalloc(&p->Linv, sizeof(double) * (size_t)n * n));
   if (!eigen) chk(cudaMalloc(&p->LinvT, sizeof(double) * (size_t)n * n));
   if (!eigen) chk(cudaMalloc(&p->sqsum, sizeof(float2) * (size_t)(p->Mpad / 32) * p->Ncap));
   if (r == cudaSuccess) chk(cudaMemset(p->A, 0, (size_t)p->S * p->Mpad * p->Kpad));
@@ -2111,7 +2102,7 @@ cudaError_t ozaki_create(OzakiPlan** out, int n, int t, int wXL, int wXR, int x_
 void ozaki_destroy(OzakiPlan* p) {
   if (!p) return;
   void* ptrs[] = {p->A,    p->G,     p->scale, p->scale_run, p->C, p->U, p->D,    p->dmax, p->amax,
-                  p->part, p->Linv,  p->LinvT, p->err,   p->Adig, p->Ddig, p->aexp, p->dexp, p->qpart,
+                  p->part, p->LinvT, p->err,   p->Adig, p->Ddig, p->aexp, p->dexp, p->qpart,
                   p->sqsum};
   for (void* q : ptrs)
     if (q) cudaFree(q);
@@ -2242,29 +2233,13 @@ cudaError_t ozaki_set_eigen(OzakiPlan* p, cudaStream_t s, DigitGemm* dg, const d
   return cudaGetLastError();
 }
 
-// L^-1 (lower, FP64) by blocked TRSM on the identity.  Column panel
-// [c0, c0 + w) of L^-1 is zero above row c0, so each panel solves only the
-// trailing system L[c0:, c0:] X = I[c0:, c0:c0+w]: n^3/3 flops instead of n^3.
-cudaError_t lower_inverse(cudaStream_t s, int n, const double* L, double* Linv) {
-  eye_kernel<<<grid_for((long long)n * n), 256, 0, s>>>(n, Linv);
-  note_launch();
-  constexpr int W = 512;
-  for (int c0 = 0; c0 < n; c0 += W) {
-    const int w = std::min(W, n - c0);
-    const long long off = (long long)c0 + (long long)c0 * n;
-    FGLS_CUDA_TRY(dtrsm_llnn(s, n - c0, w, L + off, n, Linv + off, n));
-  }
-  return cudaGetLastError();
-}
-
-cudaError_t ozaki_set_chol(OzakiPlan* p, cudaStream_t s, const double* L, const double* WY) {
+cudaError_t ozaki_set_chol(OzakiPlan* p, cudaStream_t s, DigitGemm* dg, const double* Linv, const double* WY) {
   const int n = p->n;
-  // L^-1 by the FP64 blocked TRSM on the identity, then U = L^-T [y~ | XL~]
-  FGLS_CUDA_TRY(lower_inverse(s, n, L, p->Linv));
-  FGLS_CUDA_TRY(dgemm(s, true, false, n, p->nU, n, 1.0, p->Linv, n, WY, n, 0.0, p->U, n));
+  // U = L^-T [y~ | XL~]
+  FGLS_CUDA_TRY(digit_dgemm(dg, s, true, false, n, p->nU, n, 1.0, Linv, n, WY, n, 0.0, p->U, n));
   // rows of L^-1 contiguous: transpose, then slice
   dim3 tg((n + 31) / 32, (n + 31) / 32);
-  transpose_kernel<<<tg, dim3(32, 8), 0, s>>>(n, p->Linv, p->LinvT);
+  transpose_kernel<<<tg, dim3(32, 8), 0, s>>>(n, Linv, p->LinvT);
   note_launch();
   FGLS_CUDA_TRY(slice_operands(p, s, p->LinvT, n, n));
   return cudaGetLastError();
@@ -2320,11 +2295,10 @@ int split_rows_padded(int rows) { return (rows + BM - 1) / BM * BM; }
 int split_k_padded(int n) { return (n + KALIGN - 1) / KALIGN * KALIGN; }
 int split_cols_padded(int x) { return (x + BN - 1) / BN * BN; }
 
-cudaError_t split_chol_operand(cudaStream_t s, int n, int wXL, const double* L, const double* WY, int S, int Mpad,
-                               int Kpad, uint8_t* A, double* scale, double* Linv, double* LinvT, double* U) {
+cudaError_t split_chol_operand(cudaStream_t s, DigitGemm* dg, int n, int wXL, const double* Linv, const double* WY, int S,
+                               int Mpad, int Kpad, uint8_t* A, double* scale, double* LinvT, double* U) {
   const int nU = 1 + wXL;
-  FGLS_CUDA_TRY(lower_inverse(s, n, L, Linv));
-  FGLS_CUDA_TRY(dgemm(s, true, false, n, nU, n, 1.0, Linv, n, WY, n, 0.0, U, n));
+  FGLS_CUDA_TRY(digit_dgemm(dg, s, true, false, n, nU, n, 1.0, Linv, n, WY, n, 0.0, U, n));
   dim3 tg((n + 31) / 32, (n + 31) / 32);
   transpose_kernel<<<tg, dim3(32, 8), 0, s>>>(n, Linv, LinvT);
   note_launch();

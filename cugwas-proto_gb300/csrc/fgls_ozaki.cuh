@@ -21,8 +21,8 @@ void ozaki_destroy(OzakiPlan* p);
 struct DigitGemm;
 cudaError_t ozaki_set_eigen(OzakiPlan* p, cudaStream_t s, DigitGemm* dg, const double* Z, const double* AYL,
                             const double* dinv);
-// chol: L (n x n lower), WY = [y~ | XL~] (n x (1+wXL)) of the selected trait
-cudaError_t ozaki_set_chol(OzakiPlan* p, cudaStream_t s, const double* L, const double* WY);
+// chol: L^-1 (n x n lower), WY = [y~ | XL~] (n x (1+wXL)) of the selected trait
+cudaError_t ozaki_set_chol(OzakiPlan* p, cudaStream_t s, DigitGemm* dg, const double* Linv, const double* WY);
 // A genotype block on the device in one of three formats (exactly one
 // pointer set): FP64 or bytes, n values per column, or 2-bit packed as a
 // SNP-major PLINK .bed body (ceil(n/4) bytes per column; a missing call sets
@@ -73,10 +73,10 @@ int split_rows_padded(int rows);
 int split_k_padded(int n);
 int split_cols_padded(int x);
 // [L^-1 ; (L^-T WY)^T] of one chol problem cut into S E4M3 five-bit digit slices at A
-// (S x Mpad x Kpad) with row scales; Linv, LinvT (n x n) and U (n x (1+wXL))
-// are caller scratch.
-cudaError_t split_chol_operand(cudaStream_t s, int n, int wXL, const double* L, const double* WY, int S, int Mpad,
-                               int Kpad, uint8_t* A, double* scale, double* Linv, double* LinvT, double* U);
+// (S x Mpad x Kpad) with row scales; LinvT (n x n) and U (n x (1+wXL)) are
+// caller scratch.
+cudaError_t split_chol_operand(cudaStream_t s, DigitGemm* dg, int n, int wXL, const double* Linv, const double* WY, int S,
+                               int Mpad, int Kpad, uint8_t* A, double* scale, double* LinvT, double* U);
 // row scales of the first S slices of an operand cut into S_built slices
 cudaError_t split_rescale_rows(cudaStream_t s, int rows, const double* built_scale, int S_built, int S,
                                double* scale);
