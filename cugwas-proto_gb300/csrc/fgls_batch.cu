@@ -477,17 +477,12 @@ cudaError_t setup_problem(fglsgpu_batch* b, Scratch& w, const CohortInputs& ci, 
   FGLS_CUDA_TRY(build_shifted(s, n, ci.Phi, n, h * sg, (1.0 - h) * sg, w.L, n));
   FGLS_CUDA_TRY(dpotrf_lower(s, w.dg, n, w.L, n, w.diag, w.st));
   FGLS_CUDA_TRY(lower_inverse(s, w.dg, n, w.L, n, w.Linv));
-  // [y | XL] whitened: a product with L^-1, or the solve for small cohorts
-  const bool product = w.dg && n >= 1024;
-  double* raw = product ? w.U : w.WY;
-  FGLS_CUDA_TRY(cudaMemcpyAsync(raw, ci.Y + (size_t)q.j * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-  FGLS_CUDA_TRY(cudaMemcpyAsync(raw + n, ci.XL, sizeof(double) * n * wXL, cudaMemcpyDeviceToDevice, s));
-  if (product)
-    FGLS_CUDA_TRY(digit_dgemm(w.dg, s, false, false, n, 1 + wXL, n, 1.0, w.Linv, n, w.U, n, 0.0, w.WY, n));
-  else
-    FGLS_CUDA_TRY(dtrsm_llnn(s, n, 1 + wXL, w.L, n, w.WY, n));
+  // [y | XL] whitened by a product with L^-1
+  FGLS_CUDA_TRY(cudaMemcpyAsync(w.U, ci.Y + (size_t)q.j * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+  FGLS_CUDA_TRY(cudaMemcpyAsync(w.U + n, ci.XL, sizeof(double) * n * wXL, cudaMemcpyDeviceToDevice, s));
+  FGLS_CUDA_TRY(lower_mul(s, false, n, 1 + wXL, w.Linv, w.U, w.WY));
   FGLS_CUDA_TRY(null_model_chol(s, n, wXL, w.WY, q.top, w.st, 0));
-  FGLS_CUDA_TRY(split_chol_operand(s, w.dg, n, wXL, w.Linv, w.WY, S_BUILT, q.Mpad, c.Kpad, q.A, q.scale_built, w.LinvT,
+  FGLS_CUDA_TRY(split_chol_operand(s, n, wXL, w.Linv, w.WY, S_BUILT, q.Mpad, c.Kpad, q.A, q.scale_built, w.LinvT,
                                    w.U));
   // FP64 path on the probe block (the reference's chol per-block loop)
   FGLS_CUDA_TRY(digit_dgemm(w.dg, s, false, false, n, PROBE, n, 1.0, w.Linv, n, w.X64, n, 0.0, w.Xw, n));

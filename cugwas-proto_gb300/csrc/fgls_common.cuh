@@ -59,6 +59,8 @@ struct DigitGemm;
 cudaError_t dpotrf_lower(cudaStream_t s, DigitGemm* dg, int n, double* A, long long lda, double* dinv, DevStatus* st);
 // Linv = L^-1 (n x n, ld n, zero above the diagonal) of the lower triangle of L.
 cudaError_t lower_inverse(cudaStream_t s, DigitGemm* dg, int n, const double* L, long long ldl, double* Linv);
+// Y = Linv X or Linv^T X for few columns (n x N, ld n; Y must not be X).
+cudaError_t lower_mul(cudaStream_t s, bool trans, int n, int N, const double* Linv, const double* X, double* Y);
 cudaError_t build_shifted(cudaStream_t s, int n, const double* Src, long long lds, double alpha,
                           double beta, double* A, long long lda);
 

@@ -1,5 +1,5 @@
-// FP64 dense kernels for the plain (all-FP64) path: tiled DGEMM, blocked
-// lower Cholesky (the reference's dpotrf of M, src/fgls_chol.c:252-271) and
+// FP64 dense kernels: tiled DGEMM for products too small for the digit form
+// (fgls_digit_gemm.cu), blocked lower Cholesky (the reference's dpotrf of M, src/fgls_chol.c:252-271) and
 // blocked lower-triangular solve X := L^-1 X (the reference's per-block
 // dtrsm, src/fgls_chol.c:365-368 and cublasDtrsm in
 // src/fgls_chol_gpu.c:543-555).
@@ -124,12 +124,84 @@ __global__ void __launch_bounds__(GT) dgemm_kernel(int M, int N, int K, double a
   }
 }
 
+// The same product on 32 x 8 tiles, for outputs of less than a wave of 64 x 64
+// tiles: an SM issues about two FP64 FMAs a clock, so a 64 x 64 tile takes 1.0 us
+// per element of K on one SM while the others idle (301 x 74 x 301: 135 us; on
+// 100 tiles of 32 x 8 20 us).
+constexpr int SM_ = 32, SN_ = 8, SK_ = 32, ST_ = 128;
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(ST_) dgemm_small_kernel(int M, int N, int K, double alpha, const double* __restrict__ A,
+                                                          long long lda, const double* __restrict__ B, long long ldb,
+                                                          double beta, double* __restrict__ C, long long ldc) {
+  __shared__ double As[2][SK_][SM_ + 1], Bs[2][SK_][SN_ + 1];
+  const int i0 = blockIdx.x * SM_, j0 = blockIdx.y * SN_;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  double ra[8], rb[2], acc[2] = {0.0, 0.0};
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+      const int ii = TA ? ty + 4 * r : tx, kk = TA ? tx : ty + 4 * r;
+      ra[r] = (i0 + ii < M && k0 + kk < K) ? ldA(A, lda, TA, i0 + ii, k0 + kk) : 0.0;
+    }
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const int e = threadIdx.x + r * ST_;
+      const int jj = TB ? e % SN_ : e / SK_, kk = TB ? e / SN_ : e % SK_;
+      rb[r] = (j0 + jj < N && k0 + kk < K) ? ldA(B, ldb, !TB, j0 + jj, k0 + kk) : 0.0;
+    }
+  };
+  auto store = [&](int buf) {
+#pragma unroll
+    for (int r = 0; r < 8; r++) As[buf][TA ? tx : ty + 4 * r][TA ? ty + 4 * r : tx] = ra[r];
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const int e = threadIdx.x + r * ST_;
+      Bs[buf][TB ? e / SN_ : e % SK_][TB ? e % SN_ : e / SK_] = rb[r];
+    }
+  };
+  const int nk = (K + SK_ - 1) / SK_;
+  if (nk > 0) {
+    load(0);
+    store(0);
+  }
+  __syncthreads();
+  for (int kt = 0; kt < nk; kt++) {
+    const int buf = kt & 1;
+    if (kt + 1 < nk) load((kt + 1) * SK_);
+#pragma unroll
+    for (int k = 0; k < SK_; k++) {
+      const double a = As[buf][k][tx];
+      acc[0] = fma(a, Bs[buf][k][2 * ty], acc[0]);
+      acc[1] = fma(a, Bs[buf][k][2 * ty + 1], acc[1]);
+    }
+    if (kt + 1 < nk) store(buf ^ 1);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int i = i0 + tx, j = j0 + 2 * ty + u;
+    if (i >= M || j >= N) continue;
+    double* cp = C + i + (long long)j * ldc;
+    const double v = alpha * acc[u];
+    *cp = beta != 0.0 ? fma(beta, *cp, v) : v;
+  }
+}
+
 template <bool LOWER>
 cudaError_t launch_dgemm(cudaStream_t s, bool tA, bool tB, int M, int N, int K, double alpha,
                          const double* A, long long lda, const double* B, long long ldb,
                          double beta, double* C, long long ldc) {
   if (M <= 0 || N <= 0) return cudaSuccess;
   dim3 grid(ceil_div(M, GM), ceil_div(N, GN));
+  if (!LOWER && grid.x * grid.y < 152) {
+    const dim3 sg(ceil_div(M, SM_), ceil_div(N, SN_));
+    if (!tA && !tB) dgemm_small_kernel<false, false><<<sg, ST_, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+    else if (!tA) dgemm_small_kernel<false, true><<<sg, ST_, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+    else if (!tB) dgemm_small_kernel<true, false><<<sg, ST_, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+    else dgemm_small_kernel<true, true><<<sg, ST_, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+    note_launch();
+    return cudaGetLastError();
+  }
   if (!tA && !tB) dgemm_kernel<false, false, LOWER><<<grid, GT, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
   else if (!tA && tB) dgemm_kernel<false, true, LOWER><<<grid, GT, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
   else if (tA && !tB) dgemm_kernel<true, false, LOWER><<<grid, GT, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
@@ -147,63 +219,124 @@ constexpr int DT = 256;       // threads of the diagonal kernels
 constexpr int PB = 64;        // diagonal block of potrf and of the inverse
 constexpr int PO = 512;       // outer panel of potrf, base block of the inverse
 
-// Inverse of the kb x kb lower triangle in Ls ([c][r], rdiag[j] = 1 / L_jj) into
-// Xs ([c][r], zero above the diagonal): thread (c, g) holds column c's rows g,
-// g + 4, ..; all threads of the CTA call it.
-__device__ __forceinline__ void tri_inverse(int kb, const double (*Ls)[PB + 1], const double* rdiag,
-                                            double (*Xs)[PB + 1]) {
-  const int c = threadIdx.x & (PB - 1), g = threadIdx.x / PB;
-  for (int r = g; r < PB; r += DT / PB) Xs[c][r] = r == c ? 1.0 : 0.0;
-  __syncthreads();
-  for (int j = 0; j < kb; j++) {
-    const double x = Xs[c][j] * rdiag[j];
-    __syncthreads();
-    if (g == (j & 3)) Xs[c][j] = x;
-    if (c <= j)
-      for (int r = j + 1 + ((g - (j + 1)) & 3); r < kb; r += 4) Xs[c][r] = fma(-Ls[j][r], x, Xs[c][r]);
-    __syncthreads();
+// 1 / sqrt(d) on a short chain: dependent FP64 instructions take some 150 cycles
+// each here, and the library function is a chain of two dozen.  Seed from the FP32
+// reciprocal square root of the mantissa (moved in and out by integer
+// instructions), then one third-order step y (1 + e/2 + 3 e^2 / 8), e = 1 - d y^2
+// (the binomial series of (1 - e)^(-1/2)): |e| < 2^-21 leaves 2^-63.
+__device__ __forceinline__ double chain_rsqrt(double d) {
+  const long long b = __double_as_longlong(d);
+  const int ex = (int)(b >> 52);
+  if (ex <= 0 || ex >= 0x7ff) return rsqrt(d);  // zero, subnormal, negative, infinite, NaN
+  const int k = ex - 1023, odd = k & 1;
+  const float m = __int_as_float(((127 + odd) << 23) | ((int)(b >> 29) & 0x7fffff));  // in [1, 4)
+  const int f = __float_as_int(rsqrtf(m));
+  const double y = __longlong_as_double(((long long)((f >> 23) - 127 + 1023 - (k >> 1)) << 52) |
+                                        ((long long)(f & 0x7fffff) << 29));
+  const double e = fma(-(d * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// Cholesky factor of a 64 x 64 block and its inverse, one CTA of eight warps
+// (FACTOR = false: the inverse alone, Ls and rdiag given).
+//   Ls[c][r]: finished columns of the factor, Xs[r][c]: finished rows of the
+//   inverse, rdiag[j] = 1 / L_jj; identity past kb.
+// Bound by FP64 issue (a sub-core starts a warp's FP64 instruction every 64
+// cycles) and each pivot's reciprocal square root, so what is unfinished lives in
+// registers (warp w: columns w, w + 8, .. with a row pair per lane, rows w, w + 8,
+// .. of the inverse with a column pair per lane), one barrier a step, and the next
+// column is finished while the others are updated.  Through shared memory, column
+// by column, the pair took 0.158 ms; now 0.097 (the inverse alone 0.046).
+template <bool FACTOR>
+__device__ __forceinline__ void factor_invert(int kb, double (&L0)[8], double (&L1)[8], double (*Ls)[PB + 1],
+                                              double (*Xs)[PB + 1], double* rdiag, int col0, DevStatus* st) {
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  double X0[8], X1[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    X0[i] = wp + 8 * i == lane ? 1.0 : 0.0;
+    X1[i] = wp + 8 * i == lane + 32 ? 1.0 : 0.0;
   }
+  // column j of the factor from its updated values (rows lane, lane + 32)
+  auto finish = [&](int j, double c0, double c1) {
+    const double d = __shfl_sync(0xffffffffu, j < 32 ? c0 : c1, j & 31);
+    if (!(d > 0.0) && lane == 0 && j < kb) set_status(st, FGLSGPU_ENOTSPD, col0 + j + 1, -1);
+    const double ri = chain_rsqrt(d);
+    double piv = d * ri;
+    piv = fma(0.5 * ri, fma(-piv, piv, d), piv);
+    Ls[j][lane] = lane > j ? c0 * ri : lane == j ? piv : 0.0;
+    Ls[j][lane + 32] = lane + 32 > j ? c1 * ri : lane + 32 == j ? piv : 0.0;
+    if (lane == 0) rdiag[j] = ri;
+  };
+  if (FACTOR && wp == 0) finish(0, L0[0], L1[0]);
+  // j = 8 jb + j8, jb unrolled: register arrays take constant indexes only, and
+  // what is finished costs nothing
+#pragma unroll
+  for (int jb = 0; jb < 8; jb++) {
+#pragma unroll 1
+    for (int j8 = 0; j8 < 8; j8++) {
+      const int j = 8 * jb + j8;
+      __syncthreads();
+      if (FACTOR && j + 1 < PB) {
+        const double l0 = -Ls[j][lane], l1 = -Ls[j][lane + 32];
+        if (((j + 1) & 7) == wp) {
+          const double f = Ls[j][j + 1];
+          const int nx = jb < 7 ? jb + 1 : 7;
+          finish(j + 1, jb < 4 ? fma(l0, f, j8 < 7 ? L0[jb] : L0[nx]) : 0.0, fma(l1, f, j8 < 7 ? L1[jb] : L1[nx]));
+        }
+#pragma unroll
+        for (int i = jb; i < 8; i++) {
+          const int c = wp + 8 * i;
+          if (i <= jb + 1 && c <= j + 1) continue;
+          const double f = Ls[j][c];
+          if (i < 4) L0[i] = fma(l0, f, L0[i]);  // columns from 32 on have no row below 32
+          L1[i] = fma(l1, f, L1[i]);
+        }
+      }
+      if (j > 0) {  // row j - 1 of the inverse, finished a step ago, from the rows below
+        const double x0 = Xs[j - 1][lane], x1 = Xs[j - 1][lane + 32];
+#pragma unroll
+        for (int i = jb; i < 8; i++) {
+          const int r = wp + 8 * i;
+          if (i == jb && r < j) continue;
+          const double l = -Ls[j - 1][r];
+          X0[i] = fma(l, x0, X0[i]);
+          if (jb >= 4) X1[i] = fma(l, x1, X1[i]);
+        }
+      }
+      if (j8 == wp) {
+        const double rd = rdiag[j];
+        Xs[j][lane] = X0[jb] * rd;
+        Xs[j][lane + 32] = X1[jb] * rd;
+      }
+    }
+  }
+  __syncthreads();
 }
 
 // Factors the kb x kb diagonal block at A (lower, in place) and writes the
 // inverse of its factor to dinv (PB x PB, row c at dinv + c*PB, zero above the
-// diagonal and past kb).  One CTA, a serial chain of 2 kb steps: 64 columns
-// take 0.04 ms; the 128-column form was bound by one SM's FP64 rate.
+// diagonal and past kb).
 __global__ void __launch_bounds__(DT) potf2_inv_kernel(int kb, double* A, long long lda, int col0,
                                                        double* __restrict__ dinv, DevStatus* st) {
   extern __shared__ double sm[];
-  double(*Ls)[PB + 1] = (double(*)[PB + 1])sm;              // Ls[c][r] = A(r, c)
+  double(*Ls)[PB + 1] = (double(*)[PB + 1])sm;
   double(*Xs)[PB + 1] = (double(*)[PB + 1])(sm + PB * (PB + 1));
   __shared__ double rdiag[PB];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  double L0[8], L1[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int c = wp + 8 * i;
+    const double* a = A + (long long)c * lda;
+    L0[i] = (lane >= c && lane < kb) ? a[lane] : lane == c ? 1.0 : 0.0;
+    L1[i] = (lane + 32 >= c && lane + 32 < kb) ? a[lane + 32] : lane + 32 == c ? 1.0 : 0.0;
+  }
+  factor_invert<true>(kb, L0, L1, Ls, Xs, rdiag, col0, st);
   for (int e = threadIdx.x; e < PB * PB; e += DT) {
     const int r = e & (PB - 1), c = e / PB;
-    Ls[c][r] = (r >= c && r < kb) ? A[r + (long long)c * lda] : 0.0;
-  }
-  __syncthreads();
-  const int r = threadIdx.x & (PB - 1), g = threadIdx.x / PB;
-  bool bad = false;
-  for (int j = 0; j < kb; j++) {
-    const double d = Ls[j][j];
-    if (!(d > 0.0) && threadIdx.x == 0 && !bad) {
-      bad = true;
-      set_status(st, FGLSGPU_ENOTSPD, col0 + j + 1, -1);
-    }
-    const double piv = sqrt(d), ri = 1.0 / piv;
-    const double v = r > j ? Ls[j][r] * ri : r == j ? piv : 0.0;
-    __syncthreads();
-    if (g == 0 && r >= j) Ls[j][r] = v;
-    if (threadIdx.x == 0) rdiag[j] = ri;
-    __syncthreads();
-    // columns c > j of row r (the factor's column j in shared memory)
-    for (int c = j + 1 + ((g - (j + 1)) & 3); c <= r; c += DT / PB) Ls[c][r] = fma(-v, Ls[j][c], Ls[c][r]);
-    __syncthreads();
-  }
-  tri_inverse(kb, Ls, rdiag, Xs);
-  for (int e = threadIdx.x; e < PB * PB; e += DT) {
-    const int rr = e & (PB - 1), c = e / PB;
-    if (rr >= c && rr < kb) A[rr + (long long)c * lda] = Ls[c][rr];
-    // row c' = e / PB of dinv, element q = e % PB: Linv(c', q)
-    dinv[e] = (c < kb && rr <= c) ? Xs[rr][c] : 0.0;
+    if (r >= c && r < kb) A[r + (long long)c * lda] = Ls[c][r];
+    dinv[e] = (c < kb && r <= c) ? Xs[c][r] : 0.0;  // row c, element r
   }
 }
 
@@ -244,15 +377,16 @@ __global__ void __launch_bounds__(DT) tri_inv_kernel(int n, const double* __rest
   const int o = blockIdx.x * PB, kb = min(PB, n - o);
   for (int e = threadIdx.x; e < PB * PB; e += DT) {
     const int r = e & (PB - 1), c = e / PB;
-    Ls[c][r] = (r >= c && r < kb) ? L[(o + r) + (long long)(o + c) * ldl] : 0.0;
+    Ls[c][r] = (r >= c && r < kb) ? L[(o + r) + (long long)(o + c) * ldl] : r == c ? 1.0 : 0.0;
   }
   __syncthreads();
-  if (threadIdx.x < kb) rdiag[threadIdx.x] = 1.0 / Ls[threadIdx.x][threadIdx.x];
+  if (threadIdx.x < PB) rdiag[threadIdx.x] = 1.0 / Ls[threadIdx.x][threadIdx.x];
   __syncthreads();
-  tri_inverse(kb, Ls, rdiag, Xs);
+  double none[8];
+  factor_invert<false>(kb, none, none, Ls, Xs, rdiag, 0, nullptr);
   for (int e = threadIdx.x; e < PB * PB; e += DT) {
     const int r = e & (PB - 1), c = e / PB;
-    if (r >= c && r < kb && c < kb) Linv[(o + r) + (long long)(o + c) * n] = Xs[c][r];
+    if (r >= c && r < kb && c < kb) Linv[(o + r) + (long long)(o + c) * n] = Xs[r][c];
   }
 }
 
@@ -298,6 +432,63 @@ __global__ void __launch_bounds__(256) tri_merge_kernel(int n, int w, const doub
     if (i >= M || j >= N) continue;
     if (FIRST) Linv[(o + i) + (long long)(o + w + j) * n] = acc[u];
     else Linv[(o + w + i) + (long long)(o + j) * n] = -acc[u];
+  }
+}
+
+// Y (n x N, ld n) = Linv X: 32 rows a CTA, a row per lane, the columns of Linv up
+// to the diagonal dealt to the eight warps, N <= 8 columns of X at a time.
+// n^2 N / 2 FMAs and one read of the triangle (n = 6000, N = 3: 0.83 ms on 32 x 8
+// tiles of the general product).
+constexpr int LM = 8;
+__global__ void __launch_bounds__(256) lower_mul_kernel(int n, int N, const double* __restrict__ Linv,
+                                                        const double* __restrict__ X, double* __restrict__ Y) {
+  __shared__ double red[8][LM][32];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int r0 = (gridDim.x - 1 - blockIdx.x) * 32, r = r0 + lane;  // longest rows first
+  const int kend = min(n, r0 + 32);
+  double acc[LM];
+#pragma unroll
+  for (int q = 0; q < LM; q++) acc[q] = 0.0;
+#pragma unroll 4
+  for (int k = wp; k < kend; k += 8) {
+    const double l = r < n ? Linv[r + (long long)k * n] : 0.0;
+#pragma unroll
+    for (int q = 0; q < LM; q++)
+      if (q < N) acc[q] = fma(l, X[k + (long long)q * n], acc[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < LM; q++) red[wp][q][lane] = acc[q];
+  __syncthreads();
+  if (wp < N && r < n) {
+    double v = 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; u++) v += red[u][wp][lane];
+    Y[r + (long long)wp * n] = v;
+  }
+}
+// Y (n x N, ld n) = Linv^T X: a warp per column of Linv.
+__global__ void __launch_bounds__(256) lower_tmul_kernel(int n, int N, const double* __restrict__ Linv,
+                                                         const double* __restrict__ X, double* __restrict__ Y) {
+  const int lane = threadIdx.x & 31, j = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (j >= n) return;
+  const double* l = Linv + (long long)j * n;
+  double acc[LM];
+#pragma unroll
+  for (int q = 0; q < LM; q++) acc[q] = 0.0;
+#pragma unroll 4
+  for (int i = (j & ~31) + lane; i < n; i += 32) {
+    const double v = l[i];  // zero above the diagonal
+#pragma unroll
+    for (int q = 0; q < LM; q++)
+      if (q < N) acc[q] = fma(v, X[i + (long long)q * n], acc[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < LM; q++) {
+    if (q >= N) break;
+    double v = acc[q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) Y[j + (long long)q * n] = v;
   }
 }
 
@@ -469,8 +660,7 @@ cudaError_t build_shifted(cudaStream_t s, int n, const double* Src, long long ld
 // Blocked Cholesky: 64-column blocks (factor and its inverse in one CTA, the
 // panel below as a product with the inverse), updates within 512-column panels
 // after each block and of the whole trailing triangle after each panel, so that
-// the big update has K = 512.  With digits, n = 10000 takes ~30 ms against
-// 360 ms when every update ran on the FP64 kernel.
+// the big update has K = 512.  With digits, n = 6000 takes about 22 ms.
 cudaError_t dpotrf_lower(cudaStream_t s, DigitGemm* dg, int n, double* A, long long lda, double* dinv, DevStatus* st) {
   FGLS_CUDA_TRY(ensure_attrs());
   for (int k0 = 0; k0 < n; k0 += PO) {
@@ -558,6 +748,16 @@ cudaError_t lower_inverse(cudaStream_t s, DigitGemm* dg, int n, const double* L,
   }
   FGLS_CUDA_TRY(cudaGetLastError());
   return inverse_range(s, dg, n, L, ldl, Linv, 0, n);
+}
+
+cudaError_t lower_mul(cudaStream_t s, bool trans, int n, int N, const double* Linv, const double* X, double* Y) {
+  for (int q = 0; q < N; q += LM) {
+    const int m = std::min(LM, N - q);
+    if (trans) lower_tmul_kernel<<<ceil_div(n, 8), 256, 0, s>>>(n, m, Linv, X + (long long)q * n, Y + (long long)q * n);
+    else lower_mul_kernel<<<ceil_div(n, 32), 256, 0, s>>>(n, m, Linv, X + (long long)q * n, Y + (long long)q * n);
+    note_launch();
+  }
+  return cudaGetLastError();
 }
 
 cudaError_t dtrsm_llnn(cudaStream_t s, int n, int nrhs, const double* L, long long ldl, double* X,

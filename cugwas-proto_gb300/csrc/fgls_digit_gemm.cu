@@ -37,7 +37,7 @@
 // MMAs would take.
 //   warp 0     TMA producer (each CTA its own 128 rows), six stages
 //   warp 1     MMA issue (pair leader), TMEM allocation
-//   warps 2-9  epilogue: q = 32 P_L + P_{L+1} as int32 into the CTA's own
+//   warps 2-17 epilogue: q = 32 P_L + P_{L+1} as int32 into the CTA's own
 //              planes (L2-resident, 4 bytes per element and level pair); once a
 //              tile's last pass is stored its TMEM is released and the planes
 //              are combined while the next tile's MMAs run.
@@ -72,13 +72,17 @@ constexpr int TILE = 128 * ROW;        // 16 KB: 128 rows of one digit plane
 constexpr int STAGE = 2 * TILE;        // an A and a B tile
 constexpr int STAGES = 6;
 constexpr int SMEM = STAGES * STAGE + 1024 + 256;
-constexpr int NTHREADS = 320;
-constexpr int EPI_WARPS = 8;
+constexpr int EPI_WARPS = 16;
+constexpr int EPI_COLS = 256 * 4 / EPI_WARPS;  // columns of an epilogue warp (32 rows)
+constexpr int NTHREADS = 64 + 32 * EPI_WARPS;
 constexpr int MAXPASS = (ND + 1) / 2;  // level pairs
-constexpr int PLANE = 128 * 256;       // ints of one CTA's plane
-constexpr int BAD_ROW = 0x7fffffff;    // exponent of a row that holds a NaN or an infinity
+constexpr int PLANE4 = 128 * 256 / 4;   // int4s of one CTA's plane
 constexpr int PAIR_K = 512;            // K-steps x pairs one FP32 accumulator takes exactly (65536 elements)
 // int32 planes: 33 * 2^8 * pairs * K < 2^31 for 12 pairs
+// tiles per cluster up to which the split form runs: with whole tiles as units the
+// other clusters idle and a tile's six passes and its epilogue are one chain
+// (301 x 74 x 301 with both cuts: 0.173 ms, split 0.080; 1000 x 512 x 64 0.144, 0.064)
+constexpr double SPLIT_TILES = 1.0;
 constexpr int K_MAX_STEPS = 160;       // 20480 elements of K per launch
 // kind::f8f6f4: D=F32, A=B=E4M3, K-major, N=256, M=256 (the pair)
 constexpr uint32_t DG_IDESC = (1u << 4) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
@@ -94,34 +98,35 @@ __device__ __forceinline__ void tma_load_3d_cg2(void* dst, const CUtensorMap* tm
 struct DgArgs {
   int M, N;
   int kb0, nk;            // K-steps of this launch: [kb0, kb0 + nk)
-  int ksplit, kper;       // K split over units: split z takes steps [z*kper, ..) of the range
+  // Split form (few tiles): a unit is one level pair of a tile over a part of K;
+  // level pair i is cut into zs[i] parts of kper[i] steps and every unit writes
+  // its own plane.  zsum = 0: a unit is a whole tile.
+  int zsum, zs[MAXPASS], kper[MAXPASS];
   int tiles_m, tiles_n;   // 256 x 256 tiles
   int lower_tiles;        // tiles are those with n_tile <= m_tile only, and only r >= c is written
   int a_lower;            // row r of A is zero beyond column r
   const int *exA, *exB, *ndA, *ndB;
   double alpha, beta;
-  double* C;              // ksplit > 1: partial plane z at C + z * M * N
+  double* C;
   long long ldc;
-  int* planes;
+  int4* planes;
   int* err;
   unsigned long long wait_ns;
 };
 
-// What the three roles need of a unit (an output tile and a range of K).
+// What the roles need of a unit: an output tile, level pairs [i0, i1) and a
+// range of K; `slot`: the plane of a split unit.
 struct Unit {
-  int mt, nt, z, kb, nk, da, db;
+  int mt, nt, kb, nk, da, db, i0, i1, slot;
 };
-__device__ __forceinline__ int dg_units(const DgArgs& g) {
-  const int t = g.lower_tiles ? g.tiles_m * (g.tiles_m + 1) / 2 : g.tiles_m * g.tiles_n;
-  return t * g.ksplit;
+__device__ __forceinline__ int dg_tiles(const DgArgs& g) {
+  return g.lower_tiles ? g.tiles_m * (g.tiles_m + 1) / 2 : g.tiles_m * g.tiles_n;
 }
-// Unit u.  Lower-triangular A: row tiles with the most K first (the units are
+__device__ __forceinline__ int dg_units(const DgArgs& g) { return dg_tiles(g) * max(1, g.zsum); }
+// Tile t.  Lower-triangular A: row tiles with the most K first (the units are
 // dealt in order); else groups of eight row tiles, so that the tiles in flight
 // share operand tiles in L2.
-__device__ __forceinline__ Unit dg_unit(const DgArgs& g, int u) {
-  Unit U;
-  U.z = u % g.ksplit;
-  int t = u / g.ksplit;
+__device__ __forceinline__ void dg_tile(const DgArgs& g, int t, Unit& U) {
   if (g.lower_tiles) {
     int m = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
     while (m * (m + 1) / 2 > t) m--;
@@ -138,11 +143,31 @@ __device__ __forceinline__ Unit dg_unit(const DgArgs& g, int u) {
     U.mt = grp * 8 + in % gm;
     U.nt = in / gm;
   }
-  U.kb = g.kb0 + U.z * g.kper;
-  U.nk = min(g.kper, g.nk - U.z * g.kper);
-  if (g.a_lower) U.nk = min(U.nk, 2 * (U.mt + 1) - U.kb);  // 256 rows: 2 K-steps a row tile
   U.da = max(1, g.ndA[U.mt]);
   U.db = max(1, g.ndB[U.nt]);
+  U.i0 = 0;
+  U.i1 = min(ND + 1, U.da + U.db) / 2;
+  U.kb = g.kb0;
+  U.nk = g.nk;
+  if (g.a_lower) U.nk = min(U.nk, 2 * (U.mt + 1) - U.kb);  // 256 rows: 2 K-steps a row tile
+  U.slot = 0;
+}
+// Unit u.  Split form: the level pairs with the most digit pairs first.
+__device__ __forceinline__ Unit dg_unit(const DgArgs& g, int u) {
+  Unit U;
+  if (g.zsum == 0) {
+    dg_tile(g, u, U);
+    return U;
+  }
+  const int tiles = dg_tiles(g), t = u % tiles;
+  int z = u / tiles, i = MAXPASS - 1;
+  dg_tile(g, t, U);
+  U.slot = t * g.zsum + z;
+  while (z >= g.zs[i]) z -= g.zs[i--];
+  U.i0 = i;
+  U.i1 = min(i + 1, U.i1);
+  U.kb += z * g.kper[i];
+  U.nk = min(U.nk - z * g.kper[i], g.kper[i]);
   return U;
 }
 
@@ -150,7 +175,6 @@ __device__ __forceinline__ Unit dg_unit(const DgArgs& g, int u) {
 struct Pass {
   int L, tlo, thi, has1, pro, chunk;  // pro: an A tile (digit L + 1 - tlo) precedes step tlo; chunk: K-steps a pass
 };
-__device__ __forceinline__ int dg_passes(const Unit& U) { return (min(ND + 1, U.da + U.db)) / 2; }
 __device__ __forceinline__ Pass dg_pass(const Unit& U, int i) {
   Pass P;
   const int lmax = min(ND + 1, U.da + U.db);
@@ -175,32 +199,76 @@ __device__ __forceinline__ int exact_f2i(float v) {
   return (int)(((uint32_t)__float_as_int(t) - 0x4C400000u) * 4u + ((uint32_t)__float_as_int(u) - 0x4B400000u));
 }
 
-// T * 2^e rounded to FP64 (to nearest even), in integer instructions.
-__device__ __forceinline__ double i128_to_double(__int128 T, int e) {
-  const bool neg = T < 0;
-  const unsigned __int128 U = neg ? (unsigned __int128)0 - (unsigned __int128)T : (unsigned __int128)T;
-  uint64_t hi = (uint64_t)(U >> 64), lo = (uint64_t)U;
-  int top;  // index of the highest set bit
+// exponent of a row's scale from the largest biased exponent in it (what a
+// DigitMat keeps per row)
+__device__ __forceinline__ int row_exponent(int top) { return top - 1021; }
+
+// (W 2^sh + V) 2^e rounded to FP64 (to nearest even) in integer instructions;
+// |W|, |V| < 2^52, sh <= 30.
+__device__ __forceinline__ double combine_words(long long W, int sh, long long V, int e) {
+  uint64_t lo = (uint64_t)W << sh;
+  long long hi = sh ? W >> (64 - sh) : W >> 63;
+  const uint64_t sum = lo + (uint64_t)V;
+  hi += (V >> 63) + (sum < lo);
+  lo = sum;
+  const bool neg = hi < 0;
+  if (neg) {
+    lo = 0 - lo;
+    hi = ~hi + (lo == 0);
+  }
+  // the magnitude (below 2^83) with its highest bit at bit 63 of m
+  uint64_t m;
+  int top;
+  bool sticky = false;
   if (hi) {
-    const int z = __clzll((long long)hi);
-    top = 127 - z;
-    if (z) {
-      hi = (hi << z) | (lo >> (64 - z));
-      lo <<= z;
-    }
+    const int s = 32 - __clz((int)hi);  // 1 .. 19 bits above bit 63
+    top = 63 + s;
+    m = ((uint64_t)hi << (64 - s)) | (lo >> s);
+    sticky = (lo << (64 - s)) != 0;
   } else {
     if (!lo) return 0.0;
     const int z = __clzll((long long)lo);
     top = 63 - z;
-    hi = lo << z;
-    lo = 0;
+    m = lo << z;
   }
-  uint64_t m = hi >> 11;
-  const uint32_t rest = (uint32_t)hi & 0x7ffu;
-  if (rest > 0x400u || (rest == 0x400u && (lo != 0 || (m & 1)))) m++;
+  const uint32_t rest = (uint32_t)m & 0x7ffu;
+  m >>= 11;
+  m += (rest > 0x400u || (rest == 0x400u && (sticky || (m & 1)))) ? 1 : 0;
   const int ex = top + e;  // m in [2^52, 2^53]
   if (ex < -1000 || ex > 1000) return ldexp(neg ? -(double)m : (double)m, ex - 52);
   return __longlong_as_double((long long)((m + ((uint64_t)(ex + 1022) << 52)) | (neg ? 1ull << 63 : 0ull)));
+}
+
+// Four elements of row r from column c on: T = sum_i q_i 2^(10 (np - 1 - i)),
+// the element is T 2^(exA + exB - 5 (2 np + 1)); alpha, beta and the write.
+__device__ __forceinline__ void store_four(const DgArgs& g, const int4 (&q)[MAXPASS], int np, int r, int c) {
+  const int ea = g.exA[r], e0 = row_exponent(ea) - 5 * (2 * np + 1);
+  const int h = min(np, 3), sh = 10 * (np - h);
+  const int most = min(4, (g.lower_tiles ? min(g.N, r + 1) : g.N) - c);
+  double* cp = g.C + r + (long long)c * g.ldc;
+  double old[4];
+  if (g.beta != 0.0) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) old[j] = j < most ? cp[j * g.ldc] : 0.0;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    if (j >= most) break;
+    long long W = 0, V = 0;
+#pragma unroll
+    for (int i = 0; i < MAXPASS; i++) {
+      const int x = j == 0 ? q[i].x : j == 1 ? q[i].y : j == 2 ? q[i].z : q[i].w;
+      if (i < h) W = W * 1024 + x;
+      else if (i < np) V = V * 1024 + x;
+    }
+    const int eb = g.exB[c + j];
+    double v;
+    if (ea == 0x7ff || eb == 0x7ff) v = __longlong_as_double(0x7ff8000000000000ll);  // a NaN or an infinity in the row
+    else v = combine_words(W, sh, V, e0 + row_exponent(eb));
+    if (g.alpha != 1.0) v = g.alpha == -1.0 ? -v : v * g.alpha;
+    if (g.beta != 0.0) v = fma(g.beta, old[j], v);
+    cp[j * g.ldc] = v;
+  }
 }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
@@ -274,9 +342,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
       for (int u = cid; u < units && ok; u += ncl) {
         const Unit U = dg_unit(g, u);
         const int ra = U.mt * 256 + (int)rank * 128, rb = U.nt * 256 + (int)rank * 128;
-        const int np = dg_passes(U);
 #pragma unroll 1
-        for (int i = 0; i < np && ok; i++) {
+        for (int i = U.i0; i < U.i1 && ok; i++) {
           const Pass P = dg_pass(U, i);
 #pragma unroll 1
           for (int kb = 0; kb < U.nk && ok; kb++) {
@@ -308,9 +375,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
 #pragma unroll 1
       for (int u = cid; u < units && ok; u += ncl) {
         const Unit U = dg_unit(g, u);
-        const int np = dg_passes(U);
 #pragma unroll 1
-        for (int i = 0; i < np && ok; i++) {
+        for (int i = U.i0; i < U.i1 && ok; i++) {
           const Pass P = dg_pass(U, i);
 #pragma unroll 1
           for (int k0 = 0; k0 < U.nk && ok; k0 += P.chunk, q++) {
@@ -386,21 +452,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
     __syncwarp();
   } else {
     const int lq = warp & 3;
-    const int cbeg = ((warp - 2) >> 2) * 128;
+    const int cbeg = ((warp - 2) >> 2) * EPI_COLS;
     const int row = lq * 32 + lane;
     const uint32_t ta = tbase + ((uint32_t)(lq * 32) << 16) + (uint32_t)cbeg;
     const uint32_t lead_tempty = cluster_addr(tempty, 0);
-    int* plane0 = g.planes + (size_t)blockIdx.x * (MAXPASS * PLANE) + cbeg * 128 + row;
+    // planes as [column / 4][row][column % 4]: sixteen bytes a thread, 512 a warp
+    const bool split = g.zsum > 0;
     uint32_t q = 0;
     bool ok = true;
 #pragma unroll 1
     for (int u = cid; u < units && ok; u += ncl) {
       const Unit U = dg_unit(g, u);
-      const int np = dg_passes(U);
+      const int np = U.i1;
+      // (split: the unit's one plane, addressed as level pair i0)
+      int4* plane0 = g.planes + cbeg / 4 * 128 + row +
+                     (split ? (2 * (size_t)U.slot + rank) * PLANE4 - (ptrdiff_t)U.i0 * PLANE4
+                            : (size_t)blockIdx.x * (MAXPASS * PLANE4));
+      const int r = U.mt * 256 + (int)rank * 128 + row;
+      const int n0 = U.nt * 256 + cbeg;
+      const int ncols = max(0, min(EPI_COLS, g.N - n0));
 #pragma unroll 1
-      for (int i = 0; i < np && ok; i++) {
+      for (int i = U.i0; i < np && ok; i++) {
         const Pass P = dg_pass(U, i);
-        int* pl = plane0 + i * PLANE;
+        int4* pl = plane0 + i * PLANE4;
 #pragma unroll 1
         for (int k0 = 0; k0 < U.nk; k0 += P.chunk, q++) {
           int okw = 1;
@@ -409,26 +483,33 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
           if (!okw) { ok = false; break; }
           tc_fence_after();
 #pragma unroll 1
-          for (int c0 = 0; c0 < 128; c0 += 32) {
-            uint32_t v[32], w[32];
-            tmem_ld32(ta + c0, v);
-            if (P.has1) {
-              tmem_ld32(ta + 256 + c0, w);
-              tmem_ld_wait();
+          for (int c0 = 0; c0 < ncols; c0 += 32) {
+            uint32_t v[32];
+            {
+              uint32_t w[32];
+              tmem_ld32(ta + c0, v);
+              if (P.has1) {
+                tmem_ld32(ta + 256 + c0, w);
+                tmem_ld_wait();
 #pragma unroll
-              for (int j = 0; j < 32; j++)
-                v[j] = (uint32_t)(exact_f2i(__uint_as_float(v[j])) * 32 + exact_f2i(__uint_as_float(w[j])));
-            } else {
-              tmem_ld_wait();
+                for (int j = 0; j < 32; j++)
+                  v[j] = (uint32_t)(exact_f2i(__uint_as_float(v[j])) * 32 + exact_f2i(__uint_as_float(w[j])));
+              } else {
+                tmem_ld_wait();
 #pragma unroll
-              for (int j = 0; j < 32; j++) v[j] = (uint32_t)(exact_f2i(__uint_as_float(v[j])) * 32);
+                for (int j = 0; j < 32; j++) v[j] = (uint32_t)(exact_f2i(__uint_as_float(v[j])) * 32);
+              }
             }
-            if (k0 > 0) {
 #pragma unroll
-              for (int j = 0; j < 32; j++) v[j] += (uint32_t)pl[(c0 + j) * 128];
+            for (int j = 0; j < 8; j++) {
+              int4* p4 = pl + (c0 / 4 + j) * 128;
+              int4 t = make_int4((int)v[4 * j], (int)v[4 * j + 1], (int)v[4 * j + 2], (int)v[4 * j + 3]);
+              if (k0 > 0) {
+                const int4 o = *p4;
+                t = make_int4(t.x + o.x, t.y + o.y, t.z + o.z, t.w + o.w);
+              }
+              *p4 = t;
             }
-#pragma unroll
-            for (int j = 0; j < 32; j++) pl[(c0 + j) * 128] = (int)v[j];
           }
           tc_fence_before();
           __syncwarp();
@@ -436,43 +517,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
         }
       }
       if (!ok) break;
-      // combine the planes: T = sum_i q_i 2^(10 (np - 1 - i)), the element is
-      // T 2^(exA + exB - 5 (2 np + 1))
-      const int r = U.mt * 256 + (int)rank * 128 + row;
-      const int n0 = U.nt * 256 + cbeg;
-      const int ncols = min(128, g.N - n0);
-      if (r < g.M && ncols > 0) {
-        const int ea = g.exA[r];
-        const int h = min(np, 3);
-        double* crow = g.C + (g.ksplit > 1 ? (size_t)U.z * g.M * g.N : 0) + r + (long long)n0 * g.ldc;
+      if (!split && r < g.M) {
 #pragma unroll 1
         for (int c0 = 0; c0 < ncols; c0 += 4) {
-          int qv[4][MAXPASS];
+          int4 qv[MAXPASS];
 #pragma unroll
-          for (int j = 0; j < 4; j++)
-#pragma unroll
-            for (int i = 0; i < MAXPASS; i++) qv[j][i] = (i < np && U.nk > 0) ? plane0[i * PLANE + (c0 + j) * 128] : 0;
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const int c = c0 + j;
-            if (c >= ncols) break;
-            if (g.lower_tiles && r < n0 + c) continue;
-            long long W = 0, V = 0;
-#pragma unroll
-            for (int i = 0; i < MAXPASS; i++) {
-              if (i < h) W = W * 1024 + qv[j][i];
-              else if (i < np) V = V * 1024 + qv[j][i];
-            }
-            const __int128 T = ((__int128)W << (10 * (np - h))) + V;
-            const int eb = g.exB[n0 + c];
-            double v;
-            if (ea == BAD_ROW || eb == BAD_ROW) v = __longlong_as_double(0x7ff8000000000000ll);
-            else v = i128_to_double(T, ea + eb - 5 * (2 * np + 1));
-            double* cp = crow + (long long)c * g.ldc;
-            if (g.alpha != 1.0) v = g.alpha == -1.0 ? -v : v * g.alpha;
-            if (g.beta != 0.0) v = fma(g.beta, *cp, v);
-            *cp = v;
-          }
+          for (int i = 0; i < MAXPASS; i++)
+            qv[i] = (i < np && U.nk > 0) ? plane0[i * PLANE4 + c0 / 4 * 128] : make_int4(0, 0, 0, 0);
+          store_four(g, qv, np, r, n0 + c0);
         }
       }
       __syncwarp();
@@ -493,18 +545,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
   }
 }
 
-// C = alpha * sum_z P_z + beta * C, z ascending (P_z: M x N, ld M)
-__global__ void __launch_bounds__(256) digit_split_sum_kernel(int M, int N, int splits, const double* __restrict__ P,
-                                                              double alpha, double beta, double* __restrict__ C,
-                                                              long long ldc) {
-  const long long total = (long long)M * N;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    double v = 0.0;
-    for (int z = 0; z < splits; z++) v += P[e + (long long)z * total];
-    double* c = C + e % M + (e / M) * ldc;
-    *c = beta != 0.0 ? fma(beta, *c, alpha * v) : alpha * v;
+// Split form: the planes of a tile's level pairs and K parts, four columns of a
+// row per thread; the parts are added as integers, exactly.
+__global__ void __launch_bounds__(256) digit_combine_kernel(const __grid_constant__ DgArgs g) {
+  const int t = blockIdx.x / (2 * PLANE4 / 256);
+  const int e = (blockIdx.x % (2 * PLANE4 / 256)) * 256 + threadIdx.x;  // int4 of the tile: rank, column / 4, row
+  Unit U;
+  dg_tile(g, t, U);
+  const int r = U.mt * 256 + e / PLANE4 * 128 + e % 128, c = U.nt * 256 + (e % PLANE4) / 128 * 4;
+  if (r >= g.M || c >= (g.lower_tiles ? min(g.N, r + 1) : g.N)) return;
+  int4 q[MAXPASS];
+  int slot = t * g.zsum;
+#pragma unroll
+  for (int i = MAXPASS - 1; i >= 0; i--) {
+    q[i] = make_int4(0, 0, 0, 0);
+    if (i < U.i1) {
+      for (int z = 0; z < g.zs[i] && z * g.kper[i] < U.nk; z++) {
+        const int4 v = g.planes[(2 * (size_t)(slot + z)) * PLANE4 + e];
+        q[i] = make_int4(q[i].x + v.x, q[i].y + v.y, q[i].z + v.z, q[i].w + v.w);
+      }
+    }
+    slot += g.zs[i];
   }
+  store_four(g, q, U.i1, r, c);
 }
 
 // ------------------------------------------------------------------- digits
@@ -542,8 +605,6 @@ __device__ __forceinline__ uint32_t digit_word(const uint64_t (&u)[4], const uin
   const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(f[2], f[3]), __NV_SATFINITE, __NV_E4M3);
   return lo | (hi << 16);
 }
-// exponent of a row's scale from the largest biased exponent in it
-__device__ __forceinline__ int row_exponent(int top) { return top == 0x7ff ? BAD_ROW : top - 1021; }
 __device__ __forceinline__ int digits_used(unsigned long long bits) {  // of the OR of a row's fixed-point magnitudes
   return bits ? ND - (__ffsll((long long)bits) - 1) / 5 : 0;
 }
@@ -576,9 +637,8 @@ __global__ void __launch_bounds__(256) cut_contig_kernel(const double* __restric
     __syncthreads();
     for (int q = 0; q < 8; q++) top = max(top, stop[q]);
   }
-  const int e = row_exponent(top);
-  if (l == 0) ex[r] = e;
-  const int es = e == BAD_ROW ? 1024 : e;  // finite digits in a bad row too
+  if (l == 0) ex[r] = top;
+  const int es = row_exponent(top);
   unsigned long long bits = 0;
   for (int g = l; g < Kpad / 4; g += TPR) {
     uint64_t u[4];
@@ -603,43 +663,61 @@ __global__ void __launch_bounds__(256) cut_contig_kernel(const double* __restric
   if (l == 0) atomicMax(nd + (r >> 8), digits_used(bits));
 }
 
-// 32 rows per CTA, elements contiguous over the rows: digits of 32 x 64 tiles
-// turned in shared memory, so that both the loads (256 bytes a warp) and the
-// stores (64 bytes a row and plane) are coalesced.
-__global__ void __launch_bounds__(256) cut_strided_kernel(const double* __restrict__ X, long long ld, int rows, int K,
-                                                          int Kpad, uint8_t* __restrict__ D, int* __restrict__ ex,
-                                                          int* __restrict__ nd) {
-  __shared__ uint32_t t[ND][32][17];
+// Largest biased exponent of each row of a matrix whose elements are contiguous
+// over the rows: 32 rows and a slice of K a CTA, into ex (zero before).
+__global__ void __launch_bounds__(256) strided_top_kernel(const double* __restrict__ X, long long ld, int rows, int K,
+                                                          int slice, int* __restrict__ ex) {
   __shared__ int stop[8][32];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int r = blockIdx.x * 32 + lane, k1 = min(K, ((int)blockIdx.y + 1) * slice);
+  int top = 0;
+  if (r < rows) {
+#pragma unroll 4
+    for (int k = blockIdx.y * slice + wp; k < k1; k += 8)
+      top = max(top, (int)((__double_as_longlong(X[r + (long long)k * ld]) >> 52) & 0x7ff));
+  }
+  stop[wp][lane] = top;
+  __syncthreads();
+  if (wp == 0 && r < rows) {
+    for (int q = 1; q < 8; q++) top = max(top, stop[q][lane]);
+    atomicMax(ex + r, top);
+  }
+}
+
+// Digits of such a matrix, ex holding its rows' exponents: 32 x 64 tiles turned
+// in shared memory, so that both the loads (256 bytes a warp) and the stores (64
+// bytes a row and plane) are coalesced; 32 rows and a slice of K (a multiple of
+// 64) a CTA.  (One CTA per 32 rows for all of K: 0.62 ms for 6000 x 6000.)
+__global__ void __launch_bounds__(256) cut_strided_kernel(const double* __restrict__ X, long long ld, int rows, int K,
+                                                          int Kpad, int slice, uint8_t* __restrict__ D,
+                                                          const int* __restrict__ ex, int* __restrict__ nd) {
+  __shared__ uint32_t t[ND][32][17];
   __shared__ unsigned long long sbits[8];
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   const int r0 = blockIdx.x * 32, r = r0 + lane;
   const double* x = X + r;
-  int top = 0;
-  if (r < rows)
-    for (int k = wp; k < K; k += 8) top = max(top, (int)((__double_as_longlong(x[(long long)k * ld]) >> 52) & 0x7ff));
-  stop[wp][lane] = top;
-  __syncthreads();
-  for (int q = 0; q < 8; q++) top = max(top, stop[q][lane]);
-  const int e = row_exponent(top);
-  if (wp == 0 && r < rows) ex[r] = e;
-  const int es = e == BAD_ROW ? 1024 : e;
+  const int es = row_exponent(r < rows ? ex[r] : 0);
+  const int kend = min(Kpad, ((int)blockIdx.y + 1) * slice);
   unsigned long long bits = 0;
-  for (int k0 = 0; k0 < Kpad; k0 += 64) {
+  for (int k0 = blockIdx.y * slice; k0 < kend; k0 += 64) {
+    double v[8];
 #pragma unroll
-    for (int h = 0; h < 2; h++) {  // two groups of four elements a thread
-      const int g = wp * 2 + h;
+    for (int j = 0; j < 8; j++) {  // two groups of four elements a thread
+      const int k = k0 + 8 * wp + j;
+      v[j] = (r < rows && k < K) ? x[(long long)k * ld] : 0.0;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
       uint64_t u[4];
       uint32_t sg[4];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        const int k = k0 + 4 * g + j;
-        const unsigned long long f = to_fixed((r < rows && k < K) ? x[(long long)k * ld] : 0.0, es, sg[j]);
+        const unsigned long long f = to_fixed(v[4 * h + j], es, sg[j]);
         bits |= f;
         u[j] = f + DIGIT_BIAS;
       }
 #pragma unroll
-      for (int s = 0; s < ND; s++) t[s][lane][g] = digit_word(u, sg, s);
+      for (int s = 0; s < ND; s++) t[s][lane][2 * wp + h] = digit_word(u, sg, s);
     }
     __syncthreads();
     // 12 planes x 32 rows of 16 words: two rows a warp and step
@@ -718,10 +796,8 @@ int dg_clusters() {
 
 struct DigitGemm {
   int clusters = 0;
-  int* planes = nullptr;
+  int4* planes = nullptr;      // MAXPASS planes a CTA, or one a unit and CTA in the split form
   int* err = nullptr;
-  double* part = nullptr;
-  size_t part_elems = 0;
   void* op[2] = {nullptr, nullptr};
   size_t op_bytes[2] = {0, 0};
 };
@@ -745,10 +821,18 @@ DigitMat digit_mat_at(void* mem, int rows, int K) {
 namespace {
 cudaError_t cut(cudaStream_t s, const DigitMat& m, const double* X, long long ld, bool kcontig, int w) {
   if (m.rows <= 0 || m.K <= 0 || m.prow != m.rows) return cudaErrorInvalidValue;
-  FGLS_CUDA_TRY(cudaMemsetAsync(m.nd, 0, sizeof(int) * ((m.rows + 255) / 256), s));
-  if (!kcontig)
-    cut_strided_kernel<<<ceil_div(m.rows, 32), 256, 0, s>>>(X, ld, m.rows, m.K, m.Kpad, m.d, m.ex, m.nd);
-  else if (m.K <= 1024)
+  // nd and, behind it, ex
+  FGLS_CUDA_TRY(cudaMemsetAsync(m.nd, 0, sizeof(int) * ((m.rows + 255) / 256 + (kcontig ? 0 : m.rows)), s));
+  if (!kcontig) {
+    // slices of K: about four CTAs an SM
+    const int blocks = ceil_div(m.rows, 32);
+    const int want = std::max(1, std::min(ceil_div(608, blocks), m.Kpad / 64));
+    const int slice = ceil_div(m.Kpad / 64, want) * 64;
+    const dim3 grid(blocks, ceil_div(m.Kpad, slice));
+    strided_top_kernel<<<grid, 256, 0, s>>>(X, ld, m.rows, m.K, slice, m.ex);
+    cut_strided_kernel<<<grid, 256, 0, s>>>(X, ld, m.rows, m.K, m.Kpad, slice, m.d, m.ex, m.nd);
+    note_launch();
+  } else if (m.K <= 1024)
     cut_contig_kernel<32><<<ceil_div(m.rows, 8), 256, 0, s>>>(X, ld, m.rows, m.K, m.Kpad, w, m.d, m.ex, m.nd);
   else
     cut_contig_kernel<256><<<m.rows, 256, 0, s>>>(X, ld, m.rows, m.K, m.Kpad, w, m.d, m.ex, m.nd);
@@ -771,7 +855,7 @@ cudaError_t digit_gemm_create(DigitGemm** out) {
   if (n <= 0 || !encoder()) return cudaErrorNotSupported;
   DigitGemm* g = new DigitGemm();
   g->clusters = n;
-  cudaError_t r = cudaMalloc(&g->planes, sizeof(int) * (size_t)MAXPASS * PLANE * 2 * n);
+  cudaError_t r = cudaMalloc(&g->planes, sizeof(int4) * (size_t)MAXPASS * PLANE4 * 2 * n);
   if (r == cudaSuccess) r = cudaMalloc(&g->err, sizeof(int));
   if (r == cudaSuccess) r = cudaMemset(g->err, 0, sizeof(int));
   if (r == cudaSuccess) r = cudaDeviceSynchronize();  // the memset ran on the default stream
@@ -785,7 +869,7 @@ cudaError_t digit_gemm_create(DigitGemm** out) {
 
 void digit_gemm_destroy(DigitGemm* g) {
   if (!g) return;
-  void* ptrs[] = {g->planes, g->err, g->part, g->op[0], g->op[1]};
+  void* ptrs[] = {g->planes, g->err, g->op[0], g->op[1]};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete g;
@@ -820,35 +904,32 @@ cudaError_t digit_mul(DigitGemm* g, cudaStream_t s, const DigitMat& A, const Dig
     a.kb0 = kb;
     a.nk = std::min(K_MAX_STEPS, nk_all - kb);
     a.beta = kb > 0 ? 1.0 : beta;
-    // few tiles: split K over the idle clusters, at least four K-steps each
-    int z = 1;
-    if (!o.a_lower && !o.c_lower && 2 * tiles <= g->clusters) z = std::min(g->clusters / tiles, a.nk / 4);
-    const size_t elems = (size_t)a.M * a.N;
-    if (z > 1 && g->part_elems < elems * z) {
-      if (g->part) cudaFree(g->part);
-      g->part = nullptr;
-      g->part_elems = 0;
-      if (cudaMalloc(&g->part, sizeof(double) * elems * z) == cudaSuccess) g->part_elems = elems * z;
-      else (void)cudaGetLastError();
-    }
-    if (z < 2 || g->part_elems < elems * z) z = 1;
-    a.kper = ceil_div(a.nk, z);
-    a.ksplit = ceil_div(a.nk, a.kper);
     a.C = C;
     a.ldc = ldc;
-    DgArgs b = a;
-    if (a.ksplit > 1) {
-      b.alpha = 1.0;
-      b.beta = 0.0;
-      b.C = g->part;
-      b.ldc = a.M;
+    // Few tiles for the clusters: level pairs become units of their own, the
+    // larger ones (2 i + 3 stages a K-step) cut along K into parts of at most
+    // an even share, as long as the planes of six per cluster hold them.
+    a.zsum = 0;
+    if (tiles <= SPLIT_TILES * g->clusters) {
+      const long long all = (long long)MAXPASS * (MAXPASS + 2) * a.nk * tiles;  // stages of the product
+      long long share = std::max(24LL, (all + g->clusters - 1) / g->clusters);
+      for (;; share += share / 4) {
+        a.zsum = 0;
+        for (int i = 0; i < MAXPASS; i++) {
+          const int st = (2 * i + 3) * a.nk;
+          a.kper[i] = ceil_div(a.nk, std::min<long long>(a.nk, (st + share - 1) / share));
+          a.zs[i] = ceil_div(a.nk, a.kper[i]);
+          a.zsum += a.zs[i];
+        }
+        if ((long long)a.zsum * tiles <= (long long)MAXPASS * g->clusters || a.zsum == MAXPASS) break;
+      }
+      if ((long long)a.zsum * tiles > (long long)MAXPASS * g->clusters) a.zsum = 0;
     }
-    const int cl = std::max(1, std::min(g->clusters, tiles * a.ksplit));
-    digit_gemm_kernel<<<2 * cl, NTHREADS, SMEM, s>>>(ma, mb, b);
+    const int units = tiles * std::max(1, a.zsum);
+    digit_gemm_kernel<<<2 * std::min(g->clusters, units), NTHREADS, SMEM, s>>>(ma, mb, a);
     note_launch();
-    if (a.ksplit > 1) {
-      digit_split_sum_kernel<<<(int)std::min<long long>((elems + 255) / 256, 152LL * 16), 256, 0, s>>>(
-          a.M, a.N, a.ksplit, g->part, a.alpha, a.beta, C, ldc);
+    if (a.zsum) {
+      digit_combine_kernel<<<tiles * (2 * PLANE4 / 256), 256, 0, s>>>(a);
       note_launch();
     }
     FGLS_CUDA_TRY(cudaGetLastError());
@@ -856,20 +937,23 @@ cudaError_t digit_mul(DigitGemm* g, cudaStream_t s, const DigitMat& A, const Dig
   return cudaSuccess;
 }
 
-// Estimates in microseconds, from measured products of 64 .. 10000 rows:
-//   FP64 kernel: 64 x 64 tiles, one wave of up to 152 takes 1.0 us per element
-//     of K (300 x 513 x 5000: 5.06 ms; 4096 x 4096 x 5000: 134.6 ms);
-//   digits: five launches (40 us), cutting at 6 ps an element, 0.16 us per
-//     element of K and wave of 76 tiles of 256 x 256, K split when there are
-//     fewer (300 x 513 x 5000: 0.31 ms; 4096 x 4096 x 5000: 4.2 ms).
-// They cross near K = 60 for one tile; 256 x 256 x 128 measures 0.16 ms both ways.
+// Estimates in microseconds, from measured products:
+//   FP64 kernels: an SM takes 1.0 us per element of K for a 64 x 64 tile (a wave
+//     of up to 152; 4096 x 4096 x 5000: 134.6 ms), 0.064 us for a 32 x 8 tile
+//     (used below a wave of the others);
+//   digits: five launches (60 us), cutting at 6 ps an element, 0.16 us per
+//     element of K and wave of 76 tiles of 256 x 256, shared out evenly below a
+//     wave, and 50 us a wave for the epilogue beyond it (301 x 74 x 301: 80 us;
+//     5000 x 256 x 5000: 0.53 ms; 4096 x 4096 x 64: 0.43 ms, FP64 1.77 ms).
 bool digit_gemm_pays(long long M, long long N, long long K) {
+  const double k = (double)K;
   const double t64 = (double)((M + 63) / 64) * (double)((N + 63) / 64);
+  const double t32 = (double)((M + 31) / 32) * (double)((N + 7) / 8);
   const double t256 = (double)((M + 255) / 256) * (double)((N + 255) / 256);
-  const double fp64 = std::max(1.0, t64 / 152.0) * (double)K;
-  const double waves = t256 < 38.0 ? std::max(t256 / 76.0, 512.0 / (double)std::max(K, 512LL)) : std::ceil(t256 / 76.0);
-  const double digits = 40.0 + 6e-6 * (double)(M + N) * (double)K + 0.16 * (double)K * waves;
-  return K >= 64 && digits < fp64;
+  const double fp64 = t64 < 152.0 ? 5.0 + 0.064 * k * std::max(1.0, t32 / 152.0) : k * t64 / 152.0;
+  const double waves = t256 <= 76.0 ? t256 / 76.0 : std::ceil(t256 / 76.0);
+  const double digits = 60.0 + 6e-6 * (double)(M + N) * k + 0.16 * k * waves + (t256 > 76.0 ? 50.0 * waves : 0.0);
+  return digits < fp64;
 }
 
 namespace {

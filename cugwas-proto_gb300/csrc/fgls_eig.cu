@@ -12,8 +12,8 @@
 //     per column.
 //  2. Eigenpairs of the tridiagonal by divide and conquer (fgls_dc.cu):
 //     eigenvalues ascending, eigenvectors V of T.
-//  3. Z = H_0 H_1 ... H_{n-3} V applied in blocks of 256 reflectors in
-//     compact-WY form (Y, T from tau and Y^T Y): DGEMMs only.
+//  3. Z = H_0 H_1 ... H_{n-3} V applied in blocks of 512 reflectors in
+//     compact-WY form (Y, T from tau and Y^T Y): products only.
 #include <algorithm>
 #include <cfloat>
 #include <cstdio>
@@ -448,7 +448,7 @@ cudaError_t dsyev_device(cudaStream_t s, DigitGemm* dg, int n, const double* Phi
   // 3. eigenpairs of T by divide and conquer (fgls_dc.cu) into Z; A keeps the reflectors
   // one workspace for the divide and conquer, then for the back-transform
   // (Y: n x NBT, G, T: NBT x NBT, W, W2: NBT x n)
-  constexpr int NBT = 256;
+  constexpr int NBT = 512;  // K of the widest product; the back-transform at n = 5000: 35 ms with 256, 18 with 512
   const size_t bt_bytes = sizeof(double) * ((size_t)3 * NBT * n + (size_t)2 * NBT * NBT);
   void* dcw = nullptr;
   FGLS_CUDA_TRY(cudaMalloc(&dcw, std::max(dc_workspace_bytes(n), bt_bytes)));

@@ -80,7 +80,7 @@ struct fglsgpu_engine {
   DigitMat zdig, ayldig, ddig;  // eigen: Z^T, AYL^T, dinv^T rows
   // chol: the selected trait's L^-1 (null: no memory for it, the blocks then
   // run a blocked TRSM) and its rows' digits (valid when linv_cut), 64 x 64 scratch
-  double *dLinv = nullptr, *ddiag = nullptr;
+  double *dLinv = nullptr, *ddiag = nullptr, *dWraw = nullptr;
   DigitMat ldig;
   bool linv_cut = false;
   void *zmem = nullptr, *wmem = nullptr, *blkmem = nullptr;
@@ -173,7 +173,7 @@ void free_all(fglsgpu_engine* e) {
                   e->dQ,   e->dGYL, e->dGR,  e->dB[0], e->dB[1], e->dV[0], e->dV[1], e->dU8, e->dst,
                   e->aWc, e->aAYLc, e->aAYLs, e->atopc, e->atops, e->areml, e->aGYLc, e->aGYLs, e->aGRc,
                   e->aGRs, e->acontrib, e->ag, e->agR, e->aacc, e->aU, e->aV2, e->dSE[0], e->dSE[1], e->dP[0],
-                  e->dP[1], e->dXw, e->zmem, e->wmem, e->blkmem, e->dLinv, e->ddiag};
+                  e->dP[1], e->dXw, e->zmem, e->wmem, e->blkmem, e->dLinv, e->ddiag, e->dWraw};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (e->hst) cudaFreeHost(e->hst);
@@ -677,6 +677,7 @@ int fglsgpu_create(const fglsgpu_config* cfg, fglsgpu_engine** out) {
     chk(dalloc(&e->dWY, n * (1 + wXL)));
     chk(dalloc(&e->dWork, n * xb * wXR));
     chk(dalloc(&e->ddiag, 64 * 64));
+    chk(dalloc(&e->dWraw, n * (1 + wXL)));
   } else {
     chk(dalloc(&e->dL, n * n));  // eigensolver scratch
     chk(dalloc(&e->dZ, n * n));
@@ -803,15 +804,11 @@ int fglsgpu_select_trait(fglsgpu_engine* e, int j) {
   bool digits = false;
   rc = chol_digits(e, split(e) ? std::min((long long)TUNE_SNPS, (long long)c.x_b) : (long long)c.x_b * c.wXR, &digits);
   if (rc) return rc;
-  if (digits && c.n >= 1024) {
-    // whitening as a product: four columns cost one tile column, the solve a
-    // chain of 128-column steps (24 ms at n = 10000)
-    DigitMat w = digit_gemm_operand(e->dg, 0, 1 + c.wXL, c.n);
-    if (!w.d) return fail(e, FGLSGPU_ENOMEM, "no memory for the whitening");
-    DigitMulOpts lower;
-    lower.a_lower = true;
-    ENG_TRY(e, digit_cut(s, w, e->dWY, n, true), "whiten y, XL");
-    ENG_TRY(e, digit_mul(e->dg, s, e->ldig, w, 1.0, 0.0, e->dWY, n, lower), "whiten y, XL");
+  if (e->dLinv && !e->dg_off) {
+    // whitening as a product with L^-1: the solve is a chain of 128-column steps
+    // (24 ms at n = 10000, 2.2 ms at n = 1000)
+    ENG_TRY(e, cudaMemcpyAsync(e->dWraw, e->dWY, sizeof(double) * n * (1 + c.wXL), cudaMemcpyDeviceToDevice, s), "copy");
+    ENG_TRY(e, lower_mul(s, false, c.n, 1 + c.wXL, e->dLinv, e->dWraw, e->dWY), "whiten y, XL");
   } else {
     ENG_TRY(e, dtrsm_llnn(s, c.n, 1 + c.wXL, e->dL, n, e->dWY, n), "whiten y, XL");
   }
@@ -821,7 +818,7 @@ int fglsgpu_select_trait(fglsgpu_engine* e, int j) {
   if (split(e)) {
     if (!e->oz) ENG_TRY(e, ozaki_create(&e->oz, c.n, 1, c.wXL, c.wXR, c.x_b, c.slices, /*eigen=*/0), "split plan");
     ozaki_set_wait_limit(e->oz, e->wait_ns);
-    ENG_TRY(e, ozaki_set_chol(e->oz, s, e->dg, e->dLinv, e->dWY), "split operands");
+    ENG_TRY(e, ozaki_set_chol(e->oz, s, e->dLinv, e->dWY), "split operands");
     ENG_TRY(e, cudaStreamSynchronize(s), "split operands");
     e->trait_sel = j;
     rc = tune_slices(e);

@@ -2233,10 +2233,10 @@ cudaError_t ozaki_set_eigen(OzakiPlan* p, cudaStream_t s, DigitGemm* dg, const d
   return cudaGetLastError();
 }
 
-cudaError_t ozaki_set_chol(OzakiPlan* p, cudaStream_t s, DigitGemm* dg, const double* Linv, const double* WY) {
+cudaError_t ozaki_set_chol(OzakiPlan* p, cudaStream_t s, const double* Linv, const double* WY) {
   const int n = p->n;
   // U = L^-T [y~ | XL~]
-  FGLS_CUDA_TRY(digit_dgemm(dg, s, true, false, n, p->nU, n, 1.0, Linv, n, WY, n, 0.0, p->U, n));
+  FGLS_CUDA_TRY(lower_mul(s, true, n, p->nU, Linv, WY, p->U));
   // rows of L^-1 contiguous: transpose, then slice
   dim3 tg((n + 31) / 32, (n + 31) / 32);
   transpose_kernel<<<tg, dim3(32, 8), 0, s>>>(n, Linv, p->LinvT);
@@ -2295,10 +2295,10 @@ int split_rows_padded(int rows) { return (rows + BM - 1) / BM * BM; }
 int split_k_padded(int n) { return (n + KALIGN - 1) / KALIGN * KALIGN; }
 int split_cols_padded(int x) { return (x + BN - 1) / BN * BN; }
 
-cudaError_t split_chol_operand(cudaStream_t s, DigitGemm* dg, int n, int wXL, const double* Linv, const double* WY, int S,
+cudaError_t split_chol_operand(cudaStream_t s, int n, int wXL, const double* Linv, const double* WY, int S,
                                int Mpad, int Kpad, uint8_t* A, double* scale, double* LinvT, double* U) {
   const int nU = 1 + wXL;
-  FGLS_CUDA_TRY(digit_dgemm(dg, s, true, false, n, nU, n, 1.0, Linv, n, WY, n, 0.0, U, n));
+  FGLS_CUDA_TRY(lower_mul(s, true, n, nU, Linv, WY, U));
   dim3 tg((n + 31) / 32, (n + 31) / 32);
   transpose_kernel<<<tg, dim3(32, 8), 0, s>>>(n, Linv, LinvT);
   note_launch();

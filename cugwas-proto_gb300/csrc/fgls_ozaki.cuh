@@ -17,12 +17,12 @@ struct OzakiPlan;
 cudaError_t ozaki_create(OzakiPlan** out, int n, int t, int wXL, int wXR, int x_b, int slices, int eigen);
 void ozaki_destroy(OzakiPlan* p);
 // eigen: Z (n x n), AYL (n x t(1+wXL)), dinv (n x t)
-// (dg, here and below: digit products for the FP64 operand setup; may be null)
+// (dg: digit products for the FP64 operand setup; may be null)
 struct DigitGemm;
 cudaError_t ozaki_set_eigen(OzakiPlan* p, cudaStream_t s, DigitGemm* dg, const double* Z, const double* AYL,
                             const double* dinv);
 // chol: L^-1 (n x n lower), WY = [y~ | XL~] (n x (1+wXL)) of the selected trait
-cudaError_t ozaki_set_chol(OzakiPlan* p, cudaStream_t s, DigitGemm* dg, const double* Linv, const double* WY);
+cudaError_t ozaki_set_chol(OzakiPlan* p, cudaStream_t s, const double* Linv, const double* WY);
 // A genotype block on the device in one of three formats (exactly one
 // pointer set): FP64 or bytes, n values per column, or 2-bit packed as a
 // SNP-major PLINK .bed body (ceil(n/4) bytes per column; a missing call sets
@@ -75,7 +75,7 @@ int split_cols_padded(int x);
 // [L^-1 ; (L^-T WY)^T] of one chol problem cut into S E4M3 five-bit digit slices at A
 // (S x Mpad x Kpad) with row scales; LinvT (n x n) and U (n x (1+wXL)) are
 // caller scratch.
-cudaError_t split_chol_operand(cudaStream_t s, DigitGemm* dg, int n, int wXL, const double* Linv, const double* WY, int S,
+cudaError_t split_chol_operand(cudaStream_t s, int n, int wXL, const double* Linv, const double* WY, int S,
                                int Mpad, int Kpad, uint8_t* A, double* scale, double* LinvT, double* U);
 // row scales of the first S slices of an operand cut into S_built slices
 cudaError_t split_rescale_rows(cudaStream_t s, int rows, const double* built_scale, int S_built, int S,

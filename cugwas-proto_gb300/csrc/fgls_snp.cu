@@ -187,55 +187,71 @@ __global__ void __launch_bounds__(256) eigen_trait_kernel(int n, int t, int wXL,
   }
 }
 
-// Skinny Gram for the chol variant (one trait).  X: n x (x*wXR) whitened SNP
-// columns; C = [y~ | XL~] (n x (1+wXL)).  One warp per SNP (its wXR columns),
-// 8 warps per CTA share a shared-memory copy of a 256-row chunk of C.
+// Skinny Gram for the chol variant (one trait).  X: n x (x*WR) whitened SNP
+// columns; C = [y~ | XL~] (n x NC, NC = 1 + wXL).  One warp per SNP (its WR
+// columns), 8 warps per CTA share a shared-memory copy of a 256-row chunk of C.
+// The sums stay in registers (sizes are template arguments; indexed at run time
+// they went through local memory: 57 us for 37 SNPs at n = 301, now 20).
 constexpr int SG_ROWS = 256;
-__global__ void __launch_bounds__(256) gram_skinny_kernel(int n, int x, int wXL, int wXR,
-                                                          const double* __restrict__ X, long long ldx,
+template <int NC, int WR>
+__global__ void __launch_bounds__(256) gram_skinny_kernel(int n, int x, const double* __restrict__ X, long long ldx,
                                                           const double* __restrict__ C,
                                                           double* __restrict__ GYL, double* __restrict__ GR) {
-  __shared__ double Cs[SG_ROWS * (FGLS_MAX_P + 1)];
-  const int nc = 1 + wXL;
+  __shared__ double Cs[SG_ROWS * NC];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int snp = blockIdx.x * 8 + warp;
   const bool active = snp < x;
-  double acc_c[FGLS_MAX_WXR][FGLS_MAX_P + 1];
-  double acc_r[FGLS_MAX_WXR][FGLS_MAX_WXR];
-  for (int c = 0; c < FGLS_MAX_WXR; c++) {
-    for (int q = 0; q <= FGLS_MAX_P; q++) acc_c[c][q] = 0.0;
-    for (int d = 0; d < FGLS_MAX_WXR; d++) acc_r[c][d] = 0.0;
+  double acc_c[WR][NC], acc_r[WR][WR];
+#pragma unroll
+  for (int c = 0; c < WR; c++) {
+#pragma unroll
+    for (int q = 0; q < NC; q++) acc_c[c][q] = 0.0;
+#pragma unroll
+    for (int d = 0; d < WR; d++) acc_r[c][d] = 0.0;
   }
+  const double* xs = X + (long long)snp * WR * ldx;
   for (int l0 = 0; l0 < n; l0 += SG_ROWS) {
     const int rows = min(SG_ROWS, n - l0);
+    // this warp's genotype rows are in flight while the chunk of C is copied
+    double xv[SG_ROWS / 32][WR];
+#pragma unroll
+    for (int k = 0; k < SG_ROWS / 32; k++)
+#pragma unroll
+      for (int c = 0; c < WR; c++) {
+        const int r = lane + 32 * k;
+        xv[k][c] = active && r < rows ? xs[(l0 + r) + c * ldx] : 0.0;
+      }
     __syncthreads();
-    for (int e = threadIdx.x; e < rows * nc; e += blockDim.x) {
-      int r = e % rows, q = e / rows;
-      Cs[q * SG_ROWS + r] = C[(l0 + r) + (long long)q * n];
-    }
+#pragma unroll
+    for (int q = 0; q < NC; q++)
+      Cs[q * SG_ROWS + threadIdx.x] = (int)threadIdx.x < rows ? C[(l0 + threadIdx.x) + (long long)q * n] : 0.0;
     __syncthreads();
-    if (!active) continue;
-    for (int r = lane; r < rows; r += 32) {
-      double xv[FGLS_MAX_WXR];
-      for (int c = 0; c < wXR; c++) xv[c] = X[(l0 + r) + (long long)(snp * wXR + c) * ldx];
-      for (int c = 0; c < wXR; c++) {
-        for (int q = 0; q < nc; q++) acc_c[c][q] = fma(xv[c], Cs[q * SG_ROWS + r], acc_c[c][q]);
-        for (int d = 0; d <= c; d++) acc_r[c][d] = fma(xv[c], xv[d], acc_r[c][d]);
+#pragma unroll
+    for (int k = 0; k < SG_ROWS / 32; k++) {
+#pragma unroll
+      for (int c = 0; c < WR; c++) {
+#pragma unroll
+        for (int q = 0; q < NC; q++) acc_c[c][q] = fma(xv[k][c], Cs[q * SG_ROWS + lane + 32 * k], acc_c[c][q]);
+#pragma unroll
+        for (int d = 0; d <= c; d++) acc_r[c][d] = fma(xv[k][c], xv[k][d], acc_r[c][d]);
       }
     }
   }
   if (!active) return;
-  const long long ld = (long long)x * wXR;
-  for (int c = 0; c < wXR; c++) {
-    for (int q = 0; q < nc; q++) {
-      double v = warp_sum(acc_c[c][q]);
-      if (lane == 0) GYL[(snp * wXR + c) + q * ld] = v;
+  const long long ld = (long long)x * WR;
+#pragma unroll
+  for (int c = 0; c < WR; c++) {
+#pragma unroll
+    for (int q = 0; q < NC; q++) {
+      const double v = warp_sum(acc_c[c][q]);
+      if (lane == 0) GYL[(snp * WR + c) + q * ld] = v;
     }
+#pragma unroll
     for (int d = 0; d <= c; d++) {
-      double v = warp_sum(acc_r[c][d]);
+      const double v = warp_sum(acc_r[c][d]);
       if (lane == 0) {
-        GR[((long long)(snp * wXR + c)) * wXR + d] = v;
-        GR[((long long)(snp * wXR + d)) * wXR + c] = v;
+        GR[((long long)(snp * WR + c)) * WR + d] = v;
+        GR[((long long)(snp * WR + d)) * WR + c] = v;
       }
     }
   }
@@ -619,9 +635,35 @@ cudaError_t eigen_traits(cudaStream_t s, int n, int t, int wXL, const double* W,
   return cudaGetLastError();
 }
 
+namespace {
+template <int NC, int WR>
+void launch_gram_skinny(cudaStream_t s, int n, int x, const double* X, long long ldx, const double* C, double* GYL,
+                        double* GR) {
+  if constexpr (NC - 1 + WR <= FGLS_MAX_P)
+    gram_skinny_kernel<NC, WR><<<ceil_div(x, 8), 256, 0, s>>>(n, x, X, ldx, C, GYL, GR);
+}
+template <int WR>
+void gram_skinny_cols(cudaStream_t s, int nc, int n, int x, const double* X, long long ldx, const double* C, double* GYL,
+                      double* GR) {
+  switch (nc) {
+    case 2: launch_gram_skinny<2, WR>(s, n, x, X, ldx, C, GYL, GR); break;
+    case 3: launch_gram_skinny<3, WR>(s, n, x, X, ldx, C, GYL, GR); break;
+    case 4: launch_gram_skinny<4, WR>(s, n, x, X, ldx, C, GYL, GR); break;
+    case 5: launch_gram_skinny<5, WR>(s, n, x, X, ldx, C, GYL, GR); break;
+    case 6: launch_gram_skinny<6, WR>(s, n, x, X, ldx, C, GYL, GR); break;
+    case 7: launch_gram_skinny<7, WR>(s, n, x, X, ldx, C, GYL, GR); break;
+    default: launch_gram_skinny<8, WR>(s, n, x, X, ldx, C, GYL, GR); break;
+  }
+}
+}  // namespace
+
 cudaError_t gram_skinny(cudaStream_t s, int n, int x, int wXL, int wXR, const double* X, long long ldx,
                         const double* C, double* GYL, double* GR) {
-  gram_skinny_kernel<<<ceil_div(x, 8), 256, 0, s>>>(n, x, wXL, wXR, X, ldx, C, GYL, GR);
+  if (wXL < 1 || wXR < 1 || wXR > FGLS_MAX_WXR || wXL + wXR > FGLS_MAX_P) return cudaErrorInvalidValue;
+  if (wXR == 1) gram_skinny_cols<1>(s, 1 + wXL, n, x, X, ldx, C, GYL, GR);
+  else if (wXR == 2) gram_skinny_cols<2>(s, 1 + wXL, n, x, X, ldx, C, GYL, GR);
+  else if (wXR == 3) gram_skinny_cols<3>(s, 1 + wXL, n, x, X, ldx, C, GYL, GR);
+  else gram_skinny_cols<4>(s, 1 + wXL, n, x, X, ldx, C, GYL, GR);
   note_launch();
   return cudaGetLastError();
 }
