@@ -251,6 +251,19 @@ long long geno_bytes_per_col(int fmt, int n) {
   return fmt == GENO_F64 ? 8LL * n : fmt == GENO_U8 ? (long long)n : (long long)(n + 3) / 4;
 }
 
+// Results of `rows` traits (width elements each, contiguous on the device) to a
+// host array with `pitch` elements between traits.  The last trait goes as a plain
+// copy: a strided copy into pageable memory touches its last row up to the pitch,
+// which ends past the caller's array when the block is not its first (a
+// segmentation fault where nothing is mapped there).
+cudaError_t download(double* dst, long long pitch, const double* src, long long width, int rows, cudaStream_t s) {
+  if (rows > 1)
+    FGLS_CUDA_TRY(cudaMemcpy2DAsync(dst, sizeof(double) * pitch, src, sizeof(double) * width, sizeof(double) * width,
+                                    rows - 1, cudaMemcpyDeviceToHost, s));
+  return cudaMemcpyAsync(dst + (rows - 1) * pitch, src + (rows - 1) * width, sizeof(double) * width,
+                         cudaMemcpyDeviceToHost, s);
+}
+
 // Device memory of `bytes` at *p, kept in *have; false when there is none.
 bool grow(void** p, size_t* have, size_t bytes) {
   if (*have >= bytes) return true;
@@ -888,11 +901,9 @@ int fglsgpu_run_block(fglsgpu_engine* e, const double* XR, int x_inc, double* B,
   rc = compute_block(e, e->dX[0], GENO_F64, x_inc, e->dB[0], e->dV[0], db, dv, 0);
   if (rc) return rc;
   const int nt = out_traits(e);
-  ENG_TRY(e, cudaMemcpy2DAsync(B, sizeof(double) * bstr, e->dB[0], sizeof(double) * db, sizeof(double) * db, nt,
-                               cudaMemcpyDeviceToHost, s),
+  ENG_TRY(e, download(B, bstr, e->dB[0], db, nt, s),
           "B download");
-  ENG_TRY(e, cudaMemcpy2DAsync(V, sizeof(double) * vstr, e->dV[0], sizeof(double) * dv, sizeof(double) * dv, nt,
-                               cudaMemcpyDeviceToHost, s),
+  ENG_TRY(e, download(V, vstr, e->dV[0], dv, nt, s),
           "V download");
   return check_status(e, "block");
 }
@@ -956,19 +967,15 @@ int run_snps_impl(fglsgpu_engine* e, const void* XR, int fmt, long long m, doubl
       ENG_TRY(e, snp_compact(e->comp, x, nt, p, e->dB[k], db, e->dV[k], dv, e->dSE[k], e->dP[k], db), "compact");
     ENG_TRY(e, cudaEventRecord(e->evC[k], e->comp), "event");
     ENG_TRY(e, cudaStreamWaitEvent(e->d2h, e->evC[k], 0), "wait");
-    ENG_TRY(e, cudaMemcpy2DAsync(B + ib * p, sizeof(double) * m * p, e->dB[k], sizeof(double) * db,
-                                 sizeof(double) * db, nt, cudaMemcpyDeviceToHost, e->d2h),
+    ENG_TRY(e, download(B + ib * p, m * p, e->dB[k], db, nt, e->d2h),
             "B download");
     if (!compact) {
-      ENG_TRY(e, cudaMemcpy2DAsync(V + ib * p * p, sizeof(double) * m * p * p, e->dV[k], sizeof(double) * dv,
-                                   sizeof(double) * dv, nt, cudaMemcpyDeviceToHost, e->d2h),
+      ENG_TRY(e, download(V + ib * p * p, m * p * p, e->dV[k], dv, nt, e->d2h),
               "V download");
     } else {
-      ENG_TRY(e, cudaMemcpy2DAsync(SE + ib * p, sizeof(double) * m * p, e->dSE[k], sizeof(double) * db,
-                                   sizeof(double) * db, nt, cudaMemcpyDeviceToHost, e->d2h),
+      ENG_TRY(e, download(SE + ib * p, m * p, e->dSE[k], db, nt, e->d2h),
               "SE download");
-      ENG_TRY(e, cudaMemcpy2DAsync(P + ib * p, sizeof(double) * m * p, e->dP[k], sizeof(double) * db,
-                                   sizeof(double) * db, nt, cudaMemcpyDeviceToHost, e->d2h),
+      ENG_TRY(e, download(P + ib * p, m * p, e->dP[k], db, nt, e->d2h),
               "P download");
     }
     ENG_TRY(e, cudaEventRecord(e->evD[k], e->d2h), "event");
