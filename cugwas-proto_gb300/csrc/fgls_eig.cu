@@ -3,13 +3,13 @@
 // 861-893).  W ascending, Z orthonormal columns.
 //
 // Algorithm (all FP64, no vendor library):
-//  1. Householder reduction to tridiagonal form on the lower triangle
-//     (A := H A H per column).  Each column's rank-2 update is deferred by
-//     one step: step k first applies update k-1 to column k (reflector
-//     kernel), then one pass over the trailing matrix applies update k-1 and
-//     forms A v_k by 32 x 32 lower tiles with a fixed-order reduction.
-//     Memory-bound: one read and one write of the trailing lower triangle
-//     per column.
+//  1. Householder reduction to tridiagonal form in panels of 64 columns (the
+//     scheme of LAPACK's dsytrd/dlatrd): within a panel a column is brought up to
+//     date from the panel's V and W, and A v runs over the trailing matrix as it
+//     was at the panel's start; then A -= V W^T + W V^T in one product of K = 128.
+//     A is kept in full storage, so that A v is one contiguous dot product per
+//     column; its power-of-two scale keeps V and W of one size (the product cuts
+//     rows of [V W] into digits under one scale).
 //  2. Eigenpairs of the tridiagonal by divide and conquer (fgls_dc.cu):
 //     eigenvalues ascending, eigenvectors V of T.
 //  3. Z = H_0 H_1 ... H_{n-3} V applied in blocks of 512 reflectors in
@@ -33,42 +33,54 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-__device__ double block_sum(double v, double* red) {
-  v = warp_sum(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double s = (l < (int)(blockDim.x >> 5)) ? red[l] : 0.0;
-    s = warp_sum(s);
-    if (l == 0) red[32] = s;
-  }
-  __syncthreads();
-  return red[32];
+// Largest |element| of the lower triangle, as the bits of a non-negative double
+// (ordered like integers; a NaN or an infinity is the largest), into *top.
+__global__ void __launch_bounds__(256) lower_max_kernel(int n, const double* __restrict__ A, long long lda,
+                                                        unsigned long long* __restrict__ top) {
+  unsigned long long m = 0;
+  for (int c = blockIdx.x; c < n; c += gridDim.x)
+    for (int r = c + threadIdx.x; r < n; r += 256)
+      m = max(m, (unsigned long long)__double_as_longlong(A[r + (long long)c * lda]) & 0x7fffffffffffffffull);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(top, m);
+}
+// Exponent of the power of two that brings the largest element to about
+// 1 / sqrt(n), so that the largest eigenvalue lies in about [1 / sqrt(n), sqrt(n)];
+// 0 where there is none.
+__device__ __forceinline__ int norm_shift(int n, unsigned long long top) {
+  const int ex = (int)(top >> 52);
+  return ex == 0 || ex == 0x7ff ? 0 : 1023 - ex - (31 - __clz(n)) / 2;
 }
 
-// Fill the strict upper triangle from the lower one (A symmetric in full storage).
-__global__ void symmetrize_kernel(int n, double* A, long long lda) {
-  const long long total = (long long)n * n;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    int r = (int)(e % n), c = (int)(e / n);
-    if (r < c) A[r + (long long)c * lda] = A[c + (long long)r * lda];
+// A := the symmetric matrix of Src's lower triangle times 2^norm_shift, full
+// storage, 32 x 32 tiles turned in shared memory (src == dst allowed: the mirror
+// image of the lower triangle, unscaled with top == nullptr).
+__global__ void __launch_bounds__(256) symmetrize_kernel(int n, const double* Src, long long lds, double* A,
+                                                         long long lda, const unsigned long long* __restrict__ top) {
+  if (blockIdx.x < blockIdx.y) return;
+  __shared__ double t[32][33];
+  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int sh = top ? norm_shift(n, *top) : 0;
+  for (int c = ty; c < 32; c += 8) {
+    const int r = r0 + tx, cc = c0 + c;
+    if (r < n && cc < n && r >= cc) {
+      double v = Src[r + (long long)cc * lds];
+      if (sh) v = ldexp(v, sh);
+      t[c][tx] = v;
+      if (top) A[r + (long long)cc * lda] = v;
+    }
+  }
+  __syncthreads();
+  for (int c = ty; c < 32; c += 8) {
+    const int r = c0 + tx, cc = r0 + c;  // row of the upper triangle
+    if (r < n && cc < n && cc > r) A[r + (long long)cc * lda] = t[tx][c];
   }
 }
-
-// Per column k the work is three launches, all spread over the SMs (a
-// single CTA would be bound by one SM's FP64 rate):
-//   tridiag_col_kernel   w_{k-1} = p + g v from the previous step's p, v and
-//                        partial dots; the pending update of step k-1 applied
-//                        to column k; partial sums of squares of column k
-//   tridiag_step_kernel  the reflector v_k from those sums (every CTA derives
-//                        the same scalars), then one pass over the trailing
-//                        matrix: pending update and A v_k
-//   tridiag_p_kernel     p_k = tau_k A v_k from the tile partials, partial
-//                        dots p_k^T v_k
-constexpr int RT = 256;  // rows per CTA of the row kernels
+__global__ void unscale_kernel(int n, double* W, const unsigned long long* __restrict__ top) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) W[i] = ldexp(W[i], -norm_shift(n, *top));
+}
 
 // Scalars of the Householder reflector of x (x[0] = alpha, |x[1:]|^2 = xnorm2):
 // beta, tau and the scale of x[1:] into v[1:].
@@ -84,224 +96,207 @@ __device__ __forceinline__ void reflector(double alpha, double xnorm2, double& b
   }
 }
 
-// Column k (rows k+1 .. n-1, i = 0 .. m-1).  With k > 0: g = -(tau_{k-1}/2)
-// sum(dpart) (p^T v of step k-1, fixed order), w_{k-1} = p + g v into wprev
-// (index 0 = row k), x_i = A[k+1+i, k] - (v[1+i] w[0] + w[1+i] v[0]) written
-// back, d[k] = A[k, k] - 2 v[0] w[0], and v_{k-1}[1:] stored below the
-// subdiagonal of column k-1.  Partial sums of x_i^2 (i >= 1) to npart.
-__global__ void __launch_bounds__(RT) tridiag_col_kernel(int n, int k, double* A, long long lda, double* d,
-                                                         const double* __restrict__ tau,
-                                                         const double* __restrict__ pprev,
-                                                         const double* __restrict__ vprev,
-                                                         double* __restrict__ wprev,
-                                                         const double* __restrict__ dpart, int ndp,
-                                                         double* __restrict__ npart) {
-  __shared__ double red[33];
-  const int m = n - k - 1;
-  const int i = blockIdx.x * RT + threadIdx.x;
-  const bool upd = k > 0;
-  double* x = A + (k + 1) + (long long)k * lda;
-  double sq = 0.0;
-  __shared__ double dot_s;
-  if (upd && threadIdx.x == 0) {
-    double dot = 0.0;
-    for (int c = 0; c < ndp; c++) dot += dpart[c];
-    dot_s = dot;
-  }
-  __syncthreads();
-  if (upd) {
-    const double g = -0.5 * tau[k - 1] * dot_s;
-    const double v0 = vprev[0];
-    const double w0 = pprev[0] + g * v0;
-    if (i < m) {
-      const double vi = vprev[1 + i];
-      const double wi = pprev[1 + i] + g * vi;
-      wprev[1 + i] = wi;
-      const double xi = x[i] - (vi * w0 + wi * v0);
-      x[i] = xi;
-      if (i >= 1) sq = xi * xi;
-      A[(k + 1 + i) + (long long)(k - 1) * lda] = vi;  // reflector k-1, row k+1+i
+// Panel of columns k0 .. k0 + TB - 1: P = [V W V] (n x 3 TB, ld n), column q of V
+// the reflector of column k0 + q (1 at row k0 + q + 1, zero above), W the vectors
+// of the rank-2 updates.  Two launches a column:
+//   tridiag_col   column i - 1's w from y = A v and the dot products of v with V
+//                 and W, then column i of A brought up to date
+//   tridiag_mv    the reflector of that column (every CTA derives the same
+//                 scalars), y = A v, t = [W^T v ; V^T v] and the parts of y^T v
+// Sums over CTAs are taken from arrays of parts in a fixed order.
+constexpr int TB = 64;
+constexpr int TR = 32;  // rows per CTA of tridiag_col, one per lane; the panel's columns are dealt to the warps
+
+// Panel column i = k - k0.  pend: w of column i - 1 is due,
+//   w = tau (y - V t1 - W t2) + g v,  g = -tau/2 p^T v,  p^T v = tau (y^T v - 2 t1 . t2)
+// (p the bracket times tau; V, W the columns before i - 1).  live: column k is
+// wanted, x_r = A[r, k] - sum_q V[r, q] W[k, q] + W[r, q] V[k, q]; x_k is d[k],
+// and the parts of |x[k+2:]|^2 go to npart.
+__global__ void __launch_bounds__(256) tridiag_col_kernel(int n, int k, int i, bool pend, bool live,
+                                                          const double* __restrict__ A, long long lda,
+                                                          double* __restrict__ P, const double* __restrict__ y,
+                                                          const double* __restrict__ t, const double* __restrict__ yvpart,
+                                                          int nyv, const double* __restrict__ tau,
+                                                          double* __restrict__ d, double* __restrict__ x,
+                                                          double* __restrict__ npart) {
+  __shared__ double st1[TB], st2[TB], vk[TB], wk[TB], part[2][8][TR], yvs[8], wsum;
+  const int q1 = pend ? i - 1 : 0;  // panel columns that are complete
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int r = k + blockIdx.x * TR + lane;
+  const double *V = P, *W = P + (long long)TB * n;
+  double yr = 0.0, vr = 0.0, ar = 0.0, tk = 0.0, yk = 0.0;  // what the last part needs, in flight early
+  if (wp == 0 && r < n) {
+    if (live) ar = A[r + (long long)k * lda];
+    if (pend) {
+      yr = y[r];
+      vr = V[r + (long long)q1 * n];
     }
-    if (i == 0) {
-      wprev[0] = w0;
-      d[k] = A[k + (long long)k * lda] - 2.0 * v0 * w0;
-    }
-  } else {
-    if (i < m && i >= 1) sq = x[i] * x[i];
-    if (i == 0) d[k] = A[k + (long long)k * lda];
   }
-  sq = block_sum(sq, red);
-  if (threadIdx.x == 0) npart[blockIdx.x] = sq;
+  if (pend) {
+    tk = tau[k - 1];
+    yk = y[k];
+    if (threadIdx.x < q1) {
+      st1[threadIdx.x] = t[threadIdx.x];
+      st2[threadIdx.x] = t[TB + threadIdx.x];
+      vk[threadIdx.x] = V[k + (long long)threadIdx.x * n];
+      wk[threadIdx.x] = W[k + (long long)threadIdx.x * n];
+    }
+    double yv = 0.0;
+    for (int c = threadIdx.x; c < nyv; c += 256) yv += yvpart[c];
+    __syncthreads();
+    if (threadIdx.x < q1) yv = fma(-2.0 * st1[threadIdx.x], st2[threadIdx.x], yv);
+    double a1 = 0.0, a2 = 0.0;
+    if (r < n) {
+#pragma unroll
+      for (int u = 0; u < TB / 8; u++) {
+        const int q = wp + 8 * u;
+        if (q >= q1) break;
+        const double v = V[r + (long long)q * n], w = W[r + (long long)q * n];
+        a1 = fma(v, st1[q], fma(w, st2[q], a1));
+        a2 = fma(v, wk[q], fma(w, vk[q], a2));
+      }
+    }
+    part[0][wp][lane] = a1;
+    part[1][wp][lane] = a2;
+    yv = warp_sum(yv);
+    if (lane == 0) yvs[wp] = yv;
+    if (wp == 7) {  // the bracket's sum for row k, whose w every row's update needs
+      double a = 0.0;
+      for (int q = lane; q < q1; q += 32) a = fma(vk[q], st1[q], fma(wk[q], st2[q], a));
+      a = warp_sum(a);
+      if (lane == 0) wsum = a;
+    }
+    __syncthreads();
+  }
+  if (wp > 0) return;
+  double sq = 0.0, xr = ar;
+  if (pend) {
+    double a1 = 0.0, a2 = 0.0, yv = 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      a1 += part[0][u][lane];
+      a2 += part[1][u][lane];
+      yv += yvs[u];
+    }
+    const double g = -0.5 * tk * tk * yv;
+    const double wlast = fma(tk, yk - wsum, g);  // v_k = 1
+    const double w = fma(tk, yr - a1, g * vr);
+    if (r < n) P[r + (long long)(TB + q1) * n] = w;
+    xr -= a2 + fma(vr, wlast, w);
+  }
+  if (!live) return;
+  if (r < n) {
+    if (r == k) d[k] = xr;
+    else x[r] = xr;
+    if (r >= k + 2) sq = xr * xr;
+  }
+  sq = warp_sum(sq);
+  if (lane == 0) npart[blockIdx.x] = sq;
 }
 
-// The last 2 x 2 block.  n >= 3: w of step n-3 from its p, v and partial
-// dots, its reflector stored (A[n-1, n-3]), and its pending update applied.
-__global__ void tridiag_tail_kernel(int n, double* A, long long lda, double* d, double* e, const double* tau,
-                                    const double* p, const double* v, const double* dpart, int ndp) {
-  if (n >= 3) {
-    double dot = 0.0;
-    for (int c = 0; c < ndp; c++) dot += dpart[c];
-    const double g = -0.5 * tau[n - 3] * dot;
-    const double v0 = v[0], v1 = v[1];
-    const double w0 = p[0] + g * v0, w1 = p[1] + g * v1;
-    A[(n - 1) + (long long)(n - 3) * lda] = v1;
-    d[n - 2] = A[(n - 2) + (long long)(n - 2) * lda] - 2.0 * v0 * w0;
-    e[n - 2] = A[(n - 1) + (long long)(n - 2) * lda] - (v1 * w0 + w1 * v0);
-    d[n - 1] = A[(n - 1) + (long long)(n - 1) * lda] - 2.0 * v1 * w1;
-  } else if (n == 2) {
-    d[0] = A[0];
-    e[0] = A[1];
-    d[1] = A[1 + lda];
+// y = A22 v, t = [W^T v ; V^T v] over rows and columns k+1 .. (i complete panel
+// columns), a warp per column, and the parts of y^T v.  v = scal x below its
+// leading 1, so the dot products run on x at once and take the scale at the end;
+// the ninth warp derives the reflector meanwhile.  Bound by the m^2 FP64 FMAs (an
+// SM takes a warp's in 16 cycles: 20 us at m = 3500) and, below m of about 1500,
+// by latency.
+constexpr int MV_THREADS = 288;
+__global__ void __launch_bounds__(MV_THREADS) tridiag_mv_kernel(int n, int k, int i, double* A, long long lda, double* P,
+                                                                const double* __restrict__ x,
+                                                                const double* __restrict__ npart, int nnp,
+                                                                double* __restrict__ tau_out, double* __restrict__ e_out,
+                                                                double* __restrict__ y, double* __restrict__ t,
+                                                                double* __restrict__ yvpart) {
+  __shared__ double sscal, yvs[8];
+  const int m = n - k - 1, r0 = k + 1;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int warps = gridDim.x * 8, cols = m + 2 * i;
+  const double* xs = x + r0;
+  auto column = [&](int j) -> const double* {
+    return j < m ? A + r0 + (long long)(r0 + j) * lda
+                 : j < m + i ? P + r0 + (long long)(TB + j - m) * n : P + r0 + (long long)(j - m - i) * n;
+  };
+  auto dot = [&](int j) -> double {  // x[1:] with the column, every lane
+    const double* a = column(j);
+    double s0 = 0.0, s1 = 0.0;
+    int r = lane;
+    if (lane == 0) r = 32;  // row 0 goes in apart
+#pragma unroll 4
+    for (; r + 32 < m; r += 64) {
+      s0 = fma(a[r], xs[r], s0);
+      s1 = fma(a[r + 32], xs[r + 32], s1);
+    }
+    if (r < m) s0 = fma(a[r], xs[r], s0);
+    return warp_sum(s0 + s1);
+  };
+  const int j0 = blockIdx.x * 8 + wp;
+  double first = 0.0, head = 0.0;
+  if (wp < 8) {
+    if (j0 < cols) {
+      head = column(j0)[0];
+      first = dot(j0);
+    }
   } else {
-    d[0] = A[0];
+    double xn2 = 0.0;
+    for (int c = lane; c < nnp; c += 32) xn2 += npart[c];
+    xn2 = warp_sum(xn2);
+    double beta, tau, scal;
+    reflector(xs[0], xn2, beta, tau, scal);
+    if (lane == 0) sscal = scal;
+    if (blockIdx.x == 0 && lane == 0) {
+      tau_out[k] = tau;
+      e_out[k] = beta;
+    }
   }
+  __syncthreads();
+  const double scal = sscal;
+  // the reflector: the panel's two copies and column k of A (for the back-transform)
+  for (int j = blockIdx.x * MV_THREADS + threadIdx.x; j < m + i + 1; j += gridDim.x * MV_THREADS) {
+    const int r = k - i + j;
+    const double v = r < r0 ? 0.0 : r == r0 ? 1.0 : x[r] * scal;
+    P[r + (long long)i * n] = v;
+    P[r + (long long)(2 * TB + i) * n] = v;
+    if (r > r0) A[r + (long long)k * lda] = v;
+  }
+  if (wp == 8) return;
+  double yv = 0.0;
+  for (int j = j0; j < cols; j += warps) {
+    if (j != j0) {
+      head = column(j)[0];
+      first = dot(j);
+    }
+    const double s = fma(scal, first, head);
+    if (lane == 0) {
+      if (j < m) {
+        y[r0 + j] = s;
+        yv = fma(s, j == 0 ? 1.0 : xs[j] * scal, yv);
+      } else {
+        t[j < m + i ? j - m : TB + j - m - i] = s;
+      }
+    }
+  }
+  if (lane == 0) yvs[wp] = yv;
+  asm volatile("bar.sync 1, 256;" ::: "memory");  // the eight column warps
+  if (threadIdx.x == 0) {
+    double v = 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; u++) v += yvs[u];
+    yvpart[blockIdx.x] = v;
+  }
+}
+constexpr int EIG_CTAS = 608;  // most CTAs of tridiag_mv: four an SM
+
+// The last 2 x 2 block.
+__global__ void tridiag_tail_kernel(int n, const double* A, long long lda, double* d, double* e) {
+  if (n >= 2) {
+    d[n - 2] = A[(n - 2) + (long long)(n - 2) * lda];
+    e[n - 2] = A[(n - 1) + (long long)(n - 2) * lda];
+  }
+  d[n - 1] = A[(n - 1) + (long long)(n - 1) * lda];
   e[n - 1] = 0.0;
 }
 
 int grid_for(long long total) { return (int)std::min<long long>((total + 255) / 256, 152LL * 32); }
-
-// One pass over the trailing lower triangle (m x m, 32 x 32 tiles) per
-// column: apply the pending rank-2 update A -= vo wo^T + wo vo^T (vo, wo:
-// the previous step's vectors shifted to this trailing matrix; nullptr at
-// step 0) and form A v with the updated values.  v is the reflector of
-// column x (x[0] = alpha, rows below: the updated column), derived by every
-// CTA from the same fixed-order sum of npart; CTAs Jc = 0 store it (vout),
-// CTA (0, 0) stores tau and e.  CTA (Jc, I) takes the lower tiles (I, J), J
-// in [Jc*SS, min(Jc*SS + SS, I + 1)).  Row block I's partial of A v from the
-// strip goes to slot (I, Jc), and the below-diagonal tiles' A_IJ^T v_I to
-// slot (J, I) (> J), each written exactly once: part[(R * nt + K) * 32 + r].
-// The reduction sums them in a fixed order (deterministic, no atomics).
-constexpr int ST = 32;
-constexpr int SS = 4;
-__global__ void __launch_bounds__(256) tridiag_step_kernel(int m, double* __restrict__ A, long long lda,
-                                                           const double* __restrict__ vo,
-                                                           const double* __restrict__ wo,
-                                                           const double* __restrict__ x,
-                                                           const double* __restrict__ npart, int nnp,
-                                                           double* __restrict__ vout, double* __restrict__ tau_out,
-                                                           double* __restrict__ e_out, double* __restrict__ part) {
-  const int I = blockIdx.y, Jc = blockIdx.x, J0 = Jc * SS;
-  if (J0 > I) return;
-  __shared__ double scal_s;
-  if (threadIdx.x == 0) {
-    double xn2 = 0.0;
-    for (int c = 0; c < nnp; c++) xn2 += npart[c];
-    double beta, tau, scal;
-    reflector(x[0], xn2, beta, tau, scal);
-    scal_s = scal;
-    if (blockIdx.x == 0 && blockIdx.y == 0) {
-      *tau_out = tau;
-      *e_out = beta;
-    }
-  }
-  __syncthreads();
-  const double scal = scal_s;
-  // v_i: 1 at i = 0, x_i * scal below, 0 past the matrix
-  auto vval = [&](int i) { return i < m ? (i == 0 ? 1.0 : x[i] * scal) : 0.0; };
-  const int J1 = min(J0 + SS, I + 1);
-  const int nt = gridDim.y;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-  __shared__ double a[ST][ST + 1];  // a[c][r] = A[I*32 + r, J*32 + c]
-  __shared__ double vr[ST], vor[ST], wor[ST], vc[ST], voc[ST], woc[ST];
-  __shared__ double red[8][ST];
-  const bool upd = vo != nullptr;
-  const int gr = I * ST + tx;
-  if (ty == 0) {
-    const double vi = vval(gr);
-    vr[tx] = vi;
-    if (Jc == 0 && gr < m) vout[gr] = vi;
-    vor[tx] = (upd && gr < m) ? vo[gr] : 0.0;
-    wor[tx] = (upd && gr < m) ? wo[gr] : 0.0;
-  }
-  double rs = 0.0;  // row tx of this strip's A_I. v, over this thread's columns
-  for (int J = J0; J < J1; J++) {
-    __syncthreads();  // the previous tile's shared reads are done
-    if (ty == 1) {
-      const int gc = J * ST + tx;
-      vc[tx] = vval(gc);
-      voc[tx] = (upd && gc < m) ? vo[gc] : 0.0;
-      woc[tx] = (upd && gc < m) ? wo[gc] : 0.0;
-    }
-    __syncthreads();
-    for (int c = ty; c < ST; c += 8) {
-      const int gc = J * ST + c;
-      double av = 0.0;
-      if (gr < m && gc < m && (I != J || tx >= c)) {
-        double* pa = A + gr + (long long)gc * lda;
-        av = *pa;
-        if (upd) {
-          // two FMAs (FP64 issue rate bounds this pass)
-          av = fma(-vor[tx], woc[c], av);
-          av = fma(-wor[tx], voc[c], av);
-          *pa = av;
-        }
-      }
-      a[c][tx] = av;
-    }
-    __syncthreads();
-    if (I == J) {
-      // diagonal tile: the symmetric block from its lower part
-      for (int c = ty; c < ST; c += 8) rs += (tx >= c ? a[c][tx] : a[tx][c]) * vc[c];
-    } else {
-      for (int c = ty; c < ST; c += 8) rs += a[c][tx] * vc[c];
-      // column tx of A_IJ^T v_I: rows ty, ty+8, ... here, the eight partial
-      // sums added by one thread (FP64 issue rate is the bound: no shuffles)
-      double cs = 0.0;
-      for (int r = ty; r < ST; r += 8) cs += a[tx][r] * vr[r];
-      red[ty][tx] = cs;
-      __syncthreads();
-      if (ty == 0) {
-        double t = 0.0;
-#pragma unroll
-        for (int q = 0; q < 8; q++) t += red[q][tx];
-        part[((long long)J * nt + I) * ST + tx] = t;
-      }
-    }
-  }
-  __syncthreads();  // the last tile's column reduction has read red
-  red[ty][tx] = rs;
-  __syncthreads();
-  if (ty == 0) {
-    double t = 0.0;
-#pragma unroll
-    for (int q = 0; q < 8; q++) t += red[q][tx];
-    part[((long long)I * nt + Jc) * ST + tx] = t;
-  }
-}
-
-// p[i] = tau_k * sum of row block R = i / 32's slots (strip slots K = 0 ..
-// R/SS, then tile slots K = R+1 .. nt-1).  One CTA per row block: thread
-// (r, c) sums slots c, c+8, ... of row r, the eight partial sums are added in
-// c order (fixed order); the CTA's p^T v goes to dpart[R].
-__global__ void __launch_bounds__(256) tridiag_p_kernel(int m, int nt, const double* __restrict__ part,
-                                                        const double* __restrict__ tau_ptr,
-                                                        const double* __restrict__ v, double* __restrict__ p,
-                                                        double* __restrict__ dpart) {
-  __shared__ double red[8][ST];
-  const int R = blockIdx.x;
-  const int r = threadIdx.x & 31, c = threadIdx.x >> 5;
-  const int i = R * ST + r;
-  const int ns = R / SS + 1;          // strip slots 0 .. R/SS
-  const int nslots = ns + (nt - R - 1);  // then tile slots R+1 .. nt-1
-  const double* q = part + ((long long)R * nt) * ST + r;
-  double sum = 0.0;
-  for (int e = c; e < nslots; e += 8) {
-    const int K = e < ns ? e : R + 1 + (e - ns);
-    sum += q[(long long)K * ST];
-  }
-  red[c][r] = sum;
-  __syncthreads();
-  if (c == 0) {
-    double t = 0.0;
-#pragma unroll
-    for (int u = 0; u < 8; u++) t += red[u][r];
-    const double pi = i < m ? *tau_ptr * t : 0.0;
-    if (i < m) p[i] = pi;
-    double pv = i < m ? pi * v[i] : 0.0;
-    pv = warp_sum(pv);
-    if (r == 0) dpart[R] = pv;
-  }
-}
 
 // Y (mr x nb, ld mr): reflectors b .. b+nb-1 as explicit columns over rows
 // b+1 .. n-1: column c is zero above row c, 1 at row c, A[b+c+1+i, b+c] below.
@@ -383,11 +378,9 @@ cudaError_t larft(cudaStream_t s, int nb, const double* tau, const double* G, do
 }  // namespace
 
 size_t eig_workspace_bytes(int n) {
-  // d, e, tau, two v and two w buffers, p (n each), per-CTA dot and norm
-  // partials (n / RT each) + n ints of scratch + symv partials (nt^2 x 32)
-  const size_t nt = (size_t)(n + ST - 1) / ST;
-  const size_t nr = (size_t)(n + RT - 1) / RT;
-  return sizeof(double) * ((size_t)n * 8 + nt + nr + nt * nt * ST) + sizeof(int) * (size_t)n + 256;
+  // d, e, tau, x, y (n each), t (2 TB), parts of the column norm (n / TR) and of
+  // y^T v (up to EIG_CTAS), the panel (n x 3 TB), the norm and the failure flag
+  return sizeof(double) * ((size_t)n * (5 + 3 * TB) + 2 * TB + (n + TR - 1) / TR + 2 + EIG_CTAS + 2) + 256;
 }
 
 cudaError_t dsyev_device(cudaStream_t s, DigitGemm* dg, int n, const double* Phi, long long ldp, double* A, double* Z,
@@ -395,13 +388,14 @@ cudaError_t dsyev_device(cudaStream_t s, DigitGemm* dg, int n, const double* Phi
   double* d = (double*)work;
   double* e = d + n;
   double* tau = e + n;
-  double* vb[2] = {tau + n, tau + 2 * (size_t)n};      // reflectors of even / odd steps
-  double* wb[2] = {tau + 3 * (size_t)n, tau + 4 * (size_t)n};  // their w vectors
-  double* pbuf = tau + 5 * (size_t)n;                  // p of the current step
-  double* dpart = pbuf + n;                            // p^T v per 32-row block
-  double* npart = dpart + (n + ST - 1) / ST;           // per-CTA sums of squares of the column
-  int* rank = (int*)(npart + (n + RT - 1) / RT);
-  double* part = (double*)(((uintptr_t)(rank + n) + 15) & ~(uintptr_t)15);  // symv partials
+  double* xb = tau + n;                             // the current column
+  double* yb = xb + n;                              // A v
+  double* tb = yb + n;                              // W^T v, V^T v
+  double* npart = tb + 2 * TB;                      // parts of the column's sum of squares
+  double* yvpart = npart + (n + TR - 1) / TR + 2;   // parts of y^T v
+  double* P = yvpart + EIG_CTAS;                    // [V W V]
+  unsigned long long* top = (unsigned long long*)(P + (size_t)n * 3 * TB);
+  int* dfail = (int*)(top + 1);
   long long nl = 0;
   // FGLS_EIG_TIMING=1 prints the phase times (CUDA events on s) to stderr
   const bool timing = getenv("FGLS_EIG_TIMING") != nullptr;
@@ -417,30 +411,47 @@ cudaError_t dsyev_device(cudaStream_t s, DigitGemm* dg, int n, const double* Phi
     dg = nullptr;
   }
   mark(0);
-  // A := Phi (lower) symmetrized
-  FGLS_CUDA_TRY(cudaMemcpy2DAsync(A, sizeof(double) * n, Phi, sizeof(double) * ldp, sizeof(double) * n, n,
-                                  cudaMemcpyDeviceToDevice, s));
-  symmetrize_kernel<<<grid_for((long long)n * n), 256, 0, s>>>(n, A, n);
-  nl++;
+  // A := Phi's lower triangle, scaled, in full storage
+  FGLS_CUDA_TRY(cudaMemsetAsync(top, 0, sizeof(*top), s));
+  lower_max_kernel<<<std::min(n, 1216), 256, 0, s>>>(n, Phi, ldp, top);
+  const dim3 tiles(ceil_div(n, 32), ceil_div(n, 32));
+  symmetrize_kernel<<<tiles, 256, 0, s>>>(n, Phi, ldp, A, n, top);
+  nl += 2;
   FGLS_CUDA_TRY(cudaGetLastError());
   // 1. tridiagonalization
-  int ndp = 0;  // CTAs of the previous step's p kernel
-  for (int k = 0; k + 2 < n; k++) {
-    const int m = n - k - 1;
-    const int cur = k & 1, prv = cur ^ 1;
-    const int nr = ceil_div(m, RT);
-    tridiag_col_kernel<<<nr, RT, 0, s>>>(n, k, A, n, d, tau, pbuf, vb[prv], wb[prv], dpart, ndp, npart);
-    double* Asub = A + (k + 1) + (long long)(k + 1) * n;
-    const int nt = ceil_div(m, ST);
-    const double* vo = k > 0 ? vb[prv] + 1 : nullptr;  // pending update of step k-1, shifted to rows k+1..
-    const double* wo = k > 0 ? wb[prv] + 1 : nullptr;
-    tridiag_step_kernel<<<dim3(ceil_div(nt, SS), nt), 256, 0, s>>>(m, Asub, n, vo, wo, A + (k + 1) + (long long)k * n,
-                                                                    npart, nr, vb[cur], tau + k, e + k, part);
-    tridiag_p_kernel<<<nt, 256, 0, s>>>(m, nt, part, tau + k, vb[cur], pbuf, dpart);
-    ndp = nt;
-    nl += 3;
+  for (int k0 = 0; k0 + 2 < n; k0 += TB) {
+    const int nb = std::min(TB, n - 2 - k0);
+    int nyv = 0;
+    for (int i = 0; i < nb; i++) {
+      const int k = k0 + i, m = n - k - 1;
+      const int nr = ceil_div(n - k, TR);
+      tridiag_col_kernel<<<nr, 256, 0, s>>>(n, k, i, i > 0, true, A, n, P, yb, tb, yvpart, nyv, tau, d, xb, npart);
+      nyv = std::min(ceil_div(m + 2 * i, 8), EIG_CTAS);
+      tridiag_mv_kernel<<<nyv, MV_THREADS, 0, s>>>(n, k, i, A, n, P, xb, npart, nr, tau, e, yb, tb, yvpart);
+      nl += 2;
+    }
+    const int kn = k0 + nb, m = n - kn;  // the trailing matrix
+    tridiag_col_kernel<<<ceil_div(m, TR), 256, 0, s>>>(n, kn, nb, true, false, A, n, P, yb, tb, yvpart, nyv, tau, d, xb,
+                                                        npart);
+    nl++;
+    FGLS_CUDA_TRY(cudaGetLastError());
+    // A -= [V W] [W V]^T; a short last panel leaves columns of P beyond nb unset
+    double* T = A + kn + (long long)kn * n;
+    if (nb == TB && dg && digit_gemm_pays(m, m, 2 * TB)) {
+      DigitMulOpts lower;
+      lower.c_lower = true;
+      FGLS_CUDA_TRY(digit_dgemm(dg, s, false, true, m, m, 2 * TB, -1.0, P + kn, n, P + kn + (long long)TB * n, n, 1.0, T,
+                                n, lower));
+      symmetrize_kernel<<<dim3(ceil_div(m, 32), ceil_div(m, 32)), 256, 0, s>>>(m, T, n, T, n, nullptr);
+      nl++;
+    } else if (nb == TB) {
+      FGLS_CUDA_TRY(dgemm(s, false, true, m, m, 2 * TB, -1.0, P + kn, n, P + kn + (long long)TB * n, n, 1.0, T, n));
+    } else {
+      FGLS_CUDA_TRY(dgemm(s, false, true, m, m, nb, -1.0, P + kn, n, P + kn + (long long)TB * n, n, 1.0, T, n));
+      FGLS_CUDA_TRY(dgemm(s, false, true, m, m, nb, -1.0, P + kn + (long long)TB * n, n, P + kn, n, 1.0, T, n));
+    }
   }
-  tridiag_tail_kernel<<<1, 1, 0, s>>>(n, A, n, d, e, tau, pbuf, n >= 3 ? vb[(n - 3) & 1] : nullptr, dpart, ndp);
+  tridiag_tail_kernel<<<1, 1, 0, s>>>(n, A, n, d, e);
   nl++;
   FGLS_CUDA_TRY(cudaGetLastError());
   mark(1);
@@ -452,9 +463,10 @@ cudaError_t dsyev_device(cudaStream_t s, DigitGemm* dg, int n, const double* Phi
   const size_t bt_bytes = sizeof(double) * ((size_t)3 * NBT * n + (size_t)2 * NBT * NBT);
   void* dcw = nullptr;
   FGLS_CUDA_TRY(cudaMalloc(&dcw, std::max(dc_workspace_bytes(n), bt_bytes)));
-  int* dfail = rank;  // n ints of scratch; first used as the failure flag
   FGLS_CUDA_TRY(cudaMemsetAsync(dfail, 0, sizeof(int), s));
   cudaError_t rc = dc_tridiag_eig(s, dg, n, d, e, W, Z, dcw, dfail, &nl);
+  unscale_kernel<<<ceil_div(n, 256), 256, 0, s>>>(n, W, top);
+  nl++;
   mark(3);
   // 4. Z := H_0 H_1 ... H_{n-3} Z, blocks of NB reflectors from the last one
   //    in compact-WY form (I - Y T Y^T): three DGEMMs per block, 2 n^3 flops
