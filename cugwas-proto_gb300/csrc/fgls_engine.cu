@@ -84,6 +84,8 @@ struct fglsgpu_engine {
   DigitMat ldig;
   bool linv_cut = false;
   void *zmem = nullptr, *wmem = nullptr, *blkmem = nullptr;
+  void* remlmem = nullptr;
+  size_t reml_bytes = 0;
   size_t blk_bytes = 0;
   bool z_cut = false, w_cut = false;
   bool probing = false;  // the autotuner's FP64 block: no room for x_b SNPs
@@ -173,7 +175,7 @@ void free_all(fglsgpu_engine* e) {
                   e->dQ,   e->dGYL, e->dGR,  e->dB[0], e->dB[1], e->dV[0], e->dV[1], e->dU8, e->dst,
                   e->aWc, e->aAYLc, e->aAYLs, e->atopc, e->atops, e->areml, e->aGYLc, e->aGYLs, e->aGRc,
                   e->aGRs, e->acontrib, e->ag, e->agR, e->aacc, e->aU, e->aV2, e->dSE[0], e->dSE[1], e->dP[0],
-                  e->dP[1], e->dXw, e->zmem, e->wmem, e->blkmem, e->dLinv, e->ddiag, e->dWraw};
+                  e->dP[1], e->dXw, e->zmem, e->wmem, e->blkmem, e->dLinv, e->ddiag, e->dWraw, e->remlmem};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (e->hst) cudaFreeHost(e->hst);
@@ -1212,13 +1214,16 @@ int fglsgpu_reml_fit(fglsgpu_engine* e, double h_lo, double h_hi, int grid, doub
   const int t = c.t;
   int rc = reset_status(e);
   if (rc) return rc;
-  double* dout = nullptr;
-  ENG_TRY(e, dalloc(&dout, 4 * (size_t)t), "reml_fit output");
+  // the outputs and the grid's workspace, kept for the next fit
+  const size_t outb = (sizeof(double) * 4 * (size_t)t + 255) & ~(size_t)255;
+  if (!grow(&e->remlmem, &e->reml_bytes, outb + reml_workspace_bytes(c.n, t, grid)))
+    return fail(e, FGLSGPU_ENOMEM, "no memory for the REML grid");
+  double* dout = (double*)e->remlmem;
   std::vector<double> r(4 * (size_t)t);
-  cudaError_t ce = reml_fit(e->comp, c.n, t, c.wXL, e->dW, e->dZtXL, e->dZtY, h_lo, h_hi, grid, dout, e->dst);
+  cudaError_t ce = reml_fit(e->comp, c.n, t, c.wXL, e->dW, e->dZtXL, e->dZtY, h_lo, h_hi, grid,
+                            (double*)((char*)e->remlmem + outb), dout, e->dst);
   if (ce == cudaSuccess) ce = cudaMemcpyAsync(r.data(), dout, sizeof(double) * 4 * t, cudaMemcpyDeviceToHost, e->comp);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->comp);
-  cudaFree(dout);
   if (ce != cudaSuccess) return cuda_fail(e, ce, "reml_fit");
   ENG_TRY(e, cudaMemcpy(e->hst, e->dst, sizeof(DevStatus), cudaMemcpyDeviceToHost), "status copy");
   const DevStatus st = *e->hst;

@@ -91,8 +91,10 @@ cudaError_t adjoint_ybar(cudaStream_t s, int n, int t, int wXL, const double* di
 // 2 <= grid <= FGLS_REML_MAX_GRID, then root refinement of the h-gradient).
 // out (4 x t): h, sigma_hat, profiled log-likelihood, its h-gradient there.
 #define FGLS_REML_MAX_GRID 256
+// work: reml_workspace_bytes.
+size_t reml_workspace_bytes(int n, int t, int grid);
 cudaError_t reml_fit(cudaStream_t s, int n, int t, int wXL, const double* W, const double* ZtXL, const double* ZtY,
-                     double lo, double hi, int grid, double* out, DevStatus* st);
+                     double lo, double hi, int grid, double* work, double* out, DevStatus* st);
 
 // Genotype conversion: FP64 or u8 hard calls -> FP64 (device to device).
 cudaError_t u8_to_f64(cudaStream_t s, const unsigned char* in, double* out, long long count);
