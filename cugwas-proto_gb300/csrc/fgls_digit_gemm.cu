@@ -31,11 +31,11 @@
 // rows of A and 128 of B.  Two levels run at once, L in TMEM columns 0-255 and
 // L + 1 in 256-511.  For a K-block the digits of B ascend, t = 1, 2, ..: the
 // A tile that level L + 1 needs at step t, digit L + 1 - t, is the one level L
-// used at step t - 1, so each 32 KB stage (one A tile, one B tile) feeds eight
-// MMAs and the previous stage's A tile is kept one step longer.  That is 28
-// bytes per clock and SM from L2, half of what one A and one B tile per four
-// MMAs would take.
-//   warp 0     TMA producer (each CTA its own 128 rows), six stages
+// used at step t - 1, so each step (one A tile, one B tile, at the first a second A
+// tile) feeds eight MMAs and the previous step's A tile is kept one step
+// longer.  That is 28 bytes per clock and SM from L2, half of what one A and one
+// B tile per four MMAs would take.
+//   warp 0     TMA producer (each CTA its own 128 rows), a ring of fourteen tiles
 //   warp 1     MMA issue (pair leader), TMEM allocation
 //   warps 2-17 epilogue: q = 32 P_L + P_{L+1} as int32 into the CTA's own
 //              planes (L2-resident, 4 bytes per element and level pair); once a
@@ -69,9 +69,14 @@ using namespace oz;
 constexpr int ND = DG_DIGITS;
 constexpr int ROW = 128;               // bytes (digits) of a K-step
 constexpr int TILE = 128 * ROW;        // 16 KB: 128 rows of one digit plane
-constexpr int STAGE = 2 * TILE;        // an A and a B tile
-constexpr int STAGES = 6;
-constexpr int SMEM = STAGES * STAGE + 1024 + 256;
+// Ring of tiles; a step takes two or three of them (an A tile, at a K-block's first
+// step the A tile level L + 1 starts with, a B tile) and one of the barriers.  In
+// fixed stages of three tiles four fit, in stages of two six, with a stage to
+// itself for the third: 10000 x 4096 x 10000 took 19.1 and 18.6 ms, with hard calls
+// (three tiles every step) 3.67 and 4.37; tile by tile 18.7 and 3.72.
+constexpr int TILES = 14;
+constexpr int STEPS = 8;               // at most TILES / 2 in flight
+constexpr int SMEM = TILES * TILE + 1024 + 256;
 constexpr int EPI_WARPS = 16;
 constexpr int EPI_COLS = 256 * 4 / EPI_WARPS;  // columns of an epilogue warp (32 rows)
 constexpr int NTHREADS = 64 + 32 * EPI_WARPS;
@@ -173,7 +178,7 @@ __device__ __forceinline__ Unit dg_unit(const DgArgs& g, int u) {
 
 // Level pair i of a unit: levels L and L + 1, the B digits t that take part.
 struct Pass {
-  int L, tlo, thi, has1, pro, chunk;  // pro: an A tile (digit L + 1 - tlo) precedes step tlo; chunk: K-steps a pass
+  int L, tlo, thi, has1, pro, chunk;  // pro: step tlo brings A digit L + 1 - tlo too; chunk: K-steps a pass
 };
 __device__ __forceinline__ Pass dg_pass(const Unit& U, int i) {
   Pass P;
@@ -276,14 +281,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
                       const __grid_constant__ DgArgs g) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = (uint64_t*)(smem + STAGES * STAGE);  // [STAGES], used in the leader
-  uint64_t* empty = full + STAGES;                       // [STAGES]
-  uint64_t* tfull = empty + STAGES;
+  uint64_t* full = (uint64_t*)(smem + TILES * TILE);  // [STEPS], used in the leader
+  uint64_t* empty = full + STEPS;                      // [STEPS]
+  uint64_t* tfull = empty + STEPS;
   uint64_t* tempty = tfull + 1;  // used in the leader
   uint64_t* drain = tempty + 1;
   uint32_t* tbase_slot = (uint32_t*)(drain + 1);
   volatile int* abort_flag = (volatile int*)(tbase_slot + 1);
-  static_assert((STAGES * 2 + 3) * 8 + 8 <= 256, "barriers fit the 256-byte tail");
+  static_assert((STEPS * 2 + 3) * 8 + 8 <= 256, "barriers fit the 256-byte tail");
 
   const uint32_t rank = cluster_rank();
   const bool lead = rank == 0;
@@ -293,7 +298,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
   const uint16_t BOTH = 0x3;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; s++) {
+    for (int s = 0; s < STEPS; s++) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -314,28 +319,38 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
   tc_fence_after();
   const uint32_t tbase = *tbase_slot;
   const uint32_t lead_full = cluster_addr(full, 0);
+  const uint64_t ring = desc_sw128(smem);  // tile i is (TILE >> 4) * i further
 
   if (warp == 0) {
     if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int issued[STAGES];
-      uint32_t issued_phase[STAGES];
-      for (int s = 0; s < STAGES; s++) issued[s] = 0;
+      // steps [head, tail) hold their tiles; their counts, four bits a step
+      uint32_t head = 0, tail = 0, counts = 0;
+      int room = TILES, pos = 0;
       bool ok = true;
-      // one stage: A digit sa (0: none) and B digit tb (0: none) of K-step kb
-      auto fill = [&](int kb, int ra, int sa, int rb, int tb) -> bool {
-        if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, g.err, 41, g.wait_ns)) return false;
-        issued[stage] = 0;
-        uint8_t* sb = smem + stage * STAGE;
-        const uint32_t fb = lead_full + 8u * (uint32_t)stage;
-        const int bytes = (sa > 0 ? TILE : 0) + (tb > 0 ? TILE : 0);
-        if (lead) mbar_expect_tx(&full[stage], 2 * bytes);  // both CTAs' copies
-        if (sa > 0) tma_load_3d_cg2(sb, &tmA, kb * ROW, ra, sa - 1, fb);
-        if (tb > 0) tma_load_3d_cg2(sb + TILE, &tmB, kb * ROW, rb, tb - 1, fb);
-        issued[stage] = 1;
-        issued_phase[stage] = phase;
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      auto release = [&](int site) -> bool {  // waits for the oldest step
+        if (!mbar_wait(&empty[head % STEPS], (head / STEPS) & 1, abort_flag, g.err, site, g.wait_ns)) return false;
+        room += (counts >> (4 * (head % STEPS))) & 15;
+        head++;
+        return true;
+      };
+      // a step: A digits sa and s1 (0: none) and B digit tb of K-step kb
+      auto fill = [&](int kb, int ra, int sa, int s1, int rb, int tb) -> bool {
+        const int count = (sa > 0) + (s1 > 0) + 1;
+        while (room < count || tail - head == STEPS)
+          if (!release(41)) return false;
+        const int s = tail % STEPS;
+        const uint32_t fb = lead_full + 8u * (uint32_t)s;
+        if (lead) mbar_expect_tx(&full[s], 2 * count * TILE);  // both CTAs' copies
+        auto load = [&](const CUtensorMap* tm, int row, int digit) {
+          tma_load_3d_cg2(smem + pos * TILE, tm, kb * ROW, row, digit - 1, fb);
+          if (++pos == TILES) pos = 0;
+        };
+        if (sa > 0) load(&tmA, ra, sa);
+        if (s1 > 0) load(&tmA, ra, s1);
+        load(&tmB, rb, tb);
+        counts = (counts & ~(15u << (4 * s))) | ((uint32_t)count << (4 * s));
+        room -= count;
+        tail++;
         return true;
       };
 #pragma unroll 1
@@ -347,30 +362,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
           const Pass P = dg_pass(U, i);
 #pragma unroll 1
           for (int kb = 0; kb < U.nk && ok; kb++) {
-            if (P.pro) ok = fill(U.kb + kb, ra, P.L + 1 - P.tlo, rb, 0);
 #pragma unroll 1
-            for (int t = P.tlo; t <= P.thi && ok; t++) ok = fill(U.kb + kb, ra, P.L - t, rb, t);
+            for (int t = P.tlo; t <= P.thi && ok; t++)
+              ok = fill(U.kb + kb, ra, P.L - t, P.pro && t == P.tlo ? P.L + 1 - t : 0, rb, t);
           }
         }
       }
       if (ok) {
-        // every stage filled so far has been released by the leader's MMAs:
-        // no multicast commit is still on its way to this CTA
-#pragma unroll 1
-        for (int i = 0; i < STAGES; i++) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, g.err, 45, g.wait_ns)) break;
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
-        }
+        // every step filled so far has been released by the leader's MMAs: no
+        // multicast commit is still on its way to this CTA
+        while (head != tail)
+          if (!release(45)) break;
       } else if (lead) {
         const uint64_t deadline = globaltimer_ns() + WAIT_NS;
-        for (int s = 0; s < STAGES; s++)
-          if (issued[s]) mbar_drain_until(&full[s], issued_phase[s], deadline);
+        for (; head != tail; head++) mbar_drain_until(&full[head % STEPS], (head / STEPS) & 1, deadline);
       }
     }
   } else if (warp == 1) {
     if (lane == 0 && lead) {
-      int stage = 0;
-      uint32_t phase = 0, q = 0;
+      uint32_t step = 0, q = 0;
+      int pos = 0;
       bool ok = true, any = false;
 #pragma unroll 1
       for (int u = cid; u < units && ok; u += ncl) {
@@ -401,42 +412,45 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
             const int k1 = min(U.nk, k0 + P.chunk);
 #pragma unroll 1
             for (int kb = k0; kb < k1 && ok; kb++) {
-              int prev = -1;  // the stage whose A tile level L + 1 uses next
-              if (P.pro) {
-                if (!mbar_wait(&full[stage], phase, abort_flag, g.err, 43, g.wait_ns)) { ok = false; break; }
-                prev = stage;
-                if (++stage == STAGES) { stage = 0; phase ^= 1; }
-              }
+              // the A tile level L + 1 uses next and the step it came with
+              uint64_t a1 = 0;
+              int from = -1;
 #pragma unroll 1
-              for (int t = P.tlo; t <= P.thi; t++) {
-                if (!mbar_wait(&full[stage], phase, abort_flag, g.err, 43, g.wait_ns)) { ok = false; break; }
+              for (int t = P.tlo; t <= P.thi; t++, step++) {
+                const int s = step % STEPS;
+                if (!mbar_wait(&full[s], (step / STEPS) & 1, abort_flag, g.err, 43, g.wait_ns)) { ok = false; break; }
                 tc_fence_after();
-                uint8_t* sb = smem + stage * STAGE;
-                const uint64_t b = desc_sw128(sb + TILE);
-                if (P.L - t >= 1) {
-                  const uint64_t a = desc_sw128(sb);
+                auto next = [&]() {
+                  const uint64_t d = ring + (uint64_t)(pos * (TILE >> 4));
+                  if (++pos == TILES) pos = 0;
+                  return d;
+                };
+                const bool has0 = P.L - t >= 1, first = P.pro && t == P.tlo;
+                const uint64_t a0 = has0 ? next() : 0;
+                if (first) a1 = next();
+                const uint64_t b = next();
+                if (has0) {
 #pragma unroll
                   for (int kk = 0; kk < ROW / 32; kk++) {
-                    mma_f8_cg2(tbase, a + 2 * kk, b + 2 * kk, DG_IDESC, use0);
+                    mma_f8_cg2(tbase, a0 + 2 * kk, b + 2 * kk, DG_IDESC, use0);
                     use0 = 1;
                   }
                 }
-                if (prev >= 0) {
-                  const uint64_t a = desc_sw128(smem + prev * STAGE);
+                if (first || from >= 0) {
 #pragma unroll
                   for (int kk = 0; kk < ROW / 32; kk++) {
-                    mma_f8_cg2(tbase + 256, a + 2 * kk, b + 2 * kk, DG_IDESC, use1);
+                    mma_f8_cg2(tbase + 256, a1 + 2 * kk, b + 2 * kk, DG_IDESC, use1);
                     use1 = 1;
                   }
-                  mma_commit_cg2(&empty[prev], BOTH);
+                  if (from >= 0) mma_commit_cg2(&empty[from], BOTH);
                 }
                 any = true;
-                prev = P.has1 ? stage : -1;
-                if (!P.has1) mma_commit_cg2(&empty[stage], BOTH);
-                if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                // (the last step's A tile has no further use)
+                a1 = a0;
+                from = P.has1 && t < P.thi ? s : -1;
+                if (from < 0) mma_commit_cg2(&empty[s], BOTH);
               }
               if (!ok) break;
-              if (prev >= 0) mma_commit_cg2(&empty[prev], BOTH);
             }
             if (!ok) break;
             mma_commit_cg2(tfull, BOTH);
