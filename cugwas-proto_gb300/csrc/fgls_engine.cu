@@ -69,8 +69,13 @@ struct fglsgpu_engine {
   double prof_ms[FGLSGPU_PROF_CLASSES] = {0};
   long long prof_cnt[FGLSGPU_PROF_CLASSES] = {0};
   // adjoint state (eigen, FP64): allocated by fglsgpu_adjoint_reset
-  double *aWc = nullptr, *aAYLc = nullptr, *aAYLs = nullptr, *atopc = nullptr, *atops = nullptr, *areml = nullptr;
-  double *aGYLc = nullptr, *aGYLs = nullptr, *aGRc = nullptr, *aGRs = nullptr, *acontrib = nullptr, *ag = nullptr;
+  // the d-, c- and s-weighted operands side by side, so that a block's Gram terms
+  // are two products: aAYL3 n x 3 t(1+wXL), aW3 n x 3 t, their results aG3
+  double *aAYL3 = nullptr, *aW3 = nullptr, *atopc = nullptr, *atops = nullptr, *areml = nullptr;
+  double *aG3 = nullptr, *acontrib = nullptr, *ag = nullptr;
+  void* adjmem = nullptr;  // their digits
+  DigitMat aayl3, aw3;
+  bool adj_cut = false;
   double *agR = nullptr, *aacc = nullptr, *aU = nullptr, *aV2 = nullptr;
   bool adj_ready = false;
   // FP64 products through digits (fgls_digit_gemm.cu): the resident operands,
@@ -173,8 +178,7 @@ void free_all(fglsgpu_engine* e) {
   void* ptrs[] = {e->dPhi, e->dL,   e->dZ,    e->dW,    e->dXL,   e->dY,    e->dh,    e->dsig, e->dWY,
                   e->dZtXL, e->dZtY, e->ddinv, e->dAYL, e->dtop, e->deigwork, e->dX[0], e->dX[1], e->dWork,
                   e->dQ,   e->dGYL, e->dGR,  e->dB[0], e->dB[1], e->dV[0], e->dV[1], e->dU8, e->dst,
-                  e->aWc, e->aAYLc, e->aAYLs, e->atopc, e->atops, e->areml, e->aGYLc, e->aGYLs, e->aGRc,
-                  e->aGRs, e->acontrib, e->ag, e->agR, e->aacc, e->aU, e->aV2, e->dSE[0], e->dSE[1], e->dP[0],
+                  e->aAYL3, e->aW3, e->atopc, e->atops, e->areml, e->aG3, e->adjmem, e->acontrib, e->ag, e->agR, e->aacc, e->aU, e->aV2, e->dSE[0], e->dSE[1], e->dP[0],
                   e->dP[1], e->dXw, e->zmem, e->wmem, e->blkmem, e->dLinv, e->ddiag, e->dWraw, e->remlmem};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -287,7 +291,7 @@ void drop_digits(fglsgpu_engine* e) {
     *q = nullptr;
   }
   e->blk_bytes = 0;
-  e->z_cut = e->w_cut = e->linv_cut = false;
+  e->z_cut = e->w_cut = e->linv_cut = e->adj_cut = false;
 }
 
 // The workspace of the digit products; null when the device cannot run them.
@@ -1102,16 +1106,12 @@ int fglsgpu_adjoint_reset(fglsgpu_engine* e) {
     auto chk = [&](cudaError_t x) {
       if (r == cudaSuccess) r = x;
     };
-    chk(dalloc(&e->aWc, n * 2 * t));
-    chk(dalloc(&e->aAYLc, n * t * (1 + wXL)));
-    chk(dalloc(&e->aAYLs, n * t * (1 + wXL)));
+    chk(dalloc(&e->aW3, n * 3 * t));
+    chk(dalloc(&e->aAYL3, n * 3 * t * (1 + wXL)));
     chk(dalloc(&e->atopc, t * (wXL + wXL * wXL)));
     chk(dalloc(&e->atops, t * (wXL + wXL * wXL)));
     chk(dalloc(&e->areml, 2 * t));
-    chk(dalloc(&e->aGYLc, xb * t * (1 + wXL)));
-    chk(dalloc(&e->aGYLs, xb * t * (1 + wXL)));
-    chk(dalloc(&e->aGRc, xb * t));
-    chk(dalloc(&e->aGRs, xb * t));
+    chk(dalloc(&e->aG3, xb * 3 * t * (2 + wXL)));
     chk(dalloc(&e->acontrib, 2 * t * xb));
     chk(dalloc(&e->ag, t * xb * p));
     chk(dalloc(&e->agR, xb * t));
@@ -1124,9 +1124,28 @@ int fglsgpu_adjoint_reset(fglsgpu_engine* e) {
   cudaStream_t s = e->comp;
   ENG_TRY(e, cudaMemsetAsync(e->aacc, 0, sizeof(double) * (2 * t + t * wXL), s), "adjoint reset");
   ENG_TRY(e, cudaMemsetAsync(e->aU, 0, sizeof(double) * n * t, s), "adjoint reset");
-  ENG_TRY(e, adjoint_traits(s, c.n, c.t, c.wXL, e->dW, e->dh, e->dsig, e->dZtXL, e->dZtY, e->ddinv, e->aWc,
-                            e->aAYLc, e->aAYLs, e->atopc, e->atops, e->areml),
+  const long long nyl = n * t * (1 + wXL);
+  ENG_TRY(e, cudaMemcpyAsync(e->aAYL3, e->dAYL, sizeof(double) * nyl, cudaMemcpyDeviceToDevice, s), "adjoint weights");
+  ENG_TRY(e, cudaMemcpyAsync(e->aW3, e->ddinv, sizeof(double) * n * t, cudaMemcpyDeviceToDevice, s), "adjoint weights");
+  ENG_TRY(e, adjoint_traits(s, c.n, c.t, c.wXL, e->dW, e->dh, e->dsig, e->dZtXL, e->dZtY, e->ddinv, e->aW3 + n * t,
+                            e->aAYL3 + nyl, e->aAYL3 + 2 * nyl, e->atopc, e->atops, e->areml),
           "adjoint weights");
+  // digits of the weighted operands, when the blocks run on digits
+  e->adj_cut = false;
+  bool digits = false;
+  const int rc = eigen_digits(e, xb, &digits);
+  if (rc) return rc;
+  if (digits) {
+    const size_t yb = (digit_mat_bytes((int)(3 * t * (1 + wXL)), c.n) + 255) & ~(size_t)255;
+    size_t none = 0;
+    if (e->adjmem || grow(&e->adjmem, &none, yb + digit_mat_bytes((int)(3 * t), c.n))) {
+      e->aayl3 = digit_mat_at(e->adjmem, (int)(3 * t * (1 + wXL)), c.n);
+      e->aw3 = digit_mat_at((char*)e->adjmem + yb, (int)(3 * t), c.n);
+      ENG_TRY(e, digit_cut(s, e->aayl3, e->aAYL3, n, true), "adjoint digits");
+      ENG_TRY(e, digit_cut(s, e->aw3, e->aW3, n, true), "adjoint digits");
+      e->adj_cut = true;
+    }
+  }
   ENG_TRY(e, cudaStreamSynchronize(s), "adjoint reset");
   return FGLSGPU_OK;
 }
@@ -1140,21 +1159,35 @@ int fglsgpu_adjoint_block_device(fglsgpu_engine* e, const double* dXR, int x, co
   const int n = c.n, t = c.t, wXL = c.wXL, p = e->p, nq = t * (1 + wXL);
   cudaStream_t s = e->comp;
   // recompute R = Z^T X and the d-, c- and s-weighted Gram blocks (never stored per SNP)
-  ENG_TRY(e, dgemm(s, true, false, n, x, n, 1.0, e->dZ, n, dXR, n, 0.0, e->dWork, n), "Z^T XR");
-  ENG_TRY(e, quad_products(s, n, x, 1, e->dWork, n, e->dQ, n), "quad");
-  ENG_TRY(e, dgemm(s, true, false, x, nq, n, 1.0, e->dWork, n, e->dAYL, n, 0.0, e->dGYL, x), "gram");
-  ENG_TRY(e, dgemm(s, true, false, x, t, n, 1.0, e->dQ, n, e->ddinv, n, 0.0, e->dGR, x), "gram");
-  ENG_TRY(e, dgemm(s, true, false, x, nq, n, 1.0, e->dWork, n, e->aAYLc, n, 0.0, e->aGYLc, x), "gram c");
-  ENG_TRY(e, dgemm(s, true, false, x, t, n, 1.0, e->dQ, n, e->aWc, n, 0.0, e->aGRc, x), "gram c");
-  ENG_TRY(e, dgemm(s, true, false, x, nq, n, 1.0, e->dWork, n, e->aAYLs, n, 0.0, e->aGYLs, x), "gram s");
-  ENG_TRY(e, dgemm(s, true, false, x, t, n, 1.0, e->dQ, n, e->aWc + (long long)n * t, n, 0.0, e->aGRs, x),
-          "gram s");
-  ENG_TRY(e, adjoint_snps(s, p, x, t, wXL, e->dtop, e->dGYL, e->dGR, e->atopc, e->aGYLc, e->aGRc, e->atops,
-                          e->aGYLs, e->aGRs, dBbar, bstr, e->acontrib, e->ag, e->dst),
+  double* GYL = e->aG3;
+  double* GR = e->aG3 + (long long)x * 3 * nq;
+  bool digits = false;
+  if (e->adj_cut) {
+    const int rc = eigen_digits(e, x, &digits);
+    if (rc) return rc;
+  }
+  if (digits) {
+    const DigitMat xd = digit_mat_at(e->blkmem, x, n);
+    ENG_TRY(e, digit_cut(s, xd, dXR, n, true), "digits of XR");
+    ENG_TRY(e, digit_mul(e->dg, s, e->zdig, xd, 1.0, 0.0, e->dWork, n), "Z^T XR");
+    ENG_TRY(e, digit_cut(s, xd, e->dWork, n, true), "digits of Z^T XR");
+    ENG_TRY(e, digit_mul(e->dg, s, xd, e->aayl3, 1.0, 0.0, GYL, x), "gram");
+    ENG_TRY(e, digit_cut_products(s, xd, e->dWork, n, 1), "digits of the squares");
+    ENG_TRY(e, digit_mul(e->dg, s, xd, e->aw3, 1.0, 0.0, GR, x), "gram");
+  } else {
+    ENG_TRY(e, dgemm(s, true, false, n, x, n, 1.0, e->dZ, n, dXR, n, 0.0, e->dWork, n), "Z^T XR");
+    ENG_TRY(e, quad_products(s, n, x, 1, e->dWork, n, e->dQ, n), "quad");
+    ENG_TRY(e, dgemm(s, true, false, x, 3 * nq, n, 1.0, e->dWork, n, e->aAYL3, n, 0.0, GYL, x), "gram");
+    ENG_TRY(e, dgemm(s, true, false, x, 3 * t, n, 1.0, e->dQ, n, e->aW3, n, 0.0, GR, x), "gram");
+  }
+  const long long yl = (long long)x * nq, r = (long long)x * t;
+  ENG_TRY(e, adjoint_snps(s, p, x, t, wXL, e->dtop, GYL, GR, e->atopc, GYL + yl, GR + r, e->atops, GYL + 2 * yl,
+                          GR + 2 * r, dBbar, bstr, e->acontrib, e->ag, e->dst),
           "adjoint solve");
   ENG_TRY(e, adjoint_reduce(s, x, t, p, wXL, e->acontrib, e->ag, e->aacc, e->agR), "adjoint reduce");
   // U += R gR  (the SNP part of sum_i V_i g_i, accumulated over blocks)
-  ENG_TRY(e, dgemm(s, false, false, n, t, x, 1.0, e->dWork, n, e->agR, x, 1.0, e->aU, n), "dy accumulate");
+  ENG_TRY(e, digit_dgemm(digits ? e->dg : nullptr, s, false, false, n, t, x, 1.0, e->dWork, n, e->agR, x, 1.0, e->aU, n),
+          "dy accumulate");
   return FGLSGPU_OK;
 }
 
@@ -1172,7 +1205,8 @@ int fglsgpu_adjoint_read(fglsgpu_engine* e, double* dh, double* dsigma, double* 
     // dY = Z V2 (original basis), through dQ as scratch (n x t <= n x x_b when t <= x_b)
     double* out = e->dQ;
     if ((long long)t > (long long)c.x_b) return fail(e, FGLSGPU_EINVAL, "dy needs t <= x_b");
-    ENG_TRY(e, dgemm(s, false, false, n, t, n, 1.0, e->dZ, n, e->aV2, n, 0.0, out, n), "dy");
+    ENG_TRY(e, digit_dgemm(e->adj_cut ? e->dg : nullptr, s, false, false, n, t, n, 1.0, e->dZ, n, e->aV2, n, 0.0, out, n),
+            "dy");
     ENG_TRY(e, cudaMemcpyAsync(dY, out, sizeof(double) * (size_t)n * t, cudaMemcpyDeviceToHost, s), "dy");
   }
   std::vector<double> acc(2 * t);
