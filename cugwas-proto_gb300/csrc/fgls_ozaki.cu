@@ -21,7 +21,7 @@
 // (and eight-bit digits would need 29 bits for a fused pair).
 //
 // Kernel ozaki_gemm_kernel (persistent: one CTA per SM takes 128 x 256
-// output tiles from a launch-wide counter, 10 warps):
+// output tiles from a launch-wide counter, 18 warps):
 //   warp 0      TMA producer: per K-step of 128 bytes (128 digits), two
 //               A-slice tiles (128 x 128) and one genotype tile (256 x 128),
 //               128B-swizzled, three 64 KB stages.
@@ -30,9 +30,9 @@
 //               slices of pass p into accumulator p % 2 (columns
 //               [256 (p % 2), 256 (p % 2) + 256)), so the MMAs of one pass run
 //               while the epilogue drains the previous one.
-//   warps 2-9   epilogue: tcgen05.ld the pass's accumulator, convert it
+//   the others  epilogue: tcgen05.ld the pass's accumulator, convert it
 //               exactly to the int32 q = 32 v = P_2p * 32 + P_2p+1,
-//               Horner-accumulate the passes in int64 in the output buffer
+//               Horner-accumulate the passes in int64 in the CTA's own part
 //               (V = V * 2^10 + q), and on the last pass write
 //               V * 2^(e_r - 9 - 10 (passes-1)) as FP64.  |V| < 2^62 for S <= 9.
 // Every mbarrier wait is bounded; on expiry the kernel raises an error flag,
@@ -94,7 +94,18 @@ struct GemmRing {
 };
 constexpr int GBK = GemmRing::ROW;  // digits per K-step (the tensor maps' box)
 constexpr int SMEM_BYTES = GemmRing::SMEM;
-constexpr int THREADS = 320;  // producer, MMA, 8 epilogue warps
+constexpr int THREADS = 320;  // producer, MMA, 8 epilogue warps (quadratic Gram)
+// Epilogue warps of the split GEMM (32 rows x 1024 / warps columns each).  Sixteen
+// hide the latency of a pass's partial sums where the passes are short (16 cohorts of
+// 500 .. 4000: 1.50 ms a step, 1.61 with eight; n = 750: 102 and 105 us); over long
+// uniform K the epilogue is hidden anyway and eight leave the MMAs more (n = 10000,
+// 16384 SNPs: 9.8 ms a step, 10.1 with sixteen).
+constexpr int EPI_WARPS = 16;
+constexpr int EPI_WARPS_LONG = 8;
+constexpr int LONG_K = 4096;  // from this K on, uniform tiles run with EPI_WARPS_LONG
+constexpr int gemm_threads(int epi_warps) { return 64 + 32 * epi_warps; }
+constexpr int GEMM_THREADS = gemm_threads(EPI_WARPS);
+constexpr int PART = BM * BN / 2;               // longlong2 partial sums of a CTA's tile (256 KB)
 constexpr int MAX_SLICES = 9;   // FP8 digit slices; |V| < 2^62 in the epilogue
 constexpr int FUSED_KMAX = 16368;  // K of the FP8 split GEMM: (32 + 1/32) K < 2^19
 constexpr int DEFAULT_SLICES = 9;
@@ -114,7 +125,8 @@ struct GemmArgs {
   int tiles_m, tiles_n;
   int tri_rows;     // rows [0, tri_rows) of A are lower triangular in K (0: none)
   const double* row_scale;  // per row 2^(e_r - 9 - 10 (passes-1))
-  double* C;        // output, column-major, ld = ldc (int64 between passes)
+  double* C;        // output, column-major, ld = ldc
+  longlong2* part;  // PART partial sums of each CTA of the launch, [column / 2][row]
   long long ldc;
   int col0;         // first genotype column of this launch (TMA row offset of G)
   int sq_rows;      // rows [0, sq_rows): write (C^2) as an error-free float pair (hi, lo)
@@ -269,100 +281,93 @@ __device__ __forceinline__ void pair_add(float ah, float al, float bh, float bl,
   l = __fadd_rn(e, __fadd_rn(al, bl));
 }
 
-// Column sums over a warp's 32 rows.  Five exchange-and-add rounds with
-// lane offsets 16, 8, 4, 2, 1, each lane keeping the half of its columns
-// named by its lane bit, leave the sum of column `lane` with that lane; the
-// order of the additions is fixed.  The caller runs the first round (offset
-// 16, 32 -> 16 columns) as it forms the values; this runs the other four on
-// lane k's 16 partial sums (h[c], l[c]), leaving column `lane` in (h[0], l[0]).
+// Sixteen columns' sums over a warp's 32 rows (float pairs h, l): lane bit 4, 3, 2, 1
+// picks the half of the columns a lane keeps, the last round adds lane pairs; lane
+// ends with column (lane >> 1)'s sum, bits 4..1 of the lane in that order.  Rows are
+// paired by offsets 16, 8, 4, 2, 1.
 __device__ __forceinline__ void warp_column_sums(float (&h)[16], float (&l)[16], int lane) {
 #pragma unroll
-  for (int o = 8; o >= 1; o >>= 1) {
+  for (int o = 16; o >= 2; o >>= 1) {
     const bool up = (lane & o) != 0;
 #pragma unroll
-    for (int k = 0; k < o; k++) {
-      const float sh = up ? h[k] : h[k + o], sl = up ? l[k] : l[k + o];
-      const float kh = up ? h[k + o] : h[k], kl = up ? l[k + o] : l[k];
+    for (int k = 0; k < o / 2; k++) {
+      const float sh = up ? h[k] : h[k + o / 2], sl = up ? l[k] : l[k + o / 2];
+      const float kh = up ? h[k + o / 2] : h[k], kl = up ? l[k + o / 2] : l[k];
       const float rh = __shfl_xor_sync(0xffffffffu, sh, o), rl = __shfl_xor_sync(0xffffffffu, sl, o);
       pair_add(kh, kl, rh, rl, h[k], l[k]);
     }
   }
+  const float rh = __shfl_xor_sync(0xffffffffu, h[0], 1), rl = __shfl_xor_sync(0xffffffffu, l[0], 1);
+  pair_add(h[0], l[0], rh, rl, h[0], l[0]);
 }
 
-// One pass of the split GEMM's epilogue for one thread (one output row,
-// `cend` columns of its half tile from `crow`, stride ldc): read the pass's
-// accumulator (P_2p + P_2p+1 / 32) from TMEM at `tacc` 32 columns at a time,
-// form the exact int32 q = 32 v = P_2p * 32 + P_2p+1, and fold it into the
-// int64 partial sums in C (V = V * 2^10 + q), or on the last pass write V
-// times the row scale (FP64, or squared as a float pair for rows `sq`).
+// Pass p of a tile for one epilogue warp (32 rows, its columns from the first): V = V * 2^10 + q with the exact pair sum q in TMEM at tacc.  Between
+// passes V lives in the CTA's own part (16 bytes a thread, 512 a warp and access;
+// L2-resident, since a CTA writes the same 256 KB for every tile), not in C: there
+// the sums of a launch are as large as C, and each went to DRAM and back.  The last
+// pass writes C, V times the row scale (FP64, or squared as a float pair for rows
+// `sq`); `cols` of the warp's columns are valid for all rows, `cend` of this row's.
 // With `qrow` set (warp-uniform: the warp's 32-row group holds rows `sq` of a
-// unit-weight problem) the last pass writes no squares: the warp sums them
-// over its rows and lane k writes column c0 + k's sum to qrow[c0 + k] for
-// the `qend` valid columns of the half tile; rows not `sq` still write FP64.
+// unit-weight problem) the last pass writes no squares: the warp sums them over its
+// rows and writes column c's sum to qrow[c]; rows not `sq` still write FP64.
 __device__ __forceinline__ void epilogue_pass(uint32_t tacc, int p, bool last, bool sq, double scale, float fscale,
-                                              long long* crow, long long ldc, int cend, float2* qrow, int qend) {
+                                              longlong2* part, double* crow, long long ldc, int cols, int cend,
+                                              float2* qrow) {
   const int lane = threadIdx.x & 31;
-  // The int64 partial sums live from one pass to the next (~50 us, while the
-  // other CTAs stream ~0.5 GB of operand tiles through L2): stored with
-  // evict-last priority and read back, their last use, with evict-first, so
-  // that they stay in L2 instead of making a DRAM round trip.
-  uint64_t pol_keep, pol_drop;
+  uint64_t pol_keep;  // the operand stream (~0.5 GB a pass over all CTAs) must not push the sums out
   asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_keep));
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_drop));
 #pragma unroll 1
-  for (int ch = 0; ch < BN / 64; ch++) {
-    const int c0 = ch * 32;
-    long long prev[32];
+  for (int c0 = 0; c0 < cols; c0 += 16) {
+    longlong2 prev[8];
+    longlong2* pp = part + (c0 >> 1) * BM;
     if (p > 0) {
-      // all 32 partial sums in flight at once, before the TMEM reads
 #pragma unroll
-      for (int j = 0; j < 32; j++) {
-        long long t = 0;
-        if (c0 + j < cend)
-          asm volatile("ld.global.cg.L2::cache_hint.b64 %0, [%1], %2;"
-                       : "=l"(t)
-                       : "l"(crow + (long long)(c0 + j) * ldc), "l"(pol_drop));
-        prev[j] = t;
-      }
+      for (int j = 0; j < 8; j++)
+        asm volatile("ld.global.cg.L2::cache_hint.v2.b64 {%0, %1}, [%2], %3;"
+                     : "=l"(prev[j].x), "=l"(prev[j].y)
+                     : "l"(pp + j * BM), "l"(pol_keep));
     }
-    uint32_t v[32];
-    tmem_ld32(tacc + c0, v);
+    uint32_t v[16];
+    tmem_ld16(tacc + c0, v);
     tmem_ld_wait();
-    if (last && qrow != nullptr) {
-      // column j's square as a float pair (0 past cend; rows not sq write FP64)
-      auto term = [&](int j) -> float2 {
-        if (c0 + j >= cend) return make_float2(0.0f, 0.0f);
-        const int qv = fused_pair_f2i(__uint_as_float(v[j]));
-        const long long V = (p == 0) ? (long long)qv : prev[j] * 1024ll + (long long)qv;
-        if (sq) return square_pair(V, fscale);
-        *(double*)(crow + (long long)(c0 + j) * ldc) = (double)V * scale;
-        return make_float2(0.0f, 0.0f);
-      };
-      float h[16], l[16];
-      const bool up = (lane & 16) != 0;
+    auto value = [&](int j) -> long long {
+      const long long q = fused_pair_f2i(__uint_as_float(v[j]));
+      if (p == 0) return q;
+      return (j & 1 ? prev[j >> 1].y : prev[j >> 1].x) * 1024ll + q;
+    };
+    if (!last) {
 #pragma unroll
-      for (int k = 0; k < 16; k++) {  // the offset-16 round: columns k and k + 16
-        const float2 a = term(k), b = term(k + 16);
-        const float2 send = up ? a : b, keep = up ? b : a;
-        const float rh = __shfl_xor_sync(0xffffffffu, send.x, 16), rl = __shfl_xor_sync(0xffffffffu, send.y, 16);
-        pair_add(keep.x, keep.y, rh, rl, h[k], l[k]);
+      for (int j = 0; j < 8; j++)
+        asm volatile("st.global.L2::cache_hint.v2.b64 [%0], {%1, %2}, %3;" ::"l"(pp + j * BM), "l"(value(2 * j)),
+                     "l"(value(2 * j + 1)), "l"(pol_keep)
+                     : "memory");
+    } else if (qrow != nullptr) {
+      float h[16], l[16];
+#pragma unroll
+      for (int j = 0; j < 16; j++) {  // column j's square as a float pair (0 past cend; rows not sq write FP64)
+        h[j] = l[j] = 0.0f;
+        if (c0 + j >= cend) continue;
+        const long long V = value(j);
+        if (sq) {
+          const float2 t = square_pair(V, fscale);
+          h[j] = t.x;
+          l[j] = t.y;
+        } else {
+          crow[(long long)(c0 + j) * ldc] = (double)V * scale;
+        }
       }
       warp_column_sums(h, l, lane);
-      if (c0 + lane < qend) qrow[c0 + lane] = make_float2(h[0], l[0]);
-      continue;
-    }
+      const int c = c0 + (lane >> 1);
+      if (!(lane & 1) && c < cols) qrow[c] = make_float2(h[0], l[0]);
+    } else {
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
-      if (c0 + j >= cend) break;
-      const int qv = fused_pair_f2i(__uint_as_float(v[j]));
-      long long* cp = crow + (long long)(c0 + j) * ldc;
-      const long long V = (p == 0) ? (long long)qv : prev[j] * 1024ll + (long long)qv;
-      if (!last)
-        asm volatile("st.global.L2::cache_hint.b64 [%0], %1, %2;" ::"l"(cp), "l"(V), "l"(pol_keep) : "memory");
-      else if (sq)
-        *(float2*)cp = square_pair(V, fscale);
-      else
-        *(double*)cp = (double)V * scale;
+      for (int j = 0; j < 16; j++) {
+        if (c0 + j >= cend) break;
+        const long long V = value(j);
+        double* cp = crow + (long long)(c0 + j) * ldc;
+        if (sq) *(float2*)cp = square_pair(V, fscale);
+        else *cp = (double)V * scale;
+      }
     }
   }
 }
@@ -379,7 +384,7 @@ __device__ __forceinline__ void epilogue_pass(uint32_t tacc, int p, bool last, b
 // pair (next tile, finished CTAs) starts at zero; the last CTA to finish
 // zeroes it again for the next launch on the stream, so no reset is enqueued.
 constexpr int TQ = 4;                // tile-queue slots
-constexpr int TQ_CONSUMERS = 1 + 8;  // the MMA thread and lane 0 of each epilogue warp
+constexpr int TQ_CONSUMERS = 1 + EPI_WARPS;  // the MMA thread and lane 0 of each epilogue warp
 
 // Persistent one-SM split GEMM: each CTA takes tiles from the launch-wide
 // counter (or a static deal) until none are left; per tile, (S + 1) / 2
@@ -420,7 +425,7 @@ __device__ __forceinline__ void gemm_persistent(const Src& src, int* tile_counte
     }
     for (int b = 0; b < 2; b++) {
       mbar_init(&tfull[b], 1);
-      mbar_init(&tempty[b], THREADS - 64);
+      mbar_init(&tempty[b], GEMM_THREADS - 64);
     }
     mbar_init(drain, 1);
     for (int s = 0; s < TQ; s++) {
@@ -568,12 +573,13 @@ __device__ __forceinline__ void gemm_persistent(const Src& src, int* tile_counte
     }
     __syncwarp();
   } else {
-    // epilogue: warps 2..9.  Warp w reads TMEM lane quarter w % 4 (the
+    // epilogue: the other warps.  Warp w reads TMEM lane quarter w % 4 (the
     // quarter a warp may access is fixed by its rank modulo 4) and column
-    // half (w - 2) / 4; thread = one output row.
+    // range (w - 2) / 4; thread = one output row.
     const int lq = warp & 3;
-    const int cbeg = ((warp - 2) >> 2) * (BN / 2);
+    const int cbeg = ((warp - 2) >> 2) * (BN * 4 / EPI_WARPS);
     const int row = lq * 32 + lane;
+    longlong2* part = nullptr;
     const uint32_t ta = tbase + ((uint32_t)(lq * 32) << 16) + (uint32_t)cbeg;
     uint32_t q = 0;
     bool ok = true;
@@ -604,32 +610,25 @@ __device__ __forceinline__ void gemm_persistent(const Src& src, int* tile_counte
       const bool sq = r < g.sq_rows;
       const float fscale = (float)scale;  // power of two: exact while >= 2^-149
       const int ncols = rvalid ? min(BN, T.N - n0) : 0;  // valid columns of this tile for this row
-      const int cend = min(BN / 2, ncols - cbeg);        // of this thread's half (may be <= 0)
-      long long* crow = (long long*)(g.C + (long long)r + (long long)(g.col0 + n0 + cbeg) * g.ldc);
+      const int cend = min((BN * 4 / EPI_WARPS), ncols - cbeg);      // of this warp's columns (may be <= 0)
+      double* crow = g.C + (long long)r + (long long)(g.col0 + n0 + cbeg) * g.ldc;
+      part = g.part + (size_t)blockIdx.x * PART + (cbeg >> 1) * BM + row;
       // unit weights: this warp's 32-row group (rows r & ~31 ..) sums its squares
       float2* qrow = (g.sqsum != nullptr && (r & ~31) < g.sq_rows)
                          ? g.sqsum + (long long)(r >> 5) * g.ldq + (g.col0 + n0 + cbeg)
                          : nullptr;
-      const int qend = min(BN / 2, min(BN, T.N - n0) - cbeg);
+      const int cols = min((BN * 4 / EPI_WARPS), min(BN, T.N - n0) - cbeg);
       const int passes = (g.S + 1) / 2;
 #pragma unroll 1
       for (int p = 0; p < passes; p++, q++) {
         const bool last = p == passes - 1;
         const uint32_t buf = q & 1, par = (q >> 1) & 1;
-        // pull this row's partial sums (written a pass ago) back into L2
-        // while the pass's MMAs run, if the evict-last policy did not keep
-        // them.  Only for uniform long-K tiles: with the short passes of the
-        // triangular and grouped operands the instructions cost more than
-        // they save (grouped cohorts: 29.5 against 27.9 ms per launch).
-        if (p > 0 && !src.dynamic())
-          for (int c = 0; c < cend; c++)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(crow + (long long)c * g.ldc));
         int okw = 1;
         if (lane == 0) okw = mbar_wait(&tfull[buf], par, abort_flag, g.err, 4, g.wait_ns) ? 1 : 0;
         okw = __shfl_sync(0xffffffffu, okw, 0);  // warp-uniform: tcgen05.ld is .sync.aligned
         if (!okw) { ok = false; break; }
         tc_fence_after();
-        epilogue_pass(ta + 256 * buf, p, last, sq, scale, fscale, crow, g.ldc, cend, qrow, qend);
+        epilogue_pass(ta + 256 * buf, p, last, sq, scale, fscale, part, crow, g.ldc, cols, cend, qrow);
         tc_fence_before();
         mbar_arrive(&tempty[buf]);
       }
@@ -652,7 +651,7 @@ __device__ __forceinline__ void gemm_persistent(const Src& src, int* tile_counte
 
 // Single problem: at most one CTA per SM (launch with min(tiles, SMs) CTAs);
 // tile_counter: two ints, zero before the first launch.
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
     ozaki_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ GemmArgs g, int* tile_counter) {
   const SingleTiles src{&tmA, &tmB, &g, -1};
@@ -692,13 +691,11 @@ constexpr int STAGES = 4;
 constexpr int SMEM = STAGES * STAGE + 1024 + 256;
 // kind::f8f6f4: D=F32, A=B=E4M3, K-major, N=256, M=256 (the pair)
 constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
-constexpr int EPI_WARPS = 8;
 }  // namespace p2
 
-template <class Src>
+template <int EW, class Src>
 __device__ __forceinline__ void gemm_pair(const Src& src, int* tile_counter) {
   constexpr int ROW = p2::ROW, A = p2::A, B = p2::B, STAGE = p2::STAGE, STAGES = p2::STAGES;
-  constexpr int EPI_WARPS = p2::EPI_WARPS;
   constexpr uint32_t IDESC = p2::IDESC;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -727,14 +724,14 @@ __device__ __forceinline__ void gemm_pair(const Src& src, int* tile_counter) {
     }
     for (int b = 0; b < 2; b++) {
       mbar_init(&tfull[b], 1);
-      mbar_init(&tempty[b], 2 * EPI_WARPS);
+      mbar_init(&tempty[b], 2 * EW);
     }
     mbar_init(drain, 1);
     for (int s = 0; s < TQ; s++) {
       mbar_init(&tq_full[s], 1);
       // consumers of a queue slot: the leader's MMA thread and both CTAs'
       // epilogue warps and the peer's producer
-      mbar_init(&tq_empty[s], 2 * (1 + EPI_WARPS));
+      mbar_init(&tq_empty[s], 2 * (1 + EW));
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -938,11 +935,12 @@ __device__ __forceinline__ void gemm_pair(const Src& src, int* tile_counter) {
     }
     __syncwarp();
   } else {
-    // epilogue: warps 2..9 of each CTA drain that CTA's 128 rows, as in the
+    // epilogue: the other warps of each CTA drain that CTA's 128 rows, as in the
     // one-SM kernel; one arrival per warp on the leader's tempty
     const int lq = warp & 3;
-    const int cbeg = ((warp - 2) >> 2) * (BN / 2);
+    const int cbeg = ((warp - 2) >> 2) * (BN * 4 / EW);
     const int row = lq * 32 + lane;
+    longlong2* part = nullptr;
     const uint32_t ta = tbase + ((uint32_t)(lq * 32) << 16) + (uint32_t)cbeg;
     const uint32_t lead_tempty = cluster_addr(tempty, 0);
     uint32_t q = 0;
@@ -974,27 +972,25 @@ __device__ __forceinline__ void gemm_pair(const Src& src, int* tile_counter) {
       const bool sq = r < g.sq_rows;
       const float fscale = (float)scale;
       const int ncols = rvalid ? min(BN, T.N - n0) : 0;
-      const int cend = min(BN / 2, ncols - cbeg);
-      long long* crow = (long long*)(g.C + (long long)r + (long long)(g.col0 + n0 + cbeg) * g.ldc);
+      const int cend = min((BN * 4 / EW), ncols - cbeg);
+      double* crow = g.C + (long long)r + (long long)(g.col0 + n0 + cbeg) * g.ldc;
+      part = g.part + (size_t)blockIdx.x * PART + (cbeg >> 1) * BM + row;
       // unit weights: this warp's 32-row group (rows r & ~31 ..) sums its squares
       float2* qrow = (g.sqsum != nullptr && (r & ~31) < g.sq_rows)
                          ? g.sqsum + (long long)(r >> 5) * g.ldq + (g.col0 + n0 + cbeg)
                          : nullptr;
-      const int qend = min(BN / 2, min(BN, T.N - n0) - cbeg);
+      const int cols = min((BN * 4 / EW), min(BN, T.N - n0) - cbeg);
       const int passes = (g.S + 1) / 2;
 #pragma unroll 1
       for (int p = 0; p < passes; p++, q++) {
         const bool last = p == passes - 1;
         const uint32_t buf = q & 1, par = (q >> 1) & 1;
-        if (p > 0 && !src.dynamic())  // as in the one-SM kernel
-          for (int c = 0; c < cend; c++)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(crow + (long long)c * g.ldc));
         int okw = 1;
         if (lane == 0) okw = mbar_wait(&tfull[buf], par, abort_flag, g.err, 4, g.wait_ns) ? 1 : 0;
         okw = __shfl_sync(0xffffffffu, okw, 0);
         if (!okw) { ok = false; break; }
         tc_fence_after();
-        epilogue_pass(ta + 256 * buf, p, last, sq, scale, fscale, crow, g.ldc, cend, qrow, qend);
+        epilogue_pass(ta + 256 * buf, p, last, sq, scale, fscale, part, crow, g.ldc, cols, cend, qrow);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(lead_tempty + 8u * buf);
@@ -1035,26 +1031,27 @@ __device__ __forceinline__ void gemm_pair(const Src& src, int* tile_counter) {
 // as many clusters as fit at once.  Uniform tiles are dealt statically per
 // cluster, those of the triangular L^-1 operand (and of grouped problems)
 // taken from the launch-wide counter (two ints, zero before the first launch).
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+template <int EW>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(EW), 1)
     ozaki_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBh,
                        const __grid_constant__ GemmArgs g, int* tile_counter) {
   const SingleTiles src{&tmA, &tmBh, &g, (int)cluster_rank()};
-  gemm_pair(src, tile_counter);
+  gemm_pair<EW>(src, tile_counter);
 }
 
 // Many independent problems over a table of row-tile pairs; genotype maps in
 // 128-row boxes.
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     ozaki_grouped_gemm2_kernel(const GroupedTile* __restrict__ tiles, const GroupedProblem* __restrict__ probs,
                                const CUtensorMap* __restrict__ maps, const int* __restrict__ cols, int ntiles,
                                int* tile_counter) {
   const GroupedTiles src{tiles, probs, maps, cols, ntiles, (int)cluster_rank()};
-  gemm_pair(src, tile_counter);
+  gemm_pair<EPI_WARPS>(src, tile_counter);
 }
 
 // Many independent problems in one persistent launch over a tile table;
 // tiles past a problem's valid columns this launch are skipped by all roles.
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
     ozaki_grouped_gemm_kernel(const GroupedTile* __restrict__ tiles, const GroupedProblem* __restrict__ probs,
                               const CUtensorMap* __restrict__ maps, const int* __restrict__ cols, int ntiles,
                               int* tile_counter) {
@@ -1938,12 +1935,14 @@ int pair_clusters() {
   if (v > 0) return v - 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2);
-  cfg.blockDim = dim3(THREADS);
+  cfg.blockDim = dim3(GEMM_THREADS);
   cfg.dynamicSmemBytes = p2::SMEM;
   int n = 0;
-  if (cudaFuncSetAttribute(ozaki_gemm2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, p2::SMEM) !=
+  if (cudaFuncSetAttribute(ozaki_gemm2_kernel<EPI_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, p2::SMEM) !=
           cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, (void*)ozaki_gemm2_kernel, &cfg) != cudaSuccess) {
+      cudaFuncSetAttribute(ozaki_gemm2_kernel<EPI_WARPS_LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           p2::SMEM) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, (void*)ozaki_gemm2_kernel<EPI_WARPS>, &cfg) != cudaSuccess) {
     (void)cudaGetLastError();
     n = 0;
   }
@@ -1965,6 +1964,7 @@ struct OzakiPlan {
   uint8_t* G = nullptr;         // Ncap x Kpad E4M3 genotypes
   double* scale = nullptr;      // Mpad
   double* C = nullptr;          // Mpad x Ncap (ld Mpad)
+  longlong2* gpart = nullptr;   // the split GEMM's partial sums, PART a CTA
   double* U = nullptr;          // n x nU
   float2* D = nullptr;          // n x t weights as float pairs (eigen d_j; chol: ones)
   float* dmax = nullptr;        // t: max_l of the high part of D[:, j]
@@ -2049,6 +2049,7 @@ cudaError_t ozaki_create(OzakiPlan** out, int n, int t, int wXL, int wXR, int x_
     chk(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev));
   }
   chk(cudaMalloc(&p->err, 3 * sizeof(int)));  // [wait error word, GEMM tile counter, finished CTAs]
+  chk(cudaMalloc(&p->gpart, sizeof(longlong2) * (size_t)PART * persistent_grid(1 << 20)));
   if (!eigen) chk(cudaMalloc(&p->LinvT, sizeof(double) * (size_t)n * n));
   if (!eigen) chk(cudaMalloc(&p->sqsum, sizeof(float2) * (size_t)(p->Mpad / 32) * p->Ncap));
   if (r == cudaSuccess) chk(cudaMemset(p->A, 0, (size_t)p->S * p->Mpad * p->Kpad));
@@ -2103,7 +2104,7 @@ void ozaki_destroy(OzakiPlan* p) {
   if (!p) return;
   void* ptrs[] = {p->A,    p->G,     p->scale, p->scale_run, p->C, p->U, p->D,    p->dmax, p->amax,
                   p->part, p->LinvT, p->err,   p->Adig, p->Ddig, p->aexp, p->dexp, p->qpart,
-                  p->sqsum};
+                  p->sqsum, p->gpart};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   delete p;
@@ -2140,6 +2141,7 @@ cudaError_t run_gemm(OzakiPlan* p, cudaStream_t s, int col0, int x, int tri_rows
   g.tri_rows = tri_rows;
   g.row_scale = S_run == p->S ? p->scale : p->scale_run;
   g.C = p->C;
+  g.part = p->gpart;
   g.ldc = p->Mpad;
   g.err = p->err;
   g.wait_ns = p->wait_ns;
@@ -2151,10 +2153,14 @@ cudaError_t run_gemm(OzakiPlan* p, cudaStream_t s, int col0, int x, int tri_rows
   // else one CTA per tile
   const int pairs = ((g.tiles_m + 1) / 2) * g.tiles_n;
   const int clusters = p->has_mapBh ? pair_clusters() : 0;
-  if (clusters > 0)
-    ozaki_gemm2_kernel<<<2 * std::min(pairs, clusters), THREADS, p2::SMEM, s>>>(p->mapA, p->mapBh, g, p->err + 1);
+  if (clusters > 0 && tri_rows == 0 && p->Kpad >= LONG_K)
+    ozaki_gemm2_kernel<EPI_WARPS_LONG><<<2 * std::min(pairs, clusters), gemm_threads(EPI_WARPS_LONG), p2::SMEM, s>>>(
+        p->mapA, p->mapBh, g, p->err + 1);
+  else if (clusters > 0)
+    ozaki_gemm2_kernel<EPI_WARPS><<<2 * std::min(pairs, clusters), GEMM_THREADS, p2::SMEM, s>>>(p->mapA, p->mapBh, g,
+                                                                                              p->err + 1);
   else
-    ozaki_gemm_kernel<<<persistent_grid(g.tiles_m * g.tiles_n), THREADS, SMEM_BYTES, s>>>(p->mapA, p->mapB, g,
+    ozaki_gemm_kernel<<<persistent_grid(g.tiles_m * g.tiles_n), GEMM_THREADS, SMEM_BYTES, s>>>(p->mapA, p->mapB, g,
                                                                                           p->err + 1);
   note_launch();
   return cudaGetLastError();
@@ -2395,12 +2401,21 @@ struct GroupedGemm {
   GroupedProblem* probs = nullptr;
   CUtensorMap* maps = nullptr;
   int* counter = nullptr;  // tile counter and finished CTAs of the persistent launch
+  longlong2* part = nullptr;  // partial sums, PART a CTA
 };
 
 cudaError_t grouped_gemm_create(GroupedGemm** out, const GroupedGemmDesc* d, int count, int x_b, int* err,
                                 bool want_pair) {
   *out = nullptr;
   const bool pair = want_pair && pair_clusters() > 0;
+  longlong2* part = nullptr;
+  FGLS_CUDA_TRY(cudaMalloc(&part, sizeof(longlong2) * (size_t)PART * persistent_grid(1 << 20)));
+  struct Give {  // given back unless the plan takes it
+    longlong2** p;
+    ~Give() {
+      if (*p) cudaFree(*p);
+    }
+  } give{&part};
   std::vector<GroupedProblem> probs(count);
   std::vector<CUtensorMap> maps(2 * (size_t)count);
   std::vector<int> order(count);
@@ -2417,6 +2432,7 @@ cudaError_t grouped_gemm_create(GroupedGemm** out, const GroupedGemmDesc* d, int
     g.tri_rows = d[i].tri_rows;
     g.row_scale = d[i].scale;
     g.C = d[i].C;
+    g.part = part;
     g.ldc = d[i].Mpad;
     g.col0 = 0;
     g.sq_rows = d[i].sq_rows;
@@ -2447,6 +2463,8 @@ cudaError_t grouped_gemm_create(GroupedGemm** out, const GroupedGemmDesc* d, int
     }
   }
   GroupedGemm* gg = new GroupedGemm();
+  gg->part = part;
+  part = nullptr;
   gg->pair = pair;
   gg->ntiles = (int)tiles.size();
   gg->nprob = count;
@@ -2482,10 +2500,10 @@ cudaError_t grouped_gemm_create(GroupedGemm** out, const GroupedGemmDesc* d, int
 cudaError_t grouped_gemm_run(GroupedGemm* gg, cudaStream_t s, const int* dcols) {
   if (gg->ntiles == 0) return cudaSuccess;
   if (gg->pair)
-    ozaki_grouped_gemm2_kernel<<<2 * std::min(gg->ntiles, pair_clusters()), THREADS, p2::SMEM, s>>>(
+    ozaki_grouped_gemm2_kernel<<<2 * std::min(gg->ntiles, pair_clusters()), GEMM_THREADS, p2::SMEM, s>>>(
         gg->tiles, gg->probs, gg->maps, dcols, gg->ntiles, gg->counter);
   else
-    ozaki_grouped_gemm_kernel<<<persistent_grid(gg->ntiles), THREADS, SMEM_BYTES, s>>>(
+    ozaki_grouped_gemm_kernel<<<persistent_grid(gg->ntiles), GEMM_THREADS, SMEM_BYTES, s>>>(
         gg->tiles, gg->probs, gg->maps, dcols, gg->ntiles, gg->counter);
   note_launch();
   return cudaGetLastError();
@@ -2501,6 +2519,7 @@ void grouped_gemm_destroy(GroupedGemm* gg) {
   if (gg->probs) cudaFree(gg->probs);
   if (gg->maps) cudaFree(gg->maps);
   if (gg->counter) cudaFree(gg->counter);
+  if (gg->part) cudaFree(gg->part);
   delete gg;
 }
 
@@ -2532,6 +2551,7 @@ extern "C" int fglsgpu_selftest_split_gemm(int M, int K, int N, int S, const dou
   chk(cudaMalloc(&p.A, (size_t)S * p.Mpad * p.Kpad));
   chk(cudaMalloc(&p.G, (size_t)p.Ncap * p.Kpad));
   chk(cudaMalloc(&p.scale, sizeof(double) * p.Mpad));
+  chk(cudaMalloc(&p.gpart, sizeof(longlong2) * (size_t)PART * persistent_grid(1 << 20)));
   chk(cudaMalloc(&p.C, sizeof(double) * (size_t)p.Mpad * p.Ncap));
   chk(cudaMalloc(&p.err, 3 * sizeof(int)));
   chk(cudaMalloc(&dA, sizeof(double) * (size_t)M * K));
@@ -2560,10 +2580,10 @@ extern "C" int fglsgpu_selftest_split_gemm(int M, int K, int N, int S, const dou
   if (r == cudaSuccess)
     chk(cudaMemcpy2D(C, sizeof(double) * M, p.C, sizeof(double) * p.Mpad, sizeof(double) * M, N,
                      cudaMemcpyDeviceToHost));
-  void* ptrs[] = {p.A, p.G, p.scale, p.C, p.err, dA, dX};
+  void* ptrs[] = {p.A, p.G, p.scale, p.C, p.err, p.gpart, dA, dX};
   for (void* q : ptrs)
     if (q) cudaFree(q);
-  p.A = nullptr; p.G = nullptr; p.scale = nullptr; p.C = nullptr; p.err = nullptr;
+  p.A = nullptr; p.G = nullptr; p.scale = nullptr; p.C = nullptr; p.err = nullptr; p.gpart = nullptr;
   if (s) cudaStreamDestroy(s);
   if (r != cudaSuccess) return FGLSGPU_ECUDA;
   return herr ? FGLSGPU_ETIMEOUT : FGLSGPU_OK;
@@ -2578,11 +2598,11 @@ extern "C" int fglsgpu_selftest_split_gemm(int M, int K, int N, int S, const dou
 // pool has reserved the memory), and code that must not change the device's
 // memory footprint between steps.  They pass device buffers for the inputs
 // and the output; the kernel's scratch (E4M3 slices of A, the E4M3 genotype
-// operand, per-row scales, an error word and the GEMM's tile counters) lives
+// operand, per-row scales, partial sums, an error word and the GEMM's tile counters) lives
 // in the file-scope array below,
 // which every GPU that loads this library holds until the process exits.
 //
-// Limits (the array's size, 5.8 MB): M <= 256, K <= 2048, N <= 512,
+// Limits (the array's size, 6.8 MB): M <= 256, K <= 2048, N <= 512,
 // slices <= 9.  Every call shares the array and leaves its contents behind;
 // calls that overlap on the GPU (several streams or threads at once) race on
 // it and must be serialised by the caller.  The first call on a device looks
@@ -2596,7 +2616,8 @@ constexpr int NA_MAX_M = 256, NA_MAX_K = 2048, NA_MAX_N = 512, NA_MAX_S = MAX_SL
 constexpr size_t NA_A_BYTES = (size_t)NA_MAX_S * NA_MAX_M * NA_MAX_K;   // E4M3 slices
 constexpr size_t NA_G_BYTES = (size_t)NA_MAX_N * NA_MAX_K;              // E4M3 genotypes
 constexpr size_t NA_SCALE_BYTES = (size_t)NA_MAX_M * 8;                     // row scales
-constexpr size_t NA_BYTES = NA_A_BYTES + NA_G_BYTES + NA_SCALE_BYTES + 256;  // + error word, tile counters
+constexpr size_t NA_PART_BYTES = (size_t)(NA_MAX_M / BM) * (NA_MAX_N / BN) * PART * sizeof(longlong2);  // a CTA per tile
+constexpr size_t NA_BYTES = NA_A_BYTES + NA_G_BYTES + NA_SCALE_BYTES + 256 + NA_PART_BYTES;  // 256: error word, tile counters
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NA_BYTES];
 
 constexpr int NA_MAX_DEVICES = 64;
@@ -2661,9 +2682,9 @@ extern "C" int fglsgpu_split_gemm_noalloc(int M, int K, int N, int slices, const
   }
   if (r == cudaSuccess) chk(load_genotypes<double>(&p, s, dX, N));
   if (r == cudaSuccess) {
-    // the output doubles as the int64 accumulator between passes
     p.C = dC;
     GemmArgs g;
+    g.part = (longlong2*)(base + NA_A_BYTES + NA_G_BYTES + NA_SCALE_BYTES + 256);
     g.M = M;
     g.Mpad = p.Mpad;
     g.N = N;
@@ -2679,7 +2700,7 @@ extern "C" int fglsgpu_split_gemm_noalloc(int M, int K, int N, int slices, const
     g.sq_rows = 0;
     g.err = p.err;
     g.wait_ns = WAIT_NS;
-    ozaki_gemm_kernel<<<persistent_grid(g.tiles_m * g.tiles_n), THREADS, SMEM_BYTES, s>>>(p.mapA, p.mapB, g,
+    ozaki_gemm_kernel<<<persistent_grid(g.tiles_m * g.tiles_n), GEMM_THREADS, SMEM_BYTES, s>>>(p.mapA, p.mapB, g,
                                                                                           p.err + 1);
     note_launch();
     chk(cudaGetLastError());
