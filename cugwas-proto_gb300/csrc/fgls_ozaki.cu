@@ -32,8 +32,8 @@
 //               while the epilogue drains the previous one.
 //   the others  epilogue: tcgen05.ld the pass's accumulator, convert it
 //               exactly to the int32 q = 32 v = P_2p * 32 + P_2p+1,
-//               Horner-accumulate the passes in int64 in the CTA's own part
-//               (V = V * 2^10 + q), and on the last pass write
+//               keep each pass's q in the CTA's own planes, and on the last
+//               pass combine them in int64 (V = V * 2^10 + q) and write
 //               V * 2^(e_r - 9 - 10 (passes-1)) as FP64.  |V| < 2^62 for S <= 9.
 // Every mbarrier wait is bounded; on expiry the kernel raises an error flag,
 // drains its own in-flight copies and MMAs (bounded), frees TMEM and exits.
@@ -96,17 +96,20 @@ constexpr int GBK = GemmRing::ROW;  // digits per K-step (the tensor maps' box)
 constexpr int SMEM_BYTES = GemmRing::SMEM;
 constexpr int THREADS = 320;  // producer, MMA, 8 epilogue warps (quadratic Gram)
 // Epilogue warps of the split GEMM (32 rows x 1024 / warps columns each).  Sixteen
-// hide the latency of a pass's partial sums where the passes are short (16 cohorts of
-// 500 .. 4000: 1.50 ms a step, 1.61 with eight; n = 750: 102 and 105 us); over long
-// uniform K the epilogue is hidden anyway and eight leave the MMAs more (n = 10000,
-// 16384 SNPs: 9.8 ms a step, 10.1 with sixteen).
+// hide the latency of a pass's sums where the passes are short (16 cohorts of 500 ..
+// 4000: 1.49 ms a step, 1.69 with eight; n = 750: 95 and 99 us); over long uniform K
+// the epilogue is hidden anyway and eight leave the MMAs more (n = 10000, 16384 SNPs:
+// 9.55 ms a step, 9.76 with sixteen, 10.5 with four).
 constexpr int EPI_WARPS = 16;
 constexpr int EPI_WARPS_LONG = 8;
 constexpr int LONG_K = 4096;  // from this K on, uniform tiles run with EPI_WARPS_LONG
 constexpr int gemm_threads(int epi_warps) { return 64 + 32 * epi_warps; }
 constexpr int GEMM_THREADS = gemm_threads(EPI_WARPS);
-constexpr int PART = BM * BN / 2;               // longlong2 partial sums of a CTA's tile (256 KB)
+constexpr int MAX_PLANES = 4;                   // passes before the last
+constexpr int PLANE = BM * BN / 4;              // int4s of a pass's sums over a CTA's tile (128 KB)
+constexpr int PART = MAX_PLANES * PLANE;
 constexpr int MAX_SLICES = 9;   // FP8 digit slices; |V| < 2^62 in the epilogue
+static_assert((MAX_SLICES + 1) / 2 - 1 <= 4, "planes of the passes before the last");
 constexpr int FUSED_KMAX = 16368;  // K of the FP8 split GEMM: (32 + 1/32) K < 2^19
 constexpr int DEFAULT_SLICES = 9;
 constexpr int KALIGN = 128;     // K padding of the FP8 operands (one 128-byte row)
@@ -126,7 +129,7 @@ struct GemmArgs {
   int tri_rows;     // rows [0, tri_rows) of A are lower triangular in K (0: none)
   const double* row_scale;  // per row 2^(e_r - 9 - 10 (passes-1))
   double* C;        // output, column-major, ld = ldc
-  longlong2* part;  // PART partial sums of each CTA of the launch, [column / 2][row]
+  int4* part;       // each CTA's planes of pass sums, [pass][column / 4][row]
   long long ldc;
   int col0;         // first genotype column of this launch (TMA row offset of G)
   int sq_rows;      // rows [0, sq_rows): write (C^2) as an error-free float pair (hi, lo)
@@ -281,70 +284,95 @@ __device__ __forceinline__ void pair_add(float ah, float al, float bh, float bl,
   l = __fadd_rn(e, __fadd_rn(al, bl));
 }
 
-// Sixteen columns' sums over a warp's 32 rows (float pairs h, l): lane bit 4, 3, 2, 1
-// picks the half of the columns a lane keeps, the last round adds lane pairs; lane
-// ends with column (lane >> 1)'s sum, bits 4..1 of the lane in that order.  Rows are
-// paired by offsets 16, 8, 4, 2, 1.
-__device__ __forceinline__ void warp_column_sums(float (&h)[16], float (&l)[16], int lane) {
+// Eight columns' sums over a warp's 32 rows (float pairs h, l): lane bits 4, 3, 2 pick
+// the half of the columns a lane keeps, the last two rounds add lanes; lane ends with
+// column (lane >> 2)'s sum.  Rows are paired by offsets 16, 8, 4, 2, 1.
+__device__ __forceinline__ void warp_column_sums(float (&h)[8], float (&l)[8], int lane) {
 #pragma unroll
-  for (int o = 16; o >= 2; o >>= 1) {
+  for (int o = 16; o >= 4; o >>= 1) {
     const bool up = (lane & o) != 0;
 #pragma unroll
-    for (int k = 0; k < o / 2; k++) {
-      const float sh = up ? h[k] : h[k + o / 2], sl = up ? l[k] : l[k + o / 2];
-      const float kh = up ? h[k + o / 2] : h[k], kl = up ? l[k + o / 2] : l[k];
+    for (int k = 0; k < o / 4; k++) {
+      const float sh = up ? h[k] : h[k + o / 4], sl = up ? l[k] : l[k + o / 4];
+      const float kh = up ? h[k + o / 4] : h[k], kl = up ? l[k + o / 4] : l[k];
       const float rh = __shfl_xor_sync(0xffffffffu, sh, o), rl = __shfl_xor_sync(0xffffffffu, sl, o);
       pair_add(kh, kl, rh, rl, h[k], l[k]);
     }
   }
-  const float rh = __shfl_xor_sync(0xffffffffu, h[0], 1), rl = __shfl_xor_sync(0xffffffffu, l[0], 1);
-  pair_add(h[0], l[0], rh, rl, h[0], l[0]);
+#pragma unroll
+  for (int o = 2; o >= 1; o >>= 1) {
+    const float rh = __shfl_xor_sync(0xffffffffu, h[0], o), rl = __shfl_xor_sync(0xffffffffu, l[0], o);
+    pair_add(h[0], l[0], rh, rl, h[0], l[0]);
+  }
 }
 
-// Pass p of a tile for one epilogue warp (32 rows, its columns from the first): V = V * 2^10 + q with the exact pair sum q in TMEM at tacc.  Between
-// passes V lives in the CTA's own part (16 bytes a thread, 512 a warp and access;
-// L2-resident, since a CTA writes the same 256 KB for every tile), not in C: there
-// the sums of a launch are as large as C, and each went to DRAM and back.  The last
-// pass writes C, V times the row scale (FP64, or squared as a float pair for rows
-// `sq`); `cols` of the warp's columns are valid for all rows, `cend` of this row's.
+// Pass p of a tile for one epilogue warp (32 rows, its columns from the first).
+// The exact pair sum q in TMEM at tacc (an int32) of a pass before the last goes to
+// the CTA's own plane of that pass, four columns a thread, 512 bytes a warp and
+// access; a CTA writes the same planes for every tile, so they stay in L2.  The last
+// pass takes V = q_0 2^(10 p) + q_1 2^(10 (p-1)) + .. from the planes, four columns a
+// step, and writes C, V times the row scale (FP64, or squared as a float pair for
+// rows `sq`); `cols` of the warp's columns are valid for all rows, `cend` of this
+// row's.  (With the int64 sums V read and written every pass, in C, then in a part of
+// the CTA's own, an element moved 64 bytes through L2 instead of 32: n = 10000, 16384
+// SNPs 10.2 and 9.9 ms a step against 9.55, 16 cohorts of 500 .. 4000 2.17 and 1.39
+// against 1.37.)
 // With `qrow` set (warp-uniform: the warp's 32-row group holds rows `sq` of a
 // unit-weight problem) the last pass writes no squares: the warp sums them over its
 // rows and writes column c's sum to qrow[c]; rows not `sq` still write FP64.
 __device__ __forceinline__ void epilogue_pass(uint32_t tacc, int p, bool last, bool sq, double scale, float fscale,
-                                              longlong2* part, double* crow, long long ldc, int cols, int cend,
+                                              int4* part, double* crow, long long ldc, int cols, int cend,
                                               float2* qrow) {
   const int lane = threadIdx.x & 31;
   uint64_t pol_keep;  // the operand stream (~0.5 GB a pass over all CTAs) must not push the sums out
   asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_keep));
+  if (!last) {
+    part += p * PLANE;
 #pragma unroll 1
-  for (int c0 = 0; c0 < cols; c0 += 16) {
-    longlong2 prev[8];
-    longlong2* pp = part + (c0 >> 1) * BM;
-    if (p > 0) {
+    for (int c0 = 0; c0 < cols; c0 += 16) {
+      uint32_t v[16];
+      tmem_ld16(tacc + c0, v);
+      tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 8; j++)
-        asm volatile("ld.global.cg.L2::cache_hint.v2.b64 {%0, %1}, [%2], %3;"
-                     : "=l"(prev[j].x), "=l"(prev[j].y)
-                     : "l"(pp + j * BM), "l"(pol_keep));
+      for (int j = 0; j < 4; j++)
+        asm volatile("st.global.L2::cache_hint.v4.b32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(part + ((c0 >> 2) + j) * BM),
+                     "r"(fused_pair_f2i(__uint_as_float(v[4 * j]))), "r"(fused_pair_f2i(__uint_as_float(v[4 * j + 1]))),
+                     "r"(fused_pair_f2i(__uint_as_float(v[4 * j + 2]))),
+                     "r"(fused_pair_f2i(__uint_as_float(v[4 * j + 3]))), "l"(pol_keep)
+                     : "memory");
     }
-    uint32_t v[16];
-    tmem_ld16(tacc + c0, v);
+    return;
+  }
+  // V of eight columns a step: all planes' loads in flight, then TMEM
+#pragma unroll 1
+  for (int c0 = 0; c0 < cols; c0 += 8) {
+    int4 q[MAX_PLANES][2];
+#pragma unroll
+    for (int i = 0; i < MAX_PLANES; i++)
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        q[i][j] = make_int4(0, 0, 0, 0);
+        if (i < p)
+          asm volatile("ld.global.cg.L2::cache_hint.v4.b32 {%0, %1, %2, %3}, [%4], %5;"
+                       : "=r"(q[i][j].x), "=r"(q[i][j].y), "=r"(q[i][j].z), "=r"(q[i][j].w)
+                       : "l"(part + i * PLANE + ((c0 >> 2) + j) * BM), "l"(pol_keep));
+      }
+    uint32_t v[8];
+    tmem_ld8(tacc + c0, v);
     tmem_ld_wait();
     auto value = [&](int j) -> long long {
-      const long long q = fused_pair_f2i(__uint_as_float(v[j]));
-      if (p == 0) return q;
-      return (j & 1 ? prev[j >> 1].y : prev[j >> 1].x) * 1024ll + q;
+      long long V = 0;
+#pragma unroll
+      for (int i = 0; i < MAX_PLANES; i++) {
+        const int4 t = q[i][j >> 2];
+        if (i < p) V = V * 1024ll + ((j & 3) == 0 ? t.x : (j & 3) == 1 ? t.y : (j & 3) == 2 ? t.z : t.w);
+      }
+      return V * 1024ll + fused_pair_f2i(__uint_as_float(v[j]));
     };
-    if (!last) {
+    if (qrow != nullptr) {
+      float h[8], l[8];
 #pragma unroll
-      for (int j = 0; j < 8; j++)
-        asm volatile("st.global.L2::cache_hint.v2.b64 [%0], {%1, %2}, %3;" ::"l"(pp + j * BM), "l"(value(2 * j)),
-                     "l"(value(2 * j + 1)), "l"(pol_keep)
-                     : "memory");
-    } else if (qrow != nullptr) {
-      float h[16], l[16];
-#pragma unroll
-      for (int j = 0; j < 16; j++) {  // column j's square as a float pair (0 past cend; rows not sq write FP64)
+      for (int j = 0; j < 8; j++) {  // column j's square as a float pair (0 past cend; rows not sq write FP64)
         h[j] = l[j] = 0.0f;
         if (c0 + j >= cend) continue;
         const long long V = value(j);
@@ -357,11 +385,11 @@ __device__ __forceinline__ void epilogue_pass(uint32_t tacc, int p, bool last, b
         }
       }
       warp_column_sums(h, l, lane);
-      const int c = c0 + (lane >> 1);
-      if (!(lane & 1) && c < cols) qrow[c] = make_float2(h[0], l[0]);
+      const int c = c0 + (lane >> 2);
+      if (!(lane & 3) && c < cols) qrow[c] = make_float2(h[0], l[0]);
     } else {
 #pragma unroll
-      for (int j = 0; j < 16; j++) {
+      for (int j = 0; j < 8; j++) {
         if (c0 + j >= cend) break;
         const long long V = value(j);
         double* cp = crow + (long long)(c0 + j) * ldc;
@@ -579,7 +607,7 @@ __device__ __forceinline__ void gemm_persistent(const Src& src, int* tile_counte
     const int lq = warp & 3;
     const int cbeg = ((warp - 2) >> 2) * (BN * 4 / EPI_WARPS);
     const int row = lq * 32 + lane;
-    longlong2* part = nullptr;
+    int4* part = nullptr;
     const uint32_t ta = tbase + ((uint32_t)(lq * 32) << 16) + (uint32_t)cbeg;
     uint32_t q = 0;
     bool ok = true;
@@ -612,7 +640,7 @@ __device__ __forceinline__ void gemm_persistent(const Src& src, int* tile_counte
       const int ncols = rvalid ? min(BN, T.N - n0) : 0;  // valid columns of this tile for this row
       const int cend = min((BN * 4 / EPI_WARPS), ncols - cbeg);      // of this warp's columns (may be <= 0)
       double* crow = g.C + (long long)r + (long long)(g.col0 + n0 + cbeg) * g.ldc;
-      part = g.part + (size_t)blockIdx.x * PART + (cbeg >> 1) * BM + row;
+      part = g.part + (size_t)blockIdx.x * PART + (cbeg >> 2) * BM + row;
       // unit weights: this warp's 32-row group (rows r & ~31 ..) sums its squares
       float2* qrow = (g.sqsum != nullptr && (r & ~31) < g.sq_rows)
                          ? g.sqsum + (long long)(r >> 5) * g.ldq + (g.col0 + n0 + cbeg)
@@ -940,7 +968,7 @@ __device__ __forceinline__ void gemm_pair(const Src& src, int* tile_counter) {
     const int lq = warp & 3;
     const int cbeg = ((warp - 2) >> 2) * (BN * 4 / EW);
     const int row = lq * 32 + lane;
-    longlong2* part = nullptr;
+    int4* part = nullptr;
     const uint32_t ta = tbase + ((uint32_t)(lq * 32) << 16) + (uint32_t)cbeg;
     const uint32_t lead_tempty = cluster_addr(tempty, 0);
     uint32_t q = 0;
@@ -974,7 +1002,7 @@ __device__ __forceinline__ void gemm_pair(const Src& src, int* tile_counter) {
       const int ncols = rvalid ? min(BN, T.N - n0) : 0;
       const int cend = min((BN * 4 / EW), ncols - cbeg);
       double* crow = g.C + (long long)r + (long long)(g.col0 + n0 + cbeg) * g.ldc;
-      part = g.part + (size_t)blockIdx.x * PART + (cbeg >> 1) * BM + row;
+      part = g.part + (size_t)blockIdx.x * PART + (cbeg >> 2) * BM + row;
       // unit weights: this warp's 32-row group (rows r & ~31 ..) sums its squares
       float2* qrow = (g.sqsum != nullptr && (r & ~31) < g.sq_rows)
                          ? g.sqsum + (long long)(r >> 5) * g.ldq + (g.col0 + n0 + cbeg)
@@ -1128,12 +1156,6 @@ __host__ __device__ __forceinline__ int qt_range_begin(int c, int units, int cta
 }
 __host__ __device__ __forceinline__ int qt_owner(int u, int units, int ctas) {
   return (int)((((long long)u + 1) * ctas - 1) / units);
-}
-
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
 }
 
 __device__ __forceinline__ void two_sum_f(float a, float b, float& s, float& e) {
@@ -1964,7 +1986,7 @@ struct OzakiPlan {
   uint8_t* G = nullptr;         // Ncap x Kpad E4M3 genotypes
   double* scale = nullptr;      // Mpad
   double* C = nullptr;          // Mpad x Ncap (ld Mpad)
-  longlong2* gpart = nullptr;   // the split GEMM's partial sums, PART a CTA
+  int4* gpart = nullptr;   // the split GEMM's pass sums, PART a CTA
   double* U = nullptr;          // n x nU
   float2* D = nullptr;          // n x t weights as float pairs (eigen d_j; chol: ones)
   float* dmax = nullptr;        // t: max_l of the high part of D[:, j]
@@ -2049,7 +2071,7 @@ cudaError_t ozaki_create(OzakiPlan** out, int n, int t, int wXL, int wXR, int x_
     chk(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev));
   }
   chk(cudaMalloc(&p->err, 3 * sizeof(int)));  // [wait error word, GEMM tile counter, finished CTAs]
-  chk(cudaMalloc(&p->gpart, sizeof(longlong2) * (size_t)PART * persistent_grid(1 << 20)));
+  chk(cudaMalloc(&p->gpart, sizeof(int4) * (size_t)PART * persistent_grid(1 << 20)));
   if (!eigen) chk(cudaMalloc(&p->LinvT, sizeof(double) * (size_t)n * n));
   if (!eigen) chk(cudaMalloc(&p->sqsum, sizeof(float2) * (size_t)(p->Mpad / 32) * p->Ncap));
   if (r == cudaSuccess) chk(cudaMemset(p->A, 0, (size_t)p->S * p->Mpad * p->Kpad));
@@ -2401,17 +2423,17 @@ struct GroupedGemm {
   GroupedProblem* probs = nullptr;
   CUtensorMap* maps = nullptr;
   int* counter = nullptr;  // tile counter and finished CTAs of the persistent launch
-  longlong2* part = nullptr;  // partial sums, PART a CTA
+  int4* part = nullptr;  // partial sums, PART a CTA
 };
 
 cudaError_t grouped_gemm_create(GroupedGemm** out, const GroupedGemmDesc* d, int count, int x_b, int* err,
                                 bool want_pair) {
   *out = nullptr;
   const bool pair = want_pair && pair_clusters() > 0;
-  longlong2* part = nullptr;
-  FGLS_CUDA_TRY(cudaMalloc(&part, sizeof(longlong2) * (size_t)PART * persistent_grid(1 << 20)));
+  int4* part = nullptr;
+  FGLS_CUDA_TRY(cudaMalloc(&part, sizeof(int4) * (size_t)PART * persistent_grid(1 << 20)));
   struct Give {  // given back unless the plan takes it
-    longlong2** p;
+    int4** p;
     ~Give() {
       if (*p) cudaFree(*p);
     }
@@ -2551,7 +2573,7 @@ extern "C" int fglsgpu_selftest_split_gemm(int M, int K, int N, int S, const dou
   chk(cudaMalloc(&p.A, (size_t)S * p.Mpad * p.Kpad));
   chk(cudaMalloc(&p.G, (size_t)p.Ncap * p.Kpad));
   chk(cudaMalloc(&p.scale, sizeof(double) * p.Mpad));
-  chk(cudaMalloc(&p.gpart, sizeof(longlong2) * (size_t)PART * persistent_grid(1 << 20)));
+  chk(cudaMalloc(&p.gpart, sizeof(int4) * (size_t)PART * persistent_grid(1 << 20)));
   chk(cudaMalloc(&p.C, sizeof(double) * (size_t)p.Mpad * p.Ncap));
   chk(cudaMalloc(&p.err, 3 * sizeof(int)));
   chk(cudaMalloc(&dA, sizeof(double) * (size_t)M * K));
@@ -2598,11 +2620,11 @@ extern "C" int fglsgpu_selftest_split_gemm(int M, int K, int N, int S, const dou
 // pool has reserved the memory), and code that must not change the device's
 // memory footprint between steps.  They pass device buffers for the inputs
 // and the output; the kernel's scratch (E4M3 slices of A, the E4M3 genotype
-// operand, per-row scales, partial sums, an error word and the GEMM's tile counters) lives
+// operand, per-row scales, pass sums, an error word and the GEMM's tile counters) lives
 // in the file-scope array below,
 // which every GPU that loads this library holds until the process exits.
 //
-// Limits (the array's size, 6.8 MB): M <= 256, K <= 2048, N <= 512,
+// Limits (the array's size, 7.9 MB): M <= 256, K <= 2048, N <= 512,
 // slices <= 9.  Every call shares the array and leaves its contents behind;
 // calls that overlap on the GPU (several streams or threads at once) race on
 // it and must be serialised by the caller.  The first call on a device looks
@@ -2616,7 +2638,7 @@ constexpr int NA_MAX_M = 256, NA_MAX_K = 2048, NA_MAX_N = 512, NA_MAX_S = MAX_SL
 constexpr size_t NA_A_BYTES = (size_t)NA_MAX_S * NA_MAX_M * NA_MAX_K;   // E4M3 slices
 constexpr size_t NA_G_BYTES = (size_t)NA_MAX_N * NA_MAX_K;              // E4M3 genotypes
 constexpr size_t NA_SCALE_BYTES = (size_t)NA_MAX_M * 8;                     // row scales
-constexpr size_t NA_PART_BYTES = (size_t)(NA_MAX_M / BM) * (NA_MAX_N / BN) * PART * sizeof(longlong2);  // a CTA per tile
+constexpr size_t NA_PART_BYTES = (size_t)(NA_MAX_M / BM) * (NA_MAX_N / BN) * PART * sizeof(int4);  // a CTA per tile
 constexpr size_t NA_BYTES = NA_A_BYTES + NA_G_BYTES + NA_SCALE_BYTES + 256 + NA_PART_BYTES;  // 256: error word, tile counters
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NA_BYTES];
 
@@ -2684,7 +2706,7 @@ extern "C" int fglsgpu_split_gemm_noalloc(int M, int K, int N, int slices, const
   if (r == cudaSuccess) {
     p.C = dC;
     GemmArgs g;
-    g.part = (longlong2*)(base + NA_A_BYTES + NA_G_BYTES + NA_SCALE_BYTES + 256);
+    g.part = (int4*)(base + NA_A_BYTES + NA_G_BYTES + NA_SCALE_BYTES + 256);
     g.M = M;
     g.Mpad = p.Mpad;
     g.N = N;

@@ -312,7 +312,7 @@ int fglsgpu_selftest_dgemm(int transA, int transB, int M, int N, int K, double a
  * own memory pool, or that must keep the device's footprint fixed).  All
  * pointers are DEVICE pointers owned by the caller: A (M x K, row-major
  * FP64), X (K x N, column-major genotypes), C (M x N, column-major FP64 out).
- * The kernel's scratch lives in a fixed 6.8 MB array inside the library
+ * The kernel's scratch lives in a fixed 7.9 MB array inside the library
  * (held by every GPU that loads it): M <= 256, K <= 2048, N <= 512,
  * slices <= 9, else FGLSGPU_EINVAL.  Runs on `stream` (a cudaStream_t, NULL
  * for the default stream), reads the kernel's error word back and returns
