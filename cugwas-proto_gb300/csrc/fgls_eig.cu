@@ -105,6 +105,11 @@ __device__ __forceinline__ void reflector(double alpha, double xnorm2, double& b
 //                 scalars), y = A v, t = [W^T v ; V^T v] and the parts of y^T v
 // Sums over CTAs are taken from arrays of parts in a fixed order.
 constexpr int TB = 64;
+// Both kernels may be launched before the one ahead of them ends (programmatic
+// dependent launch): a column's two launches are on the chain of 2 n of them.
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 constexpr int TR = 32;  // rows per CTA of tridiag_col, one per lane; the panel's columns are dealt to the warps
 
 // Panel column i = k - k0.  pend: w of column i - 1 is due,
@@ -125,6 +130,7 @@ __global__ void __launch_bounds__(256) tridiag_col_kernel(int n, int k, int i, b
   const int r = k + blockIdx.x * TR + lane;
   const double *V = P, *W = P + (long long)TB * n;
   double yr = 0.0, vr = 0.0, ar = 0.0, tk = 0.0, yk = 0.0;  // what the last part needs, in flight early
+  wait_previous();
   if (wp == 0 && r < n) {
     if (live) ar = A[r + (long long)k * lda];
     if (pend) {
@@ -168,6 +174,7 @@ __global__ void __launch_bounds__(256) tridiag_col_kernel(int n, int k, int i, b
     }
     __syncthreads();
   }
+  launch_next();
   if (wp > 0) return;
   double sq = 0.0, xr = ar;
   if (pend) {
@@ -231,6 +238,7 @@ __global__ void __launch_bounds__(MV_THREADS) tridiag_mv_kernel(int n, int k, in
   };
   const int j0 = blockIdx.x * 8 + wp;
   double first = 0.0, head = 0.0;
+  wait_previous();
   if (wp < 8) {
     if (j0 < cols) {
       head = column(j0)[0];
@@ -258,7 +266,10 @@ __global__ void __launch_bounds__(MV_THREADS) tridiag_mv_kernel(int n, int k, in
     P[r + (long long)(2 * TB + i) * n] = v;
     if (r > r0) A[r + (long long)k * lda] = v;
   }
-  if (wp == 8) return;
+  if (wp == 8) {
+    launch_next();
+    return;
+  }
   double yv = 0.0;
   for (int j = j0; j < cols; j += warps) {
     if (j != j0) {
@@ -275,6 +286,7 @@ __global__ void __launch_bounds__(MV_THREADS) tridiag_mv_kernel(int n, int k, in
       }
     }
   }
+  launch_next();
   if (lane == 0) yvs[wp] = yv;
   asm volatile("bar.sync 1, 256;" ::: "memory");  // the eight column warps
   if (threadIdx.x == 0) {
@@ -294,6 +306,20 @@ __global__ void tridiag_tail_kernel(int n, const double* A, long long lda, doubl
   }
   d[n - 1] = A[(n - 1) + (long long)(n - 1) * lda];
   e[n - 1] = 0.0;
+}
+
+template <class... P, class... T>
+cudaError_t launch_chained(void (*kernel)(P...), int grid, int block, cudaStream_t s, T... args) {
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 int grid_for(long long total) { return (int)std::min<long long>((total + 255) / 256, 152LL * 32); }
@@ -425,14 +451,18 @@ cudaError_t dsyev_device(cudaStream_t s, DigitGemm* dg, int n, const double* Phi
     for (int i = 0; i < nb; i++) {
       const int k = k0 + i, m = n - k - 1;
       const int nr = ceil_div(n - k, TR);
-      tridiag_col_kernel<<<nr, 256, 0, s>>>(n, k, i, i > 0, true, A, n, P, yb, tb, yvpart, nyv, tau, d, xb, npart);
+      FGLS_CUDA_TRY(launch_chained(tridiag_col_kernel, nr, 256, s, n, k, i, i > 0, true, (const double*)A, (long long)n,
+                                   P, (const double*)yb, (const double*)tb, (const double*)yvpart, nyv,
+                                   (const double*)tau, d, xb, npart));
       nyv = std::min(ceil_div(m + 2 * i, 8), EIG_CTAS);
-      tridiag_mv_kernel<<<nyv, MV_THREADS, 0, s>>>(n, k, i, A, n, P, xb, npart, nr, tau, e, yb, tb, yvpart);
+      FGLS_CUDA_TRY(launch_chained(tridiag_mv_kernel, nyv, MV_THREADS, s, n, k, i, A, (long long)n, P,
+                                   (const double*)xb, (const double*)npart, nr, tau, e, yb, tb, yvpart));
       nl += 2;
     }
     const int kn = k0 + nb, m = n - kn;  // the trailing matrix
-    tridiag_col_kernel<<<ceil_div(m, TR), 256, 0, s>>>(n, kn, nb, true, false, A, n, P, yb, tb, yvpart, nyv, tau, d, xb,
-                                                        npart);
+    FGLS_CUDA_TRY(launch_chained(tridiag_col_kernel, ceil_div(m, TR), 256, s, n, kn, nb, true, false, (const double*)A,
+                                 (long long)n, P, (const double*)yb, (const double*)tb, (const double*)yvpart, nyv,
+                                 (const double*)tau, d, xb, npart));
     nl++;
     FGLS_CUDA_TRY(cudaGetLastError());
     // A -= [V W] [W V]^T; a short last panel leaves columns of P beyond nb unset
