@@ -28,6 +28,39 @@ __device__ __forceinline__ void set_status(DevStatus* st, int code, int info, lo
   }
 }
 
+// 1 / sqrt(d) on a short chain: dependent FP64 instructions take some 150 cycles
+// each here, and the library function is a chain of two dozen.  Seed from the FP32
+// reciprocal square root of the mantissa (moved in and out by integer
+// instructions), then one third-order step y (1 + e/2 + 3 e^2 / 8), e = 1 - d y^2
+// (the binomial series of (1 - e)^(-1/2)): |e| < 2^-21 leaves 2^-63.
+__device__ __forceinline__ double chain_rsqrt(double d) {
+  const long long b = __double_as_longlong(d);
+  const int ex = (int)(b >> 52);
+  if (ex <= 0 || ex >= 0x7ff) return rsqrt(d);  // zero, subnormal, negative, infinite, NaN
+  const int k = ex - 1023, odd = k & 1;
+  const float m = __int_as_float(((127 + odd) << 23) | ((int)(b >> 29) & 0x7fffff));  // in [1, 4)
+  const int f = __float_as_int(rsqrtf(m));
+  const double y = __longlong_as_double(((long long)((f >> 23) - 127 + 1023 - (k >> 1)) << 52) |
+                                        ((long long)(f & 0x7fffff) << 29));
+  const double t = d * y;
+  const double e = fma(-fma(d, y, -t), y, fma(-t, y, 1.0));  // with the rounding of d y
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// 1 / d on a short chain: FP32 reciprocal of the mantissa (moved in and out by
+// integer instructions), then y (1 + e + e^2), e = 1 - d y (the geometric series of
+// 1 / (1 - e)); |e| < 2^-22 leaves 2^-66.
+__device__ __forceinline__ double chain_rcp(double d) {
+  const long long b = __double_as_longlong(d);
+  const int ex = (int)(b >> 52) & 0x7ff;
+  if (ex <= 1 || ex >= 0x7fd) return 1.0 / d;
+  const int f = __float_as_int(__frcp_rn(__int_as_float(0x3f800000 | ((int)(b >> 29) & 0x7fffff))));  // in [0.5, 1]
+  const double y = __longlong_as_double(((long long)((f >> 23) - 127 - (ex - 1023) + 1023) << 52) |
+                                        ((long long)(f & 0x7fffff) << 29) | (b & (long long)0x8000000000000000ull));
+  const double e = fma(-d, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 // Kernel launchers (host side, defined in the .cu files).  All are

@@ -88,15 +88,20 @@ __global__ void __launch_bounds__(LEAF) dc_leaf_kernel(int n, const int* __restr
         int i, cnt = 0;
         for (i = mm - 1; i >= l; i--) {
           double f = s * se[i], b = c * se[i];
-          r = hypot(f, g);
+          // the rotation on a short chain (hypot and two divisions: 2.4 us each on
+          // this thread); tiny or huge pairs the long way
+          const double r2 = fma(f, f, g * g);
+          const bool plain = r2 > 1e-280 && r2 < 1e280;
+          const double ry = plain ? chain_rsqrt(r2) : 0.0;
+          r = plain ? r2 * ry : hypot(f, g);
           se[i + 1] = r;
           if (r == 0.0) {
             sd[i + 1] -= p;
             se[mm] = 0.0;
             break;
           }
-          s = f / r;
-          c = g / r;
+          s = plain ? f * ry : f / r;
+          c = plain ? g * ry : g / r;
           g = sd[i + 1] - p;
           r = (sd[i] - g) * s + 2.0 * c * b;
           p = s * r;
@@ -399,7 +404,7 @@ __device__ __forceinline__ void secular_warp(int K, const double* __restrict__ d
   const double org = dk[o];
   double s = 0.0, sa = 0.0, so = 0.0, sp = 0.0;
   for (int j = lane; j < K; j += 32) {
-    const double r = 1.0 / ((dk[j] - org) - tau);
+    const double r = chain_rcp((dk[j] - org) - tau);
     const double zr = zk[j] * r;
     const double term = zk[j] * zr;
     sa += fabs(term);
@@ -437,9 +442,6 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(int K, const double* __
   const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (k >= K) return;  // warp-uniform
-  double zn = 0.0;
-  for (int j = lane; j < K; j += 32) zn += zk[j] * zk[j];
-  zn = warp_sum(zn);
   int o;
   double lo, hi;
   double f, amag, psi, dpsi;
@@ -456,6 +458,9 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(int K, const double* __
       hi = 0.0;
     }
   } else {
+    double zn = 0.0;
+    for (int j = lane; j < K; j += 32) zn += zk[j] * zk[j];
+    zn = warp_sum(zn);
     o = k;
     lo = 0.0;
     hi = rho * zn;
@@ -508,7 +513,7 @@ __global__ void __launch_bounds__(256) dc_lowner_kernel(int K, const double* __r
     if (j == i) continue;
     const double num = (dk[org_idx[j]] - di) + tau[j];
     const double den = dk[j] - di;
-    prod *= num / den;
+    prod *= num / den;  // divided: the rounding of K factors is the accuracy of z
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) prod *= __shfl_xor_sync(0xffffffffu, prod, o);

@@ -219,24 +219,6 @@ constexpr int DT = 256;       // threads of the diagonal kernels
 constexpr int PB = 64;        // diagonal block of potrf and of the inverse
 constexpr int PO = 512;       // outer panel of potrf, base block of the inverse
 
-// 1 / sqrt(d) on a short chain: dependent FP64 instructions take some 150 cycles
-// each here, and the library function is a chain of two dozen.  Seed from the FP32
-// reciprocal square root of the mantissa (moved in and out by integer
-// instructions), then one third-order step y (1 + e/2 + 3 e^2 / 8), e = 1 - d y^2
-// (the binomial series of (1 - e)^(-1/2)): |e| < 2^-21 leaves 2^-63.
-__device__ __forceinline__ double chain_rsqrt(double d) {
-  const long long b = __double_as_longlong(d);
-  const int ex = (int)(b >> 52);
-  if (ex <= 0 || ex >= 0x7ff) return rsqrt(d);  // zero, subnormal, negative, infinite, NaN
-  const int k = ex - 1023, odd = k & 1;
-  const float m = __int_as_float(((127 + odd) << 23) | ((int)(b >> 29) & 0x7fffff));  // in [1, 4)
-  const int f = __float_as_int(rsqrtf(m));
-  const double y = __longlong_as_double(((long long)((f >> 23) - 127 + 1023 - (k >> 1)) << 52) |
-                                        ((long long)(f & 0x7fffff) << 29));
-  const double e = fma(-(d * y), y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 // Cholesky factor of a 64 x 64 block and its inverse, one CTA of eight warps
 // (FACTOR = false: the inverse alone, Ls and rdiag given).
 //   Ls[c][r]: finished columns of the factor, Xs[r][c]: finished rows of the

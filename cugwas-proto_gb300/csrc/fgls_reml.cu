@@ -210,20 +210,6 @@ __device__ void reml_point(int n, double h, const double* __restrict__ W, const 
   __syncthreads();
 }
 
-// 1 / d for a positive normal d on a short chain: FP32 reciprocal of the mantissa
-// (moved in and out by integer instructions), then y (1 + e + e^2), e = 1 - d y
-// (the geometric series of 1 / (1 - e)); |e| < 2^-22 leaves 2^-66.
-__device__ __forceinline__ double chain_rcp(double d) {
-  const long long b = __double_as_longlong(d);
-  const int ex = (int)(b >> 52);
-  if (ex <= 1 || ex >= 0x7fd) return 1.0 / d;
-  const int f = __float_as_int(__frcp_rn(__int_as_float(0x3f800000 | ((int)(b >> 29) & 0x7fffff))));  // in [0.5, 1]
-  const double y = __longlong_as_double(((long long)((f >> 23) - 127 - (ex - 1023) + 1023) << 52) |
-                                        ((long long)(f & 0x7fffff) << 29));
-  const double e = fma(-d, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-
 // Sums over a warp of K values a lane; value k's sum ends in v[0] of lane k (K <=
 // 32) or of lanes k, with v[1] for value 32 + k (K <= 64).  Each round halves the
 // values a lane carries: K additions instead of 5 K.
