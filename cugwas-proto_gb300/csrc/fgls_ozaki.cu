@@ -1753,9 +1753,12 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(int K, int rows, const 
   __shared__ double red[32];
   __shared__ int top_s[8];
   // Rows of normal magnitudes, in integer instructions (with FP64 rint, subtract and
-  // scale per digit the FP64 pipe bound it: 2.7 ms for 6000 x 6000, now under 0.3): |a| as a
+  // scale per digit the FP64 pipe bound it: 2.7 ms for 6000 x 6000, now 0.22): |a| as a
   // 62-bit fixed-point number with four bits before the point, each digit the
   // nearest integer, the remainder times 32; four elements a thread, one word a slice.
+  // Up to 9 slices the digits are those of the loop below but where a remainder is an
+  // exact tie (same error either way); from 10 on the number's 58 fraction bits are too few.
+  static_assert(MAX_SLICES <= 9, "digits from 58 fraction bits");
   int top = 0;
   for (int k = threadIdx.x; k < K; k += blockDim.x) top = max(top, (int)((__double_as_longlong(a[k]) >> 52) & 0x7ff));
   top = __reduce_max_sync(0xffffffffu, top);
