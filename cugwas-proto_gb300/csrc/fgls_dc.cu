@@ -9,14 +9,14 @@
 //  * leaves: implicit QL in one CTA per leaf (one thread runs the scalar
 //    sweep, 64 threads apply each rotation chain to the leaf's rows);
 //  * merge: z = Q^T u / sqrt2, rho = 2|b| > 0; sort the children's eigenvalues
-//    (rank by binary search); deflate tiny |rho z_i| and close pairs (Givens,
-//    sequential scan in one thread); secular equation 1 + rho sum z^2/(d - l)
+//    (rank by binary search); deflate tiny |rho z_i| and close pairs (Givens);
+//    secular equation 1 + rho sum z^2/(d - l)
 //    for each surviving root by a pole-aware Newton iteration in its own
 //    bisection bracket with the origin at the nearer pole (one warp per root); z
 //    recomputed from the roots by the Loewner formula (one warp per root) so
 //    that the eigenvectors are orthogonal to
 //    working precision; eigenvectors u_k = z_i/(d_i - l_k) normalised (one
-//    warp per root); new Q = Q_old[:, kept] * U by DGEMM; final rank sort.
+//    warp per root); new Q = Q_old[:, kept] * U by an FP64 product; final rank sort.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>

@@ -499,8 +499,8 @@ cudaError_t dsyev_device(cudaStream_t s, DigitGemm* dg, int n, const double* Phi
   nl++;
   mark(3);
   // 4. Z := H_0 H_1 ... H_{n-3} Z, blocks of NB reflectors from the last one
-  //    in compact-WY form (I - Y T Y^T): three DGEMMs per block, 2 n^3 flops
-  //    in all -- what a DGEMM with an explicit Q costs, without forming Q.
+  //    in compact-WY form (I - Y T Y^T): three FP64 products per block, 2 n^3
+  //    flops in all -- what one with an explicit Q costs, without forming Q.
   {
     constexpr int NB = NBT;  // wide blocks: the Y^T Z product has NB/64 x n/64 output tiles
     double* Yb = (double*)dcw;         // n x NB

@@ -334,7 +334,7 @@ int chol_digits(fglsgpu_engine* e, long long cols, bool* use) {
 // the digits of a block of x_b SNPs.  On return use = whether the block's
 // products run on them: the eigenvector product of `cols` columns is large
 // enough, and the device has the memory (twelve bytes an element).  A 4096-SNP
-// block of hard calls at n = 5000, t = 16 takes 2.0 ms on them and 179 ms on the
+// block of hard calls at n = 5000, t = 16 takes 1.7 ms on them and 179 ms on the
 // FP64 kernels, with the same error against exact arithmetic (1.4e-14).
 int eigen_digits(fglsgpu_engine* e, long long cols, bool* use) {
   *use = false;
