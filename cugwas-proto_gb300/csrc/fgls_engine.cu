@@ -71,7 +71,7 @@ struct fglsgpu_engine {
   // adjoint state (eigen, FP64): allocated by fglsgpu_adjoint_reset
   // the d-, c- and s-weighted operands side by side, so that a block's Gram terms
   // are two products: aAYL3 n x 3 t(1+wXL), aW3 n x 3 t, their results aG3
-  double *aAYL3 = nullptr, *aW3 = nullptr, *atopc = nullptr, *atops = nullptr, *areml = nullptr;
+  double *aAYL3 = nullptr, *aW3 = nullptr, *atopd = nullptr, *atopc = nullptr, *atops = nullptr, *areml = nullptr;
   double *aG3 = nullptr, *acontrib = nullptr, *ag = nullptr;
   void* adjmem = nullptr;  // their digits
   DigitMat aayl3, aw3;
@@ -178,7 +178,7 @@ void free_all(fglsgpu_engine* e) {
   void* ptrs[] = {e->dPhi, e->dL,   e->dZ,    e->dW,    e->dXL,   e->dY,    e->dh,    e->dsig, e->dWY,
                   e->dZtXL, e->dZtY, e->ddinv, e->dAYL, e->dtop, e->deigwork, e->dX[0], e->dX[1], e->dWork,
                   e->dQ,   e->dGYL, e->dGR,  e->dB[0], e->dB[1], e->dV[0], e->dV[1], e->dU8, e->dst,
-                  e->aAYL3, e->aW3, e->atopc, e->atops, e->areml, e->aG3, e->adjmem, e->acontrib, e->ag, e->agR, e->aacc, e->aU, e->aV2, e->dSE[0], e->dSE[1], e->dP[0],
+                  e->aAYL3, e->aW3, e->atopd, e->atopc, e->atops, e->areml, e->aG3, e->adjmem, e->acontrib, e->ag, e->agR, e->aacc, e->aU, e->aV2, e->dSE[0], e->dSE[1], e->dP[0],
                   e->dP[1], e->dXw, e->zmem, e->wmem, e->blkmem, e->dLinv, e->ddiag, e->dWraw, e->remlmem};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -1108,6 +1108,7 @@ int fglsgpu_adjoint_reset(fglsgpu_engine* e) {
     };
     chk(dalloc(&e->aW3, n * 3 * t));
     chk(dalloc(&e->aAYL3, n * 3 * t * (1 + wXL)));
+    chk(dalloc(&e->atopd, t * (wXL + wXL * wXL)));
     chk(dalloc(&e->atopc, t * (wXL + wXL * wXL)));
     chk(dalloc(&e->atops, t * (wXL + wXL * wXL)));
     chk(dalloc(&e->areml, 2 * t));
@@ -1127,8 +1128,8 @@ int fglsgpu_adjoint_reset(fglsgpu_engine* e) {
   const long long nyl = n * t * (1 + wXL);
   ENG_TRY(e, cudaMemcpyAsync(e->aAYL3, e->dAYL, sizeof(double) * nyl, cudaMemcpyDeviceToDevice, s), "adjoint weights");
   ENG_TRY(e, cudaMemcpyAsync(e->aW3, e->ddinv, sizeof(double) * n * t, cudaMemcpyDeviceToDevice, s), "adjoint weights");
-  ENG_TRY(e, adjoint_traits(s, c.n, c.t, c.wXL, e->dW, e->dh, e->dsig, e->dZtXL, e->dZtY, e->ddinv, e->aW3 + n * t,
-                            e->aAYL3 + nyl, e->aAYL3 + 2 * nyl, e->atopc, e->atops, e->areml),
+  ENG_TRY(e, adjoint_traits(s, c.n, c.t, c.wXL, e->dW, e->dsig, e->dZtXL, e->dZtY, e->ddinv, e->aW3 + n * t,
+                            e->aAYL3 + nyl, e->aAYL3 + 2 * nyl, e->atopd, e->atopc, e->atops, e->areml),
           "adjoint weights");
   // digits of the weighted operands, when the blocks run on digits
   e->adj_cut = false;

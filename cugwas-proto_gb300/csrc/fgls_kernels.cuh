@@ -75,9 +75,9 @@ cudaError_t snp_pvalues(cudaStream_t s, int x, int t, int p, int wXL, const doub
                         const double* V, long long vstride, double* P, long long pstride);
 
 // Adjoint of the eigen variant (fgls_adjoint.cu); layouts in that file.
-cudaError_t adjoint_traits(cudaStream_t s, int n, int t, int wXL, const double* W, const double* h,
-                           const double* sigma, const double* ZtXL, const double* ZtY, const double* dinv,
-                           double* Wc, double* AYLc, double* AYLs, double* topc, double* tops, double* reml);
+cudaError_t adjoint_traits(cudaStream_t s, int n, int t, int wXL, const double* W, const double* sigma,
+                           const double* ZtXL, const double* ZtY, const double* dinv, double* Wc, double* AYLc,
+                           double* AYLs, double* topd, double* topc, double* tops, double* reml);
 cudaError_t adjoint_snps(cudaStream_t s, int p, int x, int t, int wXL, const double* top, const double* GYL,
                          const double* GR, const double* topc, const double* GYLc, const double* GRc,
                          const double* tops, const double* GYLs, const double* GRs, const double* Bbar,
