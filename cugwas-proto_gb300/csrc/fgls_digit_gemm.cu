@@ -996,13 +996,16 @@ bool digit_gemm_reserve(DigitGemm* g, int rows, int K) {
   return reserve(g, 0, b) && reserve(g, 1, b);
 }
 
-void digit_gemm_trim(DigitGemm* g) {
-  if (!g) return;
+bool digit_gemm_trim(DigitGemm* g) {
+  if (!g) return false;
+  bool held = false;
   for (int q = 0; q < 2; q++) {
     if (g->op[q]) cudaFree(g->op[q]);
+    held |= g->op[q] != nullptr;
     g->op[q] = nullptr;
     g->op_bytes[q] = 0;
   }
+  return held;
 }
 
 cudaError_t digit_dgemm(DigitGemm* g, cudaStream_t s, bool tA, bool tB, int M, int N, int K, double alpha,

@@ -59,7 +59,7 @@ DigitMat digit_gemm_operand(DigitGemm* g, int q, int rows, int K);
 // nothing); false when the device has not the memory.  digit_gemm_trim gives
 // the operands' room back.
 bool digit_gemm_reserve(DigitGemm* g, int rows, int K);
-void digit_gemm_trim(DigitGemm* g);
+bool digit_gemm_trim(DigitGemm* g);
 // whether digit_dgemm takes the digits for this product
 bool digit_gemm_pays(long long M, long long N, long long K);
 

@@ -492,7 +492,14 @@ cudaError_t dsyev_device(cudaStream_t s, DigitGemm* dg, int n, const double* Phi
   constexpr int NBT = 512;  // K of the widest product; the back-transform at n = 5000: 35 ms with 256, 18 with 512
   const size_t bt_bytes = sizeof(double) * ((size_t)3 * NBT * n + (size_t)2 * NBT * NBT);
   void* dcw = nullptr;
-  FGLS_CUDA_TRY(cudaMalloc(&dcw, std::max(dc_workspace_bytes(n), bt_bytes)));
+  const size_t dcb = std::max(dc_workspace_bytes(n), bt_bytes);
+  cudaError_t room = cudaMalloc(&dcw, dcb);
+  if (room == cudaErrorMemoryAllocation && digit_gemm_trim(dg)) {  // FP64 products from here, in the digits' place
+    (void)cudaGetLastError();
+    dg = nullptr;
+    room = cudaMalloc(&dcw, dcb);
+  }
+  FGLS_CUDA_TRY(room);
   FGLS_CUDA_TRY(cudaMemsetAsync(dfail, 0, sizeof(int), s));
   cudaError_t rc = dc_tridiag_eig(s, dg, n, d, e, W, Z, dcw, dfail, &nl);
   unscale_kernel<<<ceil_div(n, 256), 256, 0, s>>>(n, W, top);

@@ -294,6 +294,40 @@ void drop_digits(fglsgpu_engine* e) {
   e->z_cut = e->w_cut = e->linv_cut = e->adj_cut = false;
 }
 
+// Gives back what only makes calls faster (the digits and their workspaces and, on
+// the FP64 path, L^-1), so that a call that fits without it is not refused; the
+// FP64 kernels serve from then on.  False when nothing is held.
+bool give_back(fglsgpu_engine* e) {
+  const bool inverse = e->dLinv && !split(e);
+  const bool digits = e->zmem || e->wmem || e->blkmem || e->adjmem;
+  cudaStreamSynchronize(e->comp);  // blocks in flight read them
+  if (!digit_gemm_trim(e->dg) && !digits && !inverse) return false;
+  drop_digits(e);
+  if (e->adjmem) cudaFree(e->adjmem);
+  e->adjmem = nullptr;
+  if (inverse) {
+    cudaFree(e->dLinv);
+    e->dLinv = nullptr;
+  }
+  e->dg_off = true;
+  return true;
+}
+
+// An allocation, tried again after give_back.
+template <class F>
+cudaError_t with_room(fglsgpu_engine* e, F alloc) {
+  cudaError_t r = alloc();
+  if (r == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    if (give_back(e)) r = alloc();
+  }
+  return r;
+}
+template <class T>
+cudaError_t dalloc_room(fglsgpu_engine* e, T** p, size_t count) {
+  return with_room(e, [&] { return dalloc(p, count); });
+}
+
 // The workspace of the digit products; null when the device cannot run them.
 DigitGemm* digit_work(fglsgpu_engine* e) {
   if (!e->dg && !e->dg_off && digit_gemm_create(&e->dg) != cudaSuccess) {
@@ -402,13 +436,13 @@ int compute_block(fglsgpu_engine* e, const void* dX, int fmt, int x, double* dB,
   }
   if (fmt == GENO_PACKED) {
     Prof pr(e, FGLSGPU_PROF_GENOTYPES, s);
-    if (!e->dU8) ENG_TRY(e, dalloc(&e->dU8, (size_t)c.x_b * c.wXR * c.n), "genotype bytes");
+    if (!e->dU8) ENG_TRY(e, dalloc_room(e, &e->dU8, (size_t)c.x_b * c.wXR * c.n), "genotype bytes");
     ENG_TRY(e, unpack_2bit(s, (const unsigned char*)dX, n, cols, wXR, e->dU8, e->dst, snp_base), "unpack genotypes");
     dXu8 = e->dU8;
   }
   if (dXu8) {
     Prof pr(e, FGLSGPU_PROF_GENOTYPES, s);
-    if (!e->dXw) ENG_TRY(e, dalloc(&e->dXw, (size_t)c.x_b * c.wXR * c.n), "widened genotypes");
+    if (!e->dXw) ENG_TRY(e, dalloc_room(e, &e->dXw, (size_t)c.x_b * c.wXR * c.n), "widened genotypes");
     ENG_TRY(e, u8_to_f64(s, dXu8, e->dXw, (long long)cols * n), "widen genotypes");
     dXin = e->dXw;
   }
@@ -523,14 +557,14 @@ int tune_slices(fglsgpu_engine* e) {
   auto chk = [&](cudaError_t x) {
     if (r == cudaSuccess) r = x;
   };
-  chk(dalloc(&dX, (size_t)n * xp));
-  chk(dalloc(&dBr, (size_t)nt * xp * p));
-  chk(dalloc(&dVr, (size_t)nt * xp * p * p));
-  chk(dalloc(&dBs, (size_t)nt * xp * p));
-  chk(dalloc(&dVs, (size_t)nt * xp * p * p));
+  chk(dalloc_room(e, &dX, (size_t)n * xp));
+  chk(dalloc_room(e, &dBr, (size_t)nt * xp * p));
+  chk(dalloc_room(e, &dVr, (size_t)nt * xp * p * p));
+  chk(dalloc_room(e, &dBs, (size_t)nt * xp * p));
+  chk(dalloc_room(e, &dVs, (size_t)nt * xp * p * p));
   if (c.variant == FGLSGPU_VARIANT_EIGEN) {
-    chk(dalloc(&dW, (size_t)n * xp));
-    chk(dalloc(&dQ, (size_t)n * xp));
+    chk(dalloc_room(e, &dW, (size_t)n * xp));
+    chk(dalloc_room(e, &dQ, (size_t)n * xp));
   }
   auto release = [&]() {
     for (double* q : {dX, dBr, dVr, dBs, dVs, dW, dQ})
@@ -757,7 +791,10 @@ int fglsgpu_set_problem(fglsgpu_engine* e, const double* Phi, const double* XL, 
   e->problem_set = false;
   if (c.variant == FGLSGPU_VARIANT_EIGEN) {
     int qfail = 0;
-    ENG_TRY(e, dsyev_device(s, digit_work(e), c.n, e->dPhi, n, e->dL, e->dZ, e->dW, e->deigwork, &qfail, nullptr),
+    DigitGemm* dg = digit_work(e);
+    ENG_TRY(e, with_room(e, [&] {
+              return dsyev_device(s, dg, c.n, e->dPhi, n, e->dL, e->dZ, e->dW, e->deigwork, &qfail, nullptr);
+            }),
             "eigendecomposition");
     if (qfail) return fail(e, FGLSGPU_ENOCONV, "dsyevr failed (info: 1): QL iteration did not converge");
     ENG_TRY(e, digit_dgemm(e->dg, s, true, false, c.n, c.wXL, c.n, 1.0, e->dZ, n, e->dXL, n, 0.0, e->dZtXL, n),
@@ -775,7 +812,9 @@ int fglsgpu_set_problem(fglsgpu_engine* e, const double* Phi, const double* XL, 
       if (rc) return rc;
     } else {
       if (!e->oz) {
-        ENG_TRY(e, ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, /*eigen=*/1), "split plan");
+        ENG_TRY(e, with_room(e, [&] {
+              return ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, /*eigen=*/1);
+            }), "split plan");
         ozaki_set_wait_limit(e->oz, e->wait_ns);
       }
       ENG_TRY(e, ozaki_set_eigen(e->oz, s, e->dg, e->dZ, e->dAYL, e->ddinv), "split operands");
@@ -813,7 +852,8 @@ int fglsgpu_select_trait(fglsgpu_engine* e, int j) {
           "copy XL");
   // L^-1: the split path's operand, and what the FP64 path multiplies by
   // (n^2 doubles: without the memory the FP64 path solves with L instead)
-  if (!e->dLinv && dalloc(&e->dLinv, (size_t)n * n) != cudaSuccess) {
+  if (!e->dLinv &&
+      (split(e) ? dalloc_room(e, &e->dLinv, (size_t)n * n) : dalloc(&e->dLinv, (size_t)n * n)) != cudaSuccess) {
     (void)cudaGetLastError();
     e->dLinv = nullptr;
     if (split(e)) return fail(e, FGLSGPU_ENOMEM, "no memory for the inverse of the factor");
@@ -835,7 +875,9 @@ int fglsgpu_select_trait(fglsgpu_engine* e, int j) {
   rc = check_status(e, "null model");
   if (rc) return rc;
   if (split(e)) {
-    if (!e->oz) ENG_TRY(e, ozaki_create(&e->oz, c.n, 1, c.wXL, c.wXR, c.x_b, c.slices, /*eigen=*/0), "split plan");
+    if (!e->oz) ENG_TRY(e, with_room(e, [&] {
+              return ozaki_create(&e->oz, c.n, 1, c.wXL, c.wXR, c.x_b, c.slices, /*eigen=*/0);
+            }), "split plan");
     ozaki_set_wait_limit(e->oz, e->wait_ns);
     ENG_TRY(e, ozaki_set_chol(e->oz, s, e->dLinv, e->dWY), "split operands");
     ENG_TRY(e, cudaStreamSynchronize(s), "split operands");
@@ -1025,8 +1067,8 @@ int fglsgpu_run_snps_compact(fglsgpu_engine* e, const double* XR, long long m, d
   ENG_TRY(e, cudaSetDevice(e->cfg.device), "cudaSetDevice");
   const size_t per = (size_t)out_traits(e) * e->cfg.x_b * e->p;
   for (int k = 0; k < 2; k++) {
-    if (!e->dSE[k]) ENG_TRY(e, dalloc(&e->dSE[k], per), "compact buffers");
-    if (!e->dP[k]) ENG_TRY(e, dalloc(&e->dP[k], per), "compact buffers");
+    if (!e->dSE[k]) ENG_TRY(e, dalloc_room(e, &e->dSE[k], per), "compact buffers");
+    if (!e->dP[k]) ENG_TRY(e, dalloc_room(e, &e->dP[k], per), "compact buffers");
   }
   return run_snps_impl(e, XR, GENO_F64, m, B, nullptr, SE, P);
 }
@@ -1041,12 +1083,14 @@ int fglsgpu_set_precision(fglsgpu_engine* e, int precision) {
   ENG_TRY(e, cudaStreamSynchronize(e->comp), "set_precision");
   const long long n = c.n, xb = c.x_b, wXR = c.wXR;
   if (precision == FGLSGPU_PREC_FP64 && c.variant == FGLSGPU_VARIANT_EIGEN) {
-    if (!e->dWork) ENG_TRY(e, dalloc(&e->dWork, n * xb * wXR), "FP64 buffers");
-    if (!e->dQ) ENG_TRY(e, dalloc(&e->dQ, n * xb * wXR * wXR), "FP64 buffers");
+    if (!e->dWork) ENG_TRY(e, dalloc_room(e, &e->dWork, n * xb * wXR), "FP64 buffers");
+    if (!e->dQ) ENG_TRY(e, dalloc_room(e, &e->dQ, n * xb * wXR * wXR), "FP64 buffers");
   }
   c.precision = precision;
   if (precision == FGLSGPU_PREC_SPLIT && e->problem_set && c.variant == FGLSGPU_VARIANT_EIGEN) {
-    if (!e->oz) ENG_TRY(e, ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, 1), "split plan");
+    if (!e->oz) ENG_TRY(e, with_room(e, [&] {
+              return ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, 1);
+            }), "split plan");
     ozaki_set_wait_limit(e->oz, e->wait_ns);
     ENG_TRY(e, ozaki_set_eigen(e->oz, e->comp, e->dg, e->dZ, e->dAYL, e->ddinv), "split operands");
     ENG_TRY(e, cudaStreamSynchronize(e->comp), "split operands");
@@ -1099,26 +1143,26 @@ int fglsgpu_adjoint_reset(fglsgpu_engine* e) {
   if (!e->problem_set) return fail(e, FGLSGPU_ESTATE, "set_problem must precede the adjoint");
   ENG_TRY(e, cudaSetDevice(c.device), "cudaSetDevice");
   const long long n = c.n, t = c.t, xb = c.x_b, wXL = c.wXL, p = e->p;
-  if (!e->dWork) ENG_TRY(e, dalloc(&e->dWork, n * xb), "adjoint buffers");
-  if (!e->dQ) ENG_TRY(e, dalloc(&e->dQ, n * xb), "adjoint buffers");
+  if (!e->dWork) ENG_TRY(e, dalloc_room(e, &e->dWork, n * xb), "adjoint buffers");
+  if (!e->dQ) ENG_TRY(e, dalloc_room(e, &e->dQ, n * xb), "adjoint buffers");
   if (!e->adj_ready) {
     cudaError_t r = cudaSuccess;
     auto chk = [&](cudaError_t x) {
       if (r == cudaSuccess) r = x;
     };
-    chk(dalloc(&e->aW3, n * 3 * t));
-    chk(dalloc(&e->aAYL3, n * 3 * t * (1 + wXL)));
-    chk(dalloc(&e->atopd, t * (wXL + wXL * wXL)));
-    chk(dalloc(&e->atopc, t * (wXL + wXL * wXL)));
-    chk(dalloc(&e->atops, t * (wXL + wXL * wXL)));
-    chk(dalloc(&e->areml, 2 * t));
-    chk(dalloc(&e->aG3, xb * 3 * t * (2 + wXL)));
-    chk(dalloc(&e->acontrib, 2 * t * xb));
-    chk(dalloc(&e->ag, t * xb * p));
-    chk(dalloc(&e->agR, xb * t));
-    chk(dalloc(&e->aacc, 2 * t + t * wXL));
-    chk(dalloc(&e->aU, n * t));
-    chk(dalloc(&e->aV2, n * t));
+    chk(dalloc_room(e, &e->aW3, n * 3 * t));
+    chk(dalloc_room(e, &e->aAYL3, n * 3 * t * (1 + wXL)));
+    chk(dalloc_room(e, &e->atopd, t * (wXL + wXL * wXL)));
+    chk(dalloc_room(e, &e->atopc, t * (wXL + wXL * wXL)));
+    chk(dalloc_room(e, &e->atops, t * (wXL + wXL * wXL)));
+    chk(dalloc_room(e, &e->areml, 2 * t));
+    chk(dalloc_room(e, &e->aG3, xb * 3 * t * (2 + wXL)));
+    chk(dalloc_room(e, &e->acontrib, 2 * t * xb));
+    chk(dalloc_room(e, &e->ag, t * xb * p));
+    chk(dalloc_room(e, &e->agR, xb * t));
+    chk(dalloc_room(e, &e->aacc, 2 * t + t * wXL));
+    chk(dalloc_room(e, &e->aU, n * t));
+    chk(dalloc_room(e, &e->aV2, n * t));
     if (r != cudaSuccess) return cuda_fail(e, r, "adjoint buffers");
     e->adj_ready = true;
   }
@@ -1251,7 +1295,9 @@ int fglsgpu_reml_fit(fglsgpu_engine* e, double h_lo, double h_hi, int grid, doub
   if (rc) return rc;
   // the outputs and the grid's workspace, kept for the next fit
   const size_t outb = (sizeof(double) * 4 * (size_t)t + 255) & ~(size_t)255;
-  if (!grow(&e->remlmem, &e->reml_bytes, outb + reml_workspace_bytes(c.n, t, grid)))
+  const size_t remlb = outb + reml_workspace_bytes(c.n, t, grid);
+  if (!grow(&e->remlmem, &e->reml_bytes, remlb) &&
+      !(give_back(e) && grow(&e->remlmem, &e->reml_bytes, remlb)))
     return fail(e, FGLSGPU_ENOMEM, "no memory for the REML grid");
   double* dout = (double*)e->remlmem;
   std::vector<double> r(4 * (size_t)t);
@@ -1307,7 +1353,9 @@ int fglsgpu_set_hsigma(fglsgpu_engine* e, const double* h, const double* sigma) 
   rc = check_status(e, "eigen setup");
   if (rc) return rc;
   if (split(e)) {
-    if (!e->oz) ENG_TRY(e, ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, 1), "split plan");
+    if (!e->oz) ENG_TRY(e, with_room(e, [&] {
+              return ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, 1);
+            }), "split plan");
     ozaki_set_wait_limit(e->oz, e->wait_ns);
     ENG_TRY(e, ozaki_set_eigen(e->oz, s, e->dg, e->dZ, e->dAYL, e->ddinv), "split operands");
     ENG_TRY(e, cudaStreamSynchronize(s), "split operands");
