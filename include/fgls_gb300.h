@@ -71,7 +71,7 @@ typedef struct fglsgpu_engine fglsgpu_engine;
 #define FGLSGPU_VARIANT_CHOL 0  /* per-trait Cholesky whitening (fgls_chol)  */
 #define FGLSGPU_VARIANT_EIGEN 1 /* eigenbasis of Phi, all traits per block (fgls_eigen) */
 
-#define FGLSGPU_PREC_FP64 0     /* FP64 throughout; large products as exact  
+#define FGLSGPU_PREC_FP64 0     /* FP64 throughout; large products as exact
                                    sums of digit products (60-bit operands)  */
 #define FGLSGPU_PREC_SPLIT 1    /* bulk GEMMs as 5-bit digit slices (FP8 E4M3) on
                                    tcgen05 tensor cores, exact FP32 accumulation,
