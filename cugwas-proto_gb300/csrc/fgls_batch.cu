@@ -434,11 +434,6 @@ struct Scratch {
     for (double** v : {&L, &Linv, &LinvT})
       if (e == cudaSuccess) e = dalloc(v, nn);
     if (e == cudaSuccess) e = dalloc(&diag, 64 * 64);
-    if (e == cudaSuccess && (digit_gemm_create(&dg) != cudaSuccess || !digit_gemm_reserve(dg, nmax, nmax))) {
-      (void)cudaGetLastError();
-      digit_gemm_destroy(dg);
-      dg = nullptr;
-    }
     if (e == cudaSuccess) e = dalloc(&WY, (size_t)nmax * (1 + wmax));
     if (e == cudaSuccess) e = dalloc(&U, (size_t)nmax * (1 + wmax));
     if (e == cudaSuccess) e = dalloc(&X64, (size_t)nmax * PROBE);
@@ -449,6 +444,13 @@ struct Scratch {
     if (e == cudaSuccess) e = dalloc(&st, 1);
     if (e == cudaSuccess) e = cudaMemset(st, 0, sizeof(DevStatus));
     return e;
+  }
+  // once everything the setup cannot do without is allocated
+  void digits(int nmax) {
+    if (digit_gemm_create(&dg) == cudaSuccess && digit_gemm_reserve(dg, nmax, nmax)) return;
+    (void)cudaGetLastError();
+    digit_gemm_destroy(dg);
+    dg = nullptr;
   }
   void release() {
     digit_gemm_destroy(dg);
@@ -619,6 +621,7 @@ int fglsgpu_batch_create(const fglsgpu_cohort* cohorts, int count, const fglsgpu
     if (e == cudaSuccess) e = dalloc(&ci.Y, ymax);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();  // the scratch status words' memsets
     if (e != cudaSuccess) return fail_scratch(e, "setup scratch");
+    for (int k = 0; k < ns; k++) w[k].digits(nmax);
     cudaEvent_t up = nullptr;
     if ((e = cudaEventCreateWithFlags(&up, cudaEventDisableTiming)) != cudaSuccess)
       return fail_scratch(e, "setup events");

@@ -34,3 +34,33 @@ def test_widened_genotypes_fit_in_the_digits_place(variant, t):
     se = np.abs(V0[..., i, i])
     assert np.max(np.abs(B - B0) / (np.abs(B0) + se)) <= 1e-12
     assert np.max(np.abs(np.abs(V[..., i, i]) - se) / se) <= 1e-12
+
+
+def test_batch_setup_fits_without_its_digits():
+    """One cohort of 3000 with four traits on four streams: 0.34 GB of operands and 0.94 GB
+    of FP64 scratch are needed; the digits' 0.86 GB on top are not."""
+    import torch
+    from fgls_gb300 import Batch, datagen
+    from test_gpu_batch import run_batch
+    pb = datagen.make_problem(3000, 64, 4, wXL=3, seed=9, hsig_uniform=True)
+    desc = [{"Phi": pb.Phi, "XL": pb.XL, "Y": pb.Y, "h": pb.h, "sigma": pb.sigma}]
+    with Batch(desc, x_b=256, slices=9) as b:
+        (B0, V0), = run_batch(b, [pb], 64)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    left = 1750 << 20
+    free, _ = torch.cuda.mem_get_info()
+    assert free > left
+    fill = torch.empty(free - left, dtype=torch.uint8, device="cuda")
+    try:
+        b = Batch(desc, x_b=256, slices=9)
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    with b:
+        (B, V), = run_batch(b, [pb], 64)
+    # the split path's bound, as against the oracle
+    i = np.arange(pb.p)
+    se = np.abs(V0[..., i, i])
+    assert np.max(np.abs(B - B0) / (np.abs(B0) + se)) <= 1e-10
+    assert np.max(np.abs(np.abs(V[..., i, i]) - se) / se) <= 1e-10
