@@ -786,7 +786,8 @@ def run_cohorts(args):
     # R^2 (float pairs) written once
     algo_bytes = sum(c["t"] * (S * (c["n"] * (c["n"] + 1) / 2 + c["p"] * c["n"])
                                + 8 * xb * (c["p"] + (c["n"] + 31) // 32)) + xb * c["n"] for c in co)
-    traffic = gemm_traffic(f"grouped_gemm_cohorts{C}_xb{xb}") if S == 9 else None
+    # captured for the 256 x 256 tiles
+    traffic = gemm_traffic(f"grouped_gemm_planes_cohorts{C}_xb{xb}") if S == 9 and tile[0] == 256 else None
     # end to end: host pinned genotypes -> device, step, results -> host
     Xh = [X[i][0].cpu().pin_memory() for i in range(C)]
     Bh = [torch.empty_like(d, device="cpu").pin_memory() for d in dB]
@@ -1023,7 +1024,7 @@ def run_eigen(args, rank, world, local, dist):
     timed_s = ms / 1e3
     pk_key = "bf16_tflops" if timed_s < 3.0 else "bf16_tflops_sustained"
     peak = 2.0 * float(pk.get(pk_key, FALLBACK_PEAKS[pk_key]))
-    traffic = gemm_traffic(f"ozaki_gemm_n{n}_t{t}_xb{xb}")
+    traffic = gemm_traffic(f"ozaki_gemm_planes_n{n}_t{t}_xb{xb}")
     Mpad, Kpad = -(-M_A // 128) * 128, -(-n // 128) * 128
     algo_bytes = S_used * Mpad * Kpad + xb * Kpad + 8 * Mpad * xb  # A slices + genotypes read, C written once
 
