@@ -368,12 +368,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
           }
         }
       }
-      if (ok) {
-        // every step filled so far has been released by the leader's MMAs: no
-        // multicast commit is still on its way to this CTA
-        while (head != tail)
-          if (!release(45)) break;
-      } else if (lead) {
+      // every step filled so far is released by the leader's MMAs: no multicast
+      // commit is still on its way to this CTA
+      while (ok && head != tail) ok = release(45);
+      if (!ok && lead) {  // the leader's barriers track both CTAs' copies of the steps it armed
         const uint64_t deadline = globaltimer_ns() + WAIT_NS;
         for (; head != tail; head++) mbar_drain_until(&full[head % STEPS], (head / STEPS) & 1, deadline);
       }
@@ -812,6 +810,7 @@ struct DigitGemm {
   int clusters = 0;
   int4* planes = nullptr;      // MAXPASS planes a CTA, or one a unit and CTA in the split form
   int* err = nullptr;
+  unsigned long long wait_ns = WAIT_NS;
   void* op[2] = {nullptr, nullptr};
   size_t op_bytes[2] = {0, 0};
 };
@@ -891,6 +890,8 @@ void digit_gemm_destroy(DigitGemm* g) {
 
 int* digit_gemm_error_word(DigitGemm* g) { return g->err; }
 
+void digit_gemm_set_wait_limit(DigitGemm* g, unsigned long long ns) { g->wait_ns = ns ? ns : WAIT_NS; }
+
 cudaError_t digit_mul(DigitGemm* g, cudaStream_t s, const DigitMat& A, const DigitMat& B, double alpha, double beta,
                       double* C, long long ldc, const DigitMulOpts& o) {
   if (A.K != B.K) return cudaErrorInvalidValue;
@@ -911,7 +912,7 @@ cudaError_t digit_mul(DigitGemm* g, cudaStream_t s, const DigitMat& A, const Dig
   a.alpha = alpha;
   a.planes = g->planes;
   a.err = g->err;
-  a.wait_ns = WAIT_NS;
+  a.wait_ns = g->wait_ns;
   const int tiles = o.c_lower ? a.tiles_m * (a.tiles_m + 1) / 2 : a.tiles_m * a.tiles_n;
   const int nk_all = A.Kpad / ROW;
   for (int kb = 0; kb < nk_all; kb += K_MAX_STEPS) {

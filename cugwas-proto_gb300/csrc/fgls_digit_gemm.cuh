@@ -37,6 +37,8 @@ struct DigitGemm;
 cudaError_t digit_gemm_create(DigitGemm** out);  // cudaErrorNotSupported: no clusters of two
 void digit_gemm_destroy(DigitGemm* g);
 int* digit_gemm_error_word(DigitGemm* g);
+// limit of one wait of the products launched from now on (0: the default, 2 s)
+void digit_gemm_set_wait_limit(DigitGemm* g, unsigned long long ns);
 
 struct DigitMulOpts {
   bool a_lower = false;    // row r of A is zero beyond column r

@@ -330,9 +330,13 @@ cudaError_t dalloc_room(fglsgpu_engine* e, T** p, size_t count) {
 
 // The workspace of the digit products; null when the device cannot run them.
 DigitGemm* digit_work(fglsgpu_engine* e) {
-  if (!e->dg && !e->dg_off && digit_gemm_create(&e->dg) != cudaSuccess) {
-    (void)cudaGetLastError();
-    e->dg_off = true;
+  if (!e->dg && !e->dg_off) {
+    if (digit_gemm_create(&e->dg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      e->dg_off = true;
+    } else {
+      digit_gemm_set_wait_limit(e->dg, e->wait_ns);
+    }
   }
   return e->dg;
 }
@@ -1119,6 +1123,7 @@ int fglsgpu_set_wait_limit(fglsgpu_engine* e, long long ns) {
   if (ns < 0) return fail(e, FGLSGPU_EINVAL, "wait limit %lld < 0", ns);
   e->wait_ns = (unsigned long long)ns;
   if (e->oz) ozaki_set_wait_limit(e->oz, e->wait_ns);
+  if (e->dg) digit_gemm_set_wait_limit(e->dg, e->wait_ns);
   return FGLSGPU_OK;
 }
 

@@ -1,0 +1,27 @@
+"""Bounded waits of the FP64 path's digit products (csrc/fgls_digit_gemm.cu): with a
+limit of 1 ns the kernel gives up at its first wait that does not complete at once,
+lets its copies and MMAs finish (those waits keep the 2 s limit), frees its TMEM and
+returns; the call that launched it reports FGLSGPU_ETIMEOUT, and with the default
+limit restored the same engine gives bit-identical results."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("variant,wXR", [("eigen", 1), ("eigen", 2), ("chol", 1)])
+def test_expired_wait_in_a_block(variant, wXR):
+    from fgls_gb300 import Engine, FGLSError, datagen
+    from fgls_gb300.engine import ETIMEOUT
+    pb = datagen.make_problem(1000, 400, 2, wXR=wXR, seed=5, hsig_uniform=True)  # two blocks, the second ragged
+    with Engine(pb.n, pb.wXL, wXR, pb.t, 256, variant=variant) as e:
+        e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+        e.select_trait(0)
+        B1, V1 = e.run_snps(pb.XR)
+        e.set_wait_limit(1)
+        with pytest.raises(FGLSError) as ei:
+            e.run_snps(pb.XR)
+        assert ei.value.code == ETIMEOUT and "wait expired" in str(ei.value), ei.value
+        e.set_wait_limit(0)
+        B2, V2 = e.run_snps(pb.XR)
+    assert np.array_equal(B1, B2) and np.array_equal(V1, V2)
