@@ -1261,7 +1261,8 @@ int fglsgpu_adjoint_read(fglsgpu_engine* e, double* dh, double* dsigma, double* 
   }
   std::vector<double> acc(2 * t);
   ENG_TRY(e, cudaMemcpyAsync(acc.data(), e->aacc, sizeof(double) * 2 * t, cudaMemcpyDeviceToHost, s), "dh");
-  ENG_TRY(e, cudaStreamSynchronize(s), "adjoint read");
+  rc = check_status(e, "adjoint read");  // dY's product may run on digits, whose waits are bounded
+  if (rc) return rc;
   for (int j = 0; j < t; j++) {
     if (dh) dh[j] = acc[j];
     if (dsigma) dsigma[j] = acc[t + j];

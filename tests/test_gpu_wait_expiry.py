@@ -25,3 +25,27 @@ def test_expired_wait_in_a_block(variant, wXR):
         e.set_wait_limit(0)
         B2, V2 = e.run_snps(pb.XR)
     assert np.array_equal(B1, B2) and np.array_equal(V1, V2)
+
+
+def test_expired_wait_in_the_read_of_the_adjoint():
+    """dY = Z V2 is launched by the read itself (n = 2000, t = 32: on digits)."""
+    import torch
+    from fgls_gb300 import Engine, FGLSError, datagen
+    from fgls_gb300.engine import ETIMEOUT
+    pb = datagen.make_problem(2000, 256, 32, seed=6, hsig_uniform=True)
+    bbar = torch.from_numpy(np.random.default_rng(6).standard_normal((pb.t, pb.m, pb.p))).cuda()
+    X = torch.from_numpy(np.ascontiguousarray(pb.XR.T)).cuda()
+    torch.cuda.synchronize()
+    with Engine(pb.n, pb.wXL, 1, pb.t, 256, variant="eigen") as e:
+        e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+        e.adjoint_reset()
+        e.adjoint_block_device(X.data_ptr(), pb.m, bbar.data_ptr(), bbar.stride(0))
+        first = e.adjoint_read()
+        e.set_wait_limit(1)
+        with pytest.raises(FGLSError) as ei:
+            e.adjoint_read()
+        assert ei.value.code == ETIMEOUT, ei.value
+        e.set_wait_limit(0)
+        again = e.adjoint_read()
+    for a, b in zip(first, again):
+        assert np.array_equal(a, b)
