@@ -131,10 +131,10 @@ cudaError_t dalloc(T** p, size_t count) {
   return cudaMalloc((void**)p, sizeof(T) * count);
 }
 
-// Reads the device status word after a sync; maps failures to messages that
-// follow the reference's error texts (src/fgls_chol.c:266-271, :309-314, :418-434).
-int check_status(fglsgpu_engine* e, const char* stage) {
-  ENG_TRY(e, cudaMemcpyAsync(e->hst, e->dst, sizeof(DevStatus), cudaMemcpyDeviceToHost, e->comp), "status copy");
+// Waits for the compute stream and reports an expired wait of the tcgen05
+// kernels since the last check: their outputs are invalid.  Clears the words, so
+// that the next launches run normally.
+int check_waits(fglsgpu_engine* e, const char* stage) {
   e->hst_wait[0] = e->hst_wait[1] = 0;
   if (e->oz)
     ENG_TRY(e, cudaMemcpyAsync(e->hst_wait, ozaki_error_word(e->oz), sizeof(int), cudaMemcpyDeviceToHost, e->comp),
@@ -144,17 +144,21 @@ int check_status(fglsgpu_engine* e, const char* stage) {
                                e->comp),
             "status copy");
   ENG_TRY(e, cudaStreamSynchronize(e->comp), stage);
-  const DevStatus s = *e->hst;
   const int wsite = e->hst_wait[0] ? e->hst_wait[0] : e->hst_wait[1];
-  if (wsite) {
-    // the tcgen05 kernels gave up on a pipeline wait: their outputs since the
-    // last check are invalid; clear the words so that the next launches run
-    // normally
-    if (e->oz) ENG_TRY(e, cudaMemsetAsync(ozaki_error_word(e->oz), 0, sizeof(int), e->comp), "status reset");
-    if (e->dg) ENG_TRY(e, cudaMemsetAsync(digit_gemm_error_word(e->dg), 0, sizeof(int), e->comp), "status reset");
-    ENG_TRY(e, cudaStreamSynchronize(e->comp), "status reset");
-    return fail(e, FGLSGPU_ETIMEOUT, "device wait expired in %s (tensor-core kernel wait site %d)", stage, wsite);
-  }
+  if (!wsite) return FGLSGPU_OK;
+  if (e->oz) ENG_TRY(e, cudaMemsetAsync(ozaki_error_word(e->oz), 0, sizeof(int), e->comp), "status reset");
+  if (e->dg) ENG_TRY(e, cudaMemsetAsync(digit_gemm_error_word(e->dg), 0, sizeof(int), e->comp), "status reset");
+  ENG_TRY(e, cudaStreamSynchronize(e->comp), "status reset");
+  return fail(e, FGLSGPU_ETIMEOUT, "device wait expired in %s (tensor-core kernel wait site %d)", stage, wsite);
+}
+
+// Reads the device status word after a sync; maps failures to messages that
+// follow the reference's error texts (src/fgls_chol.c:266-271, :309-314, :418-434).
+int check_status(fglsgpu_engine* e, const char* stage) {
+  ENG_TRY(e, cudaMemcpyAsync(e->hst, e->dst, sizeof(DevStatus), cudaMemcpyDeviceToHost, e->comp), "status copy");
+  const int rc = check_waits(e, stage);
+  if (rc) return rc;
+  const DevStatus s = *e->hst;
   if (s.code == FGLSGPU_OK) return FGLSGPU_OK;
   if (s.code == FGLSGPU_ENOTSPD) {
     if (!strcmp(stage, "potrf(M)"))
@@ -660,6 +664,19 @@ int tune_slices(fglsgpu_engine* e) {
   return FGLSGPU_OK;
 }
 
+// The split path's operands of the eigen variant (its plan on the first call) and the slice choice.
+int split_operands(fglsgpu_engine* e) {
+  const fglsgpu_config& c = e->cfg;
+  if (!e->oz)
+    ENG_TRY(e, with_room(e, [&] {
+              return ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, /*eigen=*/1);
+            }), "split plan");
+  ozaki_set_wait_limit(e->oz, e->wait_ns);
+  ENG_TRY(e, ozaki_set_eigen(e->oz, e->comp, e->dg, e->dZ, e->dAYL, e->ddinv), "split operands");
+  const int rc = check_waits(e, "split operands");  // U = Z AYL may run on digits
+  return rc ? rc : tune_slices(e);
+}
+
 }  // namespace
 
 extern "C" {
@@ -815,15 +832,7 @@ int fglsgpu_set_problem(fglsgpu_engine* e, const double* Phi, const double* XL, 
       rc = eigen_digits(e, (long long)c.x_b * c.wXR, &use);
       if (rc) return rc;
     } else {
-      if (!e->oz) {
-        ENG_TRY(e, with_room(e, [&] {
-              return ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, /*eigen=*/1);
-            }), "split plan");
-        ozaki_set_wait_limit(e->oz, e->wait_ns);
-      }
-      ENG_TRY(e, ozaki_set_eigen(e->oz, s, e->dg, e->dZ, e->dAYL, e->ddinv), "split operands");
-      ENG_TRY(e, cudaStreamSynchronize(s), "split operands");
-      rc = tune_slices(e);
+      rc = split_operands(e);
       if (rc) return rc;
     }
   }
@@ -1092,14 +1101,11 @@ int fglsgpu_set_precision(fglsgpu_engine* e, int precision) {
   }
   c.precision = precision;
   if (precision == FGLSGPU_PREC_SPLIT && e->problem_set && c.variant == FGLSGPU_VARIANT_EIGEN) {
-    if (!e->oz) ENG_TRY(e, with_room(e, [&] {
-              return ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, 1);
-            }), "split plan");
-    ozaki_set_wait_limit(e->oz, e->wait_ns);
-    ENG_TRY(e, ozaki_set_eigen(e->oz, e->comp, e->dg, e->dZ, e->dAYL, e->ddinv), "split operands");
-    ENG_TRY(e, cudaStreamSynchronize(e->comp), "split operands");
-    const int rc = tune_slices(e);
-    if (rc) return rc;
+    const int rc = split_operands(e);
+    if (rc) {
+      c.precision = FGLSGPU_PREC_FP64;  // whose operands are intact; the call can be repeated
+      return rc;
+    }
   }
   if (c.variant == FGLSGPU_VARIANT_CHOL) e->trait_sel = -1;  // re-select: the operands differ per path
   return FGLSGPU_OK;
@@ -1359,13 +1365,7 @@ int fglsgpu_set_hsigma(fglsgpu_engine* e, const double* h, const double* sigma) 
   rc = check_status(e, "eigen setup");
   if (rc) return rc;
   if (split(e)) {
-    if (!e->oz) ENG_TRY(e, with_room(e, [&] {
-              return ozaki_create(&e->oz, c.n, c.t, c.wXL, c.wXR, c.x_b, c.slices, 1);
-            }), "split plan");
-    ozaki_set_wait_limit(e->oz, e->wait_ns);
-    ENG_TRY(e, ozaki_set_eigen(e->oz, s, e->dg, e->dZ, e->dAYL, e->ddinv), "split operands");
-    ENG_TRY(e, cudaStreamSynchronize(s), "split operands");
-    rc = tune_slices(e);
+    rc = split_operands(e);
     if (rc) return rc;
   }
   ENG_TRY(e, cudaStreamSynchronize(s), "set_hsigma");

@@ -49,3 +49,34 @@ def test_expired_wait_in_the_read_of_the_adjoint():
         again = e.adjoint_read()
     for a, b in zip(first, again):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("call", ["set_hsigma", "set_precision"])
+def test_expired_wait_in_the_split_operands(call):
+    """U = Z [d y, d XL] (n = 1000, 160 columns: on digits) is the last product of
+    the calls that build the split path's operands; with given slices no probe
+    block follows it."""
+    from fgls_gb300 import Engine, FGLSError, datagen
+    from fgls_gb300.engine import ETIMEOUT
+    pb = datagen.make_problem(1000, 200, 40, seed=7, hsig_uniform=True)
+    first = "split" if call == "set_hsigma" else "fp64"
+    with Engine(pb.n, 3, 1, pb.t, 256, variant="eigen", precision="split", slices=9) as e:
+        e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+        B1, V1 = e.run_snps(pb.XR)
+    with Engine(pb.n, 3, 1, pb.t, 256, variant="eigen", precision=first, slices=9) as e:
+        def build():
+            if call == "set_hsigma":
+                e.set_hsigma(pb.h, pb.sigma)
+            else:
+                e.set_precision("split")
+        e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+        e.set_wait_limit(1)
+        with pytest.raises(FGLSError) as ei:
+            build()
+        assert ei.value.code == ETIMEOUT, ei.value
+        e.set_wait_limit(0)
+        if call == "set_hsigma":  # the problem's operands are gone, as after any failure of the call
+            e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+        build()
+        B2, V2 = e.run_snps(pb.XR)
+    assert np.array_equal(B1, B2) and np.array_equal(V1, V2)
