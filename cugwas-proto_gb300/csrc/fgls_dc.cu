@@ -218,8 +218,11 @@ __global__ void __launch_bounds__(256) dc_deflate_kernel(int nn, double rho, dou
     if (STAGED) {
       sd[i] = dv;
       sz[i] = zv;
-      sp[i] = perm[i];
     }
+    // NaN eigenvalues (a NaN in Phi, or vectors that a product whose wait expired
+    // left unset) are not ordered: ranks collide and perm keeps what an earlier merge
+    // or nobody wrote there.  Every column index below comes from here.
+    sp[i] = min(max(perm[i], 0), nn - 1);
     dmax = fmax(dmax, fabs(dv));
     zmax = fmax(zmax, fabs(zv));
   }
