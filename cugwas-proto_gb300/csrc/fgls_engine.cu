@@ -817,7 +817,10 @@ int fglsgpu_set_problem(fglsgpu_engine* e, const double* Phi, const double* XL, 
               return dsyev_device(s, dg, c.n, e->dPhi, n, e->dL, e->dZ, e->dW, e->deigwork, &qfail, nullptr);
             }),
             "eigendecomposition");
-    if (qfail) return fail(e, FGLSGPU_ENOCONV, "dsyevr failed (info: 1): QL iteration did not converge");
+    if (qfail) {
+      rc = check_waits(e, "eigendecomposition");  // the cause, if a product gave up
+      return rc ? rc : fail(e, FGLSGPU_ENOCONV, "dsyevr failed (info: 1): QL iteration did not converge");
+    }
     ENG_TRY(e, digit_dgemm(e->dg, s, true, false, c.n, c.wXL, c.n, 1.0, e->dZ, n, e->dXL, n, 0.0, e->dZtXL, n),
             "Z^T XL");
     ENG_TRY(e, digit_dgemm(e->dg, s, true, false, c.n, c.t, c.n, 1.0, e->dZ, n, e->dY, n, 0.0, e->dZtY, n), "Z^T Y");

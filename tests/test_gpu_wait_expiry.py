@@ -80,3 +80,21 @@ def test_expired_wait_in_the_split_operands(call):
         build()
         B2, V2 = e.run_snps(pb.XR)
     assert np.array_equal(B1, B2) and np.array_equal(V1, V2)
+
+
+def test_expired_wait_in_an_eigendecomposition_that_fails():
+    """A NaN in Phi makes the QL iteration fail as well: the expired wait is the
+    error, and it is not left for the next call to report."""
+    from fgls_gb300 import Engine, FGLSError, datagen
+    from fgls_gb300.engine import ETIMEOUT
+    pb = datagen.make_problem(1100, 64, 2, seed=8, hsig_uniform=True)
+    bad = pb.Phi.copy()
+    bad[5, 9] = bad[9, 5] = np.nan
+    with Engine(pb.n, 3, 1, 2, 64, variant="eigen") as e:
+        e.set_wait_limit(1)
+        with pytest.raises(FGLSError) as ei:
+            e.set_problem(bad, pb.XL, pb.Y, pb.h, pb.sigma)
+        assert ei.value.code == ETIMEOUT, ei.value
+        e.set_wait_limit(0)
+        e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+        e.run_snps(pb.XR)
