@@ -357,9 +357,7 @@ int chol_digits(fglsgpu_engine* e, long long cols, bool* use) {
   if (!((e->zmem || grow(&e->zmem, &none, digit_mat_bytes(n, n))) &&
         grow(&e->blkmem, &e->blk_bytes, digit_mat_bytes((int)most, n)))) {
     drop_digits(e);
-    e->dg_off = true;
-    digit_gemm_destroy(e->dg);
-    e->dg = nullptr;
+    e->dg_off = true;  // (e->dg stays: products of its are in flight, their error word is still to be read)
     return FGLSGPU_OK;
   }
   if (!e->linv_cut) {

@@ -98,3 +98,36 @@ def test_expired_wait_in_an_eigendecomposition_that_fails():
         e.set_wait_limit(0)
         e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
         e.run_snps(pb.XR)
+
+
+def test_expired_wait_in_the_inverse_when_the_block_digits_do_not_fit():
+    """n = 762: of select_trait's products only those of L^-1 run on digits.  The digits
+    of a block of 65536 SNPs (600 MB) do not fit, which must not lose their error."""
+    import torch
+    from fgls_gb300 import Engine, FGLSError, datagen
+    from fgls_gb300.engine import ETIMEOUT
+    pb = datagen.make_problem(762, 300, 1, seed=9, hsig_uniform=True)
+    with Engine(pb.n, 3, 1, 1, 300, variant="chol") as e:
+        e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+        e.select_trait(0)
+        B1, V1 = e.run_snps(pb.XR)
+    with Engine(pb.n, 3, 1, 1, 65536, variant="chol") as e:
+        e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+        free, _ = torch.cuda.mem_get_info()
+        fill = torch.empty(free - (320 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            e.set_wait_limit(1)
+            with pytest.raises(FGLSError) as ei:
+                e.select_trait(0)
+            assert ei.value.code == ETIMEOUT, ei.value
+            e.set_wait_limit(0)
+            e.select_trait(0)
+            B2, V2 = e.run_snps(pb.XR)
+        finally:
+            del fill
+            torch.cuda.empty_cache()
+    # two FP64-accurate routes of the same problem, as in test_gpu_scratch_limits.py
+    i = np.arange(pb.p)
+    se = np.abs(V1[..., i, i])
+    assert np.max(np.abs(B1 - B2) / (np.abs(B1) + se)) <= 1e-12
+    assert np.max(np.abs(np.abs(V2[..., i, i]) - se) / se) <= 1e-12
