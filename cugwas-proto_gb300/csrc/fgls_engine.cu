@@ -874,9 +874,11 @@ int fglsgpu_select_trait(fglsgpu_engine* e, int j) {
   }
   e->linv_cut = false;
   if (e->dLinv) ENG_TRY(e, lower_inverse(s, dg, c.n, e->dL, n, e->dLinv), "inverse of the factor");
-  bool digits = false;
-  rc = chol_digits(e, split(e) ? std::min((long long)TUNE_SNPS, (long long)c.x_b) : (long long)c.x_b * c.wXR, &digits);
-  if (rc) return rc;
+  if (!split(e)) {  // room for the blocks' digits (on the split path the probe block takes its own)
+    bool digits = false;
+    rc = chol_digits(e, (long long)c.x_b * c.wXR, &digits);
+    if (rc) return rc;
+  }
   if (e->dLinv && !e->dg_off) {
     // whitening as a product with L^-1: the solve is a chain of 128-column steps
     // (24 ms at n = 10000, 2.2 ms at n = 1000)

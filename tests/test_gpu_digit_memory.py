@@ -1,0 +1,63 @@
+"""Device memory that the digits of the FP64 products take: only where a call uses
+them, and not from calls that fit without."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+def free_bytes():
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.cuda.mem_get_info()[0]
+
+
+class Fill:
+    """Takes the device's memory but `left` bytes."""
+
+    def __init__(self, left):
+        import torch
+        free = free_bytes()
+        assert free > left
+        self.t = torch.empty(free - left, dtype=torch.uint8, device="cuda")
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        import torch
+        del self.t
+        torch.cuda.empty_cache()
+
+
+def same(B, V, B0, V0):
+    """Two FP64-accurate routes of one problem: 1e-12 on the standard errors' scale, as for parity."""
+    i = np.arange(B.shape[-1])
+    se = np.abs(V0[..., i, i])
+    assert np.max(np.abs(B - B0) / (np.abs(B0) + se)) <= 1e-12
+    assert np.max(np.abs(np.abs(V[..., i, i]) - se) / se) <= 1e-12
+
+
+def test_split_chol_takes_no_digits_of_a_whole_block():
+    """The split path's blocks have operands of their own; its FP64 probe block takes the
+    digits of 256 SNPs.  Those of a whole block (16384 SNPs: 590 MB) do not fit here, and
+    the next trait's set-up must not notice."""
+    from fgls_gb300 import Engine, datagen
+    from fgls_gb300.engine import launch_count
+    n = 3000
+    pb = datagen.make_problem(n, 64, 2, seed=10)
+    pb.Y[:, 1] = pb.Y[:, 0]  # the same trait twice: the same launches
+    with Engine(n, 3, 1, 2, 16384, variant="chol", precision="split") as e:
+        def launches(j):
+            a = launch_count()
+            e.select_trait(j)
+            return launch_count() - a
+        e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+        e.select_trait(0)  # the plan
+        usual = launches(1)
+        with Fill(500 * MB):
+            launches(0)
+            assert launches(1) == usual
