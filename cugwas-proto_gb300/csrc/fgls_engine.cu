@@ -81,7 +81,7 @@ struct fglsgpu_engine {
   // FP64 products through digits (fgls_digit_gemm.cu): the resident operands,
   // cut again only when they change, and the block's operand
   DigitGemm* dg = nullptr;
-  bool dg_off = false;  // no CTA pairs or no memory for the digits: FP64 kernels throughout
+  bool dg_off = false;  // no CTA pairs or no memory to hold digits: blocks run on the FP64 kernels
   DigitMat zdig, ayldig, ddig;  // eigen: Z^T, AYL^T, dinv^T rows
   // chol: the selected trait's L^-1 (null: no memory for it, the blocks then
   // run a blocked TRSM) and its rows' digits (valid when linv_cut), 64 x 64 scratch
@@ -299,8 +299,9 @@ void drop_digits(fglsgpu_engine* e) {
 }
 
 // Gives back what only makes calls faster (the digits and their workspaces and, on
-// the FP64 path, L^-1), so that a call that fits without it is not refused; the
-// FP64 kernels serve from then on.  False when nothing is held.
+// the FP64 path, L^-1), so that a call that fits without it is not refused; blocks
+// run on the FP64 kernels from then on.  (Set-up calls still cut digits where there
+// is room for the moment.)  False when nothing is held.
 bool give_back(fglsgpu_engine* e) {
   const bool inverse = e->dLinv && !split(e);
   const bool digits = e->zmem || e->wmem || e->blkmem || e->adjmem;
@@ -351,7 +352,7 @@ int chol_digits(fglsgpu_engine* e, long long cols, bool* use) {
   *use = false;
   const fglsgpu_config& c = e->cfg;
   const int n = c.n;
-  if (!e->dLinv || !digit_gemm_pays(n, cols, n) || !digit_work(e)) return FGLSGPU_OK;
+  if (e->dg_off || !e->dLinv || !digit_gemm_pays(n, cols, n) || !digit_work(e)) return FGLSGPU_OK;
   const long long most = e->probing ? cols : std::max<long long>(cols, (long long)c.x_b * c.wXR);
   size_t none = 0;
   if (!((e->zmem || grow(&e->zmem, &none, digit_mat_bytes(n, n))) &&
@@ -865,15 +866,17 @@ int fglsgpu_select_trait(fglsgpu_engine* e, int j) {
   ENG_TRY(e, cudaMemcpyAsync(e->dWY + n, e->dXL, sizeof(double) * n * c.wXL, cudaMemcpyDeviceToDevice, s),
           "copy XL");
   // L^-1: the split path's operand, and what the FP64 path multiplies by
-  // (n^2 doubles: without the memory the FP64 path solves with L instead)
-  if (!e->dLinv &&
+  // (n^2 doubles: without the memory, or where the digits are off and its blocks
+  // solve with L, the FP64 path does not form it)
+  const bool inverse = split(e) || !e->dg_off;
+  if (inverse && !e->dLinv &&
       (split(e) ? dalloc_room(e, &e->dLinv, (size_t)n * n) : dalloc(&e->dLinv, (size_t)n * n)) != cudaSuccess) {
     (void)cudaGetLastError();
     e->dLinv = nullptr;
     if (split(e)) return fail(e, FGLSGPU_ENOMEM, "no memory for the inverse of the factor");
   }
   e->linv_cut = false;
-  if (e->dLinv) ENG_TRY(e, lower_inverse(s, dg, c.n, e->dL, n, e->dLinv), "inverse of the factor");
+  if (inverse && e->dLinv) ENG_TRY(e, lower_inverse(s, dg, c.n, e->dL, n, e->dLinv), "inverse of the factor");
   if (!split(e)) {  // room for the blocks' digits (on the split path the probe block takes its own)
     bool digits = false;
     rc = chol_digits(e, (long long)c.x_b * c.wXR, &digits);

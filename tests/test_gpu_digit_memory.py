@@ -61,3 +61,25 @@ def test_split_chol_takes_no_digits_of_a_whole_block():
         with Fill(500 * MB):
             launches(0)
             assert launches(1) == usual
+
+
+def test_chol_traits_after_the_digits_were_given_back():
+    """The widened genotypes (524 MB) take the digits' place; the next select_trait must
+    not take L^-1 (128 MB) and the digits (980 MB) again, which its blocks will not use."""
+    from fgls_gb300 import Engine, datagen
+    n = 4000
+    pb = datagen.make_problem(n, 64, 2, seed=11, hsig_uniform=True)
+    G = np.ascontiguousarray(np.tile(pb.XR.astype(np.uint8), (1, 4)).T)
+    with Engine(n, 3, 1, 2, 16384, variant="chol") as e:
+        e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+        ref = []
+        for j in range(2):
+            e.select_trait(j)
+            ref.append(e.run_block(pb.XR))
+        with Fill(384 * MB):
+            e.run_snps_genotypes(G)
+        before = free_bytes()
+        for j in range(2):
+            e.select_trait(j)
+            same(*e.run_block(pb.XR), *ref[j])
+        assert before - free_bytes() < 64 * MB  # the factorization's own panels
