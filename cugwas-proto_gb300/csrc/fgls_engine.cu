@@ -554,7 +554,6 @@ constexpr int TUNE_MIN_SLICES = 6, TUNE_MIN_QDIGITS = 8;
 
 int tune_slices(fglsgpu_engine* e) {
   fglsgpu_config& c = e->cfg;
-  if (!split(e) || !e->oz || c.slices != 0) return FGLSGPU_OK;
   cudaStream_t s = e->comp;
   const int n = c.n, p = e->p, nt = out_traits(e), xp = std::min(TUNE_SNPS, c.x_b);
   int built = 0;
@@ -654,13 +653,20 @@ int tune_slices(fglsgpu_engine* e) {
   }
   release();
   if (!rc) rc = check_status(e, "slice probe");
-  drop_digits(e);  // the FP64 probe's operands: the split path needs the memory itself
-  digit_gemm_trim(e->dg);
   if (rc) return rc;
   ENG_TRY(e, ozaki_set_run_slices(e->oz, s, chosen), "slice choice");
   ENG_TRY(e, cudaStreamSynchronize(s), "slice choice");
   e->tune_err = err;
   return FGLSGPU_OK;
+}
+
+// The end of the split path's set-up: the slice choice, unless the caller made it,
+// then the FP64 products' operands, which no block of it uses, are given back.
+int finish_split(fglsgpu_engine* e) {
+  const int rc = e->cfg.slices == 0 ? tune_slices(e) : FGLSGPU_OK;
+  drop_digits(e);
+  digit_gemm_trim(e->dg);
+  return rc;
 }
 
 // The split path's operands of the eigen variant (its plan on the first call) and the slice choice.
@@ -673,7 +679,7 @@ int split_operands(fglsgpu_engine* e) {
   ozaki_set_wait_limit(e->oz, e->wait_ns);
   ENG_TRY(e, ozaki_set_eigen(e->oz, e->comp, e->dg, e->dZ, e->dAYL, e->ddinv), "split operands");
   const int rc = check_waits(e, "split operands");  // U = Z AYL may run on digits
-  return rc ? rc : tune_slices(e);
+  return rc ? rc : finish_split(e);
 }
 
 }  // namespace
@@ -901,7 +907,7 @@ int fglsgpu_select_trait(fglsgpu_engine* e, int j) {
     ENG_TRY(e, ozaki_set_chol(e->oz, s, e->dLinv, e->dWY), "split operands");
     ENG_TRY(e, cudaStreamSynchronize(s), "split operands");
     e->trait_sel = j;
-    rc = tune_slices(e);
+    rc = finish_split(e);
     if (rc) {
       e->trait_sel = -1;
       return rc;

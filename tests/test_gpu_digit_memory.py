@@ -83,3 +83,19 @@ def test_chol_traits_after_the_digits_were_given_back():
             e.select_trait(j)
             same(*e.run_block(pb.XR), *ref[j])
         assert before - free_bytes() < 64 * MB  # the factorization's own panels
+
+
+@pytest.mark.parametrize("variant", ["eigen", "chol"])
+def test_split_set_up_gives_its_operands_back(variant):
+    """A split engine of 9 given slices holds no more than one that chose its 9 by the
+    probe: the digits of the set-up's FP64 products (two operands of 108 MB) go."""
+    from fgls_gb300 import Engine, datagen
+    pb = datagen.make_problem(3000, 64, 40, seed=12, hsig_uniform=True)
+    held = {}
+    for slices in (9, 0):
+        before = free_bytes()
+        with Engine(pb.n, 3, 1, 40, 256, variant=variant, precision="split", slices=slices) as e:
+            e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+            e.select_trait(0)
+            held[slices] = before - free_bytes()
+    assert held[9] <= held[0] + 16 * MB, held
