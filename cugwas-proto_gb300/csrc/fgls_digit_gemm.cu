@@ -808,7 +808,7 @@ int dg_clusters() {
 
 struct DigitGemm {
   int clusters = 0;
-  int4* planes = nullptr;      // MAXPASS planes a CTA, or one a unit and CTA in the split form
+  int4* planes = nullptr;      // MAXPASS planes a CTA, or one a unit and CTA in the split form (120 MB)
   int* err = nullptr;
   unsigned long long wait_ns = WAIT_NS;
   void* op[2] = {nullptr, nullptr};
@@ -868,8 +868,7 @@ cudaError_t digit_gemm_create(DigitGemm** out) {
   if (n <= 0 || !encoder()) return cudaErrorNotSupported;
   DigitGemm* g = new DigitGemm();
   g->clusters = n;
-  cudaError_t r = cudaMalloc(&g->planes, sizeof(int4) * (size_t)MAXPASS * PLANE4 * 2 * n);
-  if (r == cudaSuccess) r = cudaMalloc(&g->err, sizeof(int));
+  cudaError_t r = cudaMalloc(&g->err, sizeof(int));
   if (r == cudaSuccess) r = cudaMemset(g->err, 0, sizeof(int));
   if (r == cudaSuccess) r = cudaDeviceSynchronize();  // the memset ran on the default stream
   if (r != cudaSuccess) {
@@ -888,6 +887,14 @@ void digit_gemm_destroy(DigitGemm* g) {
   delete g;
 }
 
+bool digit_gemm_ready(DigitGemm* g) {
+  if (g->planes) return true;
+  if (cudaMalloc(&g->planes, sizeof(int4) * (size_t)MAXPASS * PLANE4 * 2 * g->clusters) == cudaSuccess) return true;
+  (void)cudaGetLastError();
+  g->planes = nullptr;
+  return false;
+}
+
 int* digit_gemm_error_word(DigitGemm* g) { return g->err; }
 
 void digit_gemm_set_wait_limit(DigitGemm* g, unsigned long long ns) { g->wait_ns = ns ? ns : WAIT_NS; }
@@ -895,6 +902,7 @@ void digit_gemm_set_wait_limit(DigitGemm* g, unsigned long long ns) { g->wait_ns
 cudaError_t digit_mul(DigitGemm* g, cudaStream_t s, const DigitMat& A, const DigitMat& B, double alpha, double beta,
                       double* C, long long ldc, const DigitMulOpts& o) {
   if (A.K != B.K) return cudaErrorInvalidValue;
+  if (!digit_gemm_ready(g)) return cudaErrorMemoryAllocation;
   CUtensorMap ma, mb;
   FGLS_CUDA_TRY(digit_map(&ma, A));
   FGLS_CUDA_TRY(digit_map(&mb, B));
@@ -973,6 +981,7 @@ bool digit_gemm_pays(long long M, long long N, long long K) {
 
 namespace {
 bool reserve(DigitGemm* g, int q, size_t bytes) {
+  if (!digit_gemm_ready(g)) return false;
   if (g->op_bytes[q] >= bytes) return true;
   if (g->op[q]) cudaFree(g->op[q]);
   g->op[q] = nullptr;
@@ -1009,6 +1018,16 @@ bool digit_gemm_trim(DigitGemm* g) {
   return held;
 }
 
+bool digit_gemm_release(DigitGemm* g) {
+  bool held = digit_gemm_trim(g);
+  if (g && g->planes) {
+    cudaFree(g->planes);
+    g->planes = nullptr;
+    held = true;
+  }
+  return held;
+}
+
 cudaError_t digit_dgemm(DigitGemm* g, cudaStream_t s, bool tA, bool tB, int M, int N, int K, double alpha,
                         const double* A, long long lda, const double* B, long long ldb, double beta, double* C,
                         long long ldc, const DigitMulOpts& o) {
@@ -1041,6 +1060,7 @@ extern "C" int fglsgpu_selftest_dgemm(int transA, int transB, int M, int N, int 
   for (auto& e : ev) chk(cudaEventCreate(&e));
   if (digits) {
     chk(digit_gemm_create(&g));
+    if (g && !digit_gemm_ready(g)) chk(cudaErrorMemoryAllocation);
     chk(cudaMalloc(&mem[0], digit_mat_bytes(M, K)));
     chk(cudaMalloc(&mem[1], digit_mat_bytes(N, K)));
   }

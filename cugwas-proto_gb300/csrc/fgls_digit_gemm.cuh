@@ -35,6 +35,9 @@ cudaError_t digit_cut_products(cudaStream_t s, const DigitMat& m, const double* 
 // CTA, K-split partials, the operands of digit_dgemm, a wait error word.
 struct DigitGemm;
 cudaError_t digit_gemm_create(DigitGemm** out);  // cudaErrorNotSupported: no clusters of two
+// Takes the partial sums' memory (120 MB), which no product is run without; digit_dgemm
+// and the operands below do it themselves.  False when the device has not the memory.
+bool digit_gemm_ready(DigitGemm* g);
 void digit_gemm_destroy(DigitGemm* g);
 int* digit_gemm_error_word(DigitGemm* g);
 // limit of one wait of the products launched from now on (0: the default, 2 s)
@@ -59,9 +62,10 @@ cudaError_t digit_dgemm(DigitGemm* g, cudaStream_t s, bool tA, bool tB, int M, i
 DigitMat digit_gemm_operand(DigitGemm* g, int q, int rows, int K);
 // room for operands of up to `rows` x K each (so that digit_dgemm allocates
 // nothing); false when the device has not the memory.  digit_gemm_trim gives
-// the operands' room back.
+// the operands' room back, digit_gemm_release that of the partial sums too.
 bool digit_gemm_reserve(DigitGemm* g, int rows, int K);
 bool digit_gemm_trim(DigitGemm* g);
+bool digit_gemm_release(DigitGemm* g);
 // whether digit_dgemm takes the digits for this product
 bool digit_gemm_pays(long long M, long long N, long long K);
 

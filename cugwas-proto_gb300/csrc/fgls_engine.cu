@@ -306,7 +306,7 @@ bool give_back(fglsgpu_engine* e) {
   const bool inverse = e->dLinv && !split(e);
   const bool digits = e->zmem || e->wmem || e->blkmem || e->adjmem;
   cudaStreamSynchronize(e->comp);  // blocks in flight read them
-  if (!digit_gemm_trim(e->dg) && !digits && !inverse) return false;
+  if (!digit_gemm_release(e->dg) && !digits && !inverse) return false;
   drop_digits(e);
   if (e->adjmem) cudaFree(e->adjmem);
   e->adjmem = nullptr;
@@ -355,7 +355,7 @@ int chol_digits(fglsgpu_engine* e, long long cols, bool* use) {
   if (e->dg_off || !e->dLinv || !digit_gemm_pays(n, cols, n) || !digit_work(e)) return FGLSGPU_OK;
   const long long most = e->probing ? cols : std::max<long long>(cols, (long long)c.x_b * c.wXR);
   size_t none = 0;
-  if (!((e->zmem || grow(&e->zmem, &none, digit_mat_bytes(n, n))) &&
+  if (!(digit_gemm_ready(e->dg) && (e->zmem || grow(&e->zmem, &none, digit_mat_bytes(n, n))) &&
         grow(&e->blkmem, &e->blk_bytes, digit_mat_bytes((int)most, n)))) {
     drop_digits(e);
     e->dg_off = true;  // (e->dg stays: products of its are in flight, their error word is still to be read)
@@ -384,7 +384,7 @@ int eigen_digits(fglsgpu_engine* e, long long cols, bool* use) {
   if (e->dg_off || c.variant != FGLSGPU_VARIANT_EIGEN || !digit_gemm_pays(n, cols, n)) return FGLSGPU_OK;
   const long long most = (e->probing ? cols : std::max<long long>(cols, (long long)c.x_b * c.wXR)) * c.wXR;
   size_t none = 0;
-  bool ok = digit_work(e) != nullptr;
+  bool ok = digit_work(e) && digit_gemm_ready(e->dg);
   if (ok && !e->zmem) ok = grow(&e->zmem, &none, digit_mat_bytes(n, n));
   none = 0;
   const size_t wy = (digit_mat_bytes(nq, n) + 255) & ~(size_t)255;
@@ -661,11 +661,11 @@ int tune_slices(fglsgpu_engine* e) {
 }
 
 // The end of the split path's set-up: the slice choice, unless the caller made it,
-// then the FP64 products' operands, which no block of it uses, are given back.
+// then the FP64 products' operands and workspace, which no block of it uses, go.
 int finish_split(fglsgpu_engine* e) {
   const int rc = e->cfg.slices == 0 ? tune_slices(e) : FGLSGPU_OK;
   drop_digits(e);
-  digit_gemm_trim(e->dg);
+  digit_gemm_release(e->dg);
   return rc;
 }
 
@@ -839,6 +839,7 @@ int fglsgpu_set_problem(fglsgpu_engine* e, const double* Phi, const double* XL, 
       bool use;
       rc = eigen_digits(e, (long long)c.x_b * c.wXR, &use);
       if (rc) return rc;
+      if (e->dg_off) digit_gemm_release(e->dg);  // no block will use it
     } else {
       rc = split_operands(e);
       if (rc) return rc;
@@ -912,6 +913,8 @@ int fglsgpu_select_trait(fglsgpu_engine* e, int j) {
       e->trait_sel = -1;
       return rc;
     }
+  } else if (e->dg_off) {
+    digit_gemm_release(e->dg);  // no block will use it
   }
   e->trait_sel = j;
   return FGLSGPU_OK;

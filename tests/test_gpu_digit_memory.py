@@ -99,3 +99,21 @@ def test_split_set_up_gives_its_operands_back(variant):
             e.select_trait(0)
             held[slices] = before - free_bytes()
     assert held[9] <= held[0] + 16 * MB, held
+
+
+@pytest.mark.parametrize("variant,precision", [("eigen", "fp64"), ("chol", "fp64"), ("eigen", "split")])
+def test_no_workspace_where_no_block_uses_it(variant, precision):
+    """The digit products' workspace (120 MB) belongs to products that run on digits: not
+    to a small problem's engine, and not to a split engine once it is set up."""
+    from fgls_gb300 import Engine, datagen
+    n = 3000 if precision == "split" else 150
+    pb = datagen.make_problem(n, 64, 2, seed=13, hsig_uniform=True)
+    own = 3 * 8 * n * n + (180 * MB if precision == "split" else 0)  # matrices; the split plan
+    for _ in range(2):  # the first time the device also loads the kernels
+        before = free_bytes()
+        with Engine(n, 3, 1, 2, 64, variant=variant, precision=precision) as e:
+            e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+            e.select_trait(0)
+            e.run_block(pb.XR)
+            held = before - free_bytes()
+    assert held < own + 48 * MB
