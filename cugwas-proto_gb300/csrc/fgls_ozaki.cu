@@ -2018,6 +2018,13 @@ int pair_clusters() {
   return n;
 }
 
+// Most CTAs of a split GEMM of tiles_m x tiles_n tiles, in either form: each has a
+// part of the pass sums (512 KB; a plan holds what its largest block launches, not
+// 152 of them, so that many small engines fit one device).
+int gemm_ctas(int tiles_m, int tiles_n) {
+  return std::max(2 * std::min((tiles_m + 1) / 2 * tiles_n, pair_clusters()), persistent_grid(tiles_m * tiles_n));
+}
+
 }  // namespace oz
 
 using namespace oz;
@@ -2117,7 +2124,7 @@ cudaError_t ozaki_create(OzakiPlan** out, int n, int t, int wXL, int wXR, int x_
     chk(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev));
   }
   chk(cudaMalloc(&p->err, 3 * sizeof(int)));  // [wait error word, GEMM tile counter, finished CTAs]
-  chk(cudaMalloc(&p->gpart, sizeof(int4) * (size_t)PART * persistent_grid(1 << 20)));
+  chk(cudaMalloc(&p->gpart, sizeof(int4) * (size_t)PART * gemm_ctas(p->Mpad / BM, p->Ncap / BN)));
   if (!eigen) chk(cudaMalloc(&p->LinvT, sizeof(double) * (size_t)n * n));
   if (!eigen) chk(cudaMalloc(&p->sqsum, sizeof(float2) * (size_t)(p->Mpad / 32) * p->Ncap));
   if (r == cudaSuccess) chk(cudaMemset(p->A, 0, (size_t)p->S * p->Mpad * p->Kpad));
@@ -2477,7 +2484,10 @@ cudaError_t grouped_gemm_create(GroupedGemm** out, const GroupedGemmDesc* d, int
   *out = nullptr;
   const bool pair = want_pair && pair_clusters() > 0;
   int4* part = nullptr;
-  FGLS_CUDA_TRY(cudaMalloc(&part, sizeof(int4) * (size_t)PART * persistent_grid(1 << 20)));
+  long long rows = 0;  // row tiles of all problems, each rounded up to a pair
+  for (int i = 0; i < count; i++) rows += (d[i].Mpad / BM + 1) / 2 * 2;
+  const int ctas = gemm_ctas((int)std::min<long long>(rows, 1 << 10), (x_b + BN - 1) / BN);
+  FGLS_CUDA_TRY(cudaMalloc(&part, sizeof(int4) * (size_t)PART * ctas));
   struct Give {  // given back unless the plan takes it
     int4** p;
     ~Give() {

@@ -117,3 +117,25 @@ def test_no_workspace_where_no_block_uses_it(variant, precision):
             e.run_block(pb.XR)
             held = before - free_bytes()
     assert held < own + 48 * MB
+
+
+def test_split_plan_holds_the_pass_sums_of_its_own_tiles():
+    """512 KB a CTA that the block launches (n = 300, 64 SNPs: two pairs), not one per SM."""
+    from fgls_gb300 import Batch, Engine, datagen
+    from test_gpu_batch import run_batch
+    pb = datagen.make_problem(300, 64, 2, seed=14, hsig_uniform=True)
+    desc = [{"Phi": pb.Phi, "XL": pb.XL, "Y": pb.Y, "h": pb.h, "sigma": pb.sigma}]
+    for _ in range(2):  # the first time the device also loads the kernels
+        held = []
+        for variant in ("eigen", "chol"):
+            before = free_bytes()
+            with Engine(pb.n, 3, 1, 2, 64, variant=variant, precision="split", slices=9) as e:
+                e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+                e.select_trait(0)
+                e.run_block(pb.XR)
+                held.append(before - free_bytes())
+        before = free_bytes()
+        with Batch(desc, x_b=64, slices=9) as b:
+            held.append(before - free_bytes())
+            run_batch(b, [pb], 64)
+    assert max(held) < 48 * MB, held
