@@ -150,7 +150,7 @@ int bfail(fglsgpu_batch* b, int code, const char* fmt, ...) {
 template <class T>
 cudaError_t dalloc(T** p, size_t count) {
   *p = nullptr;
-  return cudaMalloc((void**)p, sizeof(T) * std::max<size_t>(count, 1));
+  return needed_malloc(p, sizeof(T) * std::max<size_t>(count, 1));
 }
 
 // genotype (0/1/2) of the probe block: a fixed integer hash of (cohort, SNP, individual)
@@ -377,7 +377,7 @@ int time_step(fglsgpu_batch* b, int x_b, double* rate) {
   double tests = 0.0;
   for (int c = 0; c < C && !rc; c++) {
     const Cohort& co = b->co[c];
-    if (cudaMalloc(&Xo[c], (size_t)x_b * co.n) != cudaSuccess ||
+    if (needed_malloc(&Xo[c], (size_t)x_b * co.n) != cudaSuccess ||
         dalloc(&B[c], (size_t)co.t * x_b * co.p) != cudaSuccess ||
         dalloc(&V[c], (size_t)co.t * x_b * co.p * co.p) != cudaSuccess) {
       rc = bfail(b, FGLSGPU_ENOMEM, "autotune buffers");

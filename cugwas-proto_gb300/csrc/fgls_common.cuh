@@ -63,6 +63,20 @@ __device__ __forceinline__ double chain_rcp(double d) {
 
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
+// The engines of this process on the current device that are between calls give back
+// the memory that only makes them faster (fgls_engine.cu); false if none holds any.
+bool engines_give_back();
+// Device memory that a call outside of an engine cannot do without.
+template <class T>
+cudaError_t needed_malloc(T** p, size_t bytes) {
+  cudaError_t r = cudaMalloc((void**)p, bytes);
+  if (r == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    if (engines_give_back()) r = cudaMalloc((void**)p, bytes);
+  }
+  return r;
+}
+
 // Kernel launchers (host side, defined in the .cu files).  All are
 // asynchronous on `s` and return cudaError_t of the launch.
 

@@ -51,6 +51,7 @@
 #include <thread>
 #include <vector>
 
+#include "fgls_common.cuh"
 #include "fgls_gb300.h"
 
 namespace {
@@ -258,9 +259,9 @@ int run_variant(int variant, int n, int p, int m, int t, int wXL, int wXR, int x
     cuda_check(cudaMallocHost((void**)&s.hX, (size_t)colb * x_b), "pinned XR slot");
     cuda_check(cudaMallocHost((void**)&s.hB, sizeof(double) * nt * x_b * p), "pinned B slot");
     cuda_check(cudaMallocHost((void**)&s.hV, sizeof(double) * nt * x_b * p * p), "pinned V slot");
-    cuda_check(cudaMalloc((void**)&s.dX, (size_t)colb * x_b), "XR slot");
-    cuda_check(cudaMalloc((void**)&s.dB, sizeof(double) * nt * x_b * p), "B slot");
-    cuda_check(cudaMalloc((void**)&s.dV, sizeof(double) * nt * x_b * p * p), "V slot");
+    cuda_check(fgls::needed_malloc(&s.dX, (size_t)colb * x_b), "XR slot");
+    cuda_check(fgls::needed_malloc(&s.dB, sizeof(double) * nt * x_b * p), "B slot");
+    cuda_check(fgls::needed_malloc(&s.dV, sizeof(double) * nt * x_b * p * p), "V slot");
     cuda_check(cudaEventCreateWithFlags(&s.evH, cudaEventDisableTiming), "event");
     cuda_check(cudaEventCreateWithFlags(&s.evC, cudaEventDisableTiming), "event");
     cuda_check(cudaEventCreateWithFlags(&s.evD, cudaEventDisableTiming), "event");

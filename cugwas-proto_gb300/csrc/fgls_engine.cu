@@ -17,7 +17,9 @@
 #include <string.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cmath>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -30,6 +32,7 @@ using namespace fgls;
 
 struct fglsgpu_engine {
   fglsgpu_config cfg{};
+  std::timed_mutex busy;  // held by a call on this engine
   int p = 0, topw = 0;
   cudaStream_t comp = nullptr, h2d = nullptr, d2h = nullptr;
   cudaEvent_t evH[2]{}, evC[2]{}, evD[2]{};
@@ -318,13 +321,44 @@ bool give_back(fglsgpu_engine* e) {
   return true;
 }
 
-// An allocation, tried again after give_back.
+// The process's engines, so that one short of memory can have what others hold to be
+// faster.  Never destroyed: an engine may outlive static objects.
+struct Registry {
+  std::mutex m;
+  std::vector<fglsgpu_engine*> all;
+};
+Registry& registry() {
+  static Registry* r = new Registry;
+  return *r;
+}
+
+// give_back of the other engines on `device`, each between two calls on it: a call in
+// progress is waited for, but not for long (the one in need of memory is then refused,
+// and two that wait for each other go on).  Without the wait a thread that runs block
+// after block is hardly ever met between calls: a failing allocation holds up its next.
+bool others_give_back(int device, const fglsgpu_engine* self) {
+  Registry& g = registry();
+  std::lock_guard<std::mutex> hold(g.m);
+  bool any = false;
+  for (fglsgpu_engine* e : g.all) {
+    if (e == self || e->cfg.device != device || !e->busy.try_lock_for(std::chrono::seconds(1))) continue;
+    any |= give_back(e);
+    e->busy.unlock();
+  }
+  return any;
+}
+
+// An allocation that a call cannot do without, tried again after give_back.
 template <class F>
 cudaError_t with_room(fglsgpu_engine* e, F alloc) {
   cudaError_t r = alloc();
   if (r == cudaErrorMemoryAllocation) {
     (void)cudaGetLastError();
     if (give_back(e)) r = alloc();
+  }
+  if (r == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    if (others_give_back(e->cfg.device, e)) r = alloc();
   }
   return r;
 }
@@ -684,6 +718,11 @@ int split_operands(fglsgpu_engine* e) {
 
 }  // namespace
 
+bool fgls::engines_give_back() {
+  int device = 0;
+  return cudaGetDevice(&device) == cudaSuccess && others_give_back(device, nullptr);
+}
+
 extern "C" {
 
 int fglsgpu_version(void) { return 10000; }
@@ -727,6 +766,9 @@ int fglsgpu_create(const fglsgpu_config* cfg, fglsgpu_engine** out) {
   auto chk = [&](cudaError_t x) {
     if (r == cudaSuccess) r = x;
   };
+  auto need = [&](auto** p, size_t count) {
+    if (r == cudaSuccess) r = dalloc_room(e, p, count);
+  };
   chk(cudaStreamCreateWithFlags(&e->comp, cudaStreamNonBlocking));
   chk(cudaStreamCreateWithFlags(&e->h2d, cudaStreamNonBlocking));
   chk(cudaStreamCreateWithFlags(&e->d2h, cudaStreamNonBlocking));
@@ -735,40 +777,40 @@ int fglsgpu_create(const fglsgpu_config* cfg, fglsgpu_engine** out) {
     chk(cudaEventCreateWithFlags(&e->evC[k], cudaEventDisableTiming));
     chk(cudaEventCreateWithFlags(&e->evD[k], cudaEventDisableTiming));
   }
-  chk(dalloc(&e->dPhi, n * n));
-  chk(dalloc(&e->dXL, n * wXL));
-  chk(dalloc(&e->dY, n * t));
-  chk(dalloc(&e->dh, t));
-  chk(dalloc(&e->dsig, t));
-  chk(dalloc(&e->dtop, t * e->topw));
-  chk(dalloc(&e->dst, 1));
+  need(&e->dPhi, n * n);
+  need(&e->dXL, n * wXL);
+  need(&e->dY, n * t);
+  need(&e->dh, t);
+  need(&e->dsig, t);
+  need(&e->dtop, t * e->topw);
+  need(&e->dst, 1);
   chk(cudaMallocHost((void**)&e->hst, sizeof(DevStatus)));
   chk(cudaMallocHost((void**)&e->hst_wait, 2 * sizeof(int)));
   for (int k = 0; k < 2; k++) {
-    chk(dalloc(&e->dX[k], n * xb * wXR));
-    chk(dalloc(&e->dB[k], (long long)nt * xb * p));
-    chk(dalloc(&e->dV[k], (long long)nt * xb * p * p));
+    need(&e->dX[k], n * xb * wXR);
+    need(&e->dB[k], (long long)nt * xb * p);
+    need(&e->dV[k], (long long)nt * xb * p * p);
   }
-  chk(dalloc(&e->dGYL, xb * wXR * nt * (1 + wXL)));
-  chk(dalloc(&e->dGR, xb * wXR * wXR * nt));
+  need(&e->dGYL, xb * wXR * nt * (1 + wXL));
+  need(&e->dGR, xb * wXR * wXR * nt);
   if (c.variant == FGLSGPU_VARIANT_CHOL) {
-    chk(dalloc(&e->dL, n * n));
-    chk(dalloc(&e->dWY, n * (1 + wXL)));
-    chk(dalloc(&e->dWork, n * xb * wXR));
-    chk(dalloc(&e->ddiag, 64 * 64));
-    chk(dalloc(&e->dWraw, n * (1 + wXL)));
+    need(&e->dL, n * n);
+    need(&e->dWY, n * (1 + wXL));
+    need(&e->dWork, n * xb * wXR);
+    need(&e->ddiag, 64 * 64);
+    need(&e->dWraw, n * (1 + wXL));
   } else {
-    chk(dalloc(&e->dL, n * n));  // eigensolver scratch
-    chk(dalloc(&e->dZ, n * n));
-    chk(dalloc(&e->dW, n));
-    chk(dalloc(&e->dZtXL, n * wXL));
-    chk(dalloc(&e->dZtY, n * t));
-    chk(dalloc(&e->ddinv, n * t));
-    chk(dalloc(&e->dAYL, n * t * (1 + wXL)));
-    chk(cudaMalloc(&e->deigwork, eig_workspace_bytes(c.n)));
+    need(&e->dL, n * n);  // eigensolver scratch
+    need(&e->dZ, n * n);
+    need(&e->dW, n);
+    need(&e->dZtXL, n * wXL);
+    need(&e->dZtY, n * t);
+    need(&e->ddinv, n * t);
+    need(&e->dAYL, n * t * (1 + wXL));
+    if (r == cudaSuccess) r = with_room(e, [&] { return cudaMalloc(&e->deigwork, eig_workspace_bytes(c.n)); });
     if (c.precision == FGLSGPU_PREC_FP64) {
-      chk(dalloc(&e->dWork, n * xb * wXR));
-      chk(dalloc(&e->dQ, n * xb * wXR * wXR));
+      need(&e->dWork, n * xb * wXR);
+      need(&e->dQ, n * xb * wXR * wXR);
     }
   }
   if (r == cudaSuccess) r = cudaMemsetAsync(e->dst, 0, sizeof(DevStatus), e->comp);
@@ -780,12 +822,21 @@ int fglsgpu_create(const fglsgpu_config* cfg, fglsgpu_engine** out) {
     delete e;
     return code;
   }
+  {
+    std::lock_guard<std::mutex> hold(registry().m);
+    registry().all.push_back(e);
+  }
   *out = e;
   return FGLSGPU_OK;
 }
 
 int fglsgpu_destroy(fglsgpu_engine* e) {
   if (!e) return FGLSGPU_OK;
+  {
+    std::lock_guard<std::mutex> hold(registry().m);
+    auto& all = registry().all;
+    all.erase(std::find(all.begin(), all.end(), e));
+  }
   cudaSetDevice(e->cfg.device);
   if (e->comp) cudaStreamSynchronize(e->comp);
   free_all(e);
@@ -796,6 +847,7 @@ int fglsgpu_destroy(fglsgpu_engine* e) {
 int fglsgpu_set_problem(fglsgpu_engine* e, const double* Phi, const double* XL, const double* Y, const double* h,
                         const double* sigma) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!Phi || !XL || !Y || !h || !sigma) return fail(e, FGLSGPU_EINVAL, "null input pointer");
   const fglsgpu_config& c = e->cfg;
   const long long n = c.n, t = c.t;
@@ -852,6 +904,7 @@ int fglsgpu_set_problem(fglsgpu_engine* e, const double* Phi, const double* XL, 
 
 int fglsgpu_select_trait(fglsgpu_engine* e, int j) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->problem_set) return fail(e, FGLSGPU_ESTATE, "set_problem must precede select_trait");
   const fglsgpu_config& c = e->cfg;
   if (c.variant == FGLSGPU_VARIANT_EIGEN) return FGLSGPU_OK;
@@ -923,6 +976,7 @@ int fglsgpu_select_trait(fglsgpu_engine* e, int j) {
 int fglsgpu_run_block_device(fglsgpu_engine* e, const double* dXR, int x_inc, double* dB, double* dV,
                              long long bstr, long long vstr) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->problem_set) return fail(e, FGLSGPU_ESTATE, "set_problem must precede run_block");
   if (x_inc <= 0 || x_inc > e->cfg.x_b) return fail(e, FGLSGPU_EINVAL, "x_inc=%d outside [1, %d]", x_inc, e->cfg.x_b);
   if (!dXR || !dB || !dV) return fail(e, FGLSGPU_EINVAL, "null block pointer");
@@ -934,6 +988,7 @@ int fglsgpu_run_block_device(fglsgpu_engine* e, const double* dXR, int x_inc, do
 int fglsgpu_run_block_device_u8(fglsgpu_engine* e, const unsigned char* dXR, int x_inc, double* dB, double* dV,
                                 long long bstr, long long vstr) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->problem_set) return fail(e, FGLSGPU_ESTATE, "set_problem must precede run_block");
   if (x_inc <= 0 || x_inc > e->cfg.x_b) return fail(e, FGLSGPU_EINVAL, "x_inc=%d outside [1, %d]", x_inc, e->cfg.x_b);
   ENG_TRY(e, cudaSetDevice(e->cfg.device), "cudaSetDevice");
@@ -944,6 +999,7 @@ int fglsgpu_run_block_device_u8(fglsgpu_engine* e, const unsigned char* dXR, int
 int fglsgpu_run_block_device_packed(fglsgpu_engine* e, const unsigned char* dXR2, int x_inc, double* dB, double* dV,
                                     long long bstr, long long vstr) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->problem_set) return fail(e, FGLSGPU_ESTATE, "set_problem must precede run_block");
   if (x_inc <= 0 || x_inc > e->cfg.x_b) return fail(e, FGLSGPU_EINVAL, "x_inc=%d outside [1, %d]", x_inc, e->cfg.x_b);
   if (!dXR2 || !dB || !dV) return fail(e, FGLSGPU_EINVAL, "null block pointer");
@@ -953,6 +1009,7 @@ int fglsgpu_run_block_device_packed(fglsgpu_engine* e, const unsigned char* dXR2
 
 int fglsgpu_sync(fglsgpu_engine* e) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   ENG_TRY(e, cudaSetDevice(e->cfg.device), "cudaSetDevice");
   const int rc = check_status(e, "block");
   const int rr = reset_status(e);
@@ -962,6 +1019,7 @@ int fglsgpu_sync(fglsgpu_engine* e) {
 int fglsgpu_run_block(fglsgpu_engine* e, const double* XR, int x_inc, double* B, double* V, long long bstr,
                       long long vstr) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->problem_set) return fail(e, FGLSGPU_ESTATE, "set_problem must precede run_block");
   if (x_inc <= 0 || x_inc > e->cfg.x_b) return fail(e, FGLSGPU_EINVAL, "x_inc=%d outside [1, %d]", x_inc, e->cfg.x_b);
   if (!XR || !B || !V) return fail(e, FGLSGPU_EINVAL, "null block pointer");
@@ -1069,6 +1127,7 @@ extern "C" {
 
 int fglsgpu_run_snps(fglsgpu_engine* e, const double* XR, long long m, double* B, double* V) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->problem_set) return fail(e, FGLSGPU_ESTATE, "set_problem must precede run_snps");
   if (m <= 0 || !XR || !B || !V) return fail(e, FGLSGPU_EINVAL, "invalid run_snps arguments");
   return run_snps_impl(e, XR, GENO_F64, m, B, V, nullptr, nullptr);
@@ -1076,6 +1135,7 @@ int fglsgpu_run_snps(fglsgpu_engine* e, const double* XR, long long m, double* B
 
 int fglsgpu_run_snps_u8(fglsgpu_engine* e, const unsigned char* XR, long long m, double* B, double* V) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->problem_set) return fail(e, FGLSGPU_ESTATE, "set_problem must precede run_snps");
   if (m <= 0 || !XR || !B || !V) return fail(e, FGLSGPU_EINVAL, "invalid run_snps_u8 arguments");
   return run_snps_impl(e, XR, GENO_U8, m, B, V, nullptr, nullptr);
@@ -1083,6 +1143,7 @@ int fglsgpu_run_snps_u8(fglsgpu_engine* e, const unsigned char* XR, long long m,
 
 int fglsgpu_run_snps_packed(fglsgpu_engine* e, const unsigned char* XR2, long long m, double* B, double* V) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->problem_set) return fail(e, FGLSGPU_ESTATE, "set_problem must precede run_snps");
   if (m <= 0 || !XR2 || !B || !V) return fail(e, FGLSGPU_EINVAL, "invalid run_snps_packed arguments");
   return run_snps_impl(e, XR2, GENO_PACKED, m, B, V, nullptr, nullptr);
@@ -1090,6 +1151,7 @@ int fglsgpu_run_snps_packed(fglsgpu_engine* e, const unsigned char* XR2, long lo
 
 int fglsgpu_run_snps_compact(fglsgpu_engine* e, const double* XR, long long m, double* B, double* SE, double* P) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->problem_set) return fail(e, FGLSGPU_ESTATE, "set_problem must precede run_snps");
   if (m <= 0 || !XR || !B || !SE || !P) return fail(e, FGLSGPU_EINVAL, "invalid run_snps_compact arguments");
   ENG_TRY(e, cudaSetDevice(e->cfg.device), "cudaSetDevice");
@@ -1103,6 +1165,7 @@ int fglsgpu_run_snps_compact(fglsgpu_engine* e, const double* XR, long long m, d
 
 int fglsgpu_set_precision(fglsgpu_engine* e, int precision) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (precision != FGLSGPU_PREC_FP64 && precision != FGLSGPU_PREC_SPLIT)
     return fail(e, FGLSGPU_EINVAL, "unknown precision %d", precision);
   fglsgpu_config& c = e->cfg;
@@ -1134,6 +1197,7 @@ int fglsgpu_quad_digits(fglsgpu_engine* e, int* digits) {
 
 int fglsgpu_split_params(fglsgpu_engine* e, int* slices, double* probe_err) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (slices) *slices = e->oz ? ozaki_slices(e->oz, nullptr) : 0;
   if (probe_err) *probe_err = e->tune_err;
   return FGLSGPU_OK;
@@ -1141,6 +1205,7 @@ int fglsgpu_split_params(fglsgpu_engine* e, int* slices, double* probe_err) {
 
 int fglsgpu_set_wait_limit(fglsgpu_engine* e, long long ns) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (ns < 0) return fail(e, FGLSGPU_EINVAL, "wait limit %lld < 0", ns);
   e->wait_ns = (unsigned long long)ns;
   if (e->oz) ozaki_set_wait_limit(e->oz, e->wait_ns);
@@ -1151,6 +1216,7 @@ int fglsgpu_set_wait_limit(fglsgpu_engine* e, long long ns) {
 int fglsgpu_pvalues_device(fglsgpu_engine* e, const double* dB, const double* dV, int x_inc, long long b_trait_stride,
                            long long v_trait_stride, double* dP, long long p_trait_stride) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!dB || !dV || !dP || x_inc <= 0) return fail(e, FGLSGPU_EINVAL, "invalid p-value arguments");
   ENG_TRY(e, cudaSetDevice(e->cfg.device), "cudaSetDevice");
   const int nt = e->cfg.variant == FGLSGPU_VARIANT_EIGEN ? e->cfg.t : 1;
@@ -1163,6 +1229,7 @@ int fglsgpu_pvalues_device(fglsgpu_engine* e, const double* dB, const double* dV
 // ---------------------------------------------------------------- adjoint
 int fglsgpu_adjoint_reset(fglsgpu_engine* e) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   const fglsgpu_config& c = e->cfg;
   if (c.variant != FGLSGPU_VARIANT_EIGEN || c.wXR != 1)
     return fail(e, FGLSGPU_EINVAL, "the adjoint is defined for the eigen variant with wXR = 1");
@@ -1223,6 +1290,7 @@ int fglsgpu_adjoint_reset(fglsgpu_engine* e) {
 
 int fglsgpu_adjoint_block_device(fglsgpu_engine* e, const double* dXR, int x, const double* dBbar, long long bstr) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->adj_ready) return fail(e, FGLSGPU_ESTATE, "fglsgpu_adjoint_reset must precede adjoint blocks");
   const fglsgpu_config& c = e->cfg;
   if (x <= 0 || x > c.x_b || !dXR || !dBbar) return fail(e, FGLSGPU_EINVAL, "invalid adjoint block");
@@ -1264,6 +1332,7 @@ int fglsgpu_adjoint_block_device(fglsgpu_engine* e, const double* dXR, int x, co
 
 int fglsgpu_adjoint_read(fglsgpu_engine* e, double* dh, double* dsigma, double* dY) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->adj_ready) return fail(e, FGLSGPU_ESTATE, "no adjoint accumulated");
   const fglsgpu_config& c = e->cfg;
   ENG_TRY(e, cudaSetDevice(c.device), "cudaSetDevice");
@@ -1293,6 +1362,7 @@ int fglsgpu_adjoint_read(fglsgpu_engine* e, double* dh, double* dsigma, double* 
 
 int fglsgpu_reml(fglsgpu_engine* e, double* loglik, double* dloglik_dh) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->adj_ready) return fail(e, FGLSGPU_ESTATE, "fglsgpu_adjoint_reset computes the REML terms first");
   const int t = e->cfg.t;
   ENG_TRY(e, cudaSetDevice(e->cfg.device), "cudaSetDevice");
@@ -1308,6 +1378,7 @@ int fglsgpu_reml(fglsgpu_engine* e, double* loglik, double* dloglik_dh) {
 int fglsgpu_reml_fit(fglsgpu_engine* e, double h_lo, double h_hi, int grid, double* h, double* sigma,
                      double* loglik, double* dloglik_dh) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->problem_set) return fail(e, FGLSGPU_ESTATE, "set_problem must precede reml_fit");
   const fglsgpu_config& c = e->cfg;
   if (c.variant != FGLSGPU_VARIANT_EIGEN) return fail(e, FGLSGPU_EINVAL, "reml_fit needs the eigen variant");
@@ -1323,9 +1394,9 @@ int fglsgpu_reml_fit(fglsgpu_engine* e, double h_lo, double h_hi, int grid, doub
   // the outputs and the grid's workspace, kept for the next fit
   const size_t outb = (sizeof(double) * 4 * (size_t)t + 255) & ~(size_t)255;
   const size_t remlb = outb + reml_workspace_bytes(c.n, t, grid);
-  if (!grow(&e->remlmem, &e->reml_bytes, remlb) &&
-      !(give_back(e) && grow(&e->remlmem, &e->reml_bytes, remlb)))
-    return fail(e, FGLSGPU_ENOMEM, "no memory for the REML grid");
+  ENG_TRY(e, with_room(e, [&] {
+            return grow(&e->remlmem, &e->reml_bytes, remlb) ? cudaSuccess : cudaErrorMemoryAllocation;
+          }), "REML grid");
   double* dout = (double*)e->remlmem;
   std::vector<double> r(4 * (size_t)t);
   cudaError_t ce = reml_fit(e->comp, c.n, t, c.wXL, e->dW, e->dZtXL, e->dZtY, h_lo, h_hi, grid,
@@ -1351,6 +1422,7 @@ int fglsgpu_reml_fit(fglsgpu_engine* e, double h_lo, double h_hi, int grid, doub
 
 int fglsgpu_set_hsigma(fglsgpu_engine* e, const double* h, const double* sigma) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (!e->problem_set) return fail(e, FGLSGPU_ESTATE, "set_problem must precede set_hsigma");
   if (!h || !sigma) return fail(e, FGLSGPU_EINVAL, "null input pointer");
   const fglsgpu_config& c = e->cfg;
@@ -1390,6 +1462,7 @@ int fglsgpu_set_hsigma(fglsgpu_engine* e, const double* h, const double* sigma) 
 
 int fglsgpu_profile(fglsgpu_engine* e, int enable) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   ENG_TRY(e, cudaSetDevice(e->cfg.device), "cudaSetDevice");
   ENG_TRY(e, cudaStreamSynchronize(e->comp), "profile");
   for (auto& ev : e->pev_live) e->pev_pool.push_back(ev);
@@ -1435,6 +1508,7 @@ int fglsgpu_get_res_sigma(fglsgpu_engine* e, double* out) {
 
 int fglsgpu_get_eigen(fglsgpu_engine* e, double* W, double* Z) {
   if (!e) return fail(nullptr, FGLSGPU_EINVAL, "null engine");
+  std::lock_guard<std::timed_mutex> call(e->busy);
   if (e->cfg.variant != FGLSGPU_VARIANT_EIGEN || !e->problem_set) return fail(e, FGLSGPU_ESTATE, "no eigendecomposition");
   ENG_TRY(e, cudaSetDevice(e->cfg.device), "cudaSetDevice");
   const long long n = e->cfg.n;

@@ -2487,7 +2487,7 @@ cudaError_t grouped_gemm_create(GroupedGemm** out, const GroupedGemmDesc* d, int
   long long rows = 0;  // row tiles of all problems, each rounded up to a pair
   for (int i = 0; i < count; i++) rows += (d[i].Mpad / BM + 1) / 2 * 2;
   const int ctas = gemm_ctas((int)std::min<long long>(rows, 1 << 10), (x_b + BN - 1) / BN);
-  FGLS_CUDA_TRY(cudaMalloc(&part, sizeof(int4) * (size_t)PART * ctas));
+  FGLS_CUDA_TRY(needed_malloc(&part, sizeof(int4) * (size_t)PART * ctas));
   struct Give {  // given back unless the plan takes it
     int4** p;
     ~Give() {
@@ -2550,10 +2550,10 @@ cudaError_t grouped_gemm_create(GroupedGemm** out, const GroupedGemmDesc* d, int
   auto chk = [&](cudaError_t e) {
     if (r == cudaSuccess) r = e;
   };
-  chk(cudaMalloc(&gg->tiles, sizeof(GroupedTile) * tiles.size()));
-  chk(cudaMalloc(&gg->probs, sizeof(GroupedProblem) * probs.size()));
-  chk(cudaMalloc(&gg->maps, sizeof(CUtensorMap) * maps.size()));  // 256-byte aligned: >= the 64 a map needs
-  chk(cudaMalloc(&gg->counter, 2 * sizeof(int)));
+  chk(needed_malloc(&gg->tiles, sizeof(GroupedTile) * tiles.size()));
+  chk(needed_malloc(&gg->probs, sizeof(GroupedProblem) * probs.size()));
+  chk(needed_malloc(&gg->maps, sizeof(CUtensorMap) * maps.size()));  // 256-byte aligned: >= the 64 a map needs
+  chk(needed_malloc(&gg->counter, 2 * sizeof(int)));
   if (r == cudaSuccess) chk(cudaMemset(gg->counter, 0, 2 * sizeof(int)));
   if (r == cudaSuccess) chk(cudaDeviceSynchronize());  // the memset is on the legacy default stream
   if (r == cudaSuccess)

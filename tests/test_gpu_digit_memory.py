@@ -139,3 +139,88 @@ def test_split_plan_holds_the_pass_sums_of_its_own_tiles():
             held.append(before - free_bytes())
             run_batch(b, [pb], 64)
     assert max(held) < 48 * MB, held
+
+
+@pytest.mark.parametrize("second", ["eigen", "chol", "batch"])
+def test_another_engine_fits_in_the_digits_place(second):
+    """The digits of one engine's blocks (590 MB and 108 MB of Z) give way to a second
+    engine or batch on the device that fits without them."""
+    from fgls_gb300 import Batch, Engine, datagen
+    from test_gpu_batch import run_batch
+    n, x_b = 3000, 16384
+    pb = datagen.make_problem(n, 64, 1, seed=15, hsig_uniform=True)
+    desc = [{"Phi": pb.Phi, "XL": pb.XL, "Y": pb.Y, "h": pb.h, "sigma": pb.sigma}]
+
+    class Second:
+        def __enter__(self):
+            if second == "batch":
+                self.b = Batch(desc, x_b=8192, slices=9)
+            else:
+                self.b = Engine(n, 3, 1, 1, 8192, variant=second)
+                self.b.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+                self.b.select_trait(0)
+            return self
+
+        def run(self):
+            return run_batch(self.b, [pb], 64)[0] if second == "batch" else self.b.run_block(pb.XR)
+
+        def __exit__(self, *exc):
+            self.b.close()
+
+    # what the second holds or needs while it is set up, no more: its own digits left out
+    # (megabytes of matrices, blocks, divide and conquer; of operands, output and scratch)
+    need = {"eigen": 3 * 72 + 4 * 197 + 288 + 5, "chol": 2 * 72 + 3 * 197,
+            "batch": 25 + 85 + 207 + 4 * 72 + 12}[second] * MB
+    with Second() as s:
+        ref2 = s.run()
+    with Engine(n, 3, 1, 1, x_b, variant="eigen") as e:
+        e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+        ref = e.run_block(pb.XR)
+        with Fill(need - 300 * MB):
+            with Second() as s:
+                same(*e.run_block(pb.XR), *ref)
+                tol = 1e-10 if second == "batch" else 1e-12
+                out = s.run()
+        i = np.arange(pb.p)
+        se = np.abs(ref2[1][..., i, i])
+        assert np.max(np.abs(out[0] - ref2[0]) / (np.abs(ref2[0]) + se)) <= tol
+
+
+def test_engines_on_two_threads_while_memory_is_short():
+    """One thread runs blocks while another creates and sets up engines that need the
+    first one's digits: every block is right, whatever the timing."""
+    import threading
+    from fgls_gb300 import Engine, FGLSError, datagen
+    n, x_b = 3000, 16384
+    pb = datagen.make_problem(n, 64, 1, seed=16, hsig_uniform=True)
+    with Engine(n, 3, 1, 1, x_b, variant="eigen") as e:
+        e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+        ref = e.run_block(pb.XR)
+        stop, bad = threading.Event(), []
+
+        def blocks():
+            try:
+                while not stop.is_set():
+                    same(*e.run_block(pb.XR), *ref)
+            except BaseException as x:  # noqa: BLE001
+                bad.append(x)
+        t = threading.Thread(target=blocks)
+        with Fill(1200 * MB):
+            t.start()
+            made = 0
+            try:
+                for _ in range(200):
+                    if made == 5:
+                        break
+                    try:
+                        with Engine(n, 3, 1, 1, 8192, variant="eigen") as o:
+                            o.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+                            same(*o.run_block(pb.XR), *ref)
+                            made += 1
+                    except FGLSError as x:  # refused while the other engine is in a call
+                        assert "memory" in str(x), x
+            finally:
+                stop.set()
+                t.join()
+    assert not bad, bad
+    assert made > 0
