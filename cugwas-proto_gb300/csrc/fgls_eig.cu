@@ -106,7 +106,9 @@ __device__ __forceinline__ void reflector(double alpha, double xnorm2, double& b
 // Sums over CTAs are taken from arrays of parts in a fixed order.
 constexpr int TB = 64;
 // Both kernels may be launched before the one ahead of them ends (programmatic
-// dependent launch): a column's two launches are on the chain of 2 n of them.
+// dependent launch): a column's two launches are on the chain of 2 n of them.  What
+// that one writes changes while they run, so none of their pointers is declared
+// constant or unaliased: the compiler could then read ahead of the wait.
 __device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -118,12 +120,9 @@ constexpr int TR = 32;  // rows per CTA of tridiag_col, one per lane; the panel'
 // wanted, x_r = A[r, k] - sum_q V[r, q] W[k, q] + W[r, q] V[k, q]; x_k is d[k],
 // and the parts of |x[k+2:]|^2 go to npart.
 __global__ void __launch_bounds__(256) tridiag_col_kernel(int n, int k, int i, bool pend, bool live,
-                                                          const double* __restrict__ A, long long lda,
-                                                          double* __restrict__ P, const double* __restrict__ y,
-                                                          const double* __restrict__ t, const double* __restrict__ yvpart,
-                                                          int nyv, const double* __restrict__ tau,
-                                                          double* __restrict__ d, double* __restrict__ x,
-                                                          double* __restrict__ npart) {
+                                                          double* A, long long lda, double* P, double* y, double* t,
+                                                          double* yvpart, int nyv, double* tau, double* d, double* x,
+                                                          double* npart) {
   __shared__ double st1[TB], st2[TB], vk[TB], wk[TB], part[2][8][TR], yvs[8], wsum;
   const int q1 = pend ? i - 1 : 0;  // panel columns that are complete
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
@@ -209,11 +208,8 @@ __global__ void __launch_bounds__(256) tridiag_col_kernel(int n, int k, int i, b
 // by latency.
 constexpr int MV_THREADS = 288;
 __global__ void __launch_bounds__(MV_THREADS) tridiag_mv_kernel(int n, int k, int i, double* A, long long lda, double* P,
-                                                                const double* __restrict__ x,
-                                                                const double* __restrict__ npart, int nnp,
-                                                                double* __restrict__ tau_out, double* __restrict__ e_out,
-                                                                double* __restrict__ y, double* __restrict__ t,
-                                                                double* __restrict__ yvpart) {
+                                                                double* x, double* npart, int nnp, double* tau_out,
+                                                                double* e_out, double* y, double* t, double* yvpart) {
   __shared__ double sscal, yvs[8];
   const int m = n - k - 1, r0 = k + 1;
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
@@ -451,18 +447,16 @@ cudaError_t dsyev_device(cudaStream_t s, DigitGemm* dg, int n, const double* Phi
     for (int i = 0; i < nb; i++) {
       const int k = k0 + i, m = n - k - 1;
       const int nr = ceil_div(n - k, TR);
-      FGLS_CUDA_TRY(launch_chained(tridiag_col_kernel, nr, 256, s, n, k, i, i > 0, true, (const double*)A, (long long)n,
-                                   P, (const double*)yb, (const double*)tb, (const double*)yvpart, nyv,
-                                   (const double*)tau, d, xb, npart));
+      FGLS_CUDA_TRY(launch_chained(tridiag_col_kernel, nr, 256, s, n, k, i, i > 0, true, A, (long long)n, P, yb, tb,
+                                   yvpart, nyv, tau, d, xb, npart));
       nyv = std::min(ceil_div(m + 2 * i, 8), EIG_CTAS);
-      FGLS_CUDA_TRY(launch_chained(tridiag_mv_kernel, nyv, MV_THREADS, s, n, k, i, A, (long long)n, P,
-                                   (const double*)xb, (const double*)npart, nr, tau, e, yb, tb, yvpart));
+      FGLS_CUDA_TRY(launch_chained(tridiag_mv_kernel, nyv, MV_THREADS, s, n, k, i, A, (long long)n, P, xb, npart, nr,
+                                   tau, e, yb, tb, yvpart));
       nl += 2;
     }
     const int kn = k0 + nb, m = n - kn;  // the trailing matrix
-    FGLS_CUDA_TRY(launch_chained(tridiag_col_kernel, ceil_div(m, TR), 256, s, n, kn, nb, true, false, (const double*)A,
-                                 (long long)n, P, (const double*)yb, (const double*)tb, (const double*)yvpart, nyv,
-                                 (const double*)tau, d, xb, npart));
+    FGLS_CUDA_TRY(launch_chained(tridiag_col_kernel, ceil_div(m, TR), 256, s, n, kn, nb, true, false, A, (long long)n,
+                                 P, yb, tb, yvpart, nyv, tau, d, xb, npart));
     nl++;
     FGLS_CUDA_TRY(cudaGetLastError());
     // A -= [V W] [W V]^T; a short last panel leaves columns of P beyond nb unset
