@@ -13,9 +13,11 @@
 //
 // Products.  A product of digits s and t has weight 32^-(s+t); level L is the
 // sum of all pairs with s + t = L.  Levels 2 .. 13 are kept (78 of the 144
-// pairs); what is dropped is below 2^-65 * 11 * 2^8 of the product of the row
-// scales per element, and of random sign, like the rounding of the digits:
-// less than the rounding of an FP64 accumulation.  Measured 2-norm errors over
+// pairs); what is dropped is below 11 * 2^8 * 2^-70 = 2^-58.5 of the product of
+// the row scales per element, and of random sign, like the rounding of the digits:
+// for rows of one magnitude less than the rounding of an FP64 accumulation (what
+// uses the products and holds mixed ones: the engine's diag_range_kernel).  Measured
+// 2-norm errors over
 // 150 entries against exactly rounded sums, normal data, digits / FP64 kernel:
 // K = 128 5e-15 / 5e-14, K = 1000 3e-14 / 4e-13, K = 10000 1.2e-13 / 4.1e-12
 // (hard calls as one operand 1.8e-15).  A level's sum over K is an integer;

@@ -1,7 +1,12 @@
 // FP64 matrix products on the FP8 tensor cores (fgls_digit_gemm.cu): both
 // operands are cut into twelve signed base-32 digits per row (60 bits under a
-// power-of-two scale per row) and the digit products are summed exactly, so
-// the result carries at least the accuracy of an FP64 DGEMM.
+// power-of-two scale per row) and the digit products are summed exactly.  The
+// error is normwise: below K 2^-58 2^exA 2^exB of the row scales (each between two
+// and four times the row's largest element) and one rounding, where an FP64 DGEMM's
+// is relative to sum |a||b|.  For rows whose elements are of one size that is the
+// smaller of the two; an element 2^-k of its row's largest keeps 60 - k bits, and
+// none from k = 60 on, so rows of mixed magnitude against rows mixed the other way
+// belong on the FP64 kernels (row (2^70, 1) by column (0, 1): 0 instead of 1).
 #pragma once
 
 #include <cuda_runtime.h>

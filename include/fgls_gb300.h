@@ -72,7 +72,10 @@ typedef struct fglsgpu_engine fglsgpu_engine;
 #define FGLSGPU_VARIANT_EIGEN 1 /* eigenbasis of Phi, all traits per block (fgls_eigen) */
 
 #define FGLSGPU_PREC_FP64 0     /* FP64 throughout; large products as exact
-                                   sums of digit products (60-bit operands)  */
+                                   sums of digit products (operands of 60
+                                   bits under each row's largest element;
+                                   FP64 kernels where individuals' variances
+                                   spread over more than 2^16)               */
 #define FGLSGPU_PREC_SPLIT 1    /* bulk GEMMs as 5-bit digit slices (FP8 E4M3) on
                                    tcgen05 tensor cores, exact FP32 accumulation,
                                    integer / FP64 recombination               */

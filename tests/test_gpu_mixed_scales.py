@@ -59,3 +59,23 @@ def test_chol_with_variances_of_many_sizes(decades):
     i = np.arange(w + 1)
     err = np.abs((B[0, :k].astype(Q) - ref).astype(float))
     assert np.max(err / (np.abs(ref.astype(float)) + np.abs(V[0, :k, i, i]).T)) <= 1e-12
+
+
+def test_digit_products_of_mixed_rows():
+    """The documented bound of one digit product, K 2^-58 of the row scales, holds for rows
+    of mixed magnitude, and is all that holds there: an element 2^-70 of its row's largest
+    is lost, which an FP64 product (relative to sum |a||b|) keeps."""
+    from test_gpu_digit_gemm import product, scale
+    rng = np.random.default_rng(18)
+    M, N, K = 130, 40, 256
+    A = rng.standard_normal((M, K)) * 2.0 ** rng.integers(-40, 1, (M, K))
+    B = rng.standard_normal((K, N)) * 2.0 ** rng.integers(0, 41, (K, N))
+    A[0], B[:, 0] = 0.0, 0.0
+    A[0, :2] = 2.0 ** 70, 1.0
+    B[1, 0] = 1.0
+    ref = np.array([[float(np.sum(A[i].astype(np.longdouble) * B[:, j])) for j in range(N)] for i in range(M)])
+    mag = np.abs(A) @ np.abs(B)
+    for digits, bound in ((1, K * 2.0 ** -58 * np.outer(scale(A, 1), scale(B, 0))), (0, K * 2.0 ** -53 * mag)):
+        out = product(A, B, np.zeros((M, N)), 1, 0, 1.0, 0.0, digits)
+        assert np.all(np.abs(out - ref) <= bound + 2.0 ** -52 * mag)
+        assert out[0, 0] == (0.0 if digits else 1.0)
