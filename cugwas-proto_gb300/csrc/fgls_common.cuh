@@ -32,7 +32,8 @@ __device__ __forceinline__ void set_status(DevStatus* st, int code, int info, lo
 // each here, and the library function is a chain of two dozen.  Seed from the FP32
 // reciprocal square root of the mantissa (moved in and out by integer
 // instructions), then one third-order step y (1 + e/2 + 3 e^2 / 8), e = 1 - d y^2
-// (the binomial series of (1 - e)^(-1/2)): |e| < 2^-21 leaves 2^-63.
+// (the binomial series of (1 - e)^(-1/2)): the seed's two ulps and the mantissa cut
+// to 23 bits make |e| < 2^-21 + 2^-23, which leaves 5/16 |e|^3 < 2^-63.7.
 __device__ __forceinline__ double chain_rsqrt(double d) {
   const long long b = __double_as_longlong(d);
   const int ex = (int)(b >> 52);
