@@ -32,9 +32,10 @@
 //               while the epilogue drains the previous one.
 //   the others  epilogue: tcgen05.ld the pass's accumulator, convert it
 //               exactly to the int32 q = 32 v = P_2p * 32 + P_2p+1,
-//               keep each pass's q in the CTA's own planes, and on the last
-//               pass combine them in int64 (V = V * 2^10 + q) and write
-//               V * 2^(e_r - 9 - 10 (passes-1)) as FP64.  |V| < 2^62 for S <= 9.
+//               keep each pass's q (or their int64 sum so far) in a buffer of
+//               the CTA's own, and on the last pass write V, their int64 sum
+//               (V = V * 2^10 + q), times 2^(e_r - 9 - 10 (passes-1)) as FP64.
+//               |V| < 2^62 for S <= 9.
 // Every mbarrier wait is bounded; on expiry the kernel raises an error flag,
 // drains its own in-flight copies and MMAs (bounded), frees TMEM and exits.
 //
@@ -95,19 +96,31 @@ struct GemmRing {
 constexpr int GBK = GemmRing::ROW;  // digits per K-step (the tensor maps' box)
 constexpr int SMEM_BYTES = GemmRing::SMEM;
 constexpr int THREADS = 320;  // producer, MMA, 8 epilogue warps (quadratic Gram)
-// Epilogue warps of the split GEMM (32 rows x 1024 / warps columns each).  Sixteen
-// hide the latency of a pass's sums where the passes are short (16 cohorts of 500 ..
-// 4000: 1.49 ms a step, 1.69 with eight; n = 750: 95 and 99 us); over long uniform K
-// the epilogue is hidden anyway and eight leave the MMAs more (n = 10000, 16384 SNPs:
-// 9.55 ms a step, 9.76 with sixteen, 10.5 with four).
+// Epilogue warps of the split GEMM (32 rows x 1024 / warps columns each) and what they
+// keep between passes (epilogue_pass).  Sixteen with planes hide the latency of a pass's
+// sums where the passes are short (steps timed in a host loop: 16 cohorts of 500 .. 4000
+// 1.49 ms, 1.69 with eight; n = 750 94 and 99 us); over long uniform K a pass of MMAs
+// hides the epilogue, eight warps leave the MMAs more, and what counts is the L2 that
+// the sums leave to the operands, then the traffic itself.  eigen, ms a launch, 16 with
+// planes / 8 with planes / 8 with int64 sums: 4096 SNPs n = 2000 0.203 / 0.222 / 0.209,
+// 3000 0.267 / 0.291 / 0.264, 4000 0.419 / 0.447 / 0.408, 5000 0.613 / 0.642 / 0.591,
+// 6500 0.904 / 0.914 / 0.869; 16384 SNPs, single launches and (back to back, at the power
+// limit) 8 with planes / 8 with int64 sums: 6500 3.55 (3.46) / 3.26 (3.39), 8000 5.03
+// (5.04) / 4.85 (5.06), 9000 6.27 (6.39) / 6.21 (6.47), 10000 7.50 (7.77) / 7.54 (7.93).
 constexpr int EPI_WARPS = 16;
 constexpr int EPI_WARPS_LONG = 8;
-constexpr int LONG_K = 4096;  // from this K on, uniform tiles run with EPI_WARPS_LONG
+constexpr int LONG_K = 4096;  // from this K on, uniform tiles run with EPI_WARPS_LONG ..
+constexpr int FOLD_K = 9088;  // .. and, below this one, with int64 sums
+// One wave of tiles ends with one last pass, which the int64 sums keep short: chol,
+// 512 SNPs, planes / int64 sums on sixteen warps, us a launch: n = 1000 57.3 / 61.8, 2000
+// 69.6 / 68.8, 4000 100.3 / 98.1, 8000 196.4 / 193.7.
+constexpr int ONE_WAVE_K = 2048;  // from this K on, for the triangular operand
 constexpr int gemm_threads(int epi_warps) { return 64 + 32 * epi_warps; }
 constexpr int GEMM_THREADS = gemm_threads(EPI_WARPS);
 constexpr int MAX_PLANES = 4;                   // passes before the last
 constexpr int PLANE = BM * BN / 4;              // int4s of a pass's sums over a CTA's tile (128 KB)
 constexpr int PART = MAX_PLANES * PLANE;
+constexpr int PART_FOLD = 2 * PLANE;             // int64 sums instead
 constexpr int MAX_SLICES = 9;   // FP8 digit slices; |V| < 2^62 in the epilogue
 static_assert((MAX_SLICES + 1) / 2 - 1 <= 4, "planes of the passes before the last");
 constexpr int FUSED_KMAX = 16368;  // K of the FP8 split GEMM: (32 + 1/32) K < 2^19
@@ -129,7 +142,7 @@ struct GemmArgs {
   int tri_rows;     // rows [0, tri_rows) of A are lower triangular in K (0: none)
   const double* row_scale;  // per row 2^(e_r - 9 - 10 (passes-1))
   double* C;        // output, column-major, ld = ldc
-  int4* part;       // each CTA's planes of pass sums, [pass][column / 4][row]
+  int4* part;       // each CTA's pass sums: planes [pass][column / 4][row], or int64 [column / 2][row]
   long long ldc;
   int col0;         // first genotype column of this launch (TMA row offset of G)
   int sq_rows;      // rows [0, sq_rows): write (C^2) as an error-free float pair (hi, lo)
@@ -306,27 +319,46 @@ __device__ __forceinline__ void warp_column_sums(float (&h)[8], float (&l)[8], i
   }
 }
 
-// Pass p of a tile for one epilogue warp (32 rows, its columns from the first).
-// The exact pair sum q in TMEM at tacc (an int32) of a pass before the last goes to
-// the CTA's own plane of that pass, four columns a thread, 512 bytes a warp and
-// access; a CTA writes the same planes for every tile, so they stay in L2.  The last
-// pass takes V = q_0 2^(10 p) + q_1 2^(10 (p-1)) + .. from the planes, four columns a
-// step, and writes C, V times the row scale (FP64, or squared as a float pair for
-// rows `sq`); `cols` of the warp's columns are valid for all rows, `cend` of this
-// row's.  (With the int64 sums V read and written every pass, in C, then in a part of
-// the CTA's own, an element moved 64 bytes through L2 instead of 32: n = 10000, 16384
-// SNPs 10.2 and 9.9 ms a step against 9.55, 16 cohorts of 500 .. 4000 2.17 and 1.39
-// against 1.37.)
+// Pass p of a tile for one epilogue warp (32 rows, its columns from the first): the
+// exact pair sum q in TMEM at tacc (an int32) joins those of the passes before, and
+// the last pass writes C, V = q_0 2^(10 p) + q_1 2^(10 (p-1)) + .. times the row scale
+// (FP64, or squared as a float pair for rows `sq`).  `cols` of the warp's columns are
+// valid for all rows, `cend` of this row's.  What a pass leaves for the next stays in
+// a part of the CTA's own, the same for every tile, so that it stays in L2; a thread
+// reads back what it wrote, 512 bytes a warp and access.
+//   FOLD = false: a plane of q per pass, all read by the last one.  Least traffic, 32
+//     bytes an element, but the last pass takes long and 512 KB a CTA leave the operand
+//     stream less of L2.  Best where the passes are short and the epilogue bounds them.
+//   FOLD = true: the int64 sum V, read and written every pass (64 bytes an element,
+//     256 KB a CTA), each step's sums loaded a step ahead.  Best where a pass of MMAs
+//     hides it.
+//     hides it.  (With V in C, where every tile's sums are other lines: 1 to 4 % more a
+//     launch at n = 4000 .. 10000.)
 // With `qrow` set (warp-uniform: the warp's 32-row group holds rows `sq` of a
 // unit-weight problem) the last pass writes no squares: the warp sums them over its
 // rows and writes column c's sum to qrow[c]; rows not `sq` still write FP64.
+template <bool FOLD>
 __device__ __forceinline__ void epilogue_pass(uint32_t tacc, int p, bool last, bool sq, double scale, float fscale,
                                               int4* part, double* crow, long long ldc, int cols, int cend,
                                               float2* qrow) {
   const int lane = threadIdx.x & 31;
-  uint64_t pol_keep;  // the operand stream (~0.5 GB a pass over all CTAs) must not push the sums out
+  uint64_t pol_keep, pol_read;  // the operand stream (~0.5 GB a pass over all CTAs) must not push the sums out
   asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_keep));
-  if (!last) {
+  if (FOLD) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_read));
+  else pol_read = pol_keep;
+  auto load = [&](const int4* at) {
+    int4 t;
+    asm volatile("ld.global.cg.L2::cache_hint.v4.b32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=r"(t.x), "=r"(t.y), "=r"(t.z), "=r"(t.w)
+                 : "l"(at), "l"(pol_read));
+    return t;
+  };
+  auto store = [&](int4* at, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.global.L2::cache_hint.v4.b32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(at), "r"(x), "r"(y), "r"(z),
+                 "r"(w), "l"(pol_keep)
+                 : "memory");
+  };
+  if (!FOLD && !last) {
     part += p * PLANE;
 #pragma unroll 1
     for (int c0 = 0; c0 < cols; c0 += 16) {
@@ -335,53 +367,71 @@ __device__ __forceinline__ void epilogue_pass(uint32_t tacc, int p, bool last, b
       tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 4; j++)
-        asm volatile("st.global.L2::cache_hint.v4.b32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(part + ((c0 >> 2) + j) * BM),
-                     "r"(fused_pair_f2i(__uint_as_float(v[4 * j]))), "r"(fused_pair_f2i(__uint_as_float(v[4 * j + 1]))),
-                     "r"(fused_pair_f2i(__uint_as_float(v[4 * j + 2]))),
-                     "r"(fused_pair_f2i(__uint_as_float(v[4 * j + 3]))), "l"(pol_keep)
-                     : "memory");
+        store(part + ((c0 >> 2) + j) * BM, fused_pair_f2i(__uint_as_float(v[4 * j])),
+              fused_pair_f2i(__uint_as_float(v[4 * j + 1])), fused_pair_f2i(__uint_as_float(v[4 * j + 2])),
+              fused_pair_f2i(__uint_as_float(v[4 * j + 3])));
     }
     return;
   }
-  // V of eight columns a step: all planes' loads in flight, then TMEM
+  // FOLD: V of two columns an int4, [column / 2][row]
+  int4 sums[4];
+  auto fetch = [&](int c0) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) sums[j] = p > 0 && c0 < cols ? load(part + ((c0 >> 1) + j) * BM) : make_int4(0, 0, 0, 0);
+  };
+  if (FOLD) fetch(0);
 #pragma unroll 1
   for (int c0 = 0; c0 < cols; c0 += 8) {
+    long long V[8];
     int4 q[MAX_PLANES][2];
+    if (FOLD) {
 #pragma unroll
-    for (int i = 0; i < MAX_PLANES; i++)
-#pragma unroll
-      for (int j = 0; j < 2; j++) {
-        q[i][j] = make_int4(0, 0, 0, 0);
-        if (i < p)
-          asm volatile("ld.global.cg.L2::cache_hint.v4.b32 {%0, %1, %2, %3}, [%4], %5;"
-                       : "=r"(q[i][j].x), "=r"(q[i][j].y), "=r"(q[i][j].z), "=r"(q[i][j].w)
-                       : "l"(part + i * PLANE + ((c0 >> 2) + j) * BM), "l"(pol_keep));
+      for (int j = 0; j < 4; j++) {
+        V[2 * j] = (long long)(((unsigned long long)(uint32_t)sums[j].y << 32) | (uint32_t)sums[j].x);
+        V[2 * j + 1] = (long long)(((unsigned long long)(uint32_t)sums[j].w << 32) | (uint32_t)sums[j].z);
       }
+      fetch(c0 + 8);
+    } else {  // all planes' loads in flight, then TMEM
+#pragma unroll
+      for (int i = 0; i < MAX_PLANES; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+          q[i][j] = i < p ? load(part + i * PLANE + ((c0 >> 2) + j) * BM) : make_int4(0, 0, 0, 0);
+    }
     uint32_t v[8];
     tmem_ld8(tacc + c0, v);
     tmem_ld_wait();
     auto value = [&](int j) -> long long {
-      long long V = 0;
+      long long s = 0;
+      if (FOLD) s = V[j];
+      else {
 #pragma unroll
-      for (int i = 0; i < MAX_PLANES; i++) {
-        const int4 t = q[i][j >> 2];
-        if (i < p) V = V * 1024ll + ((j & 3) == 0 ? t.x : (j & 3) == 1 ? t.y : (j & 3) == 2 ? t.z : t.w);
+        for (int i = 0; i < MAX_PLANES; i++) {
+          const int4 t = q[i][j >> 2];
+          if (i < p) s = s * 1024ll + ((j & 3) == 0 ? t.x : (j & 3) == 1 ? t.y : (j & 3) == 2 ? t.z : t.w);
+        }
       }
-      return V * 1024ll + fused_pair_f2i(__uint_as_float(v[j]));
+      return s * 1024ll + fused_pair_f2i(__uint_as_float(v[j]));
     };
-    if (qrow != nullptr) {
+    if (FOLD && !last) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const long long a = value(2 * j), b = value(2 * j + 1);
+        store(part + ((c0 >> 1) + j) * BM, (uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
+      }
+    } else if (qrow != nullptr) {
       float h[8], l[8];
 #pragma unroll
       for (int j = 0; j < 8; j++) {  // column j's square as a float pair (0 past cend; rows not sq write FP64)
         h[j] = l[j] = 0.0f;
         if (c0 + j >= cend) continue;
-        const long long V = value(j);
+        const long long s = value(j);
         if (sq) {
-          const float2 t = square_pair(V, fscale);
+          const float2 t = square_pair(s, fscale);
           h[j] = t.x;
           l[j] = t.y;
         } else {
-          crow[(long long)(c0 + j) * ldc] = (double)V * scale;
+          crow[(long long)(c0 + j) * ldc] = (double)s * scale;
         }
       }
       warp_column_sums(h, l, lane);
@@ -391,10 +441,10 @@ __device__ __forceinline__ void epilogue_pass(uint32_t tacc, int p, bool last, b
 #pragma unroll
       for (int j = 0; j < 8; j++) {
         if (c0 + j >= cend) break;
-        const long long V = value(j);
+        const long long s = value(j);
         double* cp = crow + (long long)(c0 + j) * ldc;
-        if (sq) *(float2*)cp = square_pair(V, fscale);
-        else *cp = (double)V * scale;
+        if (sq) *(float2*)cp = square_pair(s, fscale);
+        else *cp = (double)s * scale;
       }
     }
   }
@@ -656,7 +706,7 @@ __device__ __forceinline__ void gemm_persistent(const Src& src, int* tile_counte
         okw = __shfl_sync(0xffffffffu, okw, 0);  // warp-uniform: tcgen05.ld is .sync.aligned
         if (!okw) { ok = false; break; }
         tc_fence_after();
-        epilogue_pass(ta + 256 * buf, p, last, sq, scale, fscale, part, crow, g.ldc, cols, cend, qrow);
+        epilogue_pass<false>(ta + 256 * buf, p, last, sq, scale, fscale, part, crow, g.ldc, cols, cend, qrow);
         tc_fence_before();
         mbar_arrive(&tempty[buf]);
       }
@@ -721,7 +771,7 @@ constexpr int SMEM = STAGES * STAGE + 1024 + 256;
 constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 }  // namespace p2
 
-template <int EW, class Src>
+template <int EW, bool FOLD, class Src>
 __device__ __forceinline__ void gemm_pair(const Src& src, int* tile_counter) {
   constexpr int ROW = p2::ROW, A = p2::A, B = p2::B, STAGE = p2::STAGE, STAGES = p2::STAGES;
   constexpr uint32_t IDESC = p2::IDESC;
@@ -1002,7 +1052,7 @@ __device__ __forceinline__ void gemm_pair(const Src& src, int* tile_counter) {
       const int ncols = rvalid ? min(BN, T.N - n0) : 0;
       const int cend = min((BN * 4 / EW), ncols - cbeg);
       double* crow = g.C + (long long)r + (long long)(g.col0 + n0 + cbeg) * g.ldc;
-      part = g.part + (size_t)blockIdx.x * PART + (cbeg >> 2) * BM + row;
+      part = g.part + (size_t)blockIdx.x * (FOLD ? PART_FOLD : PART) + (FOLD ? cbeg >> 1 : cbeg >> 2) * BM + row;
       // unit weights: this warp's 32-row group (rows r & ~31 ..) sums its squares
       float2* qrow = (g.sqsum != nullptr && (r & ~31) < g.sq_rows)
                          ? g.sqsum + (long long)(r >> 5) * g.ldq + (g.col0 + n0 + cbeg)
@@ -1018,7 +1068,7 @@ __device__ __forceinline__ void gemm_pair(const Src& src, int* tile_counter) {
         okw = __shfl_sync(0xffffffffu, okw, 0);
         if (!okw) { ok = false; break; }
         tc_fence_after();
-        epilogue_pass(ta + 256 * buf, p, last, sq, scale, fscale, part, crow, g.ldc, cols, cend, qrow);
+        epilogue_pass<FOLD>(ta + 256 * buf, p, last, sq, scale, fscale, part, crow, g.ldc, cols, cend, qrow);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(lead_tempty + 8u * buf);
@@ -1059,12 +1109,12 @@ __device__ __forceinline__ void gemm_pair(const Src& src, int* tile_counter) {
 // as many clusters as fit at once.  Uniform tiles are dealt statically per
 // cluster, those of the triangular L^-1 operand (and of grouped problems)
 // taken from the launch-wide counter (two ints, zero before the first launch).
-template <int EW>
+template <int EW, bool FOLD>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(gemm_threads(EW), 1)
     ozaki_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBh,
                        const __grid_constant__ GemmArgs g, int* tile_counter) {
   const SingleTiles src{&tmA, &tmBh, &g, (int)cluster_rank()};
-  gemm_pair<EW>(src, tile_counter);
+  gemm_pair<EW, FOLD>(src, tile_counter);
 }
 
 // Many independent problems over a table of row-tile pairs; genotype maps in
@@ -1074,7 +1124,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
                                const CUtensorMap* __restrict__ maps, const int* __restrict__ cols, int ntiles,
                                int* tile_counter) {
   const GroupedTiles src{tiles, probs, maps, cols, ntiles, (int)cluster_rank()};
-  gemm_pair<EPI_WARPS>(src, tile_counter);
+  gemm_pair<EPI_WARPS, false>(src, tile_counter);
 }
 
 // Many independent problems in one persistent launch over a tile table;
@@ -2006,11 +2056,12 @@ int pair_clusters() {
   cfg.blockDim = dim3(GEMM_THREADS);
   cfg.dynamicSmemBytes = p2::SMEM;
   int n = 0;
-  if (cudaFuncSetAttribute(ozaki_gemm2_kernel<EPI_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, p2::SMEM) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(ozaki_gemm2_kernel<EPI_WARPS_LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           p2::SMEM) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, (void*)ozaki_gemm2_kernel<EPI_WARPS>, &cfg) != cudaSuccess) {
+  auto allow = [](auto kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, p2::SMEM) == cudaSuccess;
+  };
+  if (!allow(ozaki_gemm2_kernel<EPI_WARPS, false>) || !allow(ozaki_gemm2_kernel<EPI_WARPS_LONG, false>) ||
+      !allow(ozaki_gemm2_kernel<EPI_WARPS_LONG, true>) || !allow(ozaki_gemm2_kernel<EPI_WARPS, true>) ||
+      cudaOccupancyMaxActiveClusters(&n, (void*)ozaki_gemm2_kernel<EPI_WARPS, false>, &cfg) != cudaSuccess) {
     (void)cudaGetLastError();
     n = 0;
   }
@@ -2018,9 +2069,12 @@ int pair_clusters() {
   return n;
 }
 
+// Whether uniform tiles of Kpad run with int64 sums (the 2-SM kernel only).
+bool fold_form(int Kpad) { return Kpad >= LONG_K && Kpad < FOLD_K && pair_clusters() > 0; }
+
 // Most CTAs of a split GEMM of tiles_m x tiles_n tiles, in either form: each has a
-// part of the pass sums (512 KB; a plan holds what its largest block launches, not
-// 152 of them, so that many small engines fit one device).
+// part of the pass sums (512 KB, 256 KB of int64 sums; a plan holds what its largest
+// block launches, not 152 of them, so that many small engines fit one device).
 int gemm_ctas(int tiles_m, int tiles_n) {
   return std::max(2 * std::min((tiles_m + 1) / 2 * tiles_n, pair_clusters()), persistent_grid(tiles_m * tiles_n));
 }
@@ -2039,7 +2093,7 @@ struct OzakiPlan {
   uint8_t* G = nullptr;         // Ncap x Kpad E4M3 genotypes
   double* scale = nullptr;      // Mpad
   double* C = nullptr;          // Mpad x Ncap (ld Mpad)
-  int4* gpart = nullptr;   // the split GEMM's pass sums, PART a CTA
+  int4* gpart = nullptr;   // the split GEMM's pass sums, PART or PART_FOLD a CTA
   double* U = nullptr;          // n x nU
   float2* D = nullptr;          // n x t weights as float pairs (eigen d_j; chol: ones)
   float* dmax = nullptr;        // t: max_l of the high part of D[:, j]
@@ -2124,7 +2178,8 @@ cudaError_t ozaki_create(OzakiPlan** out, int n, int t, int wXL, int wXR, int x_
     chk(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev));
   }
   chk(cudaMalloc(&p->err, 3 * sizeof(int)));  // [wait error word, GEMM tile counter, finished CTAs]
-  chk(cudaMalloc(&p->gpart, sizeof(int4) * (size_t)PART * gemm_ctas(p->Mpad / BM, p->Ncap / BN)));
+  chk(cudaMalloc(&p->gpart, sizeof(int4) * (size_t)(eigen && fold_form(p->Kpad) ? PART_FOLD : PART) *
+                                gemm_ctas(p->Mpad / BM, p->Ncap / BN)));
   if (!eigen) chk(cudaMalloc(&p->LinvT, sizeof(double) * (size_t)n * n));
   if (!eigen) chk(cudaMalloc(&p->sqsum, sizeof(float2) * (size_t)(p->Mpad / 32) * p->Ncap));
   if (r == cudaSuccess) chk(cudaMemset(p->A, 0, (size_t)p->S * p->Mpad * p->Kpad));
@@ -2228,15 +2283,22 @@ cudaError_t run_gemm(OzakiPlan* p, cudaStream_t s, int col0, int x, int tri_rows
   // else one CTA per tile
   const int pairs = ((g.tiles_m + 1) / 2) * g.tiles_n;
   const int clusters = p->has_mapBh ? pair_clusters() : 0;
-  if (clusters > 0 && tri_rows == 0 && p->Kpad >= LONG_K)
-    ozaki_gemm2_kernel<EPI_WARPS_LONG><<<2 * std::min(pairs, clusters), gemm_threads(EPI_WARPS_LONG), p2::SMEM, s>>>(
-        p->mapA, p->mapBh, g, p->err + 1);
-  else if (clusters > 0)
-    ozaki_gemm2_kernel<EPI_WARPS><<<2 * std::min(pairs, clusters), GEMM_THREADS, p2::SMEM, s>>>(p->mapA, p->mapBh, g,
-                                                                                              p->err + 1);
-  else
+  if (clusters > 0 && tri_rows == 0 && p->Kpad >= LONG_K) {
+    const dim3 grid(2 * std::min(pairs, clusters)), block(gemm_threads(EPI_WARPS_LONG));
+    if (fold_form(p->Kpad))
+      ozaki_gemm2_kernel<EPI_WARPS_LONG, true><<<grid, block, p2::SMEM, s>>>(p->mapA, p->mapBh, g, p->err + 1);
+    else
+      ozaki_gemm2_kernel<EPI_WARPS_LONG, false><<<grid, block, p2::SMEM, s>>>(p->mapA, p->mapBh, g, p->err + 1);
+  } else if (clusters > 0) {
+    const dim3 grid(2 * std::min(pairs, clusters)), block(GEMM_THREADS);
+    if (tri_rows > 0 && pairs <= clusters && p->Kpad >= ONE_WAVE_K)
+      ozaki_gemm2_kernel<EPI_WARPS, true><<<grid, block, p2::SMEM, s>>>(p->mapA, p->mapBh, g, p->err + 1);
+    else
+      ozaki_gemm2_kernel<EPI_WARPS, false><<<grid, block, p2::SMEM, s>>>(p->mapA, p->mapBh, g, p->err + 1);
+  } else {
     ozaki_gemm_kernel<<<persistent_grid(g.tiles_m * g.tiles_n), GEMM_THREADS, SMEM_BYTES, s>>>(p->mapA, p->mapB, g,
-                                                                                          p->err + 1);
+                                                                                               p->err + 1);
+  }
   note_launch();
   return cudaGetLastError();
 }
