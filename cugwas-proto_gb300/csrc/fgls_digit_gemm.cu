@@ -813,6 +813,7 @@ struct DigitGemm {
   int4* planes = nullptr;      // MAXPASS planes a CTA, or one a unit and CTA in the split form (120 MB)
   int* err = nullptr;
   unsigned long long wait_ns = WAIT_NS;
+  bool unchecked = false;      // products were launched since digit_gemm_checked
   void* op[2] = {nullptr, nullptr};
   size_t op_bytes[2] = {0, 0};
 };
@@ -898,6 +899,8 @@ bool digit_gemm_ready(DigitGemm* g) {
 }
 
 int* digit_gemm_error_word(DigitGemm* g) { return g->err; }
+bool digit_gemm_unchecked(const DigitGemm* g) { return g && g->unchecked; }
+void digit_gemm_checked(DigitGemm* g) { g->unchecked = false; }
 
 void digit_gemm_set_wait_limit(DigitGemm* g, unsigned long long ns) { g->wait_ns = ns ? ns : WAIT_NS; }
 
@@ -905,6 +908,7 @@ cudaError_t digit_mul(DigitGemm* g, cudaStream_t s, const DigitMat& A, const Dig
                       double* C, long long ldc, const DigitMulOpts& o) {
   if (A.K != B.K) return cudaErrorInvalidValue;
   if (!digit_gemm_ready(g)) return cudaErrorMemoryAllocation;
+  g->unchecked = true;
   CUtensorMap ma, mb;
   FGLS_CUDA_TRY(digit_map(&ma, A));
   FGLS_CUDA_TRY(digit_map(&mb, B));

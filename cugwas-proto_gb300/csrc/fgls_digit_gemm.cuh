@@ -45,6 +45,9 @@ cudaError_t digit_gemm_create(DigitGemm** out);  // cudaErrorNotSupported: no cl
 bool digit_gemm_ready(DigitGemm* g);
 void digit_gemm_destroy(DigitGemm* g);
 int* digit_gemm_error_word(DigitGemm* g);
+// whether products were launched since the word was last read (digit_gemm_checked)
+bool digit_gemm_unchecked(const DigitGemm* g);
+void digit_gemm_checked(DigitGemm* g);
 // limit of one wait of the products launched from now on (0: the default, 2 s)
 void digit_gemm_set_wait_limit(DigitGemm* g, unsigned long long ns);
 

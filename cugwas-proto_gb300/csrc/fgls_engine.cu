@@ -146,11 +146,13 @@ int check_waits(fglsgpu_engine* e, const char* stage) {
   if (e->oz)
     ENG_TRY(e, cudaMemcpyAsync(e->hst_wait, ozaki_error_word(e->oz), sizeof(int), cudaMemcpyDeviceToHost, e->comp),
             "status copy");
-  if (e->dg)
+  const bool digits = digit_gemm_unchecked(e->dg);
+  if (digits)
     ENG_TRY(e, cudaMemcpyAsync(e->hst_wait + 1, digit_gemm_error_word(e->dg), sizeof(int), cudaMemcpyDeviceToHost,
                                e->comp),
             "status copy");
   ENG_TRY(e, cudaStreamSynchronize(e->comp), stage);
+  if (digits) digit_gemm_checked(e->dg);
   const int wsite = e->hst_wait[0] ? e->hst_wait[0] : e->hst_wait[1];
   if (!wsite) return FGLSGPU_OK;
   if (e->oz) ENG_TRY(e, cudaMemsetAsync(ozaki_error_word(e->oz), 0, sizeof(int), e->comp), "status reset");
