@@ -206,9 +206,21 @@ __device__ __forceinline__ int exact_f2i(float v) {
   return (int)(((uint32_t)__float_as_int(t) - 0x4C400000u) * 4u + ((uint32_t)__float_as_int(u) - 0x4B400000u));
 }
 
+constexpr int TOP = 0x7ff, ALL_PINF = 0x800, ALL_NINF = 0x1000, ALL_POS = 0x2000, ALL_NEG = 0x4000;  // below
 // exponent of a row's scale from the largest biased exponent in it (what a
 // DigitMat keeps per row)
-__device__ __forceinline__ int row_exponent(int top) { return top - 1021; }
+__device__ __forceinline__ int row_exponent(int top) { return (top & TOP) - 1021; }
+// What a DigitMat's ex holds of a row beside it: of a row with the exponent of NaN and
+// infinities, whether all its non-finite elements are +inf or all -inf; of rows cut by
+// digit_cut_signed, whether all elements are above or all below zero.
+// The product of two rows of which one or both are not finite: infinite where the signs
+// say so (what an FP64 sum gives), else NaN.
+__device__ __forceinline__ double nonfinite_product(int a, int b) {
+  const int inf = (a & TOP) == TOP ? a : b, fin = inf == a ? b : a;
+  const bool known = (fin & TOP) != TOP && (inf & (ALL_PINF | ALL_NINF)) && (fin & (ALL_POS | ALL_NEG));
+  const bool neg = ((inf & ALL_NINF) != 0) != ((fin & ALL_NEG) != 0);
+  return __longlong_as_double(!known ? 0x7ff8000000000000ll : neg ? (long long)0xfff0000000000000ull : 0x7ff0000000000000ll);
+}
 
 // (W 2^sh + V) 2^e rounded to FP64 (to nearest even) in integer instructions;
 // |W|, |V| < 2^52, sh <= 30.
@@ -270,7 +282,7 @@ __device__ __forceinline__ void store_four(const DgArgs& g, const int4 (&q)[MAXP
     }
     const int eb = g.exB[c + j];
     double v;
-    if (ea == 0x7ff || eb == 0x7ff) v = __longlong_as_double(0x7ff8000000000000ll);  // a NaN or an infinity in the row
+    if ((ea & TOP) == TOP || (eb & TOP) == TOP) v = nonfinite_product(ea, eb);
     else v = combine_words(W, sh, V, e0 + row_exponent(eb));
     if (g.alpha != 1.0) v = g.alpha == -1.0 ? -v : v * g.alpha;
     if (g.beta != 0.0) v = fma(g.beta, old[j], v);
@@ -627,7 +639,7 @@ __device__ __forceinline__ int digits_used(unsigned long long bits) {  // of the
 // elements are contiguous in K.  The row is read twice, the second time mostly
 // from L2; bound by the writes (twelve bytes an element) and integer issue.
 // w > 0: row (i*w + c)*w + d is the product of columns i*w + c and i*w + d.
-template <int TPR>
+template <int TPR, bool SIGNS>
 __global__ void __launch_bounds__(256) cut_contig_kernel(const double* __restrict__ X, long long ld, int rows, int K,
                                                          int Kpad, int w, uint8_t* __restrict__ D,
                                                          int* __restrict__ ex, int* __restrict__ nd) {
@@ -651,16 +663,36 @@ __global__ void __launch_bounds__(256) cut_contig_kernel(const double* __restric
     __syncthreads();
     for (int q = 0; q < 8; q++) top = max(top, stop[q]);
   }
-  if (l == 0) ex[r] = top;
+  int code = top;
+  if (top == TOP) {
+    int kinds = 0;  // 1: +inf, 2: -inf, 4: NaN
+    for (int k = l; k < K; k += TPR) {
+      const long long b = __double_as_longlong(value(k));
+      if (((b >> 52) & TOP) == TOP) kinds |= (b & 0xfffffffffffffll) ? 4 : b < 0 ? 2 : 1;
+    }
+    if (TPR > 32) {
+      const int p = __syncthreads_or(kinds & 1), m = __syncthreads_or(kinds & 2), n = __syncthreads_or(kinds & 4);
+      kinds = (p ? 1 : 0) | (m ? 2 : 0) | (n ? 4 : 0);
+    } else {
+      kinds = __reduce_or_sync(0xffffffffu, kinds);
+    }
+    code |= kinds == 1 ? ALL_PINF : kinds == 2 ? ALL_NINF : 0;
+  }
   const int es = row_exponent(top);
   unsigned long long bits = 0;
+  int pos = 1, neg = 1;
   for (int g = l; g < Kpad / 4; g += TPR) {
     uint64_t u[4];
     uint32_t sg[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       const int k = 4 * g + j;
-      const unsigned long long f = to_fixed(k < K ? value(k) : 0.0, es, sg[j]);
+      const double x1 = k < K ? value(k) : 0.0;
+      const unsigned long long f = to_fixed(x1, es, sg[j]);
+      if (SIGNS && k < K) {
+        pos &= x1 > 0.0;
+        neg &= x1 < 0.0;
+      }
       bits |= f;
       u[j] = f + DIGIT_BIAS;
     }
@@ -674,7 +706,15 @@ __global__ void __launch_bounds__(256) cut_contig_kernel(const double* __restric
     __syncthreads();
     for (int q = 0; q < 8; q++) bits |= sbits[q];
   }
-  if (l == 0) atomicMax(nd + (r >> 8), digits_used(bits));
+  if (SIGNS) {
+    pos = TPR > 32 ? __syncthreads_and(pos) : (int)__all_sync(0xffffffffu, pos);
+    neg = TPR > 32 ? __syncthreads_and(neg) : (int)__all_sync(0xffffffffu, neg);
+    code |= pos ? ALL_POS : neg ? ALL_NEG : 0;
+  }
+  if (l == 0) {
+    ex[r] = code;
+    atomicMax(nd + (r >> 8), digits_used(bits));
+  }
 }
 
 // Largest biased exponent of each row of a matrix whose elements are contiguous
@@ -835,7 +875,8 @@ DigitMat digit_mat_at(void* mem, int rows, int K) {
 }
 
 namespace {
-cudaError_t cut(cudaStream_t s, const DigitMat& m, const double* X, long long ld, bool kcontig, int w) {
+cudaError_t cut(cudaStream_t s, const DigitMat& m, const double* X, long long ld, bool kcontig, int w,
+                bool signs = false) {
   if (m.rows <= 0 || m.K <= 0 || m.prow != m.rows) return cudaErrorInvalidValue;
   // nd and, behind it, ex
   FGLS_CUDA_TRY(cudaMemsetAsync(m.nd, 0, sizeof(int) * ((m.rows + 255) / 256 + (kcontig ? 0 : m.rows)), s));
@@ -849,9 +890,11 @@ cudaError_t cut(cudaStream_t s, const DigitMat& m, const double* X, long long ld
     cut_strided_kernel<<<grid, 256, 0, s>>>(X, ld, m.rows, m.K, m.Kpad, slice, m.d, m.ex, m.nd);
     note_launch();
   } else if (m.K <= 1024)
-    cut_contig_kernel<32><<<ceil_div(m.rows, 8), 256, 0, s>>>(X, ld, m.rows, m.K, m.Kpad, w, m.d, m.ex, m.nd);
+    (signs ? cut_contig_kernel<32, true> : cut_contig_kernel<32, false>)<<<ceil_div(m.rows, 8), 256, 0, s>>>(
+        X, ld, m.rows, m.K, m.Kpad, w, m.d, m.ex, m.nd);
   else
-    cut_contig_kernel<256><<<m.rows, 256, 0, s>>>(X, ld, m.rows, m.K, m.Kpad, w, m.d, m.ex, m.nd);
+    (signs ? cut_contig_kernel<256, true> : cut_contig_kernel<256, false>)<<<m.rows, 256, 0, s>>>(
+        X, ld, m.rows, m.K, m.Kpad, w, m.d, m.ex, m.nd);
   note_launch();
   return cudaGetLastError();
 }
@@ -859,6 +902,10 @@ cudaError_t cut(cudaStream_t s, const DigitMat& m, const double* X, long long ld
 
 cudaError_t digit_cut(cudaStream_t s, const DigitMat& m, const double* X, long long ld, bool kcontig) {
   return cut(s, m, X, ld, kcontig, 0);
+}
+
+cudaError_t digit_cut_signed(cudaStream_t s, const DigitMat& m, const double* X, long long ld) {
+  return cut(s, m, X, ld, true, 0, true);
 }
 
 cudaError_t digit_cut_products(cudaStream_t s, const DigitMat& m, const double* X, long long ld, int w) {

@@ -31,8 +31,11 @@ size_t digit_mat_bytes(int rows, int K);
 DigitMat digit_mat_at(void* mem, int rows, int K);
 
 // Digits of a column-major FP64 matrix.  kcontig: row r's element k at
-// X[k + r*ld]; else at X[r + k*ld].  Rows holding a NaN or an infinity make every product with them NaN.
+// X[k + r*ld]; else at X[r + k*ld].  A row that holds a NaN or an infinity makes every
+// product with it NaN, but infinite where its non-finite elements are infinities of one
+// sign (kcontig only) and the other row was cut by digit_cut_signed and is of one sign.
 cudaError_t digit_cut(cudaStream_t s, const DigitMat& m, const double* X, long long ld, bool kcontig);
+cudaError_t digit_cut_signed(cudaStream_t s, const DigitMat& m, const double* X, long long ld);  // contiguous in K
 // rows r = (i*w + c)*w + d: the products of columns i*w + c and i*w + d of X
 cudaError_t digit_cut_products(cudaStream_t s, const DigitMat& m, const double* X, long long ld, int w);
 

@@ -481,7 +481,8 @@ int eigen_digits(fglsgpu_engine* e, long long cols, bool* use) {
     e->ayldig = digit_mat_at(e->wmem, nq, n);
     e->ddig = digit_mat_at((char*)e->wmem + wy, c.t, n);
     ENG_TRY(e, digit_cut(e->comp, e->ayldig, e->dAYL, n, true), "digits of the weighted columns");
-    ENG_TRY(e, digit_cut(e->comp, e->ddig, e->ddinv, n, true), "digits of the weights");
+    // (signed: squares past the range of FP64 keep their infinite sum with positive weights)
+    ENG_TRY(e, digit_cut_signed(e->comp, e->ddig, e->ddinv, n), "digits of the weights");
     e->w_cut = true;
   }
   *use = true;
@@ -1329,7 +1330,7 @@ int fglsgpu_adjoint_reset(fglsgpu_engine* e) {
       e->aayl3 = digit_mat_at(e->adjmem, (int)(3 * t * (1 + wXL)), c.n);
       e->aw3 = digit_mat_at((char*)e->adjmem + yb, (int)(3 * t), c.n);
       ENG_TRY(e, digit_cut(s, e->aayl3, e->aAYL3, n, true), "adjoint digits");
-      ENG_TRY(e, digit_cut(s, e->aw3, e->aW3, n, true), "adjoint digits");
+      ENG_TRY(e, digit_cut_signed(s, e->aw3, e->aW3, n), "adjoint digits");
       e->adj_cut = true;
     }
   }

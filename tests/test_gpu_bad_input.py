@@ -20,3 +20,21 @@ def test_kinship_that_is_not_finite(n, value):
         e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
         B2, V2 = e.run_snps(pb.XR)
     assert np.array_equal(B1, B2) and np.array_equal(V1, V2)
+
+
+@pytest.mark.parametrize("n", [200, 700])  # FP64 kernels, digits
+@pytest.mark.parametrize("wXR", [1, 2])
+def test_genotype_whose_square_overflows(n, wXR):
+    """A value of 1e300 makes its SNP's quadratic term infinite and its own effect zero or
+    NaN; the call is not refused, and the other SNPs are as without it."""
+    from fgls_gb300 import Engine, datagen
+    pb = datagen.make_problem(n, 256, 2, wXR=wXR, seed=n, hsig_uniform=True)
+    X = pb.XR.copy()
+    X[13, 7 * wXR] = 1e300
+    with Engine(n, 3, wXR, 2, 256, variant="eigen") as e:
+        e.set_problem(pb.Phi, pb.XL, pb.Y, pb.h, pb.sigma)
+        B0, V0 = e.run_snps(pb.XR)
+        B, V = e.run_snps(X)
+    others = np.arange(256) != 7
+    assert np.array_equal(B[:, others], B0[:, others]) and np.array_equal(V[:, others], V0[:, others])
+    assert np.isfinite(B[:, 7, :3]).all()
