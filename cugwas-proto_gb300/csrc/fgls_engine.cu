@@ -965,9 +965,9 @@ int fglsgpu_select_trait(fglsgpu_engine* e, int j) {
   ENG_TRY(e, build_shifted(s, c.n, e->dPhi, n, alpha, beta, e->dL, n), "build M");
   diag_range_kernel<<<1, 1024, 0, s>>>(c.n, e->dL, n, e->ddiag + 64 * 64);
   note_launch();
-  ENG_TRY(e, cudaMemcpyAsync(e->hrange, e->ddiag + 64 * 64, 2 * sizeof(double), cudaMemcpyDeviceToHost, s), "variances");
   DigitGemm* dg = digit_work(e);
   ENG_TRY(e, dpotrf_lower(s, dg, c.n, e->dL, n, e->ddiag, e->dst), "potrf");
+  ENG_TRY(e, cudaMemcpyAsync(e->hrange, e->ddiag + 64 * 64, 2 * sizeof(double), cudaMemcpyDeviceToHost, s), "variances");
   rc = check_status(e, "potrf(M)");
   if (rc) return rc;
   e->spread = e->hrange[1] > MAX_SPREAD * e->hrange[0];
@@ -987,9 +987,13 @@ int fglsgpu_select_trait(fglsgpu_engine* e, int j) {
   }
   e->linv_cut = false;
   if (inverse && e->dLinv) ENG_TRY(e, lower_inverse(s, dg, c.n, e->dL, n, e->dLinv), "inverse of the factor");
-  if (!split(e)) {  // room for the blocks' digits (on the split path the probe block takes its own)
+  if (!split(e) || c.slices == 0) {
+    // L^-1's digits and room for the blocks', on the split path for the probe block's,
+    // while the inverse is being computed
     bool digits = false;
-    rc = chol_digits(e, (long long)c.x_b * c.wXR, &digits);
+    e->probing = split(e);
+    rc = chol_digits(e, split(e) ? std::min((long long)TUNE_SNPS, (long long)c.x_b) : (long long)c.x_b * c.wXR, &digits);
+    e->probing = false;
     if (rc) return rc;
   }
   if (e->dLinv && !e->dg_off && !e->spread) {
@@ -1388,20 +1392,22 @@ int fglsgpu_adjoint_read(fglsgpu_engine* e, double* dh, double* dsigma, double* 
   ENG_TRY(e, cudaSetDevice(c.device), "cudaSetDevice");
   const int n = c.n, t = c.t;
   cudaStream_t s = e->comp;
-  int rc = check_status(e, "adjoint");
-  if (rc) return rc;
+  if (dY && (long long)t > (long long)c.x_b) {
+    const int rc = check_status(e, "adjoint");
+    return rc ? rc : fail(e, FGLSGPU_EINVAL, "dy needs t <= x_b");
+  }
   if (dY) {
     ENG_TRY(e, adjoint_ybar(s, n, t, c.wXL, e->ddinv, e->dZtXL, e->aacc, e->aU, e->aV2), "dy");
     // dY = Z V2 (original basis), through dQ as scratch (n x t <= n x x_b when t <= x_b)
     double* out = e->dQ;
-    if ((long long)t > (long long)c.x_b) return fail(e, FGLSGPU_EINVAL, "dy needs t <= x_b");
     ENG_TRY(e, digit_dgemm(e->adj_cut ? e->dg : nullptr, s, false, false, n, t, n, 1.0, e->dZ, n, e->aV2, n, 0.0, out, n),
             "dy");
     ENG_TRY(e, cudaMemcpyAsync(dY, out, sizeof(double) * (size_t)n * t, cudaMemcpyDeviceToHost, s), "dy");
   }
   std::vector<double> acc(2 * t);
   ENG_TRY(e, cudaMemcpyAsync(acc.data(), e->aacc, sizeof(double) * 2 * t, cudaMemcpyDeviceToHost, s), "dh");
-  rc = check_status(e, "adjoint read");  // dY's product may run on digits, whose waits are bounded
+  // the blocks' failures, and an expired wait of dY's product on digits
+  const int rc = check_status(e, "adjoint");
   if (rc) return rc;
   for (int j = 0; j < t; j++) {
     if (dh) dh[j] = acc[j];
