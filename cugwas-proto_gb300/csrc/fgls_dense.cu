@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(DT) diag_solve_kernel(int kb, const double* L,
 
 constexpr size_t TRI_SMEM = sizeof(double) * 2 * PB * (PB + 1);  // a diagonal block and its inverse
 constexpr size_t DSOLVE_SMEM = sizeof(double) * (NB + SCB) * (NB + 1);
-constexpr int SCB_NARROW = 16;  // RHS per CTA when few right-hand sides (e.g. the 512-wide L^-1 panels)
+constexpr int SCB_NARROW = 16;  // RHS per CTA when few right-hand sides (e.g. [y XL] of a trait)
 constexpr size_t DSOLVE_SMEM_NARROW = sizeof(double) * (NB + SCB_NARROW) * (NB + 1);
 
 // X := L_kk^-1 X for nrhs right-hand sides: 64 per CTA, or 16 when that

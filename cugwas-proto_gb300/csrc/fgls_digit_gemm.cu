@@ -46,7 +46,7 @@
 // Every wait is bounded as in fgls_ozaki.cu.
 //
 // Bound by the FP8 pipe: 10000 x 4096 x 10000 takes 18.1 ms with both cuts (78
-// pairs: 3.5 PFLOP/s, 0.92 of twice the measured BF16 rate) and 4.5 ms with
+// pairs: 3.5 PFLOP/s, 0.92 of twice the measured BF16 rate) and 3.7 ms with
 // hard calls (12 pairs), where the FP64 kernel takes 665 ms.
 #include <cuda.h>
 #include <cuda_fp8.h>

@@ -255,8 +255,8 @@ int fglsgpu_split_params(fglsgpu_engine *e, int *slices, double *probe_err);
 int fglsgpu_quad_digits(fglsgpu_engine *e, int *digits);
 
 /* Limit of one pipeline wait (on an mbarrier: a TMA copy landing, an MMA
- * finishing, an epilogue draining TMEM) inside the split path's tcgen05
- * kernels, in nanoseconds; 0 restores the default of 2 s.  A wait that
+ * finishing, an epilogue draining TMEM) inside the tcgen05 kernels (the split
+ * path's and the FP64 path's digit products), in nanoseconds; 0 restores the default of 2 s.  A wait that
  * runs out makes the kernel set an error word, let its own copies and MMAs
  * finish, free its TMEM and return; the next fglsgpu_sync (or the status
  * check of a host-API call) reports FGLSGPU_ETIMEOUT, clears the word and

@@ -1,5 +1,5 @@
 """FP64 path on inputs whose individuals differ in scale by many orders of magnitude,
-against quad arithmetic (numpy longdouble of the GPU machine)."""
+against quad arithmetic (numpy longdouble, where it is quad)."""
 import numpy as np
 import pytest
 
